@@ -2,85 +2,364 @@
 //
 // This is the true 32-bit path of every projection (no tensor cores, no
 // reduced-precision mode) and the fallback for sizes the fast kernels refuse.
-// Each output element is one float32 accumulator that walks K from 0 upward,
-// so its value does not depend on M, N, the tiling or what else is in the
-// batch.  The reference keeps weights as (in, out) and calls a library matmul
+// The reference keeps weights as (in, out) and calls a library matmul
 // (src/model.cpp:549-552); the checkpoint's (out, in) order is kept here.
+//
+// One order of summation for every output, whatever M, N, the kernel or what else is in the batch.  K is cut into
+// pieces of 8; piece q belongs to lane q mod 16.  A lane walks its pieces from K = 0 upward, one fma a product, the even
+// and the odd features on an accumulator each (neighbours in memory, so a pair of them is one fma.rn.f32x2 without any
+// packing), and adds the two at its end; lanes 4g .. 4g + 3 are added in order to group g's sum, and the four groups'
+// sums in order.  So half a warp that streams a row of w has a lane of the sum in every thread (32 bytes each), four
+// groups of threads that share a tile of outputs have a group of lanes each, and both give the same bits.  (Against one
+// accumulator over all of K the chains are also shorter: at K = 4,096 the
+// error against 64 bits is 2.1e-7, not 1.1e-6.)
 #include "api.h"
 #include "common.cuh"
 
 namespace exl3 {
 
-constexpr int BM = 64, BN = 64, BK = 16;
+constexpr int GS_PIECE = 8;                          // features of a piece
+constexpr int GS_LANES = 16;                         // lanes of an output's sum
+constexpr int GS_GROUPS = 4, GS_GROUP_LANES = 4;     // and how they are added up
 
-template <typename TI, typename TO>
-__global__ void __launch_bounds__(256)
+__device__ inline void gs_cp16(void* smem, const void* gmem, bool ok) {
+  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
+  const int bytes = ok ? 16 : 0;                     // nothing read, zeros written
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
+}
+__device__ inline void gs_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ inline void gs_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+__device__ inline float gs_load(const float* p) { return __ldcg(p); }
+__device__ inline float gs_load(const __nv_bfloat16* p) {
+  return __uint_as_float((uint32_t)__ldcg(reinterpret_cast<const unsigned short*>(p)) << 16);
+}
+
+// two products on two accumulators: lo += a.lo * b.lo, hi += a.hi * b.hi
+__device__ inline void gs_fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ inline float gs_both(unsigned long long acc) {
+  float lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc));
+  return lo + hi;
+}
+
+// Many rows: a block has a tile of 64 x 64 outputs, and each of its four groups of 128 threads (8 x 4 outputs a thread) a
+// quarter of the lanes: the groups walk different pieces of K with rings and barriers of their own, and meet once at the
+// end.  So a narrow output (1,024 columns at some hundred rows: fewer tiles than SMs) still has sixteen warps an SM.  The
+// sums of finished lanes wait in shared memory, which leaves the registers to the pairs of accumulators.
+// Bound by the fma pipe and by what shared memory returns (12 reads of 8 bytes a lane, 128 bytes a cycle, for 32 paired fma)
+// about equally: 525 x 8,192 x 1,024 (rows, columns, K) 278 us, 32 TFLOP/s; 525 x 1,024 x 4,096 130 us (one accumulator and 4 x 4
+// outputs a thread, an element a load: 442 and 390 us; this kernel with scalar fma and the lanes' sums in registers 302 and 140).
+constexpr int GT_TILE = 64, GT_STAGES = 4, GT_GROUP = 128, GT_THREADS = GS_GROUPS * GT_GROUP;
+constexpr int GT_PITCH = GS_PIECE + 4;               // floats; rows 48 bytes apart: the reads of 8 rows do not collide
+constexpr int GT_STAGE_FLOATS = 2 * GT_TILE * GT_PITCH;
+constexpr int GT_OUT_PITCH = GT_TILE + 8;
+constexpr int GT_RING_FLOATS = GS_GROUPS * GT_STAGES * GT_STAGE_FLOATS;
+constexpr int GT_SMEM = (GT_RING_FLOATS + GT_THREADS * 32) * 4;
+static_assert(GS_GROUPS * GT_TILE * GT_OUT_PITCH <= GT_RING_FLOATS, "the groups' sums go where the rings were");
+
+// VEC: float32, K % 4 == 0 and 16-byte aligned operands (16-byte asynchronous copies); else element by element.
+template <typename TI, typename TO, bool VEC>
+__global__ void __launch_bounds__(GT_THREADS, 1)
 gemm_simt_kernel(const TI* __restrict__ x, const TI* __restrict__ w, const TI* __restrict__ bias,
                  TO* __restrict__ y, int M, int N, int K) {
-  __shared__ float As[BK][BM + 4];
-  __shared__ float Bs[BK][BN + 4];
-  const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;            // 16 x 16 threads, 4 x 4 outputs each
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+  extern __shared__ __align__(16) float gt_smem[];
+  pdl_wait();
+  pdl_trigger();
+  const int g = threadIdx.x / GT_GROUP, t = threadIdx.x % GT_GROUP;
+  // a warp has 4 x 8 threads: its reads of x are four rows, of w eight, a wavefront each
+  const int tx = (t & 7) + (t >> 6) * 8, ty = ((t >> 3) & 3) + ((t >> 5) & 1) * 4;
+  const int m0 = blockIdx.y * GT_TILE, n0 = blockIdx.x * GT_TILE;
+  float* ring = gt_smem + g * GT_STAGES * GT_STAGE_FLOATS;
+  float4* sums = reinterpret_cast<float4*>(gt_smem + GT_RING_FLOATS) + threadIdx.x;    // [8][threads], this thread's own
+  const int pieces = (K + GS_PIECE - 1) / GS_PIECE;
+  const int first_lane = g * GS_GROUP_LANES, last_lane = first_lane + GS_GROUP_LANES;
 
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    // 64 rows x 16 k per operand: thread loads 4 elements of each
+  // one stage: one piece of the 64 rows of x and of w, half a row a thread
+  const int fr = t >> 1, fk = (t & 1) * 4;
+  const bool in_m = m0 + fr < M, in_n = n0 + fr < N;
+  const TI* xr = x + (int64_t)(in_m ? m0 + fr : 0) * K;
+  const TI* wr = w + (int64_t)(in_n ? n0 + fr : 0) * K;
+  auto fill = [&](int slot, int q) {
+    float* a = ring + slot * GT_STAGE_FLOATS + fr * GT_PITCH + fk;
+    float* b = a + GT_TILE * GT_PITCH;
+    const int k = q * GS_PIECE + fk;
+    if constexpr (VEC) {
+      const bool in_k = k < K;
+      gs_cp16(a, xr + (in_k ? k : 0), in_k && in_m);
+      gs_cp16(b, wr + (in_k ? k : 0), in_k && in_n);
+    } else {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int idx = tid + e * 256;
-      const int r = idx >> 4, kk = idx & 15;
-      const int k = k0 + kk;
-      float a = 0.0f, b = 0.0f;
-      if (k < K) {
-        if (m0 + r < M) a = Elem<TI>::load(x + (int64_t)(m0 + r) * K + k);
-        if (n0 + r < N) b = Elem<TI>::load(w + (int64_t)(n0 + r) * K + k);
+      for (int e = 0; e < 4; ++e) {
+        const bool in_k = k + e < K;
+        a[e] = in_k && in_m ? gs_load(xr + k + e) : 0.0f;
+        b[e] = in_k && in_n ? gs_load(wr + k + e) : 0.0f;
       }
-      As[kk][r] = a;
-      Bs[kk][r] = b;
     }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty * 4 + i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx * 4 + j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+  };
+  // the group's stages in order: lane by lane, each from its first piece on
+  int fl = first_lane, fq = fl;                               // the next stage to fill
+  auto fill_next = [&](int slot) {
+    if (fl < last_lane && fq < pieces) {
+      fill(slot, fq);
+      fq += GS_LANES;
+      if (fq >= pieces) { ++fl; fq = fl; }
     }
-    __syncthreads();
+    gs_commit();
+  };
+#pragma unroll
+  for (int s = 0; s < GT_STAGES - 1; ++s) fill_next(s);
+
+  unsigned long long acc[8][4];
+  const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    sums[i * GT_THREADS] = zero;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0;
   }
+  int slot = 0;
+  for (int lane = first_lane; lane < last_lane && lane < pieces; ++lane) {
+    for (int q = lane; q < pieces; q += GS_LANES) {
+      gs_wait<GT_STAGES - 2>();
+      asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");
+      fill_next(slot == 0 ? GT_STAGES - 1 : slot - 1);        // the slot that was read last
+      const float* a = ring + slot * GT_STAGE_FLOATS + ty * GT_PITCH;
+      const float* b = ring + slot * GT_STAGE_FLOATS + (GT_TILE + tx) * GT_PITCH;
+      slot = slot + 1 == GT_STAGES ? 0 : slot + 1;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty * 4 + i;
-    if (m >= M) continue;
+      for (int h = 0; h < GS_PIECE / 2; ++h) {
+        unsigned long long av[8];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = n0 + tx * 4 + j;
-      if (n >= N) continue;
-      float v = acc[i][j];
-      if (bias) v += Elem<TI>::load(bias + n);
-      Elem<TO>::store(y + (int64_t)m * N + n, v);
+        for (int i = 0; i < 8; ++i) av[i] = *reinterpret_cast<const unsigned long long*>(a + i * 8 * GT_PITCH + h * 2);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const unsigned long long bv = *reinterpret_cast<const unsigned long long*>(b + j * 16 * GT_PITCH + h * 2);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) gs_fma2(acc[i][j], av[i], bv);
+        }
+      }
     }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      float4 v = sums[i * GT_THREADS];
+      v.x += gs_both(acc[i][0]); v.y += gs_both(acc[i][1]); v.z += gs_both(acc[i][2]); v.w += gs_both(acc[i][3]);
+      sums[i * GT_THREADS] = v;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = 0;
+    }
+  }
+  gs_wait<0>();
+  __syncthreads();                                            // every ring has been read
+  float* mine = gt_smem + g * GT_TILE * GT_OUT_PITCH + ty * GT_OUT_PITCH + tx;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float4 v = sums[i * GT_THREADS];
+    float* o = mine + 8 * i * GT_OUT_PITCH;
+    o[0] = v.x; o[16] = v.y; o[32] = v.z; o[48] = v.w;
+  }
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < GT_TILE * GT_TILE; idx += GT_THREADS) {
+    const int r = idx >> 6, c = idx & 63;
+    if (m0 + r >= M || n0 + c >= N) continue;
+    const float* p = gt_smem + r * GT_OUT_PITCH + c;
+    constexpr int G = GT_TILE * GT_OUT_PITCH;
+    float v = ((p[0] + p[G]) + p[2 * G]) + p[3 * G];
+    if (bias) v += Elem<TI>::load(bias + n0 + c);
+    Elem<TO>::store(y + (int64_t)(m0 + r) * N + n0 + c, v);
   }
 }
 
-template <typename TI, typename TO>
+// Few rows in float32: half a warp streams R rows of w against MR rows of x, a thread a lane of every sum.  The block's
+// segment of x (1,024 features) is in shared memory, the two 16-byte halves of the pieces in planes of their own so that
+// the threads' reads do not collide; a row's next U pieces of 512 bytes are in flight in registers, the first of them before
+// the wait for the kernel before.  Bound by reading w, with eight rows by the chain of a block's segments: 8,192 x 1,024 (columns, K) takes 5.6 / 8.3 / 11.4 us
+// for 1 / 3 / 8 rows (5.2 of bytes; the tiles alone: 98 us for any), 1,024 x 4,096 4.8 / 8.7 / 16.2 us (382).
+constexpr int GF_WARPS = 8, GF_SEG = 1024;
+
+// a lane's piece of a row of w (zeros beyond K)
+template <bool V8>
+__device__ inline void gf_load_w(const float* p, int k, int K, unsigned long long (&v)[4]) {
+  if constexpr (V8) {
+    if (k < K) {
+      asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(v[0]), "=l"(v[1]), "=l"(v[2]), "=l"(v[3]) : "l"(p + k));
+    } else {
+      v[0] = v[1] = v[2] = v[3] = 0;
+    }
+  } else {
+    const ulonglong2 z = make_ulonglong2(0, 0);
+    const ulonglong2 a = k < K ? *reinterpret_cast<const ulonglong2*>(p + k) : z;
+    const ulonglong2 b = k + 4 < K ? *reinterpret_cast<const ulonglong2*>(p + k + 4) : z;
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+  }
+}
+
+template <int MR, int R, int U, bool V8>
+__global__ void __launch_bounds__(GF_WARPS * 32)
+gemm_simt_few_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias,
+                     float* __restrict__ y, int M, int N, int K) {
+  constexpr int STEP = GS_LANES * GS_PIECE;                   // features of a warp's step
+  constexpr int STEPS = GF_SEG / STEP;                        // of a segment of x
+  static_assert(STEPS % U == 0, "the register ring starts a segment at its start");
+  extern __shared__ __align__(16) float gf_smem[];            // [2][MR][STEPS][2 planes][16 lanes][4]; later the lanes' sums
+  const int tid32 = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = tid32 & (GS_LANES - 1), half = tid32 / GS_LANES;
+  const int m0 = blockIdx.y * MR;
+  const int w0 = (blockIdx.x * GF_WARPS + warp) * 2 * R, n0 = w0 + half * R;   // the warp's first row of w, and this half's
+  const float* wr[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) wr[r] = w + (int64_t)min(n0 + r, N - 1) * K;    // rows beyond N repeat the last one
+
+  unsigned long long wv[U][R][4];
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+#pragma unroll
+    for (int r = 0; r < R; ++r) gf_load_w<V8>(wr[r], u * STEP + lane * GS_PIECE, K, wv[u][r]);
+  pdl_wait();
+  pdl_trigger();
+
+  const int segs = (K + GF_SEG - 1) / GF_SEG;
+  auto fetch = [&](int seg) {
+    if (seg < segs) {
+      float* to = gf_smem + (seg & 1) * MR * GF_SEG;
+      for (int i = threadIdx.x; i < MR * (GF_SEG / 4); i += GF_WARPS * 32) {
+        const int m = i / (GF_SEG / 4), f = i % (GF_SEG / 4);          // f: 16 bytes of the segment
+        const int k = seg * GF_SEG + f * 4;
+        const bool ok = m0 + m < M && k < K;
+        gs_cp16(to + m * GF_SEG + (f / (2 * GS_LANES)) * STEP + (f & 1) * (STEP / 2) + ((f / 2) % GS_LANES) * 4,
+                x + (ok ? (int64_t)(m0 + m) * K + k : 0), ok);
+      }
+    }
+    gs_commit();
+  };
+  unsigned long long acc[R][MR];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int m = 0; m < MR; ++m) acc[r][m] = 0;
+  fetch(0);
+  for (int seg = 0; seg < segs; ++seg) {
+    fetch(seg + 1);
+    gs_wait<1>();
+    __syncthreads();
+    const float* xs = gf_smem + (seg & 1) * MR * GF_SEG + lane * 4;
+#pragma unroll
+    for (int s = 0; s < STEPS; ++s) {
+      unsigned long long cur[R][4];
+      const int k = seg * GF_SEG + s * STEP + lane * GS_PIECE;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) cur[r][e] = wv[s % U][r][e];
+        gf_load_w<V8>(wr[r], k + U * STEP, K, wv[s % U][r]);
+      }
+#pragma unroll
+      for (int m = 0; m < MR; ++m) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(xs + m * GF_SEG + s * STEP);
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(xs + m * GF_SEG + s * STEP + STEP / 2);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          gs_fma2(acc[r][m], a.x, cur[r][0]);
+          gs_fma2(acc[r][m], a.y, cur[r][1]);
+          gs_fma2(acc[r][m], b.x, cur[r][2]);
+          gs_fma2(acc[r][m], b.y, cur[r][3]);
+        }
+      }
+    }
+    __syncthreads();                                          // the segment has been read
+  }
+  gs_wait<0>();
+  // a thread per output adds its lanes in the order above
+  constexpr int OUTS = 2 * R * MR, PITCH = GS_LANES + 1;
+  float* part = gf_smem + warp * OUTS * PITCH;
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int m = 0; m < MR; ++m) part[((half * R + r) * MR + m) * PITCH + lane] = gs_both(acc[r][m]);
+  __syncwarp();
+  for (int o = tid32; o < OUTS; o += 32) {
+    const int n = w0 + o / MR, m = m0 + o % MR;
+    if (n >= N || m >= M) continue;
+    const float* p = part + o * PITCH;
+    float v = 0.0f;
+#pragma unroll
+    for (int g = 0; g < GS_GROUPS; ++g) {
+      float s = 0.0f;
+#pragma unroll
+      for (int l = 0; l < GS_GROUP_LANES; ++l) s += p[g * GS_GROUP_LANES + l];
+      v = g == 0 ? s : v + s;
+    }
+    if (bias) v += bias[n];
+    y[(int64_t)m * N + n] = v;
+  }
+}
+
+static int gs_sm_count() {
+  static thread_local int dev_of = -1, count = 0;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev != dev_of) {
+    cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
+    dev_of = dev;
+  }
+  return count;
+}
+
+template <typename Kern>
+static int gs_allow_smem(Kern kernel, size_t smem) {
+  if (smem <= 48 * 1024) return 0;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) {
+    set_error("gemm_simt: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
+    return (int)e;
+  }
+  return 0;
+}
+
+template <typename TI, typename TO, bool VEC>
 static int launch(const void* x, const void* w, const void* bias, void* y, int M, int N, int K,
                   cudaStream_t stream) {
-  dim3 grid(ceil_div(N, BN), ceil_div(M, BM));
+  dim3 grid(ceil_div(N, GT_TILE), ceil_div(M, GT_TILE));
   if (grid.y > 65535) { set_error("gemm_simt: M=%d is too large", M); return ERR_UNSUPPORTED; }
-  gemm_simt_kernel<TI, TO><<<grid, 256, 0, stream>>>(static_cast<const TI*>(x), static_cast<const TI*>(w),
-                                                      static_cast<const TI*>(bias), static_cast<TO*>(y), M, N, K);
+  int rc = gs_allow_smem(gemm_simt_kernel<TI, TO, VEC>, GT_SMEM);
+  if (rc) return rc;
+  launch_pdl(gemm_simt_kernel<TI, TO, VEC>, grid, dim3(GT_THREADS), GT_SMEM, stream, static_cast<const TI*>(x),
+             static_cast<const TI*>(w), static_cast<const TI*>(bias), static_cast<TO*>(y), M, N, K);
   return launch_status("gemm_simt");
+}
+
+template <int MR, int R, int U, bool V8>
+static int launch_few(const float* x, const float* w, const float* bias, float* y, int M, int N, int K,
+                      cudaStream_t stream) {
+  const size_t ring = (size_t)2 * MR * GF_SEG * 4, parts = (size_t)GF_WARPS * 2 * R * MR * (GS_LANES + 1) * 4;
+  const size_t smem = ring > parts ? ring : parts;
+  int rc = gs_allow_smem(gemm_simt_few_kernel<MR, R, U, V8>, smem);
+  if (rc) return rc;
+  const dim3 grid(ceil_div(N, GF_WARPS * 2 * R), ceil_div(M, MR));
+  launch_pdl(gemm_simt_few_kernel<MR, R, U, V8>, grid, dim3(GF_WARPS * 32), smem, stream, x, w, bias, y, M, N, K);
+  return launch_status("gemm_simt_few");
+}
+
+template <int MR, bool V8>
+static int launch_few_rows(const float* x, const float* w, const float* bias, float* y, int M, int N, int K,
+                           cudaStream_t stream) {
+  // rows of w a half warp: as many as leave every SM eight warps, so that the reads of x are shared
+  const int rows_an_sm = N / gs_sm_count() * ceil_div(M, MR);
+  if (rows_an_sm >= 64) return launch_few<MR, 4, 2, V8>(x, w, bias, y, M, N, K, stream);
+  if (rows_an_sm >= 32) return launch_few<MR, 2, 4, V8>(x, w, bias, y, M, N, K, stream);
+  return launch_few<MR, 1, 8, V8>(x, w, bias, y, M, N, K, stream);
+}
+
+// Which of the two kernels: where M is large both go by the fma they do, the tiles for whole waves of 64 x 64 tiles, the
+// streaming kernel at 1 / GF_COST of their rate for the rows that there are.  1,024 x 1,024: a wave of tiles 36 us, the
+// streaming kernel 31 us for 300 rows (0.5 of a wave's products); 1,024 x 4,096: 130 us, and 102.
+constexpr double GF_COST = 1.6;
+static bool few_rows(int M, int N, int sms) {
+  const double tiles = (double)ceil_div(M, GT_TILE) * ceil_div(N, GT_TILE);
+  const double waves = (double)(int64_t)((tiles + sms - 1) / sms);
+  return GF_COST * 8.0 * ceil_div(M, 8) * N <= waves * sms * GT_TILE * GT_TILE && M <= 65535;
 }
 
 }  // namespace exl3
@@ -91,10 +370,24 @@ extern "C" int exl3_gemm_simt(const void* x, const void* w, const void* bias, vo
                               int out_dtype, int M, int N, int K, cudaStream_t stream) {
   if (M == 0 || N == 0) return 0;
   if (M < 0 || N < 0 || K < 1) { set_error("gemm_simt: bad sizes M=%d N=%d K=%d", M, N, K); return ERR_BAD_ARGUMENT; }
-  if (in_dtype == DT_F32 && out_dtype == DT_F32) return launch<float, float>(x, w, bias, y, M, N, K, stream);
+  if (in_dtype == DT_F32 && out_dtype == DT_F32) {
+    if (K % 4 != 0 || !aligned16(x) || !aligned16(w)) return launch<float, float, false>(x, w, bias, y, M, N, K, stream);
+    if (!few_rows(M, N, gs_sm_count())) return launch<float, float, true>(x, w, bias, y, M, N, K, stream);
+    const float *xf = static_cast<const float*>(x), *wf = static_cast<const float*>(w), *bf = static_cast<const float*>(bias);
+    float* yf = static_cast<float*>(y);
+    const bool v8 = K % 8 == 0 && (reinterpret_cast<uintptr_t>(w) & 31u) == 0;
+    if (M == 1)
+      return v8 ? launch_few_rows<1, true>(xf, wf, bf, yf, M, N, K, stream) : launch_few_rows<1, false>(xf, wf, bf, yf, M, N, K, stream);
+    if (M == 2)
+      return v8 ? launch_few_rows<2, true>(xf, wf, bf, yf, M, N, K, stream) : launch_few_rows<2, false>(xf, wf, bf, yf, M, N, K, stream);
+    if (M <= 4)
+      return v8 ? launch_few_rows<4, true>(xf, wf, bf, yf, M, N, K, stream) : launch_few_rows<4, false>(xf, wf, bf, yf, M, N, K, stream);
+    return v8 ? launch_few_rows<8, true>(xf, wf, bf, yf, M, N, K, stream) : launch_few_rows<8, false>(xf, wf, bf, yf, M, N, K, stream);
+  }
   if (in_dtype == DT_BF16 && out_dtype == DT_BF16)
-    return launch<__nv_bfloat16, __nv_bfloat16>(x, w, bias, y, M, N, K, stream);
-  if (in_dtype == DT_BF16 && out_dtype == DT_F32) return launch<__nv_bfloat16, float>(x, w, bias, y, M, N, K, stream);
+    return launch<__nv_bfloat16, __nv_bfloat16, false>(x, w, bias, y, M, N, K, stream);
+  if (in_dtype == DT_BF16 && out_dtype == DT_F32)
+    return launch<__nv_bfloat16, float, false>(x, w, bias, y, M, N, K, stream);
   set_error("gemm_simt: unsupported element types in=%d out=%d", in_dtype, out_dtype);
   return ERR_UNSUPPORTED;
 }

@@ -95,6 +95,24 @@ def test_gemm_simt_rows_do_not_depend_on_the_batch():
         assert torch.equal(K().gemm_simt(x[r:r + 1].contiguous(), w, None, torch.float32)[0], full[r])
 
 
+# Edges of both float32 kernels: rows 1, 2, 4, 8 of the streaming one and one beyond, tiles of 64; K below a piece, with half
+# a piece at its end (16-byte rows), off 16 bytes, and around its segments of 1,024; N around a block's rows.  A lane's
+# chain is K / 32 products, so the error is below (K / 32 + 24) * 2^-24 of sum |x w| <= sqrt(K) times the result's size.
+@pytest.mark.parametrize("M", [1, 2, 3, 5, 9, 64, 65, 200])
+@pytest.mark.parametrize("N,Kd", [(1, 4), (15, 12), (129, 260), (31, 1023), (64, 1024), (70, 1028), (5000, 136)])
+def test_gemm_simt_edges(M, N, Kd):
+    g = torch.Generator(device=DEV).manual_seed(M * 10007 + N)
+    x, w = torch.randn(M, Kd, device=DEV, generator=g), torch.randn(N, Kd, device=DEV, generator=g)
+    b = torch.randn(N, device=DEV, generator=g)
+    got = K().gemm_simt(x, w, b, torch.float32)
+    bound = (Kd / 32 + 24) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T + b.double().abs())
+    assert bool(((got.double() - x.double() @ w.double().T - b.double()).abs() <= bound).all())
+    # a row alone, and a part of w's rows alone, give the same bits
+    m, n = M // 2, N // 2
+    assert torch.equal(K().gemm_simt(x[m:m + 1].contiguous(), w, b, torch.float32)[0], got[m])
+    assert torch.equal(K().gemm_simt(x, w[n:n + 1].contiguous(), b[n:n + 1].contiguous(), torch.float32)[:, 0], got[:, n])
+
+
 @pytest.mark.parametrize("M", [1, 3, 8, 9, 16])
 @pytest.mark.parametrize("N,Kd", [(2304, 2304), (263, 96), (50, 40), (1000, 5768), (16, 8)])
 def test_gemv_bf16(M, N, Kd):
