@@ -63,6 +63,14 @@ int exl3_attn_tokens(const void* q, int64_t q_row_stride, void* out, int dtype, 
                      int split_keys, int max_splits, float* scratch, size_t scratch_bytes,
                      cudaStream_t stream);
 size_t exl3_attn_tokens_scratch_bytes(int T, int nh, int hd, int max_splits);
+// The same in float32 without a window, for heads of 64 or 128, pages of 64 and at most 64 query heads a kv head.
+// tile_seq null: every token by itself.  Else the prompts' tiles of 128 new tokens (batch row and first new token of
+// each) with row_start[rows + 1], the first packed token of each batch row; the tokens of a row sit at consecutive
+// positions.
+int exl3_attn_f32(const float* q, int64_t q_row_stride, float* out, const float* k_pool, const float* v_pool,
+                  const int* block_table, int bt_stride, const int* tok_pos, const int* tok_seq, const int* row_start,
+                  const int* tile_seq, const int* tile_q0, int n_tiles, int T, int nh, int nkv, int hd, float scale,
+                  int split_keys, int max_splits, float* scratch, size_t scratch_bytes, cudaStream_t stream);
 // The same with values narrower than keys and rows of both pools kv_row elements apart (hdv <= hd <= kv_row, all
 // multiples of 16): out is [T, nh, hdv] and the scratch is sized with hdv.  With v_pool == k_pool the values are the
 // first hdv features of the keys (one latent row per token that every head reads).

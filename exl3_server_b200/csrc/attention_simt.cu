@@ -462,6 +462,295 @@ static int dispatch(const void* q, int64_t q_row_stride, void* out, const void* 
   return ERR_UNSUPPORTED;
 }
 
+// ---- float32, plain causal attention with heads of 64 or 128 ---------------------------------------------------------
+//
+// A block has up to 4 TY rows (a row: one query head of one token; the query heads of a kv head side by side, then the
+// next token of the same sequence), one kv head and one chunk of split_keys keys, which it walks a page at a time: the
+// page's scores as a product of tiles (thread: 4 rows x 4 keys, every 16th), one maximum and one rescaling a page, then
+// P V as a product of tiles (4 rows x HD / 16 features).  K of the next page is copied while the softmax and P V run, V
+// while the scores do.  What a row computes depends on its own position only: the features of a score in order, 32 at
+// a time on an accumulator for the even and one for the odd ones, a page's sum over a fixed tree, the keys of P V in
+// order, 16 at a time; so TY and what else is in the block change nothing, and the records of chunks are the general kernel's.
+// The general kernel walks one key after the other with a shuffle tree and two exponentials a key, a chain of latencies:
+// prompts of 90, 300 and 289 tokens with 16 query heads on 2 of 64 take it 256 us, this one 63; three single tokens at 250 to
+// 300 keys 79 and 25 us; prompts of 33 and 130 with 32 on 8 of 128 231 and 38 us.  Errors against 64 bits are the same
+// (1.3e-7 there).  One query head a kv head leaves a single token three quarters of the rows empty (36 heads at 1,100 keys:
+// 19 and 25 us); it takes this kernel too, so that a token's bits do not depend on the step that brought it.
+constexpr int AF_PAGE = 64, AF_TX = 16, AF_KEYS = AF_PAGE / AF_TX, AF_ROWS = 4, AF_CHAIN = 32, AF_P_PITCH = AF_PAGE + 4;
+
+__device__ inline void af_cp16(void* smem, const void* gmem, bool ok) {
+  const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
+  const int bytes = ok ? 16 : 0;                               // nothing read, zeros written
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(bytes) : "memory");
+}
+__device__ inline void af_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ inline void af_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ inline void af_fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ inline float2 af_split(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ inline unsigned long long af_pair(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+
+template <int HD, int TY>
+constexpr int af_smem_floats() {
+  return AF_ROWS * TY * (HD + 4) + AF_PAGE * (HD + 4) + AF_PAGE * HD + AF_ROWS * TY * AF_P_PITCH;
+}
+
+// tile_seq null: tile i is token i alone.  Else tile i is new tokens tile_q0[i / sub] + (i % sub) * tile_tokens on of
+// batch row tile_seq[i / sub], at most tile_tokens of them.
+template <int HD, int TY>
+__global__ void __launch_bounds__(AF_TX * TY)
+attn_f32_kernel(const float* __restrict__ q, int64_t q_row_stride, float* __restrict__ out,
+                const float* __restrict__ k_pool, const float* __restrict__ v_pool, const int* __restrict__ block_table,
+                int bt_stride, const int* __restrict__ tok_pos, const int* __restrict__ tok_seq,
+                const int* __restrict__ row_start, const int* __restrict__ tile_seq, const int* __restrict__ tile_q0,
+                int sub, int tile_tokens, int nh, int nkv, float scale, int split_keys, int max_splits,
+                float* __restrict__ scratch) {
+  constexpr int NT = AF_TX * TY, QP = HD + 4, VQ = HD / 64;    // VQ: groups of 4 features of a thread in P V
+  extern __shared__ __align__(16) float af_smem[];
+  float* sq = af_smem;
+  float* sk = sq + AF_ROWS * TY * QP;
+  float* sv = sk + AF_PAGE * QP;
+  float* sp = sv + AF_PAGE * HD;
+  pdl_wait();
+  pdl_trigger();
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int g = blockIdx.y, split = blockIdx.z, G = nh / nkv;
+  int t0, tokens;
+  if (tile_seq == nullptr) {
+    t0 = blockIdx.x;
+    tokens = 1;
+  } else {
+    const int tile = blockIdx.x / sub, b = __ldcg(tile_seq + tile);
+    t0 = __ldcg(row_start + b) + __ldcg(tile_q0 + tile) + (blockIdx.x % sub) * tile_tokens;
+    tokens = min(tile_tokens, __ldcg(row_start + b + 1) - t0);
+    tokens = min(tokens, 128 - (int)(blockIdx.x % sub) * tile_tokens);
+    if (tokens <= 0) return;
+  }
+  const int rows = tokens * G;
+  const int pos0 = __ldcg(tok_pos + t0);                              // the tile's tokens follow one another
+  const int hi_max = pos0 + tokens;
+  const int c_lo = split * split_keys;
+  const int c_hi = min(hi_max, split_keys > 0 ? c_lo + split_keys : hi_max);
+  const int* bt = block_table + (int64_t)__ldcg(tok_seq + t0) * bt_stride;
+
+  int hi[AF_ROWS];                                             // this thread's rows see keys below hi
+#pragma unroll
+  for (int i = 0; i < AF_ROWS; ++i) {
+    const int r = ty + TY * i;
+    hi[i] = pos0 + min(r, rows - 1) / G + 1;                   // rows beyond the tile's are zeros that nobody stores
+  }
+  unsigned long long acc[AF_ROWS][VQ][2];
+  float m[AF_ROWS], l[AF_ROWS];
+#pragma unroll
+  for (int i = 0; i < AF_ROWS; ++i) {
+    m[i] = -INFINITY;
+    l[i] = 0.0f;
+#pragma unroll
+    for (int v = 0; v < VQ; ++v) acc[i][v][0] = acc[i][v][1] = 0;
+  }
+
+  if (c_lo < c_hi) {
+    for (int idx = tid; idx < AF_ROWS * TY * (HD / 4); idx += NT) {
+      const int r = idx / (HD / 4), d = (idx % (HD / 4)) * 4;
+      const bool ok = r < rows;
+      af_cp16(sq + r * QP + d, q + (ok ? (int64_t)(t0 + r / G) * q_row_stride + (int64_t)(g * G + r % G) * HD + d : 0), ok);
+    }
+    // keys beyond the tile's last are not in the cache yet: zeros
+    auto fetch = [&](const float* pool, float* to, int pitch, int page) {
+      if (page * AF_PAGE < c_hi) {
+        const int pg = __ldcg(bt + page);
+        const float* from = pool + ((int64_t)max(pg, 0) * nkv + g) * AF_PAGE * HD;
+        for (int idx = tid; idx < AF_PAGE * (HD / 4); idx += NT) {
+          const int j = idx / (HD / 4), d = (idx % (HD / 4)) * 4;
+          const bool ok = pg >= 0 && page * AF_PAGE + j < c_hi;
+          af_cp16(to + j * pitch + d, from + (ok ? j * HD + d : 0), ok);
+        }
+      }
+      af_commit();
+    };
+    const int first = c_lo / AF_PAGE, last = (c_hi - 1) / AF_PAGE;
+    fetch(k_pool, sk, QP, first);
+    fetch(v_pool, sv, HD, first);
+    for (int page = first; page <= last; ++page) {
+      af_wait<1>();
+      __syncthreads();                                         // K of this page (and the queries) are here
+      float sc[AF_ROWS][AF_KEYS];
+#pragma unroll
+      for (int c = 0; c < HD / AF_CHAIN; ++c) {
+        unsigned long long s2[AF_ROWS][AF_KEYS];
+#pragma unroll
+        for (int i = 0; i < AF_ROWS; ++i)
+#pragma unroll
+          for (int j = 0; j < AF_KEYS; ++j) s2[i][j] = 0;
+#pragma unroll 4
+        for (int d = c * AF_CHAIN; d < (c + 1) * AF_CHAIN; d += 4) {
+          ulonglong2 a[AF_ROWS];
+#pragma unroll
+          for (int i = 0; i < AF_ROWS; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(sq + (ty + TY * i) * QP + d);
+#pragma unroll
+          for (int j = 0; j < AF_KEYS; ++j) {
+            const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(sk + (tx + AF_TX * j) * QP + d);
+#pragma unroll
+            for (int i = 0; i < AF_ROWS; ++i) af_fma2(s2[i][j], a[i].x, b.x);
+#pragma unroll
+            for (int i = 0; i < AF_ROWS; ++i) af_fma2(s2[i][j], a[i].y, b.y);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < AF_ROWS; ++i)
+#pragma unroll
+          for (int j = 0; j < AF_KEYS; ++j) {
+            const float2 e = af_split(s2[i][j]);
+            sc[i][j] = c == 0 ? e.x + e.y : sc[i][j] + (e.x + e.y);
+          }
+      }
+      __syncthreads();                                         // K has been read
+      fetch(k_pool, sk, QP, page + 1);
+      const int base = page * AF_PAGE;
+#pragma unroll
+      for (int i = 0; i < AF_ROWS; ++i) {
+        float s[AF_KEYS], mx = -INFINITY;
+#pragma unroll
+        for (int j = 0; j < AF_KEYS; ++j) {
+          s[j] = base + tx + AF_TX * j < hi[i] ? sc[i][j] * scale : -INFINITY;
+          mx = fmaxf(mx, s[j]);
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        const float mn = fmaxf(m[i], mx);
+        const bool any = mn > -INFINITY;
+        const float corr = any ? expf(m[i] - mn) : 1.0f;
+        float sum = 0.0f;
+#pragma unroll
+        for (int j = 0; j < AF_KEYS; ++j) {
+          const float p = any ? expf(s[j] - mn) : 0.0f;        // exp(-inf) = 0
+          sp[(ty + TY * i) * AF_P_PITCH + tx + AF_TX * j] = p;
+          sum += p;
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        l[i] = l[i] * corr + sum;
+        m[i] = mn;
+#pragma unroll
+        for (int v = 0; v < VQ; ++v)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const float2 x = af_split(acc[i][v][e]);
+            acc[i][v][e] = af_pair(x.x * corr, x.y * corr);
+          }
+      }
+      af_wait<1>();
+      __syncthreads();                                         // V of this page and P are here
+      const float* pr = sp + ty * AF_P_PITCH;
+      const float* vr = sv + tx * 4;
+      int all = AF_PAGE, most = 0;                             // keys that every row of this thread sees, that some does
+#pragma unroll
+      for (int i = 0; i < AF_ROWS; ++i) {
+        all = min(all, hi[i] - base);
+        most = max(most, hi[i] - base);
+      }
+#pragma unroll 1
+      for (int c0 = 0; c0 < AF_PAGE && c0 < most; c0 += AF_CHAIN / 2) {
+        unsigned long long pv[AF_ROWS][VQ][2];
+#pragma unroll
+        for (int i = 0; i < AF_ROWS; ++i)
+#pragma unroll
+          for (int v = 0; v < VQ; ++v) pv[i][v][0] = pv[i][v][1] = 0;
+#pragma unroll 1
+        for (int j0 = c0; j0 < c0 + AF_CHAIN / 2; j0 += 4) {
+          float4 p4[AF_ROWS];
+#pragma unroll
+          for (int i = 0; i < AF_ROWS; ++i) p4[i] = *reinterpret_cast<const float4*>(pr + i * TY * AF_P_PITCH + j0);
+          const bool some = j0 + 4 > all;                      // a key that a row does not see must not touch it,
+#pragma unroll                                                 // whatever its value holds
+          for (int jj = 0; jj < 4; ++jj) {
+#pragma unroll
+            for (int v = 0; v < VQ; ++v) {
+              const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(vr + (j0 + jj) * HD + v * 64);
+#pragma unroll
+              for (int i = 0; i < AF_ROWS; ++i) {
+                const float p = jj == 0 ? p4[i].x : (jj == 1 ? p4[i].y : (jj == 2 ? p4[i].z : p4[i].w));
+                const unsigned long long pp = af_pair(p, p);
+                if (!some || base + j0 + jj < hi[i]) {
+                  af_fma2(pv[i][v][0], pp, b.x);
+                  af_fma2(pv[i][v][1], pp, b.y);
+                }
+              }
+            }
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < AF_ROWS; ++i)
+#pragma unroll
+          for (int v = 0; v < VQ; ++v)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const float2 a = af_split(acc[i][v][e]), x = af_split(pv[i][v][e]);
+              acc[i][v][e] = af_pair(a.x + x.x, a.y + x.y);
+            }
+      }
+      __syncthreads();                                         // V and P have been read
+      fetch(v_pool, sv, HD, page + 1);
+    }
+    af_wait<0>();
+  }
+#pragma unroll
+  for (int i = 0; i < AF_ROWS; ++i) {
+    const int r = ty + TY * i;
+    if (r >= rows) continue;
+    const int64_t at = (int64_t)(t0 + r / G) * nh + g * G + r % G;
+    const float div = max_splits <= 1 ? l[i] : 1.0f;
+    float* to = max_splits <= 1 ? out + at * HD : scratch + (at * max_splits + split) * (HD + 2);
+#pragma unroll
+    for (int v = 0; v < VQ; ++v) {
+      const float2 a = af_split(acc[i][v][0]), b = af_split(acc[i][v][1]);
+      float* o = to + v * 64 + tx * 4;                         // a record's features start on 8 bytes only
+      *reinterpret_cast<float2*>(o) = make_float2(a.x / div, a.y / div);
+      *reinterpret_cast<float2*>(o + 2) = make_float2(b.x / div, b.y / div);
+    }
+    if (max_splits > 1 && tx == 0) {
+      to[HD] = m[i];
+      to[HD + 1] = l[i];
+    }
+  }
+}
+
+template <int HD, int TY>
+static int launch_f32(const float* q, int64_t q_row_stride, float* out, const float* k_pool, const float* v_pool,
+                      const int* block_table, int bt_stride, const int* tok_pos, const int* tok_seq, const int* row_start,
+                      const int* tile_seq, const int* tile_q0, int n_tiles, int T_, int nh, int nkv, float scale,
+                      int split_keys, int max_splits, float* scratch, cudaStream_t stream) {
+  const size_t smem = af_smem_floats<HD, TY>() * sizeof(float);
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(attn_f32_kernel<HD, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) {
+      set_error("attn_f32: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
+      return (int)e;
+    }
+  }
+  const int tile_tokens = tile_seq ? min(128, AF_ROWS * TY / (nh / nkv)) : 1;
+  const int sub = ceil_div(128, tile_tokens);
+  if (max_splits > 1) scratch += ATT_COUNTER_SLOTS;            // the counters' part stays as it is
+  const dim3 grid(tile_seq ? n_tiles * sub : T_, nkv, max_splits);
+  launch_pdl(attn_f32_kernel<HD, TY>, grid, dim3(AF_TX * TY), smem, stream, q, q_row_stride, out, k_pool, v_pool,
+             block_table, bt_stride, tok_pos, tok_seq, row_start, tile_seq, tile_q0, sub, tile_tokens, nh, nkv, scale,
+             split_keys, max_splits, scratch);
+  int rc = launch_status("attn_f32");
+  if (rc || max_splits <= 1) return rc;
+  launch_pdl(attn_combine_kernel<float>, dim3(T_, nh), dim3(64), (size_t)2 * max_splits * sizeof(float), stream,
+             (const float*)scratch, out, nh, HD, max_splits, 0, 0, (const float*)nullptr, (const float*)nullptr);
+  return launch_status("attn_combine");
+}
+
 }  // namespace exl3
 
 using namespace exl3;
@@ -565,4 +854,41 @@ extern "C" int exl3_attn_tokens(const void* q, int64_t q_row_stride, void* out, 
   return exl3_attn_tokens_ex(q, q_row_stride, out, dtype, k_pool, v_pool, block_table, bt_stride, tok_pos, tok_seq, T,
                              nh, nkv, hd, hd, hd, hd, page, window, 0, 0, scale, split_keys, max_splits, scratch,
                              scratch_bytes, stream);
+}
+
+extern "C" int exl3_attn_f32(const float* q, int64_t q_row_stride, float* out, const float* k_pool, const float* v_pool,
+                             const int* block_table, int bt_stride, const int* tok_pos, const int* tok_seq,
+                             const int* row_start, const int* tile_seq, const int* tile_q0, int n_tiles, int T, int nh,
+                             int nkv, int hd, float scale, int split_keys, int max_splits, float* scratch,
+                             size_t scratch_bytes, cudaStream_t stream) {
+  if (T == 0) return 0;
+  if (T < 0 || nh < 1 || nkv < 1 || nh % nkv != 0 || nh / nkv > 64 || (hd != 64 && hd != 128) || max_splits < 1 ||
+      split_keys < 0 || split_keys % AF_PAGE != 0 || (max_splits > 1 && split_keys == 0) || n_tiles < 0 ||
+      (tile_seq != nullptr && (tile_q0 == nullptr || row_start == nullptr))) {
+    set_error("attn_f32: bad sizes T=%d heads=%d kv_heads=%d head_dim=%d split_keys=%d max_splits=%d", T, nh, nkv, hd,
+              split_keys, max_splits);
+    return ERR_BAD_ARGUMENT;
+  }
+  if (nkv > 65535 || max_splits > 65535) { set_error("attn_f32: grid too large"); return ERR_UNSUPPORTED; }
+  if (!aligned16(q) || !aligned16(k_pool) || !aligned16(v_pool) || !aligned16(out) || q_row_stride % 4 != 0) {
+    set_error("attn_f32: q, k, v and out must be 16-byte aligned with a row stride in 16-byte units");
+    return ERR_ALIGNMENT;
+  }
+  if (exl3_attn_tokens_scratch_bytes(T, nh, hd, max_splits) > scratch_bytes) {
+    set_error("attn_f32: scratch of %zu bytes is too small, need %zu", scratch_bytes,
+              exl3_attn_tokens_scratch_bytes(T, nh, hd, max_splits));
+    return ERR_SCRATCH;
+  }
+  // single tokens with up to 16 query heads a kv head fill a quarter of the larger block's rows
+  const bool small = tile_seq == nullptr && nh / nkv <= 16;
+#define EXL3_AF(HD, TY)                                                                                            \
+  return launch_f32<HD, TY>(q, q_row_stride, out, k_pool, v_pool, block_table, bt_stride, tok_pos, tok_seq, row_start, \
+                            tile_seq, tile_q0, n_tiles, T, nh, nkv, scale, split_keys, max_splits, scratch, stream)
+  if (hd == 64) {
+    if (small) EXL3_AF(64, 4);
+    EXL3_AF(64, 16);
+  }
+  if (small) EXL3_AF(128, 4);
+  EXL3_AF(128, 16);
+#undef EXL3_AF
 }

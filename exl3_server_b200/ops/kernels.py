@@ -497,6 +497,31 @@ def attn_tokens(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, k_pool: t
     return out
 
 
+def attn_f32_supported(dtype: torch.dtype, heads: int, kv_heads: int, head_dim: int, page: int, window: int) -> bool:
+    """Whether ``attn_f32`` takes these sizes."""
+    return (dtype == torch.float32 and window == 0 and head_dim in (64, 128) and page == 64
+            and heads // kv_heads <= 64)
+
+
+def attn_f32(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
+             block_table: torch.Tensor, tok_pos: torch.Tensor, tok_seq: torch.Tensor, T: int, heads: int,
+             kv_heads: int, head_dim: int, scale: float, split_keys: int, max_splits: int,
+             scratch: Optional[torch.Tensor], row_start: Optional[torch.Tensor] = None, tiles=None) -> torch.Tensor:
+    """``attn_tokens`` in float32 without a window, a page of keys at a time (see attention_simt.cu).  ``tiles``: a
+    step's ``(batch row, first new token, count)`` of its tiles of 128 tokens, with ``row_start``; without, every token
+    runs by itself."""
+    if any(t.dtype != torch.float32 for t in (q, k_pool, v_pool, out)):
+        raise KernelLibraryError("attn_f32: q, cache and out must be float32")
+    tile_seq, tile_q0, n_tiles = tiles if tiles is not None else (None, None, 0)
+    nbytes = 0 if scratch is None else scratch.numel() * scratch.element_size()
+    _check(library().exl3_attn_f32(
+        _ptr(q), _c_int64(q_row_stride), _ptr(out), _ptr(k_pool), _ptr(v_pool), _ptr(block_table),
+        _c_int(block_table.stride(0)), _ptr(tok_pos), _ptr(tok_seq), _ptr(row_start), _ptr(tile_seq), _ptr(tile_q0),
+        _c_int(n_tiles), _c_int(T), _c_int(heads), _c_int(kv_heads), _c_int(head_dim), _c_float(scale),
+        _c_int(split_keys), _c_int(max_splits), _ptr(scratch), _c_size_t(nbytes), _stream()), "attn_f32")
+    return out
+
+
 def attn_tokens_kv(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, k_pool: torch.Tensor,
                    v_pool: torch.Tensor, block_table: torch.Tensor, tok_pos: torch.Tensor, tok_seq: torch.Tensor,
                    T: int, heads: int, kv_heads: int, head_dim: int, value_dim: int, kv_row: int, page: int,

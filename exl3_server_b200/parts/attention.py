@@ -192,6 +192,12 @@ class Attention:
         scratch = None
         if n > 1:
             scratch = batch.workspace.floats(K.attn_tokens_scratch_bytes(T, s.heads, s.head_dim, n) // 4)
+        if K.attn_f32_supported(qkv.dtype, s.heads, s.kv_heads, s.head_dim, kv.page_size, s.window):
+            # float32 without a window: a page of keys at a time as two products of tiles
+            K.attn_f32(qkv, qkv.stride(0), out, kv.k, kv.v, kv.block_table, batch.tok_pos, batch.tok_seq, T, s.heads,
+                       s.kv_heads, s.head_dim, self.scale, split, n, scratch, row_start=batch.row_start,
+                       tiles=batch.tiles.get(128) if batch.max_new > 1 else None)
+            return
         K.attn_tokens(qkv, qkv.stride(0), out, kv.k, kv.v, kv.block_table, batch.tok_pos, batch.tok_seq, T,
                       s.heads, s.kv_heads, s.head_dim, kv.page_size, s.window, self.scale, split, n, scratch)
 

@@ -113,6 +113,45 @@ def test_gemm_simt_edges(M, N, Kd):
     assert torch.equal(K().gemm_simt(x, w[n:n + 1].contiguous(), b[n:n + 1].contiguous(), torch.float32)[:, 0], got[:, n])
 
 
+# Tiles of several tokens against single tokens bit by bit, and both against 64 bits; places that no query may see hold NaN.
+@pytest.mark.parametrize("nh,nkv,hd,counts,starts", [(16, 2, 64, [90, 130, 1], [0, 0, 63]), (6, 2, 64, [70], [600]),
+                                                     (5, 5, 128, [257, 3], [0, 255]), (40, 1, 64, [3, 1], [33, 500]),
+                                                     (64, 1, 128, [65], [0]), (32, 2, 64, [1, 1, 1], [0, 64, 256])])
+def test_attn_f32(nh, nkv, hd, counts, starts):
+    g = torch.Generator(device=DEV).manual_seed(nh + hd)
+    B, T, page, split = len(counts), sum(counts), 64, 256
+    first = np.concatenate([[0], np.cumsum(counts)])
+    longest = max(s + c for s, c in zip(starts, counts))
+    pages = (longest + page - 1) // page
+    table = torch.randperm(B * pages, device=DEV, generator=g).to(torch.int32).view(B, pages)
+    k, v = (torch.full((B * pages, nkv, page, hd), math.nan, device=DEV) for _ in range(2))
+    q = torch.randn(T, (nh + 2 * nkv) * hd, device=DEV, generator=g)
+    want = torch.empty(T, nh * hd, dtype=torch.float64, device=DEV)
+    for b in range(B):
+        end = starts[b] + counts[b]
+        kb, vb = (torch.randn(nkv, end, hd, device=DEV, generator=g) for _ in range(2))
+        for pool, rows in ((k, kb), (v, vb)):
+            for j in range(end):
+                pool[int(table[b, j // page]), :, j % page] = rows[:, j]
+        qb = q[first[b]:first[b + 1], :nh * hd].double().view(-1, nh, hd).transpose(0, 1)
+        s = qb @ kb.double().repeat_interleave(nh // nkv, 0).transpose(1, 2) * hd ** -0.5
+        at = torch.arange(counts[b], device=DEV)[:, None] + starts[b]
+        s = s.masked_fill(torch.arange(end, device=DEV)[None] > at, -math.inf)
+        want[first[b]:first[b + 1]] = (s.softmax(-1) @ vb.double().repeat_interleave(nh // nkv, 0)).transpose(0, 1).reshape(counts[b], -1)
+    ints = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)  # noqa: E731
+    pos, seq = ints([s + i for s, c in zip(starts, counts) for i in range(c)]), ints([b for b, c in enumerate(counts) for _ in range(c)])
+    tiles = [(b, a) for b in range(B) for a in range(0, counts[b], 128)]
+    tiles = (ints([b for b, _ in tiles]), ints([a for _, a in tiles]), len(tiles))
+    n = (longest + split - 1) // split
+    scratch = torch.zeros(K().attn_tokens_scratch_bytes(T, nh, hd, n) // 4 + 1, device=DEV)
+    single, tiled = torch.empty(T, nh * hd, device=DEV), torch.empty(T, nh * hd, device=DEV)
+    args = (k, v, table, pos, seq, T, nh, nkv, hd, hd ** -0.5, split, n, scratch)
+    K().attn_f32(q, q.stride(0), single, *args)
+    K().attn_f32(q, q.stride(0), tiled, *args, row_start=ints(first.tolist()), tiles=tiles)
+    assert torch.equal(single, tiled)
+    close(single, want, 2e-6, "attention")               # scores up to 5 in size, off by some 2e-7 of it, in an exponential
+
+
 @pytest.mark.parametrize("M", [1, 3, 8, 9, 16])
 @pytest.mark.parametrize("N,Kd", [(2304, 2304), (263, 96), (50, 40), (1000, 5768), (16, 8)])
 def test_gemv_bf16(M, N, Kd):
