@@ -299,6 +299,10 @@ int exl3_argmax(const float* logits, int* out, int R, int V, void* scratch, size
 // The reference's sampler on the device (see sampling_filtered.cu).  rows: float64 [R, 5] = temperature (<= 0:
 // greedy), top_k (0: off; at most exl3_sample_filtered_cap()), top_p, min_p, uniform number in [0, 1).
 int exl3_sample_filtered(const float* logits, const double* rows, int* out, int R, int V, cudaStream_t stream);
+// The same with penalties (counts and params as exl3_sample_penalties takes them) applied as the logits are read, which
+// stay as they are, and the chosen tokens counted.
+int exl3_sample_rows(const float* logits, const double* rows, int* const* counts, const float* params, int* out, int R,
+                     int V, cudaStream_t stream);
 int exl3_sample_filtered_cap();
 // counts: R device pointers (null: none) to int32 [V] token counts of the rows' contexts; params: float32 [R, 3] =
 // repetition, presence and frequency penalty.  Changes logits in place.  exl3_sample_count adds the chosen tokens.

@@ -1,7 +1,7 @@
 // Sampling with filters on the device: the reference's sampler (sample_token,
-// src/model.cpp:667-757) step for step, one block per row of logits.
+// src/model.cpp:667-757) step for step.
 //
-//   penalties over the context (a kernel of its own, below), then
+//   penalties over the context, then
 //   the 2048 largest logits in descending order (ties: the smaller index first),
 //   p[i] = exp(logit[i] / T - max) as float32, sums in float64,
 //   min-p: cut before the first candidate whose share is below min_p * the largest share,
@@ -13,15 +13,25 @@
 // carries the whole rows there (vocabulary x 4 bytes each) and sorts them.
 //
 // The candidates are found without sorting the vocabulary: a radix select over
-// the float bits (four passes of 256 bins over the row, which stays in L2)
-// gives the 2048th largest value; when several tokens share that value the
-// select goes on over their indices, so exactly 2048 tokens pass.  They are
-// sorted in shared memory (bitonic, 64-bit keys: value bits above, inverted
-// index below, all different).
+// the float bits (digits of 11, 11 and 10 bits) gives the 2048th largest value;
+// when several tokens share that value the select goes on over their indices, so
+// exactly 2048 tokens pass.  They are sorted (bitonic, 64-bit keys: value bits
+// above, inverted index below, all different).
+//
+// A row is the work of a cluster of up to eight blocks.  Each reads its part of
+// the row once, with the penalties applied on the way, and keeps the keys in
+// shared memory, where the passes of the select find them; a pass's histograms
+// meet through distributed shared memory (every block adds all of them up and
+// finds the same digit), and the passing keys are written into the first
+// block's, which sorts and draws.  Bound by the chain of passes, barriers and the
+// sort: 32 rows of 122,753 take 43 us (one block a row that reads it five times:
+// 105 us, and the penalties were a copy of the logits and a kernel of 16 us).
 #include "api.h"
 #include "common.cuh"
 
 #include <math.h>
+
+#include <algorithm>
 
 namespace exl3 {
 
@@ -41,126 +51,211 @@ struct SfRow {            // one row's options, as the host gives them (float64 
   double temperature, top_k, top_p, min_p, u;
 };
 
-__global__ void __launch_bounds__(SF_THREADS)
-sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict__ rows, int* __restrict__ out, int V) {
-  // cand and acc hold nothing while the select runs: its histograms, one per warp, lie in their place.  (Logits
-  // crowd into a few bins of the leading byte, and additions to one address of shared memory go one after the
-  // other; a histogram per warp keeps the warps apart.  Measured, it made no difference to the kernel's time: the
-  // passes over the row through one SM's memory pipe are what it costs.)
-  __shared__ __align__(16) unsigned char raw[SF_CAP * 16];
-  unsigned long long* cand = reinterpret_cast<unsigned long long*>(raw);       // (key << 32) | ~index, sorted descending
-  double* acc = reinterpret_cast<double*>(raw + SF_CAP * 8);                   // running sums of probs
-  unsigned (*whist)[256] = reinterpret_cast<unsigned (*)[256]>(raw);           // [warps][256]
-  static_assert(sizeof(unsigned) * 256 * (SF_THREADS / 32) <= sizeof(raw), "the warps' histograms fit");
-  __shared__ float probs[SF_CAP];
-  __shared__ unsigned hist[256];
-  __shared__ double warp_tot[SF_THREADS / 32];
-  __shared__ unsigned long long sel_prefix;
-  __shared__ unsigned sel_remaining, n_cand, same;
-  __shared__ int first_below, first_hit, first_draw;
-  const float* row = logits + (int64_t)blockIdx.x * V;
-  const SfRow o = rows[blockIdx.x];
-  const int tid = threadIdx.x;
-  const int M = V < SF_CAP ? V : SF_CAP;
+constexpr double SF_FIXED_US = 36.0, SF_STAGED_US = 0.00030, SF_AGAIN_US = 0.00065;
+constexpr int SF_BINS = 2048;
+constexpr int SF_HEAD_BYTES = (2 * SF_BINS * 4) + 2 * (SF_CAP * 8);     // histograms, candidates, this block's own
 
-  // Every token's (value, inverted index) key.  One block reads its whole row several times over and an SM has
-  // only so many loads on their way: 16-byte loads, four of a thread at a time, make a pass a few round trips
-  // to L2 (rows start at any multiple of 4 bytes: the pieces before and after the aligned part go one by one).
-  auto key_of = [&](float v, int i) { return ((unsigned long long)sf_key(v) << 32) | (unsigned)(~(unsigned)i); };
-  const int head = min(V, (int)((4 - ((reinterpret_cast<uintptr_t>(row) >> 2) & 3)) & 3));
-  const int n_vec = (V - head) / 4;
-  const float4* row4 = reinterpret_cast<const float4*>(row + head);
+__device__ inline uint32_t sf_remote(const void* mine, uint32_t rank) {
+  uint32_t addr;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"((uint32_t)__cvta_generic_to_shared(mine)), "r"(rank));
+  return addr;
+}
+__device__ inline void sf_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ inline unsigned long long sf_max(unsigned long long a, unsigned long long b) { return a > b ? a : b; }
+__device__ inline unsigned long long sf_min(unsigned long long a, unsigned long long b) { return a < b ? a : b; }
+
+// A logit with its token's penalties (src/model.cpp:672-686).
+__device__ inline float sf_penalised(float x, int count, float rep, float presence, float frequency) {
+  if (count <= 0) return x;
+  if (rep != 1.0f) x = x > 0.0f ? __fdiv_rn(x, rep) : __fmul_rn(x, rep);
+  if (presence != 0.0f) x = __fsub_rn(x, presence);
+  if (frequency != 0.0f) x = __fsub_rn(x, __fmul_rn(frequency, (float)count));
+  return x;
+}
+
+// counts: null, or per row a pointer to its token counts [V] (null: the row has no penalties), which the chosen token
+// joins; params [R, 3]: repetition, presence, frequency.  STAGED: the block's part of the row is kept in shared memory;
+// else (vocabularies too long for that) every pass reads it again.
+template <bool STAGED>
+__global__ void __launch_bounds__(SF_THREADS)
+sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict__ rows, int* const* __restrict__ counts,
+                       const float* __restrict__ params, int* __restrict__ out, int V, int blocks) {
+  extern __shared__ __align__(16) unsigned char sf_smem[];
+  unsigned* hists = reinterpret_cast<unsigned*>(sf_smem);                                      // [2][SF_BINS]
+  unsigned long long* cand = reinterpret_cast<unsigned long long*>(sf_smem + 2 * SF_BINS * 4);  // the first block's: all
+  unsigned long long* found = cand + SF_CAP;                                                   // this block's
+  uint32_t* keys = reinterpret_cast<uint32_t*>(sf_smem + SF_HEAD_BYTES);                       // this block's part of the row
+  double* acc = reinterpret_cast<double*>(sf_smem);          // running sums of probs, once the histograms are done with
+  float* probs = reinterpret_cast<float*>(found);            // and once the block's own candidates are
+  __shared__ double warp_tot[SF_THREADS / 32];
+  __shared__ unsigned warp_cnt[SF_THREADS / 32];
+  __shared__ unsigned sel_digit, sel_remaining, sel_same, n_cand, n_found, at_cand;
+  __shared__ int first_below, first_hit, first_draw;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int row_id = blockIdx.x / blocks, rank = blockIdx.x % blocks;
+  const float* row = logits + (int64_t)row_id * V;
+  const SfRow o = rows[row_id];
+  const int M = V < SF_CAP ? V : SF_CAP;
+  int* count = counts ? counts[row_id] : nullptr;
+  float rep = 1.0f, presence = 0.0f, frequency = 0.0f;
+  if (count) {
+    rep = params[3 * row_id];
+    presence = params[3 * row_id + 1];
+    frequency = params[3 * row_id + 2];
+  }
+  const int per = (V + blocks - 1) / blocks;
+  const int first = min(V, rank * per), n = min(V, first + per) - first;
+  auto read_key = [&](int i) {
+    float x = row[first + i];
+    if (count) x = sf_penalised(x, count[first + i], rep, presence, frequency);
+    return sf_key(x);
+  };
+  // every token's (value, inverted index) key of this block's part
   auto for_each = [&](auto&& f) {
-    constexpr int AHEAD = 4;
-    for (int i = tid; i < head; i += SF_THREADS) f(key_of(row[i], i));
-    for (int j0 = tid; j0 < n_vec; j0 += SF_THREADS * AHEAD) {
-      float4 v[AHEAD];
+    if constexpr (STAGED) {
+      for (int i = tid; i < n; i += SF_THREADS) f(((unsigned long long)keys[i] << 32) | (unsigned)(~(unsigned)(first + i)));
+    } else {
+      for (int i = tid; i < n; i += SF_THREADS) f(((unsigned long long)read_key(i) << 32) | (unsigned)(~(unsigned)(first + i)));
+    }
+  };
+  if constexpr (STAGED) {
+    constexpr int AHEAD = 8;
+    for (int i0 = tid; i0 < n; i0 += SF_THREADS * AHEAD) {
+      float x[AHEAD];
+      int c[AHEAD];
 #pragma unroll
       for (int a = 0; a < AHEAD; ++a) {
-        const int j = j0 + a * SF_THREADS;
-        v[a] = j < n_vec ? row4[j] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        const int i = i0 + a * SF_THREADS;
+        x[a] = i < n ? row[first + i] : 0.0f;
+        c[a] = i < n && count ? count[first + i] : 0;
       }
 #pragma unroll
       for (int a = 0; a < AHEAD; ++a) {
-        const int j = j0 + a * SF_THREADS;
-        if (j < n_vec) {
-          const int i = head + 4 * j;
-          f(key_of(v[a].x, i));
-          f(key_of(v[a].y, i + 1));
-          f(key_of(v[a].z, i + 2));
-          f(key_of(v[a].w, i + 3));
-        }
+        const int i = i0 + a * SF_THREADS;
+        if (i < n) keys[i] = sf_key(sf_penalised(x[a], c[a], rep, presence, frequency));
       }
     }
-    for (int i = head + 4 * n_vec + tid; i < V; i += SF_THREADS) f(key_of(row[i], i));
-  };
+  }
+  for (int b = tid; b < SF_BINS; b += SF_THREADS) hists[b] = 0;
+  if (rank == 0)
+    for (int i = tid; i < SF_CAP; i += SF_THREADS) cand[i] = 0ull;      // padding sorts last
+  if (tid == 0) n_cand = n_found = 0;
+  __syncthreads();
 
   // ---- the M largest (value, then smaller index): radix select on the composite key -------------
   unsigned long long thresh = 0;                 // everything passes when the row is no longer than the cap
   if (V > SF_CAP) {
-    if (tid == 0) { sel_prefix = 0; sel_remaining = (unsigned)M; }
-    __syncthreads();
-    // the value's four bytes; the index's four only when tokens with the threshold's value are too many
-    for (int shift = 56; shift >= 0; shift -= 8) {
-      for (int b = tid; b < 256 * (SF_THREADS / 32); b += SF_THREADS) whist[0][b] = 0;
-      __syncthreads();
-      const unsigned long long prefix = sel_prefix;
-      const unsigned long long mask = shift == 56 ? 0ull : (~0ull << (shift + 8));
+    unsigned remaining = (unsigned)M;
+    // the value's three digits; the index's three only when tokens with the threshold's value are too many
+    for (int pass = 0; pass < 6; ++pass) {
+      const int at[6] = {53, 42, 32, 21, 10, 0}, wide[6] = {11, 11, 10, 11, 11, 10};
+      const int shift = at[pass], bits = wide[pass];
+      unsigned* hist = hists + (pass & 1) * SF_BINS;
+      if (pass > 0) {
+        // nobody reads this one any more: the blocks have met since
+        for (int b = tid; b < SF_BINS; b += SF_THREADS) hist[b] = 0;
+        __syncthreads();
+      }
+      const unsigned long long mask = shift + bits >= 64 ? 0ull : (~0ull << (shift + bits));
+      const unsigned digit_mask = (1u << bits) - 1u;
       for_each([&](unsigned long long c) {
-        if ((c & mask) == prefix) atomicAdd(&whist[tid >> 5][(unsigned)(c >> shift) & 255u], 1u);
+        if ((c & mask) == (thresh & mask)) atomicAdd(hist + ((unsigned)(c >> shift) & digit_mask), 1u);
       });
+      sf_cluster_sync();
+      // all blocks' histograms, from the largest digit down, two bins a thread
+      const int hi = SF_BINS - 1 - 2 * tid;
+      unsigned n1 = 0, n0 = 0;                    // bins hi and hi - 1
+      for (int b = 0; b < blocks; ++b) {
+        unsigned lo_bin, hi_bin;
+        asm volatile("ld.shared::cluster.v2.u32 {%0, %1}, [%2];" : "=r"(lo_bin), "=r"(hi_bin) : "r"(sf_remote(hist + hi - 1, b)));
+        n1 += hi_bin;
+        n0 += lo_bin;
+      }
+      unsigned run = n1 + n0;
+#pragma unroll
+      for (int s = 1; s < 32; s <<= 1) {
+        const unsigned v = __shfl_up_sync(0xffffffffu, run, s);
+        if (lane >= s) run += v;
+      }
+      if (lane == 31) warp_cnt[warp] = run;
       __syncthreads();
-      if (tid < 256) {
-        unsigned n = 0;
-        for (int w = 0; w < SF_THREADS / 32; ++w) n += whist[w][tid];
-        hist[tid] = n;
+      unsigned before = run - (n1 + n0);
+      for (int v = 0; v < warp; ++v) before += warp_cnt[v];
+      if (before < remaining && before + n1 >= remaining) {
+        sel_digit = hi;
+        sel_remaining = remaining - before;      // how many of this digit's tokens still pass
+        sel_same = n1;
+      } else if (before + n1 < remaining && before + n1 + n0 >= remaining) {
+        sel_digit = hi - 1;
+        sel_remaining = remaining - before - n1;
+        sel_same = n0;
       }
       __syncthreads();
-      if (tid == 0) {
-        unsigned cum = 0, rem = sel_remaining;
-        int digit = 0;
-        for (int b = 255; b >= 0; --b) {
-          if (cum + hist[b] >= rem) { digit = b; break; }
-          cum += hist[b];
-        }
-        sel_remaining = rem - cum;               // how many of this digit's tokens still pass
-        sel_prefix = prefix | ((unsigned long long)digit << shift);
-        same = hist[digit];                      // after the value's last byte: the tokens with the threshold's value
-      }
-      __syncthreads();
+      remaining = sel_remaining;
+      thresh |= (unsigned long long)sel_digit << shift;
       // if all tokens with this value pass, their indices need no select: the threshold is (value, any index)
-      if (shift == 32 && same == sel_remaining) break;
+      if (shift == 32 && sel_same == remaining) break;
+      __syncthreads();                            // before the next pass's sums
     }
-    thresh = sel_prefix;
   }
-  if (tid == 0) n_cand = 0;
-  for (int i = tid; i < SF_CAP; i += SF_THREADS) cand[i] = 0ull;   // padding sorts last
-  __syncthreads();
   for_each([&](unsigned long long c) {
     if (c >= thresh) {
-      const unsigned at = atomicAdd(&n_cand, 1u);
-      if (at < (unsigned)SF_CAP) cand[at] = c;
+      const unsigned k = atomicAdd(&n_found, 1u);
+      if (k < (unsigned)SF_CAP) found[k] = c;
     }
   });
+  if (V <= SF_CAP) sf_cluster_sync();             // the first block's candidates are cleared (else the select has met)
   __syncthreads();
+  if (tid == 0)
+    asm volatile("atom.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(at_cand) : "r"(sf_remote(&n_cand, 0)), "r"(n_found) : "memory");
+  __syncthreads();
+  for (unsigned i = tid; i < n_found; i += SF_THREADS)
+    if (at_cand + i < (unsigned)SF_CAP)
+      asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(sf_remote(cand + at_cand + i, 0)), "l"(found[i]) : "memory");
+  sf_cluster_sync();                              // all candidates are there, and nobody reads another block any more
+  if (rank != 0) return;
 
-  // ---- sorted descending: bitonic over the 2048 slots --------------------------------------------
-  for (int k = 2; k <= SF_CAP; k <<= 1) {
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = tid; i < SF_CAP; i += SF_THREADS) {
-        const int l = i ^ j;
-        if (l > i) {
-          const unsigned long long a = cand[i], b = cand[l];
-          const bool desc = (i & k) == 0;
-          if (desc ? a < b : a > b) { cand[i] = b; cand[l] = a; }
-        }
+  // ---- sorted descending: bitonic over the 2048 slots, two neighbours a thread: partners up to 32 places away are in
+  // the same warp, only the farther ones go through shared memory -----------------------------------
+  {
+    unsigned long long a = cand[2 * tid], b = cand[2 * tid + 1];
+    for (int k = 2; k <= SF_CAP; k <<= 1) {
+      const bool desc = ((2 * tid) & k) == 0;     // the same for both places: k >= 2
+      for (int j = k >> 1; j >= 64; j >>= 1) {
+        __syncthreads();
+        cand[2 * tid] = a;
+        cand[2 * tid + 1] = b;
+        __syncthreads();
+        const unsigned long long pa = cand[(2 * tid) ^ j], pb = cand[(2 * tid + 1) ^ j];
+        const bool larger = desc == (((2 * tid) & j) == 0);
+        a = larger ? sf_max(a, pa) : sf_min(a, pa);
+        b = larger ? sf_max(b, pb) : sf_min(b, pb);
       }
-      __syncthreads();
+      for (int j = min(k >> 1, 32); j >= 2; j >>= 1) {
+        const unsigned long long pa = __shfl_xor_sync(0xffffffffu, a, j >> 1), pb = __shfl_xor_sync(0xffffffffu, b, j >> 1);
+        const bool larger = desc == (((2 * tid) & j) == 0);
+        a = larger ? sf_max(a, pa) : sf_min(a, pa);
+        b = larger ? sf_max(b, pb) : sf_min(b, pb);
+      }
+      const unsigned long long top = sf_max(a, b), low = sf_min(a, b);
+      a = desc ? top : low;
+      b = desc ? low : top;
     }
+    __syncthreads();
+    cand[2 * tid] = a;
+    cand[2 * tid + 1] = b;
+    __syncthreads();
   }
   auto token_of = [&](int i) { return (int)(~(unsigned)(cand[i] & 0xffffffffull)); };
+  auto choose = [&](int i) {
+    const int t = token_of(i);
+    out[row_id] = t;
+    if (count) count[t] += 1;                     // the chosen token joins its row's context
+  };
   if (!(o.temperature > 0.0)) {                  // greedy: the first maximum
-    if (tid == 0) out[blockIdx.x] = token_of(0);
+    if (tid == 0) choose(0);
     return;
   }
 
@@ -200,7 +295,7 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
   __syncthreads();
   const double total = acc[M - 1];
   if (!(total > 0.0)) {
-    if (tid == 0) out[blockIdx.x] = token_of(0);
+    if (tid == 0) choose(0);
     return;
   }
   int keep = M;
@@ -223,7 +318,7 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
   for (int i = tid; i < keep; i += SF_THREADS)
     if (acc[i] >= r) atomicMin(&first_draw, i);
   __syncthreads();
-  if (tid == 0) out[blockIdx.x] = token_of(first_draw < keep ? first_draw : keep - 1);
+  if (tid == 0) choose(first_draw < keep ? first_draw : keep - 1);
 }
 
 // Penalties over a row's context (src/model.cpp:672-686).  counts[r] points to the row's token counts [V]
@@ -237,12 +332,8 @@ __global__ void sample_penalties_kernel(float* __restrict__ logits, int V, const
   if (tok >= V) return;
   const int count = c[tok];
   if (count <= 0) return;
-  const float rep = params[3 * row], presence = params[3 * row + 1], frequency = params[3 * row + 2];
-  float x = logits[(int64_t)row * V + tok];
-  if (rep != 1.0f) x = x > 0.0f ? __fdiv_rn(x, rep) : __fmul_rn(x, rep);
-  if (presence != 0.0f) x = __fsub_rn(x, presence);
-  if (frequency != 0.0f) x = __fsub_rn(x, __fmul_rn(frequency, (float)count));
-  logits[(int64_t)row * V + tok] = x;
+  float* x = logits + (int64_t)row * V + tok;
+  *x = sf_penalised(*x, count, params[3 * row], params[3 * row + 1], params[3 * row + 2]);
 }
 
 // The chosen tokens join their rows' contexts.
@@ -258,13 +349,63 @@ __global__ void sample_count_kernel(int* const* __restrict__ counts, const int* 
 using namespace exl3;
 
 // rows: float64 [R, 5] on the device: temperature (<= 0: greedy), top_k (0: off, at most 2048), top_p, min_p and
-// the row's uniform number in [0, 1).  out: int32 [R].
+// the row's uniform number in [0, 1).  out: int32 [R].  counts (may be null): as in exl3_sample_penalties, with params;
+// the penalties are applied as the logits are read, and the chosen tokens are counted.
+extern "C" int exl3_sample_rows(const float* logits, const double* rows, int* const* counts, const float* params, int* out,
+                                int R, int V, cudaStream_t stream) {
+  if (R == 0) return 0;
+  if (R < 0 || V < 1 || (counts != nullptr && params == nullptr)) {
+    set_error("sample_filtered: bad sizes rows=%d vocab=%d, or penalties without their constants", R, V);
+    return ERR_BAD_ARGUMENT;
+  }
+  // Blocks a row.  An SM holds one block and the SMs come in eight groups that a cluster must fit into; a wave of clusters
+  // takes some 36 us and 0.3 ns a token of a block's part, 0.65 ns where it is too long for shared memory.  With 8 / 4 / 2 / 1
+  // blocks: 32 rows of 122,753 89 / 43 / 68 / 106 us, 64 rows of 32,000 117 / 66 / 37 / 42, 256 rows 392 / 205 / 136 / 82.
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  constexpr size_t MOST = 200 * 1024 - SF_HEAD_BYTES;
+  int blocks = 8;
+  double best = 0.0;
+  for (int b = 8; b >= 1; b /= 2) {
+    const int each = ceil_div(V, b);
+    const int at_once = 8 * std::max(1, sms / 8 / b);    // clusters of b that fit: the SMs come in eight groups
+    const double waves = (double)((R + at_once - 1) / at_once);
+    const double cost = waves * (SF_FIXED_US + ((size_t)each * 4 <= MOST ? SF_STAGED_US : SF_AGAIN_US) * each);
+    if (b == 8 || cost < best) {
+      best = cost;
+      blocks = b;
+    }
+  }
+  const size_t part = (size_t)ceil_div(V, blocks) * 4;
+  const bool staged = part <= MOST;
+  auto kernel = staged ? sample_filtered_kernel<true> : sample_filtered_kernel<false>;
+  const size_t smem = SF_HEAD_BYTES + (staged ? part : 0);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) {
+    set_error("sample_filtered: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
+    return (int)e;
+  }
+  if ((long long)R * blocks > 0x7fffffffll) { set_error("sample_filtered: %d rows are too many", R); return ERR_UNSUPPORTED; }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(R * blocks);
+  cfg.blockDim = dim3(SF_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = blocks;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, logits, reinterpret_cast<const SfRow*>(rows), counts, params, out, V, blocks);
+  return launch_status("sample_filtered");
+}
+
 extern "C" int exl3_sample_filtered(const float* logits, const double* rows, int* out, int R, int V,
                                     cudaStream_t stream) {
-  if (R == 0) return 0;
-  if (R < 0 || V < 1) { set_error("sample_filtered: bad sizes rows=%d vocab=%d", R, V); return ERR_BAD_ARGUMENT; }
-  sample_filtered_kernel<<<R, SF_THREADS, 0, stream>>>(logits, reinterpret_cast<const SfRow*>(rows), out, V);
-  return launch_status("sample_filtered");
+  return exl3_sample_rows(logits, rows, nullptr, nullptr, out, R, V, stream);
 }
 
 extern "C" int exl3_sample_filtered_cap() { return SF_CAP; }

@@ -1158,6 +1158,23 @@ def sample_filtered(logits: torch.Tensor, rows: torch.Tensor, out: Optional[torc
     return out
 
 
+def sample_rows(logits: torch.Tensor, rows: torch.Tensor, counts: torch.Tensor, params: torch.Tensor) -> torch.Tensor:
+    """``sample_filtered`` of logits with penalties (``counts`` and ``params`` as ``sample_penalties`` takes them), which
+    are applied as the logits are read: the logits stay as they are.  The chosen tokens join the counts."""
+    R, V = logits.shape
+    if logits.dtype != torch.float32 or rows.dtype != torch.float64 or tuple(rows.shape) != (R, 5) or \
+            counts.dtype != torch.int64 or counts.numel() != R or params.dtype != torch.float32 or \
+            tuple(params.shape) != (R, 3):
+        raise KernelLibraryError("sample_rows: logits [R, V] and params [R, 3] must be float32, rows [R, 5] float64 and "
+                                 "counts int64 [R]")
+    for t, name in ((logits, "logits"), (rows, "rows"), (counts, "counts"), (params, "params")):
+        _contig(t, name)
+    out = torch.empty((R,), dtype=torch.int32, device=logits.device)
+    _check(library().exl3_sample_rows(_ptr(logits), _ptr(rows), _ptr(counts), _ptr(params), _ptr(out), _c_int(R),
+                                      _c_int(V), _stream()), "sample_rows")
+    return out
+
+
 def sample_penalties(logits: torch.Tensor, counts: torch.Tensor, params: torch.Tensor) -> None:
     """Repetition, presence and frequency penalties, in place.  ``counts``: int64 ``[R]`` on the device, the
     addresses of the rows' int32 ``[V]`` token counts (0: the row has none); ``params``: float32 ``[R, 3]``."""

@@ -52,7 +52,8 @@ def on_device(logits: torch.Tensor, rows: Sequence[RowSampler]) -> bool:
     if not logits.is_cuda:
         return False
     from ..ops import kernels as K
-    return all(r.opt.top_k <= K.sample_filtered_cap() for r in rows)
+    cap = K.sample_filtered_cap()
+    return all(r.opt.top_k <= cap for r in rows)
 
 
 def launch_on_device(logits: torch.Tensor, rows: Sequence[RowSampler]) -> torch.Tensor:
@@ -62,25 +63,35 @@ def launch_on_device(logits: torch.Tensor, rows: Sequence[RowSampler]) -> torch.
     from ..engine.decode import TRANSFERRED
     from ..ops import kernels as K
     R, V = logits.shape
-    counts = None
-    if any(r.opt.has_penalties for r in rows):
-        logits = logits.clone()                          # the step's own buffer stays as the model left it
-        counts = torch.tensor([r.device_counts(V, logits.device).data_ptr() if r.opt.has_penalties else 0
-                               for r in rows], dtype=torch.int64).to(logits.device)
-        params = torch.tensor([[r.opt.repetition_penalty, r.opt.presence_penalty, r.opt.frequency_penalty]
-                               for r in rows], dtype=torch.float32)
-        TRANSFERRED["h2d"] += counts.numel() * 8 + params.numel() * 4
-        K.sample_penalties(logits, counts, params.to(logits.device))
-    # a greedy row draws no number from its generator, as on the host
-    opts = torch.tensor([[r.opt.temperature, r.opt.top_k, r.opt.top_p, r.opt.min_p,
-                          0.0 if r.opt.greedy else r.rng.uniform01()] for r in rows], dtype=torch.float64)
-    ids = K.sample_filtered(logits, opts.to(logits.device))
-    if counts is not None:
-        K.sample_count(counts, ids, V)                   # the chosen tokens join the counts without a trip to the host
-        for r in rows:
-            if r.opt.has_penalties:
-                r.counted()
-    TRANSFERRED["h2d"] += opts.numel() * 8
+    opts, counts, params, penalised = [], [], [], []     # one pass over the rows: their options are read once each
+    for r in rows:
+        o = r.opt
+        # a greedy row draws no number from its generator, as on the host
+        opts.append((o.temperature, o.top_k, o.top_p, o.min_p, 0.0 if o.greedy else r.rng.uniform01()))
+        if o.has_penalties:
+            counts.append(r.device_counts(V, logits.device).data_ptr())
+            params.append((o.repetition_penalty, o.presence_penalty, o.frequency_penalty))
+            penalised.append(r)
+        else:
+            counts.append(0)
+            params.append((1.0, 0.0, 0.0))
+    if not penalised:
+        host = np.array(opts, dtype=np.float64)
+        ids = K.sample_filtered(logits, torch.from_numpy(host).to(logits.device))
+    else:
+        # options, the counts' addresses and the penalties as one buffer: one copy to the device
+        host = np.empty(R * (40 + 8 + 12), dtype=np.uint8)
+        host[:R * 40].view(np.float64).reshape(R, 5)[:] = opts
+        host[R * 40:R * 48].view(np.int64)[:] = counts
+        host[R * 48:].view(np.float32).reshape(R, 3)[:] = params
+        dev = torch.from_numpy(host).to(logits.device)
+        # the kernel reads the logits with their penalties (the step's own buffer stays as the model left it), and the
+        # chosen tokens join the counts without a trip to the host
+        ids = K.sample_rows(logits, dev[:R * 40].view(torch.float64).view(R, 5), dev[R * 40:R * 48].view(torch.int64),
+                            dev[R * 48:].view(torch.float32).view(R, 3))
+        for r in penalised:
+            r.counted()
+    TRANSFERRED["h2d"] += host.nbytes
     return ids
 
 

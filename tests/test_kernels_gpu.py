@@ -1262,3 +1262,26 @@ def test_sample_penalties_as_on_the_host():
     K().sample_count(ptrs, ids, V)
     after = [int(c[t]) for c, t in zip(counts, (5, 6, 7))]
     assert after == [before[0] + 1, before[1], before[2] + 1]
+
+
+@pytest.mark.parametrize("V,R", [(7, 3), (2048, 5), (2049, 2), (40001, 19), (320001, 2)])
+def test_sample_rows_applies_and_counts(V, R):
+    """Rows sampled with their penalties in one kernel against the penalties, the sampler and the counting one by one: for
+    rows shorter than the cluster, around the cap, longer than shared memory holds, and with four blocks a row."""
+    g = torch.Generator(device=DEV).manual_seed(V)
+    logits = 3.0 * torch.randn(R, V, device=DEV, generator=g)
+    counts = [torch.randint(0, 3, (V,), device=DEV, generator=g, dtype=torch.int32) for _ in range(R)]
+    ptrs = torch.tensor([0 if r % 4 == 1 else c.data_ptr() for r, c in enumerate(counts)], dtype=torch.int64, device=DEV)
+    params = torch.tensor([[1.0 + 0.1 * (r % 3), 0.1 * (r % 2), 0.05] for r in range(R)], dtype=torch.float32, device=DEV)
+    rows = torch.tensor([[0.0 if r % 5 == 4 else 0.9, (0, 40)[r % 2], 0.95, 0.01, (0.37 * r + 0.2) % 1.0] for r in range(R)],
+                        dtype=torch.float64, device=DEV)
+    before = [c.clone() for c in counts]
+    changed, kept = logits.clone(), logits.clone()
+    K().sample_penalties(changed, ptrs, params)
+    want = K().sample_filtered(changed, rows)
+    got = K().sample_rows(logits, rows, ptrs, params)
+    assert torch.equal(got, want) and torch.equal(logits, kept)
+    for r in range(R):
+        if r % 4 != 1:
+            before[r][int(want[r])] += 1
+        assert torch.equal(counts[r], before[r])
