@@ -121,7 +121,7 @@ token_shift_vec_kernel(const TH* h, const float* __restrict__ mu, int n_mix, flo
 // ---- the scan ------------------------------------------------------------------------------------------------------
 
 constexpr int LS_STAGE = 8;                      // tokens staged in shared memory at a time
-constexpr int LS_CHUNK = 64;                     // tokens of a chunk when a row's tokens run side by side
+constexpr int LS_CHUNK = 64;                     // tokens of a chunk when a row's tokens run side by side: this or a multiple
 
 struct ScanArgs {
   const void* r; int64_t r_ld; const void* k; int64_t k_ld; int rk_dtype;
@@ -131,12 +131,12 @@ struct ScanArgs {
   const float* decay;
   float* state; const int* slot_ids; const int* row_start;
   float* out; float* ab; float* snap;
-  int heads, dk, dv, places;
+  int heads, dk, dv, places, chunk;              // chunk: tokens of a chunk
   int act;                                       // see ls_in
 };
 
-// Chunk j of batch row b has a place of its own among floor(T / LS_CHUNK) + B + 1 places.
-__device__ inline int ls_place(int t0, int b, int j) { return t0 / LS_CHUNK + b + j; }
+// Chunk j of batch row b has a place of its own among floor(T / chunk) + B + 1 places.
+__device__ inline int ls_place(const ScanArgs& a, int t0, int b, int j) { return t0 / a.chunk + b + j; }
 
 // phase 0: a row's tokens of the step, from its state, state written back.
 // phase 1: a chunk from zero, (A, B) to scratch (no output; the row's last chunk does nothing).
@@ -157,12 +157,12 @@ __global__ void linear_scan_kernel(ScanArgs a, int phase) {
   const int t0 = __ldcg(a.row_start + b), t1 = __ldcg(a.row_start + b + 1);
   int lo = t0, hi = t1;
   if (phase == 1) {
-    lo = t0 + c * LS_CHUNK;
-    hi = lo + LS_CHUNK;
+    lo = t0 + c * a.chunk;
+    hi = lo + a.chunk;
     if (hi >= t1) return;                        // the row's last chunk has nobody after it
   } else if (phase == 2) {
-    lo = t0 + c * LS_CHUNK;
-    hi = min(lo + LS_CHUNK, t1);
+    lo = t0 + c * a.chunk;
+    hi = min(lo + a.chunk, t1);
     if (lo >= t1) return;
   }
   const int j = threadIdx.x;
@@ -176,11 +176,11 @@ __global__ void linear_scan_kernel(ScanArgs a, int phase) {
     if (c == 0 && col) for (int i = 0; i < dk; ++i) snap[i * dv + j] = __ldcg(st + i * dv + j);
   } else {
     // a row of several chunks starts from the copy that the first launch took
-    const float* from = (phase == 2 && t1 - t0 > LS_CHUNK) ? snap : st;
+    const float* from = (phase == 2 && t1 - t0 > a.chunk) ? snap : st;
     if (col) for (int i = 0; i < dk; ++i) S[i * dv + j] = __ldcg(from + i * dv + j);
     if (phase == 2 && col) {
       for (int p = 0; p < c; ++p) {              // the chunks before this one, in order
-        const float* ab = a.ab + ((int64_t)ls_place(t0, b, p) * a.heads + hd) * rec;
+        const float* ab = a.ab + ((int64_t)ls_place(a, t0, b, p) * a.heads + hd) * rec;
         for (int i = 0; i < dk; ++i) S[i * dv + j] = fmaf(__ldcg(ab + i), S[i * dv + j], __ldcg(ab + dk + i * dv + j));
       }
     }
@@ -255,7 +255,7 @@ __global__ void linear_scan_kernel(ScanArgs a, int phase) {
   }
   if (phase == 1) {
     __syncthreads();
-    float* ab = a.ab + ((int64_t)ls_place(t0, b, c) * a.heads + hd) * rec;
+    float* ab = a.ab + ((int64_t)ls_place(a, t0, b, c) * a.heads + hd) * rec;
     for (int i = threadIdx.x; i < dk; i += blockDim.x) ab[i] = sA[i];
     if (col) for (int i = 0; i < dk; ++i) ab[dk + i * dv + j] = S[i * dv + j];
   } else if (hi == t1 && col) {
@@ -290,12 +290,12 @@ __global__ void __launch_bounds__(LS_Q * LS_MAX_DV, DK <= 64 ? 2 : 1) linear_sca
   const int t0 = __ldcg(a.row_start + b), t1 = __ldcg(a.row_start + b + 1);
   int lo = t0, hi = t1;
   if (phase == 1) {
-    lo = t0 + c * LS_CHUNK;
-    hi = lo + LS_CHUNK;
+    lo = t0 + c * a.chunk;
+    hi = lo + a.chunk;
     if (hi >= t1) return;
   } else if (phase == 2) {
-    lo = t0 + c * LS_CHUNK;
-    hi = min(lo + LS_CHUNK, t1);
+    lo = t0 + c * a.chunk;
+    hi = min(lo + a.chunk, t1);
     if (lo >= t1) return;
   }
   const int q = threadIdx.x / dvr, j = threadIdx.x - q * dvr;
@@ -314,13 +314,13 @@ __global__ void __launch_bounds__(LS_Q * LS_MAX_DV, DK <= 64 ? 2 : 1) linear_sca
       for (int i = 0; i < DKQ; ++i) snap[(i0 + i) * dv + j] = __ldcg(st + (i0 + i) * dv + j);
     }
   } else {
-    const float* from = (phase == 2 && t1 - t0 > LS_CHUNK) ? snap : st;
+    const float* from = (phase == 2 && t1 - t0 > a.chunk) ? snap : st;
 #pragma unroll
     for (int i = 0; i < DKQ; ++i) S[i] = col ? __ldcg(from + (i0 + i) * dv + j) : 0.0f;
     if (phase == 2 && col) {
 #pragma unroll 2
       for (int p = 0; p < c; ++p) {                  // the chunks before this one, in order
-        const float* ab = a.ab + ((int64_t)ls_place(t0, b, p) * a.heads + hd) * rec;
+        const float* ab = a.ab + ((int64_t)ls_place(a, t0, b, p) * a.heads + hd) * rec;
 #pragma unroll
         for (int i = 0; i < DKQ; ++i) S[i] = fmaf(__ldcg(ab + i0 + i), S[i], __ldcg(ab + DK + (i0 + i) * dv + j));
       }
@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(LS_Q * LS_MAX_DV, DK <= 64 ? 2 : 1) linear_sca
   }
   if (phase == 1) {
     __syncthreads();
-    float* ab = a.ab + ((int64_t)ls_place(t0, b, c) * a.heads + hd) * rec;
+    float* ab = a.ab + ((int64_t)ls_place(a, t0, b, c) * a.heads + hd) * rec;
     for (int i = threadIdx.x; i < DK; i += blockDim.x) ab[i] = sA[i];
     if (col) {
 #pragma unroll
@@ -449,6 +449,278 @@ __global__ void __launch_bounds__(LS_Q * LS_MAX_DV, DK <= 64 ? 2 : 1) linear_sca
   } else if (hi == t1 && col) {
 #pragma unroll
     for (int i = 0; i < DKQ; ++i) st[(i0 + i) * dv + j] = S[i];
+  }
+}
+
+// The same for key sizes of 64 and up to 128 values a head in sixteens, with 16-byte rows.  A thread has two columns of S
+// and a quarter of their key channels, as eight pairs of channels: a token costs it 48 paired fma (one and a product for the
+// update, one for the output) and 13 reads of shared memory for r, k, the decays and v.  The quarters of a column are lanes
+// of one warp (a quarter's eight lanes side by side: with the quarters side by side the same loop took 157 us instead of
+// 115), so an output's four parts meet in two shuffles and no barrier; sixteen tokens are staged at a time,
+// read 16 bytes a thread a stage ahead and widened (the decays' exponentials taken) on their way into shared memory.
+// Bound by what a warp does for one token after the other (some 270 cycles alone on its SM): rows of 520, 120, 300,
+// 400, 200, 350, 450 and 320 tokens with 32 heads of 64 x 64 and decays 114 us (the kernel above, in chunks: 368), with 16
+// heads of 64 x 128 127 us (280); one row of 8,192 tokens 474 (1,546) and 349 us (1,284).  Sixteen columns of eight channels,
+// or eight of four, a thread's work cut differently at the same sum: 119 and 150 us for the first of these.
+constexpr int LW_DK = 64, LW_STAGE = 16, LW_Q = 4, LW_COLS = 2, LW_PAIRS = LW_DK / LW_Q / 2;
+// A staged row: the quarters 20 floats apart, so that the four addresses of a warp's read do not collide.
+constexpr int LW_QP = LW_DK / LW_Q + 4, LW_ROW = LW_Q * LW_QP;
+__device__ inline int lw_at(int i) { return i / (LW_DK / LW_Q) * LW_QP + i % (LW_DK / LW_Q); }
+
+__device__ inline unsigned long long lw_dup(float v) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+  return r;
+}
+__device__ inline unsigned long long lw_mul(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ inline unsigned long long lw_fma(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ inline float2 lw_split(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ inline unsigned long long lw_pair(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+
+// TK: element type of r, k; TV: of v and the raw decays.  PHASE as above.
+template <int MODE, int PHASE, typename TK, typename TV>
+__global__ void __launch_bounds__(LW_Q * LS_MAX_DV / LW_COLS, MODE == 0 ? 1 : 2) linear_scan_wide_kernel(ScanArgs a) {
+  constexpr int VK = Elem<TK>::vec, VV = Elem<TV>::vec;
+  __shared__ __align__(16) float sr[LW_STAGE * LW_ROW];
+  __shared__ __align__(16) float sk[LW_STAGE * LW_ROW];
+  __shared__ __align__(16) float sw[MODE == 0 ? LW_STAGE * LW_ROW : 4];
+  __shared__ __align__(16) float sv[LW_STAGE * LS_MAX_DV];
+  __shared__ float sb[LW_STAGE];
+  __shared__ float su[MODE == 0 ? LW_DK : 1], sw0[MODE == 0 ? LW_DK : 1];
+  const int tid = threadIdx.x, lane = tid & 31, dv = a.dv, threads = blockDim.x;
+  const int hd = blockIdx.x, c = blockIdx.y, b = blockIdx.z;
+  if (MODE == 0 && tid < LW_DK) {
+    su[tid] = ls_load(a.u, a.wu_dtype, (int64_t)hd * LW_DK + tid);
+    sw0[tid] = ls_load(a.w0, a.wu_dtype, (int64_t)hd * LW_DK + tid);
+  }
+  pdl_wait();
+  pdl_trigger();
+  const int t0 = __ldcg(a.row_start + b), t1 = __ldcg(a.row_start + b + 1);
+  int lo = t0, hi = t1;
+  if (PHASE == 1) {
+    lo = t0 + c * a.chunk;
+    hi = lo + a.chunk;
+    if (hi >= t1) return;
+  } else if (PHASE == 2) {
+    lo = t0 + c * a.chunk;
+    hi = min(lo + a.chunk, t1);
+    if (lo >= t1) return;
+  }
+  const int q = lane >> 3, j = ((tid >> 5) * 8 + (lane & 7)) * LW_COLS;    // columns j, j + 1; channels 16 q .. 16 q + 15
+  float* st = a.state + ((int64_t)__ldcg(a.slot_ids + b) * a.heads + hd) * LW_DK * dv;
+  const int64_t rec = (int64_t)LW_DK + (int64_t)LW_DK * dv;
+  float* snap = a.snap + ((int64_t)b * a.heads + hd) * LW_DK * dv;
+  unsigned long long S[LW_COLS][LW_PAIRS];
+  float decays = 1.0f;                                                      // phase 1: channel tid's product
+  // a matrix's part of this thread: pairs of channels of both columns
+  auto pairs_of = [&](const float* from, auto&& f) {
+#pragma unroll
+    for (int p = 0; p < LW_PAIRS; ++p) {
+      const int i = q * (LW_DK / LW_Q) + 2 * p;
+      const float2 x = __ldcg(reinterpret_cast<const float2*>(from + (int64_t)i * dv + j));
+      const float2 y = __ldcg(reinterpret_cast<const float2*>(from + (int64_t)(i + 1) * dv + j));
+      const unsigned long long v[LW_COLS] = {lw_pair(x.x, y.x), lw_pair(x.y, y.y)};
+      f(p, i, v);
+    }
+  };
+  auto take = [&](int p, int, const unsigned long long (&v)[LW_COLS]) {
+#pragma unroll
+    for (int m = 0; m < LW_COLS; ++m) S[m][p] = v[m];
+  };
+  auto put_pairs = [&](float* to) {
+#pragma unroll
+    for (int p = 0; p < LW_PAIRS; ++p) {
+      const int i = q * (LW_DK / LW_Q) + 2 * p;
+      const float2 c0 = lw_split(S[0][p]), c1 = lw_split(S[1][p]);
+      *reinterpret_cast<float2*>(to + (int64_t)i * dv + j) = make_float2(c0.x, c1.x);
+      *reinterpret_cast<float2*>(to + (int64_t)(i + 1) * dv + j) = make_float2(c0.y, c1.y);
+    }
+  };
+  if (PHASE == 1) {
+    if (c == 0) {
+      pairs_of(st, take);
+      put_pairs(snap);
+    }
+#pragma unroll
+    for (int p = 0; p < LW_PAIRS; ++p)
+#pragma unroll
+      for (int m = 0; m < LW_COLS; ++m) S[m][p] = 0;
+  } else {
+    pairs_of((PHASE == 2 && t1 - t0 > a.chunk) ? snap : st, take);
+    if (PHASE == 2) {
+#pragma unroll 1
+      for (int e = 0; e < c; ++e) {                                         // the chunks before this one, in order
+        const float* ab = a.ab + ((int64_t)ls_place(a, t0, b, e) * a.heads + hd) * rec;
+        pairs_of(ab + LW_DK, [&](int p, int i, const unsigned long long (&v)[LW_COLS]) {
+          const float2 w = __ldcg(reinterpret_cast<const float2*>(ab + i));
+          const unsigned long long ww = lw_pair(w.x, w.y);
+#pragma unroll
+          for (int m = 0; m < LW_COLS; ++m) S[m][p] = lw_fma(ww, S[m][p], v[m]);
+        });
+      }
+    }
+  }
+  const float gamma = MODE == 1 ? a.decay[hd] : 0.0f;
+  const unsigned long long gamma2 = lw_dup(gamma);
+
+  // a stage's inputs a stage ahead in registers, 16 bytes a thread
+  constexpr int NK = LW_STAGE * LW_DK / VK, NW = LW_STAGE * LW_DK / VV;     // pieces of r or k, of the raw decays
+  constexpr int HK = NK / 128, HW = NW / 128, HV = LW_STAGE / (2 * VV);     // a block has 2 dv >= 128 threads
+  uint4 pr[HK], pk[HK], pw[MODE == 0 ? HW : 1], pv[HV];
+  const int vpieces = dv / VV;                                              // of a token's values
+  auto fetch = [&](int s0) {
+    const int n = min(LW_STAGE, hi - s0);
+#pragma unroll
+    for (int e = 0; e < HK; ++e) {
+      const int idx = tid + e * threads, tt = idx / (LW_DK / VK), i = idx % (LW_DK / VK) * VK;
+      if (idx < NK && tt < n) {
+        if (PHASE != 1) pr[e] = load_raw_cg(static_cast<const TK*>(a.r) + (int64_t)(s0 + tt) * a.r_ld + hd * LW_DK + i);
+        pk[e] = load_raw_cg(static_cast<const TK*>(a.k) + (int64_t)(s0 + tt) * a.k_ld + hd * LW_DK + i);
+      }
+    }
+    if (MODE == 0) {
+#pragma unroll
+      for (int e = 0; e < HW; ++e) {
+        const int idx = tid + e * threads, tt = idx / (LW_DK / VV), i = idx % (LW_DK / VV) * VV;
+        if (idx < NW && tt < n) pw[e] = load_raw_cg(static_cast<const TV*>(a.wraw) + (int64_t)(s0 + tt) * a.w_ld + hd * LW_DK + i);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < HV; ++e) {
+      const int idx = tid + e * threads, tt = idx / vpieces;
+      if (tt < n) pv[e] = load_raw_cg(static_cast<const TV*>(a.v) + (int64_t)(s0 + tt) * a.v_ld + (int64_t)hd * dv + (idx - tt * vpieces) * VV);
+    }
+  };
+  fetch(lo);
+#pragma unroll 1
+  for (int s0 = lo; s0 < hi; s0 += LW_STAGE) {
+    const int n = min(LW_STAGE, hi - s0);
+    __syncthreads();                                                        // the stage before has been used
+#pragma unroll
+    for (int e = 0; e < HK; ++e) {
+      const int idx = tid + e * threads, tt = idx / (LW_DK / VK), i = idx % (LW_DK / VK) * VK;
+      float bonus = 0.0f;
+      if (idx < NK && tt < n) {
+        float x[VK], y[VK];
+        unpack_raw(pk[e], y, (const TK*)nullptr);
+#pragma unroll
+        for (int z = 0; z < VK; ++z) y[z] = ls_in(y[z], a.act);
+#pragma unroll
+        for (int z = 0; z < VK; z += 4)
+          *reinterpret_cast<float4*>(sk + tt * LW_ROW + lw_at(i + z)) = make_float4(y[z], y[z + 1], y[z + 2], y[z + 3]);
+        if (PHASE != 1) {
+          unpack_raw(pr[e], x, (const TK*)nullptr);
+#pragma unroll
+          for (int z = 0; z < VK; ++z) {
+            x[z] = ls_in(x[z], a.act);
+            if (MODE == 0) bonus = fmaf(x[z] * su[i + z], y[z], bonus);
+          }
+#pragma unroll
+          for (int z = 0; z < VK; z += 4)
+            *reinterpret_cast<float4*>(sr + tt * LW_ROW + lw_at(i + z)) = make_float4(x[z], x[z + 1], x[z + 2], x[z + 3]);
+        }
+      }
+      if (MODE == 0 && PHASE != 1) {                                        // a token's pieces are neighbours in a warp
+#pragma unroll
+        for (int o = LW_DK / VK / 2; o > 0; o >>= 1) bonus += __shfl_xor_sync(0xffffffffu, bonus, o);
+        if (idx < NK && tt < n && i == 0) sb[tt] = bonus;
+      }
+    }
+    if (MODE == 0) {
+#pragma unroll
+      for (int e = 0; e < HW; ++e) {
+        const int idx = tid + e * threads, tt = idx / (LW_DK / VV), i = idx % (LW_DK / VV) * VV;
+        if (idx < NW && tt < n) {
+          float x[VV];
+          unpack_raw(pw[e], x, (const TV*)nullptr);
+#pragma unroll
+          for (int z = 0; z < VV; ++z) x[z] = expf(-expf(x[z] + sw0[i + z]));
+#pragma unroll
+          for (int z = 0; z < VV; z += 4)
+            *reinterpret_cast<float4*>(sw + tt * LW_ROW + lw_at(i + z)) = make_float4(x[z], x[z + 1], x[z + 2], x[z + 3]);
+        }
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < HV; ++e) {
+      const int idx = tid + e * threads, tt = idx / vpieces;
+      if (tt < n) {
+        float x[VV];
+        unpack_raw(pv[e], x, (const TV*)nullptr);
+#pragma unroll
+        for (int z = 0; z < VV; ++z) x[z] = ls_in(x[z], a.act);
+#pragma unroll
+        for (int z = 0; z < VV; z += 4)
+          *reinterpret_cast<float4*>(sv + tt * LS_MAX_DV + (idx - tt * vpieces) * VV + z) =
+              make_float4(x[z], x[z + 1], x[z + 2], x[z + 3]);
+      }
+    }
+    __syncthreads();
+    if (s0 + LW_STAGE < hi) fetch(s0 + LW_STAGE);
+    if (PHASE == 1 && tid < LW_DK) {
+      for (int tt = 0; tt < n; ++tt)
+        decays *= MODE == 0 ? sw[tt * LW_ROW + lw_at(tid)] : gamma;
+    }
+    const bool odd = q & 1;                                                 // the column whose output ends up in this lane
+    float* to = a.out + (int64_t)s0 * a.heads * dv + (int64_t)hd * dv + j + (odd ? 1 : 0);
+#pragma unroll 2
+    for (int tt = 0; tt < n; ++tt) {
+      const float* rt = sr + tt * LW_ROW + q * LW_QP;
+      const float* kt = sk + tt * LW_ROW + q * LW_QP;
+      const float* wt = MODE == 0 ? sw + tt * LW_ROW + q * LW_QP : nullptr;
+      const float2 v = *reinterpret_cast<const float2*>(sv + tt * LS_MAX_DV + j);
+      const unsigned long long vv[LW_COLS] = {lw_dup(v.x), lw_dup(v.y)};
+      unsigned long long o[LW_COLS] = {0, 0};
+#pragma unroll
+      for (int h = 0; h < LW_PAIRS / 2; ++h) {
+        const ulonglong2 k2 = *reinterpret_cast<const ulonglong2*>(kt + h * 4);
+        const ulonglong2 w2 = MODE == 0 ? *reinterpret_cast<const ulonglong2*>(wt + h * 4) : make_ulonglong2(gamma2, gamma2);
+        const ulonglong2 r2 = PHASE != 1 ? *reinterpret_cast<const ulonglong2*>(rt + h * 4) : make_ulonglong2(0, 0);
+#pragma unroll
+        for (int z = 0; z < 2; ++z) {
+          const unsigned long long kp = z ? k2.y : k2.x, wp = z ? w2.y : w2.x, rp = z ? r2.y : r2.x;
+          const int p = 2 * h + z;
+#pragma unroll
+          for (int m = 0; m < LW_COLS; ++m) {
+            if (MODE == 0 && PHASE != 1) o[m] = lw_fma(rp, S[m][p], o[m]);  // the output sees the state before the token
+            S[m][p] = lw_fma(wp, S[m][p], lw_mul(kp, vv[m]));
+            if (MODE == 1 && PHASE != 1) o[m] = lw_fma(rp, S[m][p], o[m]);
+          }
+        }
+      }
+      if (PHASE != 1) {
+        // lanes of odd quarters go on with the second column, of even ones with the first; then both halves
+        const float2 e0 = lw_split(o[0]), e1 = lw_split(o[1]);
+        const float y0 = e0.x + e0.y, y1 = e1.x + e1.y;
+        float out = (odd ? y1 : y0) + __shfl_xor_sync(0xffffffffu, odd ? y0 : y1, 8);
+        out += __shfl_xor_sync(0xffffffffu, out, 16);
+        if (MODE == 0) out = fmaf(sb[tt], odd ? v.y : v.x, out);            // the bonus
+        if (q < 2) to[(int64_t)tt * a.heads * dv] = out;
+      }
+    }
+  }
+  if (PHASE == 1) {
+    float* ab = a.ab + ((int64_t)ls_place(a, t0, b, c) * a.heads + hd) * rec;
+    if (tid < LW_DK) ab[tid] = decays;
+    put_pairs(ab + LW_DK);
+  } else if (hi == t1) {
+    put_pairs(st);
   }
 }
 
@@ -565,11 +837,37 @@ head_norm_gate_vec_kernel(const float* o, const float* __restrict__ w, const TG*
 
 using namespace exl3;
 
-static bool ls_chunked(int max_new) { return max_new > 2 * LS_CHUNK; }
+// Sizes that the wide kernel takes (with 16-byte rows: else the kernels above run, over the same chunks).
+static bool ls_wide(int dk, int dv) { return dk == LW_DK && dv % 16 == 0 && dv >= 64 && dv <= LS_MAX_DV; }
+
+static int ls_sm_count() {
+  static thread_local int dev_of = -1, count = 0;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev != dev_of) {
+    if (cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) count = 148;
+    dev_of = dev;
+  }
+  return count;
+}
+
+// Tokens of a chunk, 0 for rows that are walked whole.  The wide kernel walks rows whole while they keep half the SMs busy
+// for as long as the longest one takes (the eight rows above: whole 114 us, in chunks of 64 / 128
+// / 256 132 / 126 / 171; four rows of 2,048 287 against 448 / 366 / 356); else chunks leave two blocks an SM, since every chunk
+// pays for folding the ones before it (one row of 8,192: chunks of 64 747 us, of 256 378, of 896 470, whole 1,137).
+static int ls_chunk_len(int T, int heads, int dk, int dv, int max_new) {
+  if (max_new <= 2 * LS_CHUNK) return 0;
+  if (!ls_wide(dk, dv)) return LS_CHUNK;
+  const int64_t work = (int64_t)T * heads, sms = ls_sm_count();
+  if (2 * work >= sms * max_new) return 0;
+  const int64_t len = (work / (2 * sms) + LS_CHUNK - 1) / LS_CHUNK * LS_CHUNK;
+  return len < LS_CHUNK ? LS_CHUNK : (len >= max_new ? 0 : (int)len);
+}
 
 extern "C" size_t exl3_linear_scan_scratch_bytes(int B, int T, int heads, int dk, int dv, int max_new) {
-  if (!ls_chunked(max_new)) return 0;
-  return ((size_t)(T / LS_CHUNK + B + 1) * heads * ((size_t)dk + (size_t)dk * dv) + (size_t)B * heads * dk * dv) *
+  const int chunk = ls_chunk_len(T, heads, dk, dv, max_new);
+  if (chunk == 0) return 0;
+  return ((size_t)(T / chunk + B + 1) * heads * ((size_t)dk + (size_t)dk * dv) + (size_t)B * heads * dk * dv) *
          sizeof(float);
 }
 
@@ -646,23 +944,47 @@ extern "C" int exl3_linear_scan(int mode, const void* r, int64_t r_ld, const voi
   a.wraw = wraw; a.w_ld = w_ld; a.w_dtype = w_dtype; a.w0 = w0; a.u = u; a.wu_dtype = wu_dtype; a.decay = decay;
   a.state = state; a.slot_ids = slot_ids; a.row_start = row_start; a.out = out; a.ab = scratch;
   a.act = in_act;
-  a.heads = heads; a.dk = dk; a.dv = dv; a.places = T / LS_CHUNK + B + 1;
+  a.heads = heads; a.dk = dk; a.dv = dv; a.chunk = ls_chunk_len(T, heads, dk, dv, max_new);
+  a.places = a.chunk > 0 ? T / a.chunk + B + 1 : 0;
   a.snap = scratch ? scratch + (size_t)a.places * heads * ((size_t)dk + (size_t)dk * dv) : nullptr;
   const int threads = regs ? LS_Q * dvr : dvr;
-  if (ls_chunked(max_new)) {
-    const int chunks = ceil_div(max_new, LS_CHUNK);
+  const int vk = rk_dtype == DT_F32 ? 4 : 8, vv = v_dtype == DT_F32 ? 4 : 8;
+  const bool wide = ls_wide(dk, dv) && r_ld % vk == 0 && k_ld % vk == 0 && v_ld % vv == 0 && aligned16(r) && aligned16(k) &&
+                    aligned16(v) && aligned16(state) && aligned16(out) && aligned16(scratch) &&
+                    (mode == 1 || (w_dtype == v_dtype && w_ld % vv == 0 && aligned16(wraw)));
+  auto go = [&](int phase, int chunks) {
+    const dim3 grid(heads, chunks, B);
+    if (!wide) {
+      launch_pdl(by_phase[phase], grid, dim3(threads), smem, stream, a, phase);
+      return;
+    }
+#define EXL3_WIDE(M, TK, TV)                                                                                          \
+  launch_pdl(phase == 0 ? linear_scan_wide_kernel<M, 0, TK, TV> : phase == 1 ? linear_scan_wide_kernel<M, 1, TK, TV>  \
+                                                                              : linear_scan_wide_kernel<M, 2, TK, TV>, \
+             grid, dim3(LW_Q * dv / LW_COLS), 0, stream, a)
+#define EXL3_WIDE_TYPES(M)                                                                    \
+  if (rk_dtype == DT_F32 && v_dtype == DT_F32) EXL3_WIDE(M, float, float);                    \
+  else if (rk_dtype == DT_F32) EXL3_WIDE(M, float, __nv_bfloat16);                            \
+  else if (v_dtype == DT_F32) EXL3_WIDE(M, __nv_bfloat16, float);                             \
+  else EXL3_WIDE(M, __nv_bfloat16, __nv_bfloat16);
+    if (mode == 0) { EXL3_WIDE_TYPES(0) } else { EXL3_WIDE_TYPES(1) }
+#undef EXL3_WIDE_TYPES
+#undef EXL3_WIDE
+  };
+  if (a.chunk > 0) {
+    const int chunks = ceil_div(max_new, a.chunk);
     if (scratch == nullptr || exl3_linear_scan_scratch_bytes(B, T, heads, dk, dv, max_new) > scratch_bytes ||
         chunks > 65535) {
       set_error("linear_scan: scratch of %zu bytes is too small for %d tokens", scratch_bytes, T);
       return ERR_SCRATCH;
     }
-    launch_pdl(by_phase[1], dim3(heads, chunks, B), dim3(threads), smem, stream, a, 1);
+    go(1, chunks);
     int rc = launch_status("linear_scan (chunks)");
     if (rc) return rc;
-    launch_pdl(by_phase[2], dim3(heads, chunks, B), dim3(threads), smem, stream, a, 2);
+    go(2, chunks);
     return launch_status("linear_scan (fold)");
   }
-  launch_pdl(by_phase[0], dim3(heads, 1, B), dim3(threads), smem, stream, a, 0);
+  go(0, 1);
   return launch_status("linear_scan");
 }
 

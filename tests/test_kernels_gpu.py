@@ -1285,3 +1285,62 @@ def test_sample_rows_applies_and_counts(V, R):
         if r % 4 != 1:
             before[r][int(want[r])] += 1
         assert torch.equal(counts[r], before[r])
+
+
+# The recurrence's wide kernel (keys of 64, values in sixteens): around its stages of sixteen tokens, rows walked whole and
+# in chunks (a long row with few heads), cut into two steps, in both types.  Everything but the inputs' type is float32: the
+# inputs are rounded first, and the chains of some hundred sums stay within 2e-5 of the largest output.
+@pytest.mark.parametrize("mode,dv,dtype", [(0, 64, torch.bfloat16), (1, 128, torch.float32), (0, 80, torch.float32),
+                                           (1, 112, torch.bfloat16)])
+@pytest.mark.parametrize("counts", [[1], [16, 1, 17], [130, 3], [700], [33] * 9])
+def test_linear_scan_wide(mode, dv, dtype, counts):
+    H, dk, B = 3, 64, len(counts)
+    g = torch.Generator(device=DEV).manual_seed(dv + sum(counts))
+    draw = lambda *s: torch.randn(*s, device=DEV, generator=g)  # noqa: E731
+    T = sum(counts)
+    r, k, v, w = draw(T, H * dk).to(dtype), draw(T, H * dk).to(dtype), draw(T, H * dv).to(dtype), (draw(T, H * dk) - 2.0).to(dtype)
+    start = draw(B + 1, H, dk, dv)
+    w0, u, decay = draw(H * dk), draw(H * dk), torch.rand(H, device=DEV, generator=g) * 0.2 + 0.8
+    slots = torch.randperm(B, device=DEV, generator=g).to(torch.int32)
+
+    def scan(state, parts):
+        """Each row's tokens in ``parts`` steps."""
+        outs = [[] for _ in counts]
+        for p in range(parts):
+            cuts = [(n * p // parts, n * (p + 1) // parts) for n in counts]
+            at = torch.cat([torch.arange(sum(counts[:b]) + x, sum(counts[:b]) + y, device=DEV) for b, (x, y) in enumerate(cuts)])
+            new = [y - x for x, y in cuts]
+            rows = torch.tensor([sum(new[:b]) for b in range(B + 1)], dtype=torch.int32, device=DEV)
+            more = dict(wraw=w[at], w0=w0, u=u) if mode == 0 else dict(decay=decay)
+            need = K().linear_scan_scratch_bytes(B, len(at), H, dk, dv, max(new))
+            scratch = torch.empty(max(1, need // 4), device=DEV)
+            o = K().linear_scan(mode, r[at], k[at], v[at], state, slots, rows, B, H, dk, dv, max(new), scratch=scratch, **more)
+            for b in range(B):
+                outs[b].append(o[sum(new[:b]):sum(new[:b + 1])])
+        return torch.cat([x for row in outs for x in row])
+
+    state = start.clone()
+    got = scan(state, 1)
+    S = start.double()[slots.long()].cpu()
+    rr, kk, vv = (x.double().cpu().view(T, H, -1) for x in (r, k, v))
+    ww = torch.exp(-torch.exp(w.double().cpu() + w0.double().cpu())).view(T, H, dk)
+    uu = u.double().cpu().view(H, dk)
+    want = torch.empty(T, H, dv, dtype=torch.float64)
+    t = 0
+    for b, n in enumerate(counts):
+        for _ in range(n):
+            kv = kk[t][:, :, None] * vv[t][:, None, :]
+            if mode == 0:
+                want[t] = ((S[b] + uu[:, :, None] * kv) * rr[t][:, :, None]).sum(1)
+                S[b] = ww[t][:, :, None] * S[b] + kv
+            else:
+                S[b] = decay.double().cpu()[:, None, None] * S[b] + kv
+                want[t] = (S[b] * rr[t][:, :, None]).sum(1)
+            t += 1
+    close(got, want.reshape(T, H * dv), 2e-5, "outputs")
+    close(state[slots.long()], S, 2e-5, "states")
+    assert torch.equal(state[B], start[B])
+    if min(counts) >= 2:
+        again = start.clone()
+        close(scan(again, 2), want.reshape(T, H * dv), 2e-5, "in two steps")
+        close(again[slots.long()], S, 2e-5, "states after two steps")
