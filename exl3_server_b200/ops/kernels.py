@@ -41,7 +41,8 @@ def _ptr(t: Optional[torch.Tensor]) -> _c_void_p:
 
 
 def _stream() -> _c_void_p:
-    return _c_void_p(torch.cuda.current_stream().cuda_stream)
+    # the current device's current stream, without making a Stream object of it (a fifth of what a launch costs the host)
+    return _c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def _check(rc: int, what: str) -> None:
