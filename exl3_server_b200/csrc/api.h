@@ -296,6 +296,10 @@ int exl3_attn_decode(const void* q, int64_t q_row_stride, void* out, void* k_poo
 
 int exl3_argmax(const float* logits, int* out, int R, int V, void* scratch, size_t scratch_bytes,
                 cudaStream_t stream);
+// The end of a decode step: out[r] = feed[r] = the argmax of row r, pos[r] += inc[r] (scratch as the second function says).
+int exl3_argmax_step(const float* logits, int* out, int* feed, int* pos, const int* inc, int R, int V, void* scratch,
+                     size_t scratch_bytes, cudaStream_t stream);
+size_t exl3_argmax_step_scratch_bytes(int R, int V);
 // The reference's sampler on the device (see sampling_filtered.cu).  rows: float64 [R, 5] = temperature (<= 0:
 // greedy), top_k (0: off; at most exl3_sample_filtered_cap()), top_p, min_p, uniform number in [0, 1).
 int exl3_sample_filtered(const float* logits, const double* rows, int* out, int R, int V, cudaStream_t stream);

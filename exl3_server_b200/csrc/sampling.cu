@@ -91,8 +91,11 @@ argmax_partial_kernel(const float* __restrict__ logits, float* __restrict__ pv, 
   if (threadIdx.x == 0) { pv[(int64_t)row * nchunks + chunk] = best; pi[(int64_t)row * nchunks + chunk] = bi; }
 }
 
+// The end of a decode step, where the ids are known: feed[row] takes the id and pos[row] goes on by inc[row] (feed null:
+// neither).  They were a copy and an addition of their own at the end of every step: two launches, 5 us.
 __global__ void __launch_bounds__(ARGMAX_THREADS)
-argmax_final_kernel(const float* __restrict__ pv, const int* __restrict__ pi, int* __restrict__ out, int nchunks) {
+argmax_final_kernel(const float* __restrict__ pv, const int* __restrict__ pi, int* __restrict__ out, int nchunks, int* feed,
+                    int* pos, const int* inc) {
   __shared__ float sv[32];
   __shared__ int si[32];
   pdl_wait();
@@ -106,7 +109,27 @@ argmax_final_kernel(const float* __restrict__ pv, const int* __restrict__ pi, in
     if (i != 0x7fffffff && (bi == 0x7fffffff || argmax_better(v, i, best, bi))) { best = v; bi = i; }
   }
   argmax_block_reduce(best, bi, sv, si);
-  if (threadIdx.x == 0) out[row] = (bi == 0x7fffffff) ? 0 : bi;
+  if (threadIdx.x == 0) {
+    const int id = (bi == 0x7fffffff) ? 0 : bi;
+    out[row] = id;
+    if (feed) {
+      feed[row] = id;
+      pos[row] = __ldcg(pos + row) + __ldcg(inc + row);
+    }
+  }
+}
+
+static int argmax_two_stages(const float* logits, int* out, int R, int V, void* scratch, int* feed, int* pos, const int* inc,
+                             const char* what, cudaStream_t stream) {
+  const int nchunks = ceil_div(V, ARGMAX_CHUNK);
+  float* pv = static_cast<float*>(scratch);
+  int* pi = reinterpret_cast<int*>(pv + (size_t)R * nchunks);
+  launch_pdl(argmax_partial_kernel, dim3(nchunks, R), dim3(ARGMAX_THREADS), 0, stream, logits, pv, pi, V, nchunks);
+  int rc = launch_status(what);
+  if (rc) return rc;
+  launch_pdl(argmax_final_kernel, dim3(R), dim3(ARGMAX_THREADS), 0, stream, (const float*)pv, (const int*)pi, out, nchunks,
+             feed, pos, inc);
+  return launch_status(what);
 }
 
 }  // namespace exl3
@@ -133,15 +156,25 @@ extern "C" int exl3_argmax(const float* logits, int* out, int R, int V, void* sc
     return ERR_SCRATCH;
   }
   if (R > 65535) { set_error("argmax: too many rows (%d)", R); return ERR_UNSUPPORTED; }
-  const int nchunks = ceil_div(V, ARGMAX_CHUNK);
-  float* pv = static_cast<float*>(scratch);
-  int* pi = reinterpret_cast<int*>(pv + (size_t)R * nchunks);
-  launch_pdl(argmax_partial_kernel, dim3(nchunks, R), dim3(ARGMAX_THREADS), 0, stream, logits, pv, pi, V, nchunks);
-  int rc = launch_status("argmax_partial");
-  if (rc) return rc;
-  launch_pdl(argmax_final_kernel, dim3(R), dim3(ARGMAX_THREADS), 0, stream, (const float*)pv, (const int*)pi, out,
-             nchunks);
-  return launch_status("argmax_final");
+  return argmax_two_stages(logits, out, R, V, scratch, nullptr, nullptr, nullptr, "argmax", stream);
+}
+
+extern "C" size_t exl3_argmax_step_scratch_bytes(int R, int V) {
+  return (size_t)R * ceil_div(V, ARGMAX_CHUNK) * (sizeof(float) + sizeof(int));
+}
+
+extern "C" int exl3_argmax_step(const float* logits, int* out, int* feed, int* pos, const int* inc, int R, int V,
+                                void* scratch, size_t scratch_bytes, cudaStream_t stream) {
+  if (R == 0) return 0;
+  if (R < 0 || R > 65535 || V < 1 || feed == nullptr || pos == nullptr || inc == nullptr) {
+    set_error("argmax_step: bad sizes rows=%d vocab=%d, or a missing buffer", R, V);
+    return ERR_BAD_ARGUMENT;
+  }
+  if (scratch == nullptr || scratch_bytes < exl3_argmax_step_scratch_bytes(R, V)) {
+    set_error("argmax_step: scratch of %zu bytes is too small", scratch_bytes);
+    return ERR_SCRATCH;
+  }
+  return argmax_two_stages(logits, out, R, V, scratch, feed, pos, inc, "argmax_step", stream);
 }
 
 // ---------------------------------------------------------------------------
@@ -198,13 +231,5 @@ extern "C" int exl3_argmax_static(const float* logits, int* out, int R, int V, c
   // Same two kernels as exl3_argmax, for every vocabulary size, so that the
   // array is what the second kernel reads.  Every (row, chunk) entry that the
   // second kernel reads is written by the first in this call.
-  const int nchunks = ceil_div(V, ARGMAX_CHUNK);
-  float* pv = static_cast<float*>(scratch);
-  int* pi = reinterpret_cast<int*>(pv + (size_t)R * nchunks);
-  launch_pdl(argmax_partial_kernel, dim3(nchunks, R), dim3(ARGMAX_THREADS), 0, stream, logits, pv, pi, V, nchunks);
-  rc = launch_status("argmax_static (partial)");
-  if (rc) return rc;
-  launch_pdl(argmax_final_kernel, dim3(R), dim3(ARGMAX_THREADS), 0, stream, (const float*)pv, (const int*)pi, out,
-             nchunks);
-  return launch_status("argmax_static (final)");
+  return argmax_two_stages(logits, out, R, V, scratch, nullptr, nullptr, nullptr, "argmax_static", stream);
 }

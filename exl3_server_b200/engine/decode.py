@@ -131,9 +131,7 @@ class DecodeRunner:
         try:
             with torch.cuda.graph(g, pool=self.pool):
                 logits = model.forward(self._batch(bucket, padding=False), cache)
-                K.argmax(logits, out=self.next_ids)
-                self.token_ids.dev.copy_(self.next_ids)
-                self.tok_pos.dev.add_(self.pos_inc.dev)
+                K.argmax_step(logits, self.next_ids, self.token_ids.dev, self.tok_pos.dev, self.pos_inc.dev)
         finally:
             if gc_was_on:
                 gc.enable()

@@ -1139,6 +1139,21 @@ def argmax(logits: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Te
     return out
 
 
+def argmax_step(logits: torch.Tensor, out: torch.Tensor, feed: torch.Tensor, pos: torch.Tensor, inc: torch.Tensor) -> None:
+    """The end of a decode step: ``out`` and ``feed`` (int32 ``[R]``) take each row's argmax and ``pos += inc``."""
+    R, V = logits.shape
+    if logits.dtype != torch.float32 or any(t.dtype != torch.int32 or t.numel() != R for t in (out, feed, pos, inc)):
+        raise KernelLibraryError("argmax_step: logits must be float32 [R, V], out, feed, pos and inc int32 [R]")
+    for t, name in ((logits, "logits"), (out, "out"), (feed, "feed"), (pos, "pos"), (inc, "inc")):
+        _contig(t, name)
+    lib = library()
+    lib.exl3_argmax_step_scratch_bytes.restype = _c_size_t
+    need = int(lib.exl3_argmax_step_scratch_bytes(_c_int(R), _c_int(V)))
+    scratch = torch.empty(need // 4, dtype=torch.float32, device=logits.device)
+    _check(lib.exl3_argmax_step(_ptr(logits), _ptr(out), _ptr(feed), _ptr(pos), _ptr(inc), _c_int(R), _c_int(V),
+                                _ptr(scratch), _c_size_t(need), _stream()), "argmax_step")
+
+
 def sample_filtered_cap() -> int:
     """The most candidates the device sampler ranks (``top_k`` above it is the host sampler's)."""
     return int(library().exl3_sample_filtered_cap())

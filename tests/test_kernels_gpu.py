@@ -1344,3 +1344,15 @@ def test_linear_scan_wide(mode, dv, dtype, counts):
         again = start.clone()
         close(scan(again, 2), want.reshape(T, H * dv), 2e-5, "in two steps")
         close(again[slots.long()], S, 2e-5, "states after two steps")
+
+
+@pytest.mark.parametrize("R,V", [(1, 1), (3, 2048), (8, 2049), (5, 122753)])
+def test_argmax_step(R, V):
+    x = torch.randn(R, V, device=DEV)
+    x[0, V // 2] = x[0, V - 1] = 9.0                     # a tie: the first wins
+    ints = lambda *s: torch.randint(0, 50, s, dtype=torch.int32, device=DEV)  # noqa: E731
+    out, feed, pos, inc = ints(R), ints(R), ints(R), ints(R)
+    want = pos + inc
+    K().argmax_step(x, out, feed, pos, inc)
+    assert out.tolist() == feed.tolist() == K().argmax(x).tolist() and out[0] == V // 2
+    assert torch.equal(pos, want)
