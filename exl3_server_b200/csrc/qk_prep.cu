@@ -220,14 +220,13 @@ __device__ inline void qp_load8<__nv_bfloat16>(const __nv_bfloat16* p, float (&v
 template <typename TX, typename TS>
 __global__ void __launch_bounds__(QP_WARPS * 32) qk_prep_vec_kernel(QkPrepArgs a, int lph) {
   __shared__ float s_sn[QP_TABLE], s_cs[QP_TABLE];
-  pdl_wait();
-  pdl_trigger();
   const int t = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // before the wait: the token's position and page, its sines and cosines (the step's positions and page tables are nobody's
+  // output): a step of few tokens waits 1 us less for it
   const int pos = __ldcg(a.tok_pos + t);
   const int pg = a.nkv > 0 ? __ldcg(a.block_table + (int64_t)__ldcg(a.tok_seq + t) * a.bt_stride + pos / a.page) : -1;
   const int in_page = a.nkv > 0 ? pos % a.page : 0;
-  qp_gates(a, t);
   const int half = a.rot >> 1;
   for (int i = threadIdx.x; i < half; i += blockDim.x) {
     float sn, cs;
@@ -235,6 +234,9 @@ __global__ void __launch_bounds__(QP_WARPS * 32) qk_prep_vec_kernel(QkPrepArgs a
     s_sn[i] = sn * a.mscale;
     s_cs[i] = cs * a.mscale;
   }
+  pdl_wait();
+  pdl_trigger();
+  qp_gates(a, t);
   __syncthreads();
   const int per_warp = 32 / lph;
   const int jobs = a.nh + 2 * a.nkv;
@@ -328,6 +330,50 @@ __global__ void __launch_bounds__(QP_WARPS * 32) qk_prep_vec_kernel(QkPrepArgs a
   }
 }
 
+// What a recurrence takes: queries and keys rotated as whole heads (feature i with i + hd / 2) or not at all, as float32, without
+// norms, values, gates or a cache.  A block a token; a thread has eight features of a head's first half and their eight
+// partners.  Bound by its bytes: 2 x 16 heads of 64 of 3,163 tokens in bfloat16, 39 MB, 11.4 us = 0.52 of
+// the copy rate (the kernel above, a feature a lane: 57).
+template <typename TX>
+__global__ void __launch_bounds__(128) qk_rotate_vec_kernel(QkPrepArgs a) {
+  __shared__ float s_sn[QP_TABLE], s_cs[QP_TABLE];
+  const int t = blockIdx.x, half = a.hd >> 1, per_head = half / 8;
+  const int pos = __ldcg(a.tok_pos + t);              // before the wait: the step's positions are nobody's output
+  for (int i = threadIdx.x; i < half; i += blockDim.x) {
+    float sn = 0.0f, cs = 1.0f;
+    if (a.rot) rope_sincos((float)pos, a.f_hi[i], a.f_lo ? a.f_lo[i] : 0.0f, &sn, &cs);
+    s_sn[i] = a.rot ? sn * a.mscale : 0.0f;
+    s_cs[i] = a.rot ? cs * a.mscale : 1.0f;
+  }
+  pdl_wait();
+  pdl_trigger();
+  __syncthreads();
+  const TX* x = static_cast<const TX*>(a.x) + (int64_t)t * a.ld;
+  const float q_mul = qp_temperature(a, pos);
+  for (int job = threadIdx.x; job < (a.nh + a.nkv) * per_head; job += blockDim.x) {
+    const int head = job / per_head, i = (job - head * per_head) * 8;
+    const bool is_q = head < a.nh;
+    const int h = is_q ? head : head - a.nh;
+    const TX* from = x + (is_q ? a.q_off : a.k_off) + (int64_t)h * a.hd + i;
+    float u[8], v[8], lo[8], hi[8];
+    qp_load8<TX>(from, u);
+    qp_load8<TX>(from + half, v);
+    const float mul = is_q ? q_mul : a.k_mul;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float sn = s_sn[i + e], cs = s_cs[i + e];
+      lo[e] = fmaf(u[e], cs, -v[e] * sn) * mul;
+      hi[e] = fmaf(v[e], cs, u[e] * sn) * mul;
+    }
+    float* to = static_cast<float*>(is_q ? a.q_out : a.k_out) + ((int64_t)t * (is_q ? a.nh : a.nkv) + h) * a.hd + i;
+#pragma unroll
+    for (int e = 0; e < 8; e += 4) {
+      *reinterpret_cast<float4*>(to + e) = make_float4(lo[e], lo[e + 1], lo[e + 2], lo[e + 3]);
+      *reinterpret_cast<float4*>(to + half + e) = make_float4(hi[e], hi[e + 1], hi[e + 2], hi[e + 3]);
+    }
+  }
+}
+
 }  // namespace exl3
 
 using namespace exl3;
@@ -384,6 +430,14 @@ extern "C" int exl3_qk_prep(const void* x, int x_dtype, int64_t ld, int q_off, i
     else if (xf) launch_pdl(qk_prep_vec_kernel<float, __nv_bfloat16>, grid, threads, 0, stream, a, lph);
     else if (sf) launch_pdl(qk_prep_vec_kernel<__nv_bfloat16, float>, grid, threads, 0, stream, a, lph);
     else launch_pdl(qk_prep_vec_kernel<__nv_bfloat16, __nv_bfloat16>, grid, threads, 0, stream, a, lph);
+    return launch_status("qk_prep");
+  }
+  if (v_off < 0 && k_pool == nullptr && gate_out == nullptr && norm == 0 && (rot == 0 || (layout == 0 && rot == hd)) &&
+      hd == hd_pad && hd % 16 == 0 && hd / 2 <= QP_TABLE && q_out_dtype == DT_F32 && (nkv == 0 || k_out_dtype == DT_F32) &&
+      ld % 8 == 0 && q_off % 8 == 0 && (nkv == 0 || k_off % 8 == 0) && (x_dtype == DT_BF16 || x_dtype == DT_F32) &&
+      aligned16(x) && aligned16(q_out) && (nkv == 0 || aligned16(k_out))) {
+    if (x_dtype == DT_F32) launch_pdl(qk_rotate_vec_kernel<float>, dim3(T), dim3(128), 0, stream, a);
+    else launch_pdl(qk_rotate_vec_kernel<__nv_bfloat16>, dim3(T), dim3(128), 0, stream, a);
     return launch_status("qk_prep");
   }
   const size_t smem = (size_t)QP_WARPS * (hd > a.hdv ? hd : a.hdv) * sizeof(float);

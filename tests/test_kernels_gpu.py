@@ -1356,3 +1356,29 @@ def test_argmax_step(R, V):
     K().argmax_step(x, out, feed, pos, inc)
     assert out.tolist() == feed.tolist() == K().argmax(x).tolist() and out[0] == V // 2
     assert torch.equal(pos, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,nh,nkv,hd,rot,temp", [(1, 1, 1, 16, 16, 0.0), (7, 5, 3, 64, 64, 0.0), (3, 2, 2, 128, 0, 0.0),
+                                                  (150, 16, 16, 64, 64, 40.0)])
+def test_qk_prep_rotated_heads_for_a_recurrence(dtype, T, nh, nkv, hd, rot, temp):
+    """Whole heads rotated half by half into float32 (the kernel with 16-byte accesses): the sums are two products, and the
+    angles are right to a few 1e-9 of themselves."""
+    g = torch.Generator(device=DEV).manual_seed(T)
+    x = torch.randn(T, (nh + nkv) * hd + 24, device=DEV, generator=g).to(dtype)
+    pos = torch.randint(0, 3000, (T,), dtype=torch.int32, device=DEV, generator=g)
+    freqs = [10000.0 ** (-2.0 * i / hd) for i in range(hd // 2)]
+    table = K().rotary_table(torch.tensor(freqs, dtype=torch.float64)).to(DEV) if rot else None
+    q, k = K().qk_prep(x, 8, 8 + nh * hd, -1, nh, nkv, hd, 0, hd, 0, 0, None, None, 1e-6, rot, 0, table, 1.25, 0.5, None, pos,
+                       torch.zeros_like(pos), None, 0, torch.float32, None, None, k_dtype=torch.float32,
+                       temperature=(0.1, temp) if temp else None)
+    a = pos.double().cpu()[:, None] * torch.tensor(freqs, dtype=torch.float64)
+    c, s = (a.cos() * 1.25)[:, None], (a.sin() * 1.25)[:, None]
+    for got, off, n, mul in ((q, 8, nh, 1.0), (k, 8 + nh * hd, nkv, 0.5)):
+        want = x[:, off:off + n * hd].double().cpu().view(T, n, hd)
+        if rot:
+            u, v = want[..., :hd // 2], want[..., hd // 2:]
+            want = torch.cat([u * c - v * s, v * c + u * s], dim=-1)
+        if temp and off == 8:
+            mul = (1.0 + 0.1 * torch.log(torch.floor((pos.double().cpu() + 1) / temp) + 1.0))[:, None, None]
+        close(got.view(T, n, hd), want * mul, 1e-6, "rotated")
