@@ -106,6 +106,100 @@ latent_prep_kernel(const void* a, int a_dtype, int lda, int q_off, int q_rank, c
   }
 }
 
+// The same for few tokens, whose chain of trips to memory is what they cost: the latents are read once, kept in registers
+// (what is beyond LP_KEEP values a thread is read again) and their sums of squares taken together, and the token's place in the
+// cache is looked up before the wait (the step's positions and page tables are nobody's output).  2 tokens of 768 + 576: 8.0
+// us, the kernel above 14.9; 2,000 tokens 20.7 and 14.9 (fewer blocks an SM): so up to LP_MOST tokens, four blocks an SM.
+constexpr int LP_THREADS = 256, LP_KEEP = 4, LP_MOST = 592;
+
+__global__ void __launch_bounds__(LP_THREADS)
+latent_prep_once_kernel(const void* a, int a_dtype, int lda, int q_off, int q_rank, const void* __restrict__ wq, int wq_dtype,
+                   int kv_off, int kv_rank, int rot_dim, const void* __restrict__ wkv, int wkv_dtype, int g_off, int heads,
+                   float eps, const float* __restrict__ inv_freq, const float* __restrict__ inv_freq_lo, int rot, int layout,
+                   float mscale, const int* __restrict__ tok_pos, const int* __restrict__ tok_seq, const int* __restrict__ block_table,
+                   int bt_stride, int page, void* pool, int pool_dtype, int kv_row, int rank_pad, void* cq, int cq_dtype,
+                   float* gate) {
+  __shared__ float red[2][LP_THREADS / 32];
+  const int t = blockIdx.x, tid = threadIdx.x;
+  const int64_t row = (int64_t)t * lda;
+  int pos = 0, pg = -1;
+  if (pool != nullptr) {                            // null: a layer that reads another layer's rows
+    pos = __ldcg(tok_pos + t);
+    pg = __ldcg(block_table + (int64_t)__ldcg(tok_seq + t) * bt_stride + pos / page);
+  }
+  pdl_wait();
+  pdl_trigger();
+  const int kv_n = pool != nullptr ? kv_rank : 0;
+  float q[LP_KEEP], kv[LP_KEEP], sq = 0.0f, skv = 0.0f;
+#pragma unroll
+  for (int e = 0; e < LP_KEEP; ++e) {
+    const int i = tid + e * LP_THREADS;
+    q[e] = i < q_rank ? lt_load(a, a_dtype, row + q_off + i) : 0.0f;
+    kv[e] = i < kv_n ? lt_load(a, a_dtype, row + kv_off + i) : 0.0f;
+  }
+#pragma unroll
+  for (int e = 0; e < LP_KEEP; ++e) {
+    sq = fmaf(q[e], q[e], sq);
+    skv = fmaf(kv[e], kv[e], skv);
+  }
+  for (int i = tid + LP_KEEP * LP_THREADS; i < q_rank; i += LP_THREADS) {
+    const float v = lt_load(a, a_dtype, row + q_off + i);
+    sq = fmaf(v, v, sq);
+  }
+  for (int i = tid + LP_KEEP * LP_THREADS; i < kv_n; i += LP_THREADS) {
+    const float v = lt_load(a, a_dtype, row + kv_off + i);
+    skv = fmaf(v, v, skv);
+  }
+  // the gates
+  for (int i = tid; i < heads; i += LP_THREADS)
+    gate[(int64_t)t * heads + i] = 1.0f / (1.0f + expf(-lt_load(a, a_dtype, row + g_off + i)));
+  sq = warp_sum(sq);
+  skv = warp_sum(skv);
+  if ((tid & 31) == 0) {
+    red[0][tid >> 5] = sq;
+    red[1][tid >> 5] = skv;
+  }
+  __syncthreads();
+  sq = skv = 0.0f;
+#pragma unroll
+  for (int w = 0; w < LP_THREADS / 32; ++w) {
+    sq += red[0][w];
+    skv += red[1][w];
+  }
+  // the query latent
+  float inv = 1.0f / sqrtf(sq / (float)q_rank + eps);
+#pragma unroll
+  for (int e = 0; e < LP_KEEP; ++e) {
+    const int i = tid + e * LP_THREADS;
+    if (i < q_rank) lt_store(cq, cq_dtype, (int64_t)t * q_rank + i, q[e] * inv * lt_load_w(wq, wq_dtype, i));
+  }
+  for (int i = tid + LP_KEEP * LP_THREADS; i < q_rank; i += LP_THREADS)
+    lt_store(cq, cq_dtype, (int64_t)t * q_rank + i, lt_load(a, a_dtype, row + q_off + i) * inv * lt_load_w(wq, wq_dtype, i));
+  // the key/value latent and the shared rotated key part, into the token's row of the cache
+  if (pg < 0) return;
+  inv = 1.0f / sqrtf(skv / (float)kv_rank + eps);
+  const int64_t dst = ((int64_t)pg * page + pos % page) * kv_row;
+#pragma unroll
+  for (int e = 0; e < LP_KEEP; ++e) {
+    const int i = tid + e * LP_THREADS;
+    if (i < rank_pad) lt_store(pool, pool_dtype, dst + i, i < kv_rank ? kv[e] * inv * lt_load_w(wkv, wkv_dtype, i) : 0.0f);
+  }
+  for (int i = tid + LP_KEEP * LP_THREADS; i < rank_pad; i += LP_THREADS)
+    lt_store(pool, pool_dtype, dst + i,
+             i < kv_rank ? lt_load(a, a_dtype, row + kv_off + i) * inv * lt_load_w(wkv, wkv_dtype, i) : 0.0f);
+  const int64_t src = row + kv_off + kv_rank;
+  for (int i = threadIdx.x; i < kv_row - rank_pad; i += blockDim.x) {
+    float v = 0.0f;
+    if (i < rot) {
+      v = lt_rotated(i, rot, layout, (float)pos, inv_freq, inv_freq_lo, mscale,
+                     [&](int j) { return lt_load(a, a_dtype, src + j); });
+    } else if (i < rot_dim) {
+      v = lt_load(a, a_dtype, src + i);
+    }
+    lt_store(pool, pool_dtype, dst + rank_pad + i, v);
+  }
+}
+
 // A value that an earlier kernel of the step wrote: through L2 (see load_vec_cg in common.cuh).
 __device__ inline float lt_act(const float* p) { return __ldcg(p); }
 __device__ inline float lt_act(const __nv_bfloat16* p) { return __bfloat162float(__ldcg(p)); }
@@ -251,8 +345,8 @@ extern "C" int exl3_latent_prep(const void* a, int a_dtype, int lda, int T, int 
               kv_rank, rot_dim, rot, heads, kv_row, rank_pad);
     return ERR_BAD_ARGUMENT;
   }
-  launch_pdl(latent_prep_kernel, dim3(T), dim3(128), 0, stream, a, a_dtype, lda, q_off, q_rank, wq, wq_dtype, kv_off,
-             kv_rank, rot_dim, wkv, wkv_dtype, g_off, heads, eps, inv_freq, inv_freq_lo, rot, layout, mscale, tok_pos, tok_seq, block_table,
+  launch_pdl(T <= LP_MOST ? latent_prep_once_kernel : latent_prep_kernel, dim3(T), dim3(T <= LP_MOST ? LP_THREADS : 128), 0,
+             stream, a, a_dtype, lda, q_off, q_rank, wq, wq_dtype, kv_off, kv_rank, rot_dim, wkv, wkv_dtype, g_off, heads, eps, inv_freq, inv_freq_lo, rot, layout, mscale, tok_pos, tok_seq, block_table,
              bt_stride, page, pool, pool_dtype, kv_row, rank_pad, cq, cq_dtype, gate);
   return launch_status("latent_prep");
 }
