@@ -54,6 +54,7 @@ struct SfRow {            // one row's options, as the host gives them (float64 
 constexpr double SF_FIXED_US = 36.0, SF_STAGED_US = 0.00030, SF_AGAIN_US = 0.00065;
 constexpr int SF_BINS = 2048;
 constexpr int SF_HEAD_BYTES = (2 * SF_BINS * 4) + 2 * (SF_CAP * 8);     // histograms, candidates, this block's own
+constexpr int SF_SMEM_MOST = 200 * 1024;                                // with the staged part of a row
 
 __device__ inline uint32_t sf_remote(const void* mine, uint32_t rank) {
   uint32_t addr;
@@ -364,7 +365,7 @@ extern "C" int exl3_sample_rows(const float* logits, const double* rows, int* co
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  constexpr size_t MOST = 200 * 1024 - SF_HEAD_BYTES;
+  constexpr size_t MOST = SF_SMEM_MOST - SF_HEAD_BYTES;
   int blocks = 8;
   double best = 0.0;
   for (int b = 8; b >= 1; b /= 2) {
@@ -381,9 +382,12 @@ extern "C" int exl3_sample_rows(const float* logits, const double* rows, int* co
   const bool staged = part <= MOST;
   auto kernel = staged ? sample_filtered_kernel<true> : sample_filtered_kernel<false>;
   const size_t smem = SF_HEAD_BYTES + (staged ? part : 0);
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // The limit belongs to the function and not to this call: the same number from every thread, whatever its rows take, or a
+  // thread with shorter rows would lower it between another one's setting it and its launch.
+  const int limit = staged ? SF_SMEM_MOST : SF_HEAD_BYTES;
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
   if (e != cudaSuccess) {
-    set_error("sample_filtered: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
+    set_error("sample_filtered: %d bytes of shared memory refused: %s", limit, cudaGetErrorString(e));
     return (int)e;
   }
   if ((long long)R * blocks > 0x7fffffffll) { set_error("sample_filtered: %d rows are too many", R); return ERR_UNSUPPORTED; }

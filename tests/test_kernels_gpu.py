@@ -3,6 +3,7 @@ the same operation, at sizes other than the engine tests use (widths and
 vocabularies that are no power of two, head sizes in steps of 16, grouped
 heads, windows, ragged batches)."""
 import math
+import threading
 
 import numpy as np
 import pytest
@@ -1285,6 +1286,29 @@ def test_sample_rows_applies_and_counts(V, R):
         if r % 4 != 1:
             before[r][int(want[r])] += 1
         assert torch.equal(counts[r], before[r])
+
+
+def test_sampling_in_threads_with_rows_of_other_lengths():
+    """A row's length decides how much shared memory its launch takes: two threads with different lengths must not change
+    what the other one's launch may take."""
+    failed = []
+
+    def sample(V):
+        try:
+            logits = torch.randn(2, V, device=DEV)
+            rows = torch.tensor([[0.0, 0, 1.0, 0.0, 0.0]] * 2, dtype=torch.float64, device=DEV)
+            for _ in range(1500):
+                got = K().sample_filtered(logits, rows)
+            assert got.tolist() == logits.argmax(-1).tolist()
+        except Exception as e:  # noqa: BLE001
+            failed.append(e)
+
+    threads = [threading.Thread(target=sample, args=(V,)) for V in (2049, 122753)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
 
 
 # The recurrence's wide kernel (keys of 64, values in sixteens): around its stages of sixteen tokens, rows walked whole and
