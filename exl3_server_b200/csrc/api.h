@@ -304,7 +304,7 @@ size_t exl3_argmax_step_scratch_bytes(int R, int V);
 // greedy), top_k (0: off; at most exl3_sample_filtered_cap()), top_p, min_p, uniform number in [0, 1).
 int exl3_sample_filtered(const float* logits, const double* rows, int* out, int R, int V, cudaStream_t stream);
 // The same with penalties (counts and params as exl3_sample_penalties takes them) applied as the logits are read, which
-// stay as they are, and the chosen tokens counted.
+// stay as they are, and the chosen tokens counted once every row has been drawn (rows may share their counts).
 int exl3_sample_rows(const float* logits, const double* rows, int* const* counts, const float* params, int* out, int R,
                      int V, cudaStream_t stream);
 int exl3_sample_filtered_cap();

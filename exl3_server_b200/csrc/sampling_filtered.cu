@@ -76,12 +76,13 @@ __device__ inline float sf_penalised(float x, int count, float rep, float presen
   return x;
 }
 
-// counts: null, or per row a pointer to its token counts [V] (null: the row has no penalties), which the chosen token
-// joins; params [R, 3]: repetition, presence, frequency.  STAGED: the block's part of the row is kept in shared memory;
+// counts: null, or per row a pointer to its token counts [V] (null: the row has no penalties); params [R, 3]: repetition,
+// presence, frequency.  The counts are only read: rows may share them, so the chosen tokens join them in a kernel of their
+// own, after every row has been drawn (2 us for 32 rows).  STAGED: the block's part of the row is kept in shared memory;
 // else (vocabularies too long for that) every pass reads it again.
 template <bool STAGED>
 __global__ void __launch_bounds__(SF_THREADS)
-sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict__ rows, int* const* __restrict__ counts,
+sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict__ rows, const int* const* __restrict__ counts,
                        const float* __restrict__ params, int* __restrict__ out, int V, int blocks) {
   extern __shared__ __align__(16) unsigned char sf_smem[];
   unsigned* hists = reinterpret_cast<unsigned*>(sf_smem);                                      // [2][SF_BINS]
@@ -99,7 +100,7 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
   const float* row = logits + (int64_t)row_id * V;
   const SfRow o = rows[row_id];
   const int M = V < SF_CAP ? V : SF_CAP;
-  int* count = counts ? counts[row_id] : nullptr;
+  const int* count = counts ? counts[row_id] : nullptr;
   float rep = 1.0f, presence = 0.0f, frequency = 0.0f;
   if (count) {
     rep = params[3 * row_id];
@@ -250,13 +251,8 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
     __syncthreads();
   }
   auto token_of = [&](int i) { return (int)(~(unsigned)(cand[i] & 0xffffffffull)); };
-  auto choose = [&](int i) {
-    const int t = token_of(i);
-    out[row_id] = t;
-    if (count) count[t] += 1;                     // the chosen token joins its row's context
-  };
   if (!(o.temperature > 0.0)) {                  // greedy: the first maximum
-    if (tid == 0) choose(0);
+    if (tid == 0) out[row_id] = token_of(0);
     return;
   }
 
@@ -296,7 +292,7 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
   __syncthreads();
   const double total = acc[M - 1];
   if (!(total > 0.0)) {
-    if (tid == 0) choose(0);
+    if (tid == 0) out[row_id] = token_of(0);
     return;
   }
   int keep = M;
@@ -319,7 +315,7 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
   for (int i = tid; i < keep; i += SF_THREADS)
     if (acc[i] >= r) atomicMin(&first_draw, i);
   __syncthreads();
-  if (tid == 0) choose(first_draw < keep ? first_draw : keep - 1);
+  if (tid == 0) out[row_id] = token_of(first_draw < keep ? first_draw : keep - 1);
 }
 
 // Penalties over a row's context (src/model.cpp:672-686).  counts[r] points to the row's token counts [V]
@@ -337,12 +333,12 @@ __global__ void sample_penalties_kernel(float* __restrict__ logits, int V, const
   *x = sf_penalised(*x, count, params[3 * row], params[3 * row + 1], params[3 * row + 2]);
 }
 
-// The chosen tokens join their rows' contexts.
+// The chosen tokens join their rows' contexts (rows that share their counts may have chosen the same token).
 __global__ void sample_count_kernel(int* const* __restrict__ counts, const int* __restrict__ ids, int R, int V) {
   const int row = blockIdx.x * blockDim.x + threadIdx.x;
   if (row >= R || counts[row] == nullptr) return;
   const int t = ids[row];
-  if (t >= 0 && t < V) counts[row][t] += 1;
+  if (t >= 0 && t < V) atomicAdd(counts[row] + t, 1);
 }
 
 }  // namespace exl3
@@ -351,7 +347,7 @@ using namespace exl3;
 
 // rows: float64 [R, 5] on the device: temperature (<= 0: greedy), top_k (0: off, at most 2048), top_p, min_p and
 // the row's uniform number in [0, 1).  out: int32 [R].  counts (may be null): as in exl3_sample_penalties, with params;
-// the penalties are applied as the logits are read, and the chosen tokens are counted.
+// the penalties are applied as the logits are read, and the chosen tokens are counted when all rows have been drawn.
 extern "C" int exl3_sample_rows(const float* logits, const double* rows, int* const* counts, const float* params, int* out,
                                 int R, int V, cudaStream_t stream) {
   if (R == 0) return 0;
@@ -403,8 +399,11 @@ extern "C" int exl3_sample_rows(const float* logits, const double* rows, int* co
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kernel, logits, reinterpret_cast<const SfRow*>(rows), counts, params, out, V, blocks);
-  return launch_status("sample_filtered");
+  cudaLaunchKernelEx(&cfg, kernel, logits, reinterpret_cast<const SfRow*>(rows), (const int* const*)counts, params, out, V,
+                     blocks);
+  int rc = launch_status("sample_filtered");
+  if (rc || counts == nullptr) return rc;
+  return exl3_sample_count(counts, out, R, V, stream);
 }
 
 extern "C" int exl3_sample_filtered(const float* logits, const double* rows, int* out, int R, int V,

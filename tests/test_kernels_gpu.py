@@ -1288,6 +1288,23 @@ def test_sample_rows_applies_and_counts(V, R):
         assert torch.equal(counts[r], before[r])
 
 
+@pytest.mark.parametrize("V", [300, 40001])
+def test_rows_that_share_a_sampler(V):
+    """One request's sampler for all rows, more rows than run at once: every row sees the context as it was before the
+    step, and all the tokens join it, as on the host."""
+    from exl3_server_b200.sampling import SampleOptions
+    from exl3_server_b200.sampling.sampler import RowSampler, sample_rows
+    R = 200
+    logits = 0.3 * torch.randn(1, V, device=DEV, generator=torch.Generator(device=DEV).manual_seed(V)).repeat(R, 1)
+    logits[:, 17] = 4.0                                   # chosen by many rows
+    opt = SampleOptions(temperature=0.7, top_k=40, repetition_penalty=1.1, presence_penalty=0.2, frequency_penalty=0.01)
+    device, host = RowSampler(opt, 3, [17, 4, 4, 250]), RowSampler(opt, 3, [17, 4, 4, 250])
+    for _ in range(3):
+        assert sample_rows(logits, [device] * R) == sample_rows(logits.cpu(), [host] * R)
+        want = torch.bincount(torch.tensor(device.context), minlength=V)
+        assert len(device.context) == device._counted and torch.equal(device.device_counts(V, DEV).long().cpu(), want)
+
+
 def test_sampling_in_threads_with_rows_of_other_lengths():
     """A row's length decides how much shared memory its launch takes: two threads with different lengths must not change
     what the other one's launch may take."""
