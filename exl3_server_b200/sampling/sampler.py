@@ -62,6 +62,10 @@ def launch_on_device(logits: torch.Tensor, rows: Sequence[RowSampler]) -> torch.
     has read them (``record``).  The penalties' token counts are kept up on the device."""
     from ..engine.decode import TRANSFERRED
     from ..ops import kernels as K
+    if not logits.is_contiguous():
+        if any(r.opt.has_penalties for r in rows):
+            logits = logits.clone()                      # a slice of padded rows, or one row for all, becomes dense
+        K._contig(logits, "logits")                      # before any generator has moved on
     R, V = logits.shape
     opts, counts, params, penalised = [], [], [], []     # one pass over the rows: their options are read once each
     for r in rows:

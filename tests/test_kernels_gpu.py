@@ -1288,6 +1288,24 @@ def test_sample_rows_applies_and_counts(V, R):
         assert torch.equal(counts[r], before[r])
 
 
+def test_penalised_sampling_takes_rows_that_are_not_dense():
+    """Columns of a padded vocabulary, every other row, one row for all: with penalties these become dense first.  What is
+    dense in another order is refused, before a generator has moved on."""
+    from exl3_server_b200.sampling import SampleOptions
+    from exl3_server_b200.sampling.sampler import RowSampler, sample_rows
+    V, R = 3001, 4
+    padded = 2.0 * torch.randn(2 * R, V + 7, device=DEV, generator=torch.Generator(device=DEV).manual_seed(5))
+    opt = SampleOptions(temperature=0.8, top_k=50, repetition_penalty=1.2, frequency_penalty=0.1)
+    new = lambda: [RowSampler(opt, r, [r, 5, 5, 9]) for r in range(R)]  # noqa: E731
+    for logits in (padded[:R, :V], padded[::2, 3:3 + V], padded[:1, :V].expand(R, V)):
+        assert sample_rows(logits, new()) == sample_rows(logits.cpu(), new())
+    rows = new()
+    before = [r.rng.state for r in rows]
+    with pytest.raises(Exception, match="contiguous"):
+        sample_rows(padded[:R].T.contiguous().T, rows)
+    assert [r.rng.state for r in rows] == before
+
+
 @pytest.mark.parametrize("V", [300, 40001])
 def test_rows_that_share_a_sampler(V):
     """One request's sampler for all rows, more rows than run at once: every row sees the context as it was before the
