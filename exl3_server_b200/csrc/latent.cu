@@ -107,10 +107,15 @@ latent_prep_kernel(const void* a, int a_dtype, int lda, int q_off, int q_rank, c
 }
 
 // The same for few tokens, whose chain of trips to memory is what they cost: the latents are read once, kept in registers
-// (what is beyond LP_KEEP values a thread is read again) and their sums of squares taken together, and the token's place in the
-// cache is looked up before the wait (the step's positions and page tables are nobody's output).  2 tokens of 768 + 576: 8.0
-// us, the kernel above 14.9; 2,000 tokens 20.7 and 14.9 (fewer blocks an SM): so up to LP_MOST tokens, four blocks an SM.
-constexpr int LP_THREADS = 256, LP_KEEP = 4, LP_MOST = 592;
+// (what is beyond LP_KEEP values a thread is read again) and both sums of squares taken at once, and the token's place in the
+// cache is looked up before the wait (the step's positions and page tables are nobody's output).  The sums run in the order of the
+// kernel above (LP_SUM chains, block_sum's tree), the queries' in the first half of the threads and the keys' in the other,
+// so a token's bits do not depend on how many tokens its step has.
+// Latents of 768 + 512 in bfloat16, this kernel / the one above, back to back: 2 tokens 4.4 / 6.8 us, 592 tokens 5.9 / 7.2, 2,000
+// tokens 13.3 / 11.7 (fewer blocks an SM); 64 + 64: 2 tokens 3.5 / 3.6, 300 tokens 3.8 / 3.9, 592 tokens 4.8 / 4.1.  So it takes
+// steps of up to LP_FEW tokens (two blocks an SM) whatever the ranks, and of up to LP_MOST with LP_WIDE features or more.
+constexpr int LP_SUM = 128, LP_THREADS = 2 * LP_SUM, LP_KEEP = 4, LP_KEPT = LP_KEEP * LP_THREADS;
+constexpr int LP_FEW = 296, LP_MOST = 592, LP_WIDE = 1024;
 
 __global__ void __launch_bounds__(LP_THREADS)
 latent_prep_once_kernel(const void* a, int a_dtype, int lda, int q_off, int q_rank, const void* __restrict__ wq, int wq_dtype,
@@ -119,8 +124,8 @@ latent_prep_once_kernel(const void* a, int a_dtype, int lda, int q_off, int q_ra
                    float mscale, const int* __restrict__ tok_pos, const int* __restrict__ tok_seq, const int* __restrict__ block_table,
                    int bt_stride, int page, void* pool, int pool_dtype, int kv_row, int rank_pad, void* cq, int cq_dtype,
                    float* gate) {
-  __shared__ float red[2][LP_THREADS / 32];
-  const int t = blockIdx.x, tid = threadIdx.x;
+  __shared__ float kept[2][LP_KEPT], red[2][LP_SUM / 32];
+  const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
   const int64_t row = (int64_t)t * lda;
   int pos = 0, pg = -1;
   if (pool != nullptr) {                            // null: a layer that reads another layer's rows
@@ -130,7 +135,7 @@ latent_prep_once_kernel(const void* a, int a_dtype, int lda, int q_off, int q_ra
   pdl_wait();
   pdl_trigger();
   const int kv_n = pool != nullptr ? kv_rank : 0;
-  float q[LP_KEEP], kv[LP_KEEP], sq = 0.0f, skv = 0.0f;
+  float q[LP_KEEP], kv[LP_KEEP];
 #pragma unroll
   for (int e = 0; e < LP_KEEP; ++e) {
     const int i = tid + e * LP_THREADS;
@@ -139,33 +144,26 @@ latent_prep_once_kernel(const void* a, int a_dtype, int lda, int q_off, int q_ra
   }
 #pragma unroll
   for (int e = 0; e < LP_KEEP; ++e) {
-    sq = fmaf(q[e], q[e], sq);
-    skv = fmaf(kv[e], kv[e], skv);
-  }
-  for (int i = tid + LP_KEEP * LP_THREADS; i < q_rank; i += LP_THREADS) {
-    const float v = lt_load(a, a_dtype, row + q_off + i);
-    sq = fmaf(v, v, sq);
-  }
-  for (int i = tid + LP_KEEP * LP_THREADS; i < kv_n; i += LP_THREADS) {
-    const float v = lt_load(a, a_dtype, row + kv_off + i);
-    skv = fmaf(v, v, skv);
+    kept[0][tid + e * LP_THREADS] = q[e];
+    kept[1][tid + e * LP_THREADS] = kv[e];
   }
   // the gates
   for (int i = tid; i < heads; i += LP_THREADS)
     gate[(int64_t)t * heads + i] = 1.0f / (1.0f + expf(-lt_load(a, a_dtype, row + g_off + i)));
-  sq = warp_sum(sq);
-  skv = warp_sum(skv);
-  if ((tid & 31) == 0) {
-    red[0][tid >> 5] = sq;
-    red[1][tid >> 5] = skv;
-  }
   __syncthreads();
-  sq = skv = 0.0f;
+  const int which = tid / LP_SUM, chain = tid % LP_SUM;
+  float sum = 0.0f;
 #pragma unroll
-  for (int w = 0; w < LP_THREADS / 32; ++w) {
-    sq += red[0][w];
-    skv += red[1][w];
+  for (int i = 0; i < LP_KEPT; i += LP_SUM) sum = fmaf(kept[which][i + chain], kept[which][i + chain], sum);
+  for (int i = LP_KEPT + chain; i < (which ? kv_n : q_rank); i += LP_SUM) {
+    const float v = lt_load(a, a_dtype, row + (which ? kv_off : q_off) + i);
+    sum = fmaf(v, v, sum);
   }
+  sum = warp_sum(sum);
+  if (lane == 0) red[which][chain >> 5] = sum;
+  __syncthreads();
+  const float sq = warp_sum(lane < LP_SUM / 32 ? red[0][lane] : 0.0f);
+  const float skv = warp_sum(lane < LP_SUM / 32 ? red[1][lane] : 0.0f);
   // the query latent
   float inv = 1.0f / sqrtf(sq / (float)q_rank + eps);
 #pragma unroll
@@ -345,8 +343,9 @@ extern "C" int exl3_latent_prep(const void* a, int a_dtype, int lda, int T, int 
               kv_rank, rot_dim, rot, heads, kv_row, rank_pad);
     return ERR_BAD_ARGUMENT;
   }
-  launch_pdl(T <= LP_MOST ? latent_prep_once_kernel : latent_prep_kernel, dim3(T), dim3(T <= LP_MOST ? LP_THREADS : 128), 0,
-             stream, a, a_dtype, lda, q_off, q_rank, wq, wq_dtype, kv_off, kv_rank, rot_dim, wkv, wkv_dtype, g_off, heads, eps, inv_freq, inv_freq_lo, rot, layout, mscale, tok_pos, tok_seq, block_table,
+  const bool once = T <= LP_FEW || (T <= LP_MOST && q_rank + kv_rank >= LP_WIDE);
+  launch_pdl(once ? latent_prep_once_kernel : latent_prep_kernel, dim3(T), dim3(once ? LP_THREADS : LP_SUM), 0, stream,
+             a, a_dtype, lda, q_off, q_rank, wq, wq_dtype, kv_off, kv_rank, rot_dim, wkv, wkv_dtype, g_off, heads, eps, inv_freq, inv_freq_lo, rot, layout, mscale, tok_pos, tok_seq, block_table,
              bt_stride, page, pool, pool_dtype, kv_row, rank_pad, cq, cq_dtype, gate);
   return launch_status("latent_prep");
 }

@@ -1346,6 +1346,42 @@ def test_sampling_in_threads_with_rows_of_other_lengths():
     assert not failed, failed
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("q_rank,kv_rank", [(20, 36), (768, 512), (1024, 1025), (1300, 1100)])
+def test_latent_prep_in_steps_of_any_size(dtype, q_rank, kv_rank):
+    """Both kernels of the latent preparation (steps of few tokens, which keep 1,024 features in registers and read the rest
+    again, and of many) against float64, and bit by bit against one another: a token's latents do not depend on how many
+    tokens its step has."""
+    rot, H, page, T = 8, 3, 64, 700
+    g = torch.Generator(device=DEV).manual_seed(q_rank)
+    a = torch.randn(T, q_rank + kv_rank + rot + H, device=DEV, generator=g).to(dtype)
+    wq, wkv = (torch.randn(n, device=DEV, generator=g) for n in (q_rank, kv_rank))
+    freqs = torch.tensor([700.0 ** (-2.0 * i / rot) for i in range(rot // 2)], dtype=torch.float64)
+    table = K().rotary_table(freqs).to(DEV)
+    pages = torch.randperm(T // page + 1, device=DEV, generator=g).to(torch.int32).view(1, -1)
+    pos, seq = torch.arange(T, dtype=torch.int32, device=DEV), torch.zeros(T, dtype=torch.int32, device=DEV)
+
+    def prep(n):
+        pool = torch.full((pages.numel(), 1, page, kv_rank + rot), 9.0, device=DEV, dtype=dtype)
+        cq, gate = K().latent_prep(a[:n].contiguous(), 0, q_rank, wq, q_rank, kv_rank, rot, wkv, q_rank + kv_rank + rot, H, 1e-6,
+                                   table, rot, pos[:n], seq[:n], pages, page, pool, kv_rank + rot, kv_rank, dtype)
+        return cq, gate, pool[pages[0].long()].view(-1, kv_rank + rot)[:n]
+
+    cq, gate, rows = prep(T)
+    for n in (1, 296, 297, 592, 593):
+        for got, want in zip(prep(n), (cq, gate, rows)):
+            assert torch.equal(got, want[:n])
+    a64 = a.double().cpu()
+    rms = lambda v, w: v / torch.sqrt((v * v).mean(-1, keepdim=True) + 1e-6) * w.double().cpu()  # noqa: E731
+    ang = torch.arange(T, dtype=torch.float64)[:, None] * freqs
+    u, v = a64[:, q_rank + kv_rank:][:, :rot].chunk(2, dim=-1)
+    tail = torch.cat([u * ang.cos() - v * ang.sin(), v * ang.cos() + u * ang.sin()], dim=-1)
+    tol = 1e-6 if dtype == torch.float32 else 4e-3       # half a unit of bfloat16's eight bits, of the largest
+    close(cq, rms(a64[:, :q_rank], wq), tol, "queries")
+    close(rows, torch.cat([rms(a64[:, q_rank:q_rank + kv_rank], wkv), tail], dim=-1), tol, "rows")
+    close(gate, torch.sigmoid(a64[:, -H:]), 1e-6, "gates")
+
+
 # The recurrence's wide kernel (keys of 64, values in sixteens): around its stages of sixteen tokens, rows walked whole and
 # in chunks (a long row with few heads), cut into two steps, in both types.  Everything but the inputs' type is float32: the
 # inputs are rounded first, and the chains of some hundred sums stay within 2e-5 of the largest output.
