@@ -121,7 +121,7 @@ token_shift_vec_kernel(const TH* h, const float* __restrict__ mu, int n_mix, flo
 // ---- the scan ------------------------------------------------------------------------------------------------------
 
 constexpr int LS_STAGE = 8;                      // tokens staged in shared memory at a time
-constexpr int LS_CHUNK = 64;                     // tokens of a chunk when a row's tokens run side by side: this or a multiple
+constexpr int LS_CHUNK = 64;                     // tokens of a chunk when a row's tokens run side by side
 
 struct ScanArgs {
   const void* r; int64_t r_ld; const void* k; int64_t k_ld; int rk_dtype;
@@ -131,12 +131,12 @@ struct ScanArgs {
   const float* decay;
   float* state; const int* slot_ids; const int* row_start;
   float* out; float* ab; float* snap;
-  int heads, dk, dv, places, chunk;              // chunk: tokens of a chunk
+  int heads, dk, dv, places, chunk;              // chunk: tokens of a chunk, LS_CHUNK or (the wide kernel) a multiple
   int act;                                       // see ls_in
 };
 
 // Chunk j of batch row b has a place of its own among floor(T / chunk) + B + 1 places.
-__device__ inline int ls_place(const ScanArgs& a, int t0, int b, int j) { return t0 / a.chunk + b + j; }
+__device__ inline int ls_place(int chunk, int t0, int b, int j) { return t0 / chunk + b + j; }
 
 // phase 0: a row's tokens of the step, from its state, state written back.
 // phase 1: a chunk from zero, (A, B) to scratch (no output; the row's last chunk does nothing).
@@ -157,12 +157,12 @@ __global__ void linear_scan_kernel(ScanArgs a, int phase) {
   const int t0 = __ldcg(a.row_start + b), t1 = __ldcg(a.row_start + b + 1);
   int lo = t0, hi = t1;
   if (phase == 1) {
-    lo = t0 + c * a.chunk;
-    hi = lo + a.chunk;
+    lo = t0 + c * LS_CHUNK;
+    hi = lo + LS_CHUNK;
     if (hi >= t1) return;                        // the row's last chunk has nobody after it
   } else if (phase == 2) {
-    lo = t0 + c * a.chunk;
-    hi = min(lo + a.chunk, t1);
+    lo = t0 + c * LS_CHUNK;
+    hi = min(lo + LS_CHUNK, t1);
     if (lo >= t1) return;
   }
   const int j = threadIdx.x;
@@ -176,11 +176,11 @@ __global__ void linear_scan_kernel(ScanArgs a, int phase) {
     if (c == 0 && col) for (int i = 0; i < dk; ++i) snap[i * dv + j] = __ldcg(st + i * dv + j);
   } else {
     // a row of several chunks starts from the copy that the first launch took
-    const float* from = (phase == 2 && t1 - t0 > a.chunk) ? snap : st;
+    const float* from = (phase == 2 && t1 - t0 > LS_CHUNK) ? snap : st;
     if (col) for (int i = 0; i < dk; ++i) S[i * dv + j] = __ldcg(from + i * dv + j);
     if (phase == 2 && col) {
       for (int p = 0; p < c; ++p) {              // the chunks before this one, in order
-        const float* ab = a.ab + ((int64_t)ls_place(a, t0, b, p) * a.heads + hd) * rec;
+        const float* ab = a.ab + ((int64_t)ls_place(LS_CHUNK, t0, b, p) * a.heads + hd) * rec;
         for (int i = 0; i < dk; ++i) S[i * dv + j] = fmaf(__ldcg(ab + i), S[i * dv + j], __ldcg(ab + dk + i * dv + j));
       }
     }
@@ -255,7 +255,7 @@ __global__ void linear_scan_kernel(ScanArgs a, int phase) {
   }
   if (phase == 1) {
     __syncthreads();
-    float* ab = a.ab + ((int64_t)ls_place(a, t0, b, c) * a.heads + hd) * rec;
+    float* ab = a.ab + ((int64_t)ls_place(LS_CHUNK, t0, b, c) * a.heads + hd) * rec;
     for (int i = threadIdx.x; i < dk; i += blockDim.x) ab[i] = sA[i];
     if (col) for (int i = 0; i < dk; ++i) ab[dk + i * dv + j] = S[i * dv + j];
   } else if (hi == t1 && col) {
@@ -290,12 +290,12 @@ __global__ void __launch_bounds__(LS_Q * LS_MAX_DV, DK <= 64 ? 2 : 1) linear_sca
   const int t0 = __ldcg(a.row_start + b), t1 = __ldcg(a.row_start + b + 1);
   int lo = t0, hi = t1;
   if (phase == 1) {
-    lo = t0 + c * a.chunk;
-    hi = lo + a.chunk;
+    lo = t0 + c * LS_CHUNK;
+    hi = lo + LS_CHUNK;
     if (hi >= t1) return;
   } else if (phase == 2) {
-    lo = t0 + c * a.chunk;
-    hi = min(lo + a.chunk, t1);
+    lo = t0 + c * LS_CHUNK;
+    hi = min(lo + LS_CHUNK, t1);
     if (lo >= t1) return;
   }
   const int q = threadIdx.x / dvr, j = threadIdx.x - q * dvr;
@@ -314,13 +314,13 @@ __global__ void __launch_bounds__(LS_Q * LS_MAX_DV, DK <= 64 ? 2 : 1) linear_sca
       for (int i = 0; i < DKQ; ++i) snap[(i0 + i) * dv + j] = __ldcg(st + (i0 + i) * dv + j);
     }
   } else {
-    const float* from = (phase == 2 && t1 - t0 > a.chunk) ? snap : st;
+    const float* from = (phase == 2 && t1 - t0 > LS_CHUNK) ? snap : st;
 #pragma unroll
     for (int i = 0; i < DKQ; ++i) S[i] = col ? __ldcg(from + (i0 + i) * dv + j) : 0.0f;
     if (phase == 2 && col) {
 #pragma unroll 2
       for (int p = 0; p < c; ++p) {                  // the chunks before this one, in order
-        const float* ab = a.ab + ((int64_t)ls_place(a, t0, b, p) * a.heads + hd) * rec;
+        const float* ab = a.ab + ((int64_t)ls_place(LS_CHUNK, t0, b, p) * a.heads + hd) * rec;
 #pragma unroll
         for (int i = 0; i < DKQ; ++i) S[i] = fmaf(__ldcg(ab + i0 + i), S[i], __ldcg(ab + DK + (i0 + i) * dv + j));
       }
@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(LS_Q * LS_MAX_DV, DK <= 64 ? 2 : 1) linear_sca
   }
   if (phase == 1) {
     __syncthreads();
-    float* ab = a.ab + ((int64_t)ls_place(a, t0, b, c) * a.heads + hd) * rec;
+    float* ab = a.ab + ((int64_t)ls_place(LS_CHUNK, t0, b, c) * a.heads + hd) * rec;
     for (int i = threadIdx.x; i < DK; i += blockDim.x) ab[i] = sA[i];
     if (col) {
 #pragma unroll
@@ -566,7 +566,7 @@ __global__ void __launch_bounds__(LW_Q * LS_MAX_DV / LW_COLS, MODE == 0 ? 1 : 2)
     if (PHASE == 2) {
 #pragma unroll 1
       for (int e = 0; e < c; ++e) {                                         // the chunks before this one, in order
-        const float* ab = a.ab + ((int64_t)ls_place(a, t0, b, e) * a.heads + hd) * rec;
+        const float* ab = a.ab + ((int64_t)ls_place(a.chunk, t0, b, e) * a.heads + hd) * rec;
         pairs_of(ab + LW_DK, [&](int p, int i, const unsigned long long (&v)[LW_COLS]) {
           const float2 w = __ldcg(reinterpret_cast<const float2*>(ab + i));
           const unsigned long long ww = lw_pair(w.x, w.y);
@@ -716,7 +716,7 @@ __global__ void __launch_bounds__(LW_Q * LS_MAX_DV / LW_COLS, MODE == 0 ? 1 : 2)
     }
   }
   if (PHASE == 1) {
-    float* ab = a.ab + ((int64_t)ls_place(a, t0, b, c) * a.heads + hd) * rec;
+    float* ab = a.ab + ((int64_t)ls_place(a.chunk, t0, b, c) * a.heads + hd) * rec;
     if (tid < LW_DK) ab[tid] = decays;
     put_pairs(ab + LW_DK);
   } else if (hi == t1) {
@@ -853,7 +853,7 @@ head_norm_gate_vec_kernel(const float* o, const float* __restrict__ w, const TG*
 
 using namespace exl3;
 
-// Sizes that the wide kernel takes (with 16-byte rows: else the kernels above run, over the same chunks).
+// Sizes that the wide kernel takes (with 16-byte rows: else the kernels above run).
 static bool ls_wide(int dk, int dv) { return dk == LW_DK && dv % 16 == 0 && dv >= 64 && dv <= LS_MAX_DV; }
 
 static int ls_sm_count() {
@@ -867,24 +867,30 @@ static int ls_sm_count() {
   return count;
 }
 
-// Tokens of a chunk, 0 for rows that are walked whole.  The wide kernel walks rows whole while they keep half the SMs busy
+// Tokens of a chunk, 0 for rows that are walked whole.  The kernels above take chunks of 64 of every row beyond 128 tokens: their
+// blocks are too few to fill the GPU with whole rows (four rows of 2,048 tokens off 16 bytes, 32 heads of 64 x 64: whole 2,001
+// us, in chunks 1,113).  The wide kernel walks rows whole while they keep half the SMs busy
 // for as long as the longest one takes (the eight rows above: whole 114 us, in chunks of 64 / 128
 // / 256 132 / 126 / 171; four rows of 2,048 287 against 448 / 366 / 356); else chunks leave two blocks an SM, since every chunk
 // pays for folding the ones before it (one row of 8,192: chunks of 64 747 us, of 256 378, of 896 470, whole 1,137).
-static int ls_chunk_len(int T, int heads, int dk, int dv, int max_new) {
+static int ls_chunk_len(bool wide, int T, int heads, int max_new) {
   if (max_new <= 2 * LS_CHUNK) return 0;
-  if (!ls_wide(dk, dv)) return LS_CHUNK;
+  if (!wide) return LS_CHUNK;
   const int64_t work = (int64_t)T * heads, sms = ls_sm_count();
   if (2 * work >= sms * max_new) return 0;
   const int64_t len = (work / (2 * sms) + LS_CHUNK - 1) / LS_CHUNK * LS_CHUNK;
   return len < LS_CHUNK ? LS_CHUNK : (len >= max_new ? 0 : (int)len);
 }
 
-extern "C" size_t exl3_linear_scan_scratch_bytes(int B, int T, int heads, int dk, int dv, int max_new) {
-  const int chunk = ls_chunk_len(T, heads, dk, dv, max_new);
+static size_t ls_scratch_bytes(int chunk, int B, int T, int heads, int dk, int dv) {
   if (chunk == 0) return 0;
   return ((size_t)(T / chunk + B + 1) * heads * ((size_t)dk + (size_t)dk * dv) + (size_t)B * heads * dk * dv) *
          sizeof(float);
+}
+
+// Enough for either kernel: the shortest chunks take the most.
+extern "C" size_t exl3_linear_scan_scratch_bytes(int B, int T, int heads, int dk, int dv, int max_new) {
+  return ls_scratch_bytes(ls_chunk_len(false, T, heads, max_new), B, T, heads, dk, dv);
 }
 
 extern "C" int exl3_token_shift(const void* h, int h_dtype, const void* mu, int mu_dtype, int n_mix, float* prev,
@@ -960,14 +966,15 @@ extern "C" int exl3_linear_scan(int mode, const void* r, int64_t r_ld, const voi
   a.wraw = wraw; a.w_ld = w_ld; a.w_dtype = w_dtype; a.w0 = w0; a.u = u; a.wu_dtype = wu_dtype; a.decay = decay;
   a.state = state; a.slot_ids = slot_ids; a.row_start = row_start; a.out = out; a.ab = scratch;
   a.act = in_act;
-  a.heads = heads; a.dk = dk; a.dv = dv; a.chunk = ls_chunk_len(T, heads, dk, dv, max_new);
-  a.places = a.chunk > 0 ? T / a.chunk + B + 1 : 0;
-  a.snap = scratch ? scratch + (size_t)a.places * heads * ((size_t)dk + (size_t)dk * dv) : nullptr;
-  const int threads = regs ? LS_Q * dvr : dvr;
+  a.heads = heads; a.dk = dk; a.dv = dv;
   const int vk = rk_dtype == DT_F32 ? 4 : 8, vv = v_dtype == DT_F32 ? 4 : 8;
   const bool wide = ls_wide(dk, dv) && r_ld % vk == 0 && k_ld % vk == 0 && v_ld % vv == 0 && aligned16(r) && aligned16(k) &&
                     aligned16(v) && aligned16(state) && aligned16(out) && aligned16(scratch) &&
                     (mode == 1 || (w_dtype == v_dtype && w_ld % vv == 0 && aligned16(wraw)));
+  a.chunk = ls_chunk_len(wide, T, heads, max_new);
+  a.places = a.chunk > 0 ? T / a.chunk + B + 1 : 0;
+  a.snap = scratch ? scratch + (size_t)a.places * heads * ((size_t)dk + (size_t)dk * dv) : nullptr;
+  const int threads = regs ? LS_Q * dvr : dvr;
   auto go = [&](int phase, int chunks) {
     const dim3 grid(heads, chunks, B);
     if (!wide) {
@@ -989,8 +996,7 @@ extern "C" int exl3_linear_scan(int mode, const void* r, int64_t r_ld, const voi
   };
   if (a.chunk > 0) {
     const int chunks = ceil_div(max_new, a.chunk);
-    if (scratch == nullptr || exl3_linear_scan_scratch_bytes(B, T, heads, dk, dv, max_new) > scratch_bytes ||
-        chunks > 65535) {
+    if (scratch == nullptr || ls_scratch_bytes(a.chunk, B, T, heads, dk, dv) > scratch_bytes || chunks > 65535) {
       set_error("linear_scan: scratch of %zu bytes is too small for %d tokens", scratch_bytes, T);
       return ERR_SCRATCH;
     }
