@@ -131,7 +131,7 @@ struct ScanArgs {
   const float* decay;
   float* state; const int* slot_ids; const int* row_start;
   float* out; float* ab; float* snap;
-  int heads, dk, dv, places, chunk;              // chunk: tokens of a chunk, LS_CHUNK or (the wide kernel) a multiple
+  int heads, dk, dv, places, chunk;              // chunk: tokens of a chunk, LS_CHUNK or (the wide kernel) as lw_chunk says
   int act;                                       // see ls_in
 };
 
@@ -493,6 +493,15 @@ __device__ inline unsigned long long lw_pair(float lo, float hi) {
   return r;
 }
 
+// The tokens of a chunk of a row of n: a step's, a multiple of LS_CHUNK, or (LW_BY_ROW) what the row's own length gives:
+// up to LW_CUTS chunks of some sixty-fours, rows of up to 128 tokens whole.  Places are counted in the shortest chunks.
+constexpr int LW_BY_ROW = -1, LW_CUTS = 16;
+__device__ inline int lw_chunk(int chunk, int n) {
+  if (chunk != LW_BY_ROW) return chunk;
+  return n <= 2 * LS_CHUNK ? max(n, 1) : (n + LS_CHUNK * LW_CUTS - 1) / (LS_CHUNK * LW_CUTS) * LS_CHUNK;
+}
+__host__ __device__ inline int lw_place_len(int chunk) { return chunk == LW_BY_ROW ? LS_CHUNK : chunk; }
+
 // TK: element type of r, k; TV: of v and the raw decays.  PHASE as above.
 template <int MODE, int PHASE, typename TK, typename TV>
 __global__ void __launch_bounds__(LW_Q * LS_MAX_DV / LW_COLS, MODE == 0 ? 1 : 2) linear_scan_wide_kernel(ScanArgs a) {
@@ -513,13 +522,14 @@ __global__ void __launch_bounds__(LW_Q * LS_MAX_DV / LW_COLS, MODE == 0 ? 1 : 2)
   pdl_trigger();
   const int t0 = __ldcg(a.row_start + b), t1 = __ldcg(a.row_start + b + 1);
   int lo = t0, hi = t1;
+  const int chunk = PHASE == 0 ? 0 : lw_chunk(a.chunk, t1 - t0);
   if (PHASE == 1) {
-    lo = t0 + c * a.chunk;
-    hi = lo + a.chunk;
+    lo = t0 + c * chunk;
+    hi = lo + chunk;
     if (hi >= t1) return;
   } else if (PHASE == 2) {
-    lo = t0 + c * a.chunk;
-    hi = min(lo + a.chunk, t1);
+    lo = t0 + c * chunk;
+    hi = min(lo + chunk, t1);
     if (lo >= t1) return;
   }
   const int q = lane >> 3, j = ((tid >> 5) * 8 + (lane & 7)) * LW_COLS;    // columns j, j + 1; channels 16 q .. 16 q + 15
@@ -562,11 +572,11 @@ __global__ void __launch_bounds__(LW_Q * LS_MAX_DV / LW_COLS, MODE == 0 ? 1 : 2)
 #pragma unroll
       for (int m = 0; m < LW_COLS; ++m) S[m][p] = 0;
   } else {
-    pairs_of((PHASE == 2 && t1 - t0 > a.chunk) ? snap : st, take);
+    pairs_of((PHASE == 2 && t1 - t0 > chunk) ? snap : st, take);
     if (PHASE == 2) {
 #pragma unroll 1
       for (int e = 0; e < c; ++e) {                                         // the chunks before this one, in order
-        const float* ab = a.ab + ((int64_t)ls_place(a.chunk, t0, b, e) * a.heads + hd) * rec;
+        const float* ab = a.ab + ((int64_t)ls_place(lw_place_len(a.chunk), t0, b, e) * a.heads + hd) * rec;
         pairs_of(ab + LW_DK, [&](int p, int i, const unsigned long long (&v)[LW_COLS]) {
           const float2 w = __ldcg(reinterpret_cast<const float2*>(ab + i));
           const unsigned long long ww = lw_pair(w.x, w.y);
@@ -716,7 +726,7 @@ __global__ void __launch_bounds__(LW_Q * LS_MAX_DV / LW_COLS, MODE == 0 ? 1 : 2)
     }
   }
   if (PHASE == 1) {
-    float* ab = a.ab + ((int64_t)ls_place(a.chunk, t0, b, c) * a.heads + hd) * rec;
+    float* ab = a.ab + ((int64_t)ls_place(lw_place_len(a.chunk), t0, b, c) * a.heads + hd) * rec;
     if (tid < LW_DK) ab[tid] = decays;
     put_pairs(ab + LW_DK);
   } else if (hi == t1) {
@@ -872,10 +882,13 @@ static int ls_sm_count() {
 // us, in chunks 1,113).  The wide kernel walks rows whole while they keep half the SMs busy
 // for as long as the longest one takes (the eight rows above: whole 114 us, in chunks of 64 / 128
 // / 256 132 / 126 / 171; four rows of 2,048 287 against 448 / 366 / 356); else chunks leave two blocks an SM, since every chunk
-// pays for folding the ones before it (one row of 8,192: chunks of 64 747 us, of 256 378, of 896 470, whole 1,137).
-static int ls_chunk_len(bool wide, int T, int heads, int max_new) {
+// pays for folding the ones before it (one row of 8,192: chunks of 64 747 us, of 256 378, of 896 470, whole 1,137).  With
+// float32 values each row is cut by its own length alone, so that its bits do not depend on the rows beside it: the eight rows
+// in float32 135 us (whole 119), four rows of 2,048 364 (327), one of 8,192 401.
+static int ls_chunk_len(bool wide, int v_dtype, int T, int heads, int max_new) {
   if (max_new <= 2 * LS_CHUNK) return 0;
   if (!wide) return LS_CHUNK;
+  if (v_dtype == DT_F32) return LW_BY_ROW;
   const int64_t work = (int64_t)T * heads, sms = ls_sm_count();
   if (2 * work >= sms * max_new) return 0;
   const int64_t len = (work / (2 * sms) + LS_CHUNK - 1) / LS_CHUNK * LS_CHUNK;
@@ -884,13 +897,13 @@ static int ls_chunk_len(bool wide, int T, int heads, int max_new) {
 
 static size_t ls_scratch_bytes(int chunk, int B, int T, int heads, int dk, int dv) {
   if (chunk == 0) return 0;
-  return ((size_t)(T / chunk + B + 1) * heads * ((size_t)dk + (size_t)dk * dv) + (size_t)B * heads * dk * dv) *
+  return ((size_t)(T / lw_place_len(chunk) + B + 1) * heads * ((size_t)dk + (size_t)dk * dv) + (size_t)B * heads * dk * dv) *
          sizeof(float);
 }
 
 // Enough for either kernel: the shortest chunks take the most.
 extern "C" size_t exl3_linear_scan_scratch_bytes(int B, int T, int heads, int dk, int dv, int max_new) {
-  return ls_scratch_bytes(ls_chunk_len(false, T, heads, max_new), B, T, heads, dk, dv);
+  return ls_scratch_bytes(ls_chunk_len(false, DT_F32, T, heads, max_new), B, T, heads, dk, dv);
 }
 
 extern "C" int exl3_token_shift(const void* h, int h_dtype, const void* mu, int mu_dtype, int n_mix, float* prev,
@@ -971,8 +984,8 @@ extern "C" int exl3_linear_scan(int mode, const void* r, int64_t r_ld, const voi
   const bool wide = ls_wide(dk, dv) && r_ld % vk == 0 && k_ld % vk == 0 && v_ld % vv == 0 && aligned16(r) && aligned16(k) &&
                     aligned16(v) && aligned16(state) && aligned16(out) && aligned16(scratch) &&
                     (mode == 1 || (w_dtype == v_dtype && w_ld % vv == 0 && aligned16(wraw)));
-  a.chunk = ls_chunk_len(wide, T, heads, max_new);
-  a.places = a.chunk > 0 ? T / a.chunk + B + 1 : 0;
+  a.chunk = ls_chunk_len(wide, v_dtype, T, heads, max_new);
+  a.places = a.chunk != 0 ? T / lw_place_len(a.chunk) + B + 1 : 0;
   a.snap = scratch ? scratch + (size_t)a.places * heads * ((size_t)dk + (size_t)dk * dv) : nullptr;
   const int threads = regs ? LS_Q * dvr : dvr;
   auto go = [&](int phase, int chunks) {
@@ -994,8 +1007,9 @@ extern "C" int exl3_linear_scan(int mode, const void* r, int64_t r_ld, const voi
 #undef EXL3_WIDE_TYPES
 #undef EXL3_WIDE
   };
-  if (a.chunk > 0) {
-    const int chunks = ceil_div(max_new, a.chunk);
+  if (a.chunk != 0) {
+    int chunks = ceil_div(max_new, lw_place_len(a.chunk));
+    if (a.chunk == LW_BY_ROW && chunks > LW_CUTS) chunks = LW_CUTS;
     if (scratch == nullptr || ls_scratch_bytes(a.chunk, B, T, heads, dk, dv) > scratch_bytes || chunks > 65535) {
       set_error("linear_scan: scratch of %zu bytes is too small for %d tokens", scratch_bytes, T);
       return ERR_SCRATCH;

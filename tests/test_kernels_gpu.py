@@ -1441,27 +1441,29 @@ def test_linear_scan_wide(mode, dv, dtype, counts):
         close(again[slots.long()], S, 2e-5, "states after two steps")
 
 
-# Rows beyond 128 tokens are cut the same way whatever else is in the step: rows off 16 bytes (the older kernels).
-@pytest.mark.parametrize("mode,dtype,off", [(0, torch.bfloat16, 3), (1, torch.float32, 3)])
-def test_linear_scan_a_row_alone_and_among_others(mode, dtype, off):
-    H, dk, dv, n, B = 16, 64, 64, 300, 41
+# A float32 row's bits do not depend on the rows beside it, however long (whole up to 128 tokens, chunks of 64 up to 1,024 and
+# longer ones beyond); with rows off 16 bytes, which the older kernels take in chunks of 64, rows beyond 128 tokens in either type.
+@pytest.mark.parametrize("mode,dtype,off,n", [(0, torch.bfloat16, 3, 300), (1, torch.float32, 3, 300), (0, torch.float32, 0, 100),
+                                              (0, torch.float32, 0, 300), (1, torch.float32, 0, 1025), (0, torch.float32, 0, 2500)])
+def test_linear_scan_a_row_alone_and_among_others(mode, dtype, off, n):
+    H, dk, dv, counts = 16, 64, 64, [n] + [300] * 40
     g = torch.Generator(device=DEV).manual_seed(off)
-    draw = lambda d: torch.randn(B * n, H * d + 8, device=DEV, generator=g).to(dtype)[:, off:off + H * d]  # noqa: E731
+    draw = lambda d: torch.randn(sum(counts), H * d + 8, device=DEV, generator=g).to(dtype)[:, off:off + H * d]  # noqa: E731
     r, k, v, w = draw(dk), draw(dk), draw(dv), draw(dk)
 
     def scan(rows):
-        T = rows * n
+        T, longest = sum(counts[:rows]), max(counts[:rows])
         more = dict(decay=torch.full((H,), 0.97, device=DEV))
         if mode == 0:
             more = dict(wraw=w[:T], w0=torch.full((H * dk,), -3.0, device=DEV), u=torch.ones(H * dk, device=DEV))
         state = torch.zeros(rows, H, dk, dv, device=DEV)
-        starts = torch.arange(rows + 1, dtype=torch.int32, device=DEV) * n
-        scratch = torch.empty(K().linear_scan_scratch_bytes(rows, T, H, dk, dv, n) // 4, device=DEV)
+        starts = torch.tensor([sum(counts[:b]) for b in range(rows + 1)], dtype=torch.int32, device=DEV)
+        scratch = torch.empty(K().linear_scan_scratch_bytes(rows, T, H, dk, dv, longest) // 4, device=DEV)
         o = K().linear_scan(mode, r[:T], k[:T], v[:T], state, torch.arange(rows, dtype=torch.int32, device=DEV), starts, rows, H,
-                            dk, dv, n, scratch=scratch, **more)
+                            dk, dv, longest, scratch=scratch, **more)
         return o[:n], state[0]
 
-    for alone, among in zip(scan(1), scan(B)):
+    for alone, among in zip(scan(1), scan(len(counts))):
         assert torch.equal(alone, among)
 
 
