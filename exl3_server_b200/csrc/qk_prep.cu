@@ -339,11 +339,11 @@ __global__ void __launch_bounds__(128) qk_rotate_vec_kernel(QkPrepArgs a) {
   __shared__ float s_sn[QP_TABLE], s_cs[QP_TABLE];
   const int t = blockIdx.x, half = a.hd >> 1, per_head = half / 8;
   const int pos = __ldcg(a.tok_pos + t);              // before the wait: the step's positions are nobody's output
-  for (int i = threadIdx.x; i < half; i += blockDim.x) {
-    float sn = 0.0f, cs = 1.0f;
-    if (a.rot) rope_sincos((float)pos, a.f_hi[i], a.f_lo ? a.f_lo[i] : 0.0f, &sn, &cs);
-    s_sn[i] = a.rot ? sn * a.mscale : 0.0f;
-    s_cs[i] = a.rot ? cs * a.mscale : 1.0f;
+  for (int i = threadIdx.x; i < a.rot >> 1; i += blockDim.x) {
+    float sn, cs;
+    rope_sincos((float)pos, a.f_hi[i], a.f_lo ? a.f_lo[i] : 0.0f, &sn, &cs);
+    s_sn[i] = sn * a.mscale;
+    s_cs[i] = cs * a.mscale;
   }
   pdl_wait();
   pdl_trigger();
@@ -361,9 +361,15 @@ __global__ void __launch_bounds__(128) qk_rotate_vec_kernel(QkPrepArgs a) {
     const float mul = is_q ? q_mul : a.k_mul;
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
-      const float sn = s_sn[i + e], cs = s_cs[i + e];
-      lo[e] = fmaf(u[e], cs, -v[e] * sn) * mul;
-      hi[e] = fmaf(v[e], cs, u[e] * sn) * mul;
+      lo[e] = u[e];
+      hi[e] = v[e];
+      if (a.rot) {                                    // else a feature must not meet its partner, which may be infinite
+        const float sn = s_sn[i + e], cs = s_cs[i + e];
+        lo[e] = fmaf(u[e], cs, -v[e] * sn);
+        hi[e] = fmaf(v[e], cs, u[e] * sn);
+      }
+      lo[e] *= mul;
+      hi[e] *= mul;
     }
     float* to = static_cast<float*>(is_q ? a.q_out : a.k_out) + ((int64_t)t * (is_q ? a.nh : a.nkv) + h) * a.hd + i;
 #pragma unroll

@@ -1503,3 +1503,16 @@ def test_qk_prep_rotated_heads_for_a_recurrence(dtype, T, nh, nkv, hd, rot, temp
         if temp and off == 8:
             mul = (1.0 + 0.1 * torch.log(torch.floor((pos.double().cpu() + 1) / temp) + 1.0))[:, None, None]
         close(got.view(T, n, hd), want * mul, 1e-6, "rotated")
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_qk_prep_without_a_rotation_keeps_features_apart(dtype):
+    """Queries and keys for a recurrence without a rotation: what is infinite or NaN stays in its own feature."""
+    T, n, hd = 3, 2, 32
+    x = torch.randn(T, 2 * n * hd, device=DEV, generator=torch.Generator(device=DEV).manual_seed(1)).to(dtype)
+    x[1, 20], x[2, 3], x[0, n * hd + 31] = math.inf, -math.inf, math.nan
+    pos = torch.arange(T, dtype=torch.int32, device=DEV)
+    q, k = K().qk_prep(x, 0, n * hd, -1, n, n, hd, 0, hd, 0, 0, None, None, 1e-6, 0, 0, None, 1.0, 0.5, None, pos,
+                       torch.zeros_like(pos), None, 0, torch.float32, None, None, k_dtype=torch.float32)
+    for got, want in ((q, x[:, :n * hd].float()), (k, x[:, n * hd:].float() * 0.5)):
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.nan_to_num(7.0), want.nan_to_num(7.0))
