@@ -819,7 +819,7 @@ head_norm_gate_vec_kernel(const float* o, const float* __restrict__ w, const TG*
                           float eps, TO* out, int n_items, int heads, int dv) {
   pdl_wait();
   pdl_trigger();
-  const int item = (blockIdx.x * blockDim.x + threadIdx.x) / LANES;
+  const int item = blockIdx.x * (blockDim.x / LANES) + threadIdx.x / LANES;    // the threads may be more than 2^32
   const int t = item / heads, hd = item - t * heads;
   const int e = threadIdx.x % LANES * 4;
   const bool mine = item < n_items && e < dv;

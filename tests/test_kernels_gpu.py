@@ -1516,3 +1516,13 @@ def test_qk_prep_without_a_rotation_keeps_features_apart(dtype):
                        torch.zeros_like(pos), None, 0, torch.float32, None, None, k_dtype=torch.float32)
     for got, want in ((q, x[:, :n * hd].float()), (k, x[:, n * hd:].float() * 0.5)):
         assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.nan_to_num(7.0), want.nan_to_num(7.0))
+
+
+def test_head_norm_gate_of_very_many_heads():
+    """More threads than 32 bits count: 2^28 heads and some of four values."""
+    T, H, dv = 2 ** 20 + 1, 256, 4
+    o = torch.randn(T, H * dv, device=DEV)
+    got = K().head_norm_gate(o, None, None, 1e-5, H, dv, torch.bfloat16)
+    for t in (0, T // 2, T - 1):
+        x = o[t].view(H, dv).double()
+        close(got[t].view(H, dv), x / torch.sqrt((x * x).mean(-1, keepdim=True) + 1e-5), 4e-3, f"token {t}")
