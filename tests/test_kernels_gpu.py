@@ -1518,6 +1518,23 @@ def test_qk_prep_without_a_rotation_keeps_features_apart(dtype):
         assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.nan_to_num(7.0), want.nan_to_num(7.0))
 
 
+@pytest.mark.parametrize("dv", [64, 96])
+@pytest.mark.parametrize("gate_type,out_type", [(torch.float32, torch.float32), (torch.float32, torch.bfloat16), (torch.bfloat16, torch.bfloat16)])
+def test_head_norm_gate_with_gates_anywhere(gate_type, out_type, dv):
+    """Gates that start off 16 (8, 4) bytes take the same kernel as others, with the same bits."""
+    T, H = 50, 8
+    g = torch.Generator(device=DEV).manual_seed(dv)
+    o, w = torch.randn(T, H * dv, device=DEV, generator=g), torch.randn(H * dv, device=DEV, generator=g)
+    rows = torch.randn(T, H * dv + 8, device=DEV, generator=g).to(gate_type)
+    for off in (1, 2, 4):
+        moved = torch.zeros_like(rows)
+        moved[:, :H * dv] = rows[:, off:off + H * dv]
+        for kind in ("silu", "sigmoid"):
+            got, want = (K().head_norm_gate(o, w, x, 1e-5, H, dv, out_type, gate_kind=kind)
+                         for x in (rows[:, off:off + H * dv], moved[:, :H * dv]))
+            assert torch.equal(got, want)
+
+
 def test_head_norm_gate_of_very_many_heads():
     """More threads than 32 bits count: 2^28 heads and some of four values."""
     T, H, dv = 2 ** 20 + 1, 256, 4
