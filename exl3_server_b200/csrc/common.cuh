@@ -131,9 +131,13 @@ int launch_status(const char* what);
 // while the kernel before it in the stream is still running; it must call
 // pdl_wait() before it reads anything that kernel wrote and before it writes
 // anything at all.  What comes before pdl_wait() may only touch data that no
-// kernel of the step writes (weights).  pdl_trigger() lets the next kernel in
-// the stream start early in the same way.  Without the launch attribute both
-// calls do nothing.
+// kernel writes which may still be running then: weights, and the step's
+// positions and page tables.  Those are written by copies, which every kernel
+// after them waits for, and by the last kernel of a recorded step, which does
+// not call pdl_trigger() (argmax_final_kernel): so a kernel, however many after
+// it, starts when they are written.  Any other kernel that writes such data must
+// do the same.  pdl_trigger() lets the next kernel in the stream start early in
+// the same way.  Without the launch attribute both calls do nothing.
 __device__ inline void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ inline void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

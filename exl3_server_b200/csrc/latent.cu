@@ -108,7 +108,7 @@ latent_prep_kernel(const void* a, int a_dtype, int lda, int q_off, int q_rank, c
 
 // The same for few tokens, whose chain of trips to memory is what they cost: the latents are read once, kept in registers
 // (what is beyond LP_KEEP values a thread is read again) and both sums of squares taken at once, and the token's place in the
-// cache is looked up before the wait (the step's positions and page tables are nobody's output).  The sums run in the order of the
+// cache is looked up before the wait (launch_pdl says why it may be).  The sums run in the order of the
 // kernel above (LP_SUM chains, block_sum's tree), the queries' in the first half of the threads and the keys' in the other,
 // so a token's bits do not depend on how many tokens its step has.
 // Latents of 768 + 512 in bfloat16, this kernel / the one above, back to back: 2 tokens 4.4 / 6.8 us, 592 tokens 5.9 / 7.2, 2,000

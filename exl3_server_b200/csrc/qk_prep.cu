@@ -222,8 +222,8 @@ __global__ void __launch_bounds__(QP_WARPS * 32) qk_prep_vec_kernel(QkPrepArgs a
   __shared__ float s_sn[QP_TABLE], s_cs[QP_TABLE];
   const int t = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // before the wait: the token's position and page, its sines and cosines (the step's positions and page tables are nobody's
-  // output): a step of few tokens waits 1 us less for it
+  // before the wait: the token's position and page, its sines and cosines (launch_pdl says why these may be read here): a step
+  // of few tokens waits 1 us less for it
   const int pos = __ldcg(a.tok_pos + t);
   const int pg = a.nkv > 0 ? __ldcg(a.block_table + (int64_t)__ldcg(a.tok_seq + t) * a.bt_stride + pos / a.page) : -1;
   const int in_page = a.nkv > 0 ? pos % a.page : 0;
@@ -338,7 +338,7 @@ template <typename TX>
 __global__ void __launch_bounds__(128) qk_rotate_vec_kernel(QkPrepArgs a) {
   __shared__ float s_sn[QP_TABLE], s_cs[QP_TABLE];
   const int t = blockIdx.x, half = a.hd >> 1, per_head = half / 8;
-  const int pos = __ldcg(a.tok_pos + t);              // before the wait: the step's positions are nobody's output
+  const int pos = __ldcg(a.tok_pos + t);              // before the wait: see launch_pdl
   for (int i = threadIdx.x; i < a.rot >> 1; i += blockDim.x) {
     float sn, cs;
     rope_sincos((float)pos, a.f_hi[i], a.f_lo ? a.f_lo[i] : 0.0f, &sn, &cs);

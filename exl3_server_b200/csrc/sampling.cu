@@ -92,14 +92,16 @@ argmax_partial_kernel(const float* __restrict__ logits, float* __restrict__ pv, 
 }
 
 // The end of a decode step, where the ids are known: feed[row] takes the id and pos[row] goes on by inc[row] (feed null:
-// neither).  They were a copy and an addition of their own at the end of every step: two launches, 5 us.
+// neither).  They were a copy and an addition of their own at the end of every step: two launches, 5 us.  With feed the kernel does
+// not let the next one start early: kernels read positions before their wait (see launch_pdl), so no kernel may start before
+// these are written.  As the last kernel of a recorded step it has nobody to let start.
 __global__ void __launch_bounds__(ARGMAX_THREADS)
 argmax_final_kernel(const float* __restrict__ pv, const int* __restrict__ pi, int* __restrict__ out, int nchunks, int* feed,
                     int* pos, const int* inc) {
   __shared__ float sv[32];
   __shared__ int si[32];
   pdl_wait();
-  pdl_trigger();
+  if (feed == nullptr) pdl_trigger();
   const int row = blockIdx.x;
   float best = -INFINITY;
   int bi = 0x7fffffff;
@@ -115,6 +117,7 @@ argmax_final_kernel(const float* __restrict__ pv, const int* __restrict__ pi, in
     if (feed) {
       feed[row] = id;
       pos[row] = __ldcg(pos + row) + __ldcg(inc + row);
+      __threadfence();                                // before the block ends
     }
   }
 }

@@ -1479,6 +1479,30 @@ def test_argmax_step(R, V):
     assert torch.equal(pos, want)
 
 
+def test_positions_moved_on_are_there_for_the_next_kernel():
+    """Kernels read positions before they wait for the kernel before them; the end of a step, which writes them, lets none
+    start early."""
+    T, n, hd = 8, 2, 64
+    x = torch.ones(T, n * hd, device=DEV)
+    table = K().rotary_table(torch.tensor([1.0 / (i + 1) for i in range(hd // 2)], dtype=torch.float64)).to(DEV)
+    ints = lambda v: torch.full((T,), v, dtype=torch.int32, device=DEV)  # noqa: E731
+    logits = torch.randn(T, 60000, device=DEV)
+    out, feed, pos, inc, seq = ints(0), ints(0), ints(0), ints(1), ints(0)
+
+    def rotated():
+        return K().qk_prep(x, 0, 0, -1, n, 0, hd, 0, hd, 0, 0, None, None, 1e-6, hd, 0, table, 1.0, 1.0, None, pos, seq, None, 0,
+                           torch.float32, None, None)[0]
+
+    got = []
+    for _ in range(100):
+        K().argmax_step(logits, out, feed, pos, inc)
+        got.append(rotated())
+    for i in range(100):
+        pos.fill_(i + 1)
+        torch.cuda.synchronize()
+        assert torch.equal(got[i], rotated()), i
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("T,nh,nkv,hd,rot,temp", [(1, 1, 1, 16, 16, 0.0), (7, 5, 3, 64, 64, 0.0), (3, 2, 2, 128, 0, 0.0),
                                                   (150, 16, 16, 64, 64, 40.0)])
