@@ -24,7 +24,7 @@
 // meet through distributed shared memory (every block adds all of them up and
 // finds the same digit), and the passing keys are written into the first
 // block's, which sorts and draws.  Bound by the chain of passes, barriers and the
-// sort: 32 rows of 122,753 take 43 us (one block a row that reads it five times:
+// sort: 32 rows of 122,753 take 41 us, 44 with penalties (one block a row that reads it five times:
 // 105 us, and the penalties were a copy of the logits and a kernel of 16 us).
 #include "api.h"
 #include "common.cuh"
@@ -51,7 +51,7 @@ struct SfRow {            // one row's options, as the host gives them (float64 
   double temperature, top_k, top_p, min_p, u;
 };
 
-constexpr double SF_FIXED_US = 36.0, SF_STAGED_US = 0.00030, SF_AGAIN_US = 0.00065;
+constexpr double SF_FIXED_US = 35.0, SF_STAGED_US = 0.00018, SF_AGAIN_US = 0.00033, SF_AGAIN_PENALTIES_US = 0.00075;
 constexpr int SF_BINS = 2048;
 constexpr int SF_HEAD_BYTES = (2 * SF_BINS * 4) + 2 * (SF_CAP * 8);     // histograms, candidates, this block's own
 constexpr int SF_SMEM_MOST = 200 * 1024;                                // with the staged part of a row
@@ -79,8 +79,9 @@ __device__ inline float sf_penalised(float x, int count, float rep, float presen
 // counts: null, or per row a pointer to its token counts [V] (null: the row has no penalties); params [R, 3]: repetition,
 // presence, frequency.  The counts are only read: rows may share them, so the chosen tokens join them in a kernel of their
 // own, after every row has been drawn (2 us for 32 rows).  STAGED: the block's part of the row is kept in shared memory;
-// else (vocabularies too long for that) every pass reads it again.
-template <bool STAGED>
+// else (parts too long for that) every pass reads it again, 16 bytes a load: one block a row takes 76 us for 122,753
+// tokens (4 bytes a load, and 64-bit keys compared in every pass: 107), 142 for 320,001.  PENALTIES: there may be counts.
+template <bool STAGED, bool PENALTIES>
 __global__ void __launch_bounds__(SF_THREADS)
 sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict__ rows, const int* const* __restrict__ counts,
                        const float* __restrict__ params, int* __restrict__ out, int V, int blocks) {
@@ -100,7 +101,7 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
   const float* row = logits + (int64_t)row_id * V;
   const SfRow o = rows[row_id];
   const int M = V < SF_CAP ? V : SF_CAP;
-  const int* count = counts ? counts[row_id] : nullptr;
+  const int* count = PENALTIES && counts ? counts[row_id] : nullptr;
   float rep = 1.0f, presence = 0.0f, frequency = 0.0f;
   if (count) {
     rep = params[3 * row_id];
@@ -109,17 +110,49 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
   }
   const int per = (V + blocks - 1) / blocks;
   const int first = min(V, rank * per), n = min(V, first + per) - first;
-  auto read_key = [&](int i) {
-    float x = row[first + i];
-    if (count) x = sf_penalised(x, count[first + i], rep, presence, frequency);
-    return sf_key(x);
-  };
-  // every token's (value, inverted index) key of this block's part
+  // f(value's key, place in the row) for every token of this block's part
   auto for_each = [&](auto&& f) {
     if constexpr (STAGED) {
-      for (int i = tid; i < n; i += SF_THREADS) f(((unsigned long long)keys[i] << 32) | (unsigned)(~(unsigned)(first + i)));
+      for (int i = tid; i < n; i += SF_THREADS) f(keys[i], first + i);
     } else {
-      for (int i = tid; i < n; i += SF_THREADS) f(((unsigned long long)read_key(i) << 32) | (unsigned)(~(unsigned)(first + i)));
+      // 16-byte loads, four of a thread on their way, with penalties two and as many of the counts (parts start at any
+      // multiple of 4 bytes: the pieces before and after the aligned part go one by one)
+      constexpr int AHEAD = PENALTIES ? 2 : 4;
+      const float* part = row + first;
+      auto key_of = [&](float x, int c) {
+        if constexpr (PENALTIES) return sf_key(sf_penalised(x, c, rep, presence, frequency));
+        else return sf_key(x);
+      };
+      auto counted = [&](int i) { return PENALTIES && count ? count[first + i] : 0; };
+      const int head = min(n, (int)((4 - ((reinterpret_cast<uintptr_t>(part) >> 2) & 3)) & 3)), n_vec = (n - head) / 4;
+      const float4* part4 = reinterpret_cast<const float4*>(part + head);
+      auto one = [&](int i) { f(key_of(part[i], counted(i)), first + i); };
+      if (tid < head) one(tid);
+#pragma unroll 1
+      for (int j0 = tid; j0 < n_vec; j0 += SF_THREADS * AHEAD) {
+        float4 x[AHEAD];
+        int c[AHEAD][4];
+#pragma unroll
+        for (int a = 0; a < AHEAD; ++a) {
+          const int j = j0 + a * SF_THREADS;
+          if (j < n_vec) {
+            x[a] = part4[j];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) c[a][e] = counted(head + 4 * j + e);
+          }
+        }
+#pragma unroll
+        for (int a = 0; a < AHEAD; ++a) {
+          const int j = j0 + a * SF_THREADS, i = first + head + 4 * j;
+          if (j < n_vec) {
+            f(key_of(x[a].x, c[a][0]), i);
+            f(key_of(x[a].y, c[a][1]), i + 1);
+            f(key_of(x[a].z, c[a][2]), i + 2);
+            f(key_of(x[a].w, c[a][3]), i + 3);
+          }
+        }
+      }
+      for (int i = head + 4 * n_vec + tid; i < n; i += SF_THREADS) one(i);
     }
   };
   if constexpr (STAGED) {
@@ -160,11 +193,19 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
         for (int b = tid; b < SF_BINS; b += SF_THREADS) hist[b] = 0;
         __syncthreads();
       }
-      const unsigned long long mask = shift + bits >= 64 ? 0ull : (~0ull << (shift + bits));
       const unsigned digit_mask = (1u << bits) - 1u;
-      for_each([&](unsigned long long c) {
-        if ((c & mask) == (thresh & mask)) atomicAdd(hist + ((unsigned)(c >> shift) & digit_mask), 1u);
-      });
+      const uint32_t want = (uint32_t)(thresh >> 32);
+      if (pass < 3) {
+        const uint32_t mask = pass == 0 ? 0u : ~0u << (shift - 32 + bits);
+        for_each([&](uint32_t key, int) {
+          if (((key ^ want) & mask) == 0) atomicAdd(hist + ((key >> (shift - 32)) & digit_mask), 1u);
+        });
+      } else {
+        const uint32_t mask = pass == 3 ? 0u : ~0u << (shift + bits), low = (uint32_t)thresh;
+        for_each([&](uint32_t key, int i) {
+          if (key == want && ((~(uint32_t)i ^ low) & mask) == 0) atomicAdd(hist + ((~(uint32_t)i >> shift) & digit_mask), 1u);
+        });
+      }
       sf_cluster_sync();
       // all blocks' histograms, from the largest digit down, two bins a thread
       const int hi = SF_BINS - 1 - 2 * tid;
@@ -202,10 +243,14 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
       __syncthreads();                            // before the next pass's sums
     }
   }
-  for_each([&](unsigned long long c) {
-    if (c >= thresh) {
-      const unsigned k = atomicAdd(&n_found, 1u);
-      if (k < (unsigned)SF_CAP) found[k] = c;
+  const uint32_t least = (uint32_t)(thresh >> 32);
+  for_each([&](uint32_t key, int i) {
+    if (key >= least) {
+      const unsigned long long c = ((unsigned long long)key << 32) | ~(uint32_t)i;
+      if (c >= thresh) {
+        const unsigned k = atomicAdd(&n_found, 1u);
+        if (k < (unsigned)SF_CAP) found[k] = c;
+      }
     }
   });
   if (V <= SF_CAP) sf_cluster_sync();             // the first block's candidates are cleared (else the select has met)
@@ -355,9 +400,10 @@ extern "C" int exl3_sample_rows(const float* logits, const double* rows, int* co
     set_error("sample_filtered: bad sizes rows=%d vocab=%d, or penalties without their constants", R, V);
     return ERR_BAD_ARGUMENT;
   }
-  // Blocks a row.  An SM holds one block and the SMs come in eight groups that a cluster must fit into; a wave of clusters
-  // takes some 36 us and 0.3 ns a token of a block's part, 0.65 ns where it is too long for shared memory.  With 8 / 4 / 2 / 1
-  // blocks: 32 rows of 122,753 89 / 43 / 68 / 106 us, 64 rows of 32,000 117 / 66 / 37 / 42, 256 rows 392 / 205 / 136 / 82.
+  // Blocks a row.  An SM holds one block, and the SMs come in eight groups that a cluster must fit into; a wave of rows takes
+  // some 35 us and, for a token of a block's part, 0.18 ns, or 0.33 (0.75 with penalties) where the part is too long for
+  // shared memory and read in every pass.  With 8 / 4 / 2 / 1 blocks: 32 rows of 122,753 86 / 41 / 55 / 76 us, 148 rows 280 /
+  // 168 / 108 / 77, 64 rows of 32,000 116 / 64 / 35 / 39, 100 rows of 320,001 273 / 194 / 186 / 168.
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -366,9 +412,10 @@ extern "C" int exl3_sample_rows(const float* logits, const double* rows, int* co
   double best = 0.0;
   for (int b = 8; b >= 1; b /= 2) {
     const int each = ceil_div(V, b);
-    const int at_once = 8 * std::max(1, sms / 8 / b);    // clusters of b that fit: the SMs come in eight groups
+    const int at_once = b == 1 ? sms : 8 * std::max(1, sms / 8 / b);
     const double waves = (double)((R + at_once - 1) / at_once);
-    const double cost = waves * (SF_FIXED_US + ((size_t)each * 4 <= MOST ? SF_STAGED_US : SF_AGAIN_US) * each);
+    const double a_token = (size_t)each * 4 <= MOST ? SF_STAGED_US : counts ? SF_AGAIN_PENALTIES_US : SF_AGAIN_US;
+    const double cost = waves * (SF_FIXED_US + a_token * each);
     if (b == 8 || cost < best) {
       best = cost;
       blocks = b;
@@ -376,7 +423,8 @@ extern "C" int exl3_sample_rows(const float* logits, const double* rows, int* co
   }
   const size_t part = (size_t)ceil_div(V, blocks) * 4;
   const bool staged = part <= MOST;
-  auto kernel = staged ? sample_filtered_kernel<true> : sample_filtered_kernel<false>;
+  auto kernel = staged ? sample_filtered_kernel<true, true>
+                       : counts ? sample_filtered_kernel<false, true> : sample_filtered_kernel<false, false>;
   const size_t smem = SF_HEAD_BYTES + (staged ? part : 0);
   // The limit belongs to the function and not to this call: the same number from every thread, whatever its rows take, or a
   // thread with shorter rows would lower it between another one's setting it and its launch.
@@ -398,7 +446,7 @@ extern "C" int exl3_sample_rows(const float* logits, const double* rows, int* co
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = blocks > 1 ? 1 : 0;               // without a cluster blocks are spread over the SMs first
   cudaLaunchKernelEx(&cfg, kernel, logits, reinterpret_cast<const SfRow*>(rows), (const int* const*)counts, params, out, V,
                      blocks);
   int rc = launch_status("sample_filtered");

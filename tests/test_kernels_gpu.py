@@ -1306,6 +1306,28 @@ def test_penalised_sampling_takes_rows_that_are_not_dense():
     assert [r.rng.state for r in rows] == before
 
 
+@pytest.mark.parametrize("penalties", [False, True])
+def test_sample_filtered_ranks_equal_logits_of_long_rows(penalties):
+    """Rows too long for shared memory, which every pass reads again, with few different values: the ranking goes on over the
+    indices, from rows that start at every multiple of 4 bytes."""
+    from exl3_server_b200.sampling import SampleOptions
+    from exl3_server_b200.sampling.host import sample_token
+    V, R = 330001, 5
+    logits = np.round(2.0 * np.random.default_rng(11).normal(size=(R, V))).astype(np.float32)
+    opt = SampleOptions(temperature=2.0, repetition_penalty=1.5 if penalties else 1.0)
+    contexts = [np.nonzero(logits[r] == logits[r].max())[0][:3].tolist() + [7] for r in range(R)]
+    us = [0.03, 0.2, 0.5, 0.77, 0.99]
+    rows = torch.tensor([[opt.temperature, 0, 1.0, 0.0, u] for u in us], dtype=torch.float64, device=DEV)
+    dev = torch.from_numpy(logits).to(DEV)
+    if penalties:
+        counts = [torch.bincount(torch.tensor(c), minlength=V).to(torch.int32).to(DEV) for c in contexts]
+        ptrs = torch.tensor([c.data_ptr() for c in counts], dtype=torch.int64, device=DEV)
+        got = K().sample_rows(dev, rows, ptrs, torch.tensor([[1.5, 0.0, 0.0]] * R, device=DEV))
+    else:
+        got = K().sample_filtered(dev, rows)
+    assert got.tolist() == [sample_token(logits[r], opt, contexts[r], _FixedU(us[r])) for r in range(R)]
+
+
 @pytest.mark.parametrize("V", [300, 40001])
 def test_rows_that_share_a_sampler(V):
     """One request's sampler for all rows, more rows than run at once: every row sees the context as it was before the
