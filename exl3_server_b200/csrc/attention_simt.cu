@@ -464,19 +464,22 @@ static int dispatch(const void* q, int64_t q_row_stride, void* out, const void* 
 
 // ---- float32, plain causal attention with heads of 64 or 128 ---------------------------------------------------------
 //
-// A block has up to 4 TY rows (a row: one query head of one token; the query heads of a kv head side by side, then the
+// A block has up to ROWS TY rows (a row: one query head of one token; the query heads of a kv head side by side, then the
 // next token of the same sequence), one kv head and one chunk of split_keys keys, which it walks a page at a time: the
-// page's scores as a product of tiles (thread: 4 rows x 4 keys, every 16th), one maximum and one rescaling a page, then
-// P V as a product of tiles (4 rows x HD / 16 features).  K of the next page is copied while the softmax and P V run, V
+// page's scores as a product of tiles (thread: ROWS rows x 4 keys, every 16th), one maximum and one rescaling a page, then
+// P V as a product of tiles (ROWS rows x HD / 16 features).  K of the next page is copied while the softmax and P V run, V
 // while the scores do.  What a row computes depends on its own position only: the features of a score in order, 32 at
 // a time on an accumulator for the even and one for the odd ones, a page's sum over a fixed tree, the keys of P V in
-// order, 16 at a time; so TY and what else is in the block change nothing, and the records of chunks are the general kernel's.
+// order, 16 at a time; so the block's shape and what else is in it change nothing, and the records of chunks are the general
+// kernel's.  A prompt's tiles have 64 rows (TY 16, ROWS 4).  A single token has as many as a kv head has query heads: TY 4
+// and ROWS 1, 2 or 4; with one (ONE) the four groups of threads share the row: a key of the four each, a chain of sixteen keys of
+// P V each, the chains added in order by the first.
 // The general kernel walks one key after the other with a shuffle tree and two exponentials a key, a chain of latencies:
 // prompts of 90, 300 and 289 tokens with 16 query heads on 2 of 64 take it 256 us, this one 63; three single tokens at 250 to
-// 300 keys 79 and 25 us; prompts of 33 and 130 with 32 on 8 of 128 231 and 38 us.  Errors against 64 bits are the same
-// (1.3e-7 there).  One query head a kv head leaves a single token three quarters of the rows empty (36 heads at 1,100 keys:
-// 19 and 25 us); it takes this kernel too, so that a token's bits do not depend on the step that brought it.
-constexpr int AF_PAGE = 64, AF_TX = 16, AF_KEYS = AF_PAGE / AF_TX, AF_ROWS = 4, AF_CHAIN = 32, AF_P_PITCH = AF_PAGE + 4;
+// 300 keys 79 and 18 us; prompts of 33 and 130 with 32 on 8 of 128 231 and 38 us.  Errors against 64 bits are the same
+// (1.3e-7 there).  One query head a kv head: a token at 1,100 keys with 36 of 64 19 and 12 us (in 16 rows of which one is used
+// 25), four at 4,000 keys with 16 of 128 59 and 54 us (147).
+constexpr int AF_PAGE = 64, AF_TX = 16, AF_KEYS = AF_PAGE / AF_TX, AF_CHAIN = 32, AF_P_PITCH = AF_PAGE + 4;
 
 __device__ inline void af_cp16(void* smem, const void* gmem, bool ok) {
   const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
@@ -499,14 +502,14 @@ __device__ inline unsigned long long af_pair(float lo, float hi) {
   return r;
 }
 
-template <int HD, int TY>
+template <int HD, int TY, int ROWS>
 constexpr int af_smem_floats() {
-  return AF_ROWS * TY * (HD + 4) + AF_PAGE * (HD + 4) + AF_PAGE * HD + AF_ROWS * TY * AF_P_PITCH;
+  return ROWS * TY * (HD + 4) + AF_PAGE * (HD + 4) + AF_PAGE * HD + ROWS * TY * AF_P_PITCH;
 }
 
 // tile_seq null: tile i is token i alone.  Else tile i is new tokens tile_q0[i / sub] + (i % sub) * tile_tokens on of
 // batch row tile_seq[i / sub], at most tile_tokens of them.
-template <int HD, int TY>
+template <int HD, int TY, int ROWS, bool ONE>
 __global__ void __launch_bounds__(AF_TX * TY)
 attn_f32_kernel(const float* __restrict__ q, int64_t q_row_stride, float* __restrict__ out,
                 const float* __restrict__ k_pool, const float* __restrict__ v_pool, const int* __restrict__ block_table,
@@ -515,9 +518,10 @@ attn_f32_kernel(const float* __restrict__ q, int64_t q_row_stride, float* __rest
                 int sub, int tile_tokens, int nh, int nkv, float scale, int split_keys, int max_splits,
                 float* __restrict__ scratch) {
   constexpr int NT = AF_TX * TY, QP = HD + 4, VQ = HD / 64;    // VQ: groups of 4 features of a thread in P V
+  static_assert(!ONE || (ROWS == 1 && TY == AF_KEYS && TY * AF_CHAIN / 2 == AF_PAGE), "a key, a chain of P V a group of threads");
   extern __shared__ __align__(16) float af_smem[];
   float* sq = af_smem;
-  float* sk = sq + AF_ROWS * TY * QP;
+  float* sk = sq + ROWS * TY * QP;
   float* sv = sk + AF_PAGE * QP;
   float* sp = sv + AF_PAGE * HD;
   pdl_wait();
@@ -542,16 +546,16 @@ attn_f32_kernel(const float* __restrict__ q, int64_t q_row_stride, float* __rest
   const int c_hi = min(hi_max, split_keys > 0 ? c_lo + split_keys : hi_max);
   const int* bt = block_table + (int64_t)__ldcg(tok_seq + t0) * bt_stride;
 
-  int hi[AF_ROWS];                                             // this thread's rows see keys below hi
+  int hi[ROWS];                                             // this thread's rows see keys below hi
 #pragma unroll
-  for (int i = 0; i < AF_ROWS; ++i) {
+  for (int i = 0; i < ROWS; ++i) {
     const int r = ty + TY * i;
     hi[i] = pos0 + min(r, rows - 1) / G + 1;                   // rows beyond the tile's are zeros that nobody stores
   }
-  unsigned long long acc[AF_ROWS][VQ][2];
-  float m[AF_ROWS], l[AF_ROWS];
+  unsigned long long acc[ROWS][VQ][2];
+  float m[ROWS], l[ROWS];
 #pragma unroll
-  for (int i = 0; i < AF_ROWS; ++i) {
+  for (int i = 0; i < ROWS; ++i) {
     m[i] = -INFINITY;
     l[i] = 0.0f;
 #pragma unroll
@@ -559,7 +563,7 @@ attn_f32_kernel(const float* __restrict__ q, int64_t q_row_stride, float* __rest
   }
 
   if (c_lo < c_hi) {
-    for (int idx = tid; idx < AF_ROWS * TY * (HD / 4); idx += NT) {
+    for (int idx = tid; idx < (ONE ? 1 : ROWS * TY) * (HD / 4); idx += NT) {
       const int r = idx / (HD / 4), d = (idx % (HD / 4)) * 4;
       const bool ok = r < rows;
       af_cp16(sq + r * QP + d, q + (ok ? (int64_t)(t0 + r / G) * q_row_stride + (int64_t)(g * G + r % G) * HD + d : 0), ok);
@@ -583,41 +587,49 @@ attn_f32_kernel(const float* __restrict__ q, int64_t q_row_stride, float* __rest
     for (int page = first; page <= last; ++page) {
       af_wait<1>();
       __syncthreads();                                         // K of this page (and the queries) are here
-      float sc[AF_ROWS][AF_KEYS];
+      constexpr int NS = ONE ? 1 : AF_KEYS;                    // keys of this thread's scores
+      const float* sqr = sq + (ONE ? 0 : ty * QP);
+      const float* skr = sk + (tx + (ONE ? AF_TX * ty : 0)) * QP;
+      float sc[ROWS][AF_KEYS];
 #pragma unroll
       for (int c = 0; c < HD / AF_CHAIN; ++c) {
-        unsigned long long s2[AF_ROWS][AF_KEYS];
+        unsigned long long s2[ROWS][NS];
 #pragma unroll
-        for (int i = 0; i < AF_ROWS; ++i)
+        for (int i = 0; i < ROWS; ++i)
 #pragma unroll
-          for (int j = 0; j < AF_KEYS; ++j) s2[i][j] = 0;
+          for (int j = 0; j < NS; ++j) s2[i][j] = 0;
 #pragma unroll 4
         for (int d = c * AF_CHAIN; d < (c + 1) * AF_CHAIN; d += 4) {
-          ulonglong2 a[AF_ROWS];
+          ulonglong2 a[ROWS];
 #pragma unroll
-          for (int i = 0; i < AF_ROWS; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(sq + (ty + TY * i) * QP + d);
+          for (int i = 0; i < ROWS; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(sqr + TY * i * QP + d);
 #pragma unroll
-          for (int j = 0; j < AF_KEYS; ++j) {
-            const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(sk + (tx + AF_TX * j) * QP + d);
+          for (int j = 0; j < NS; ++j) {
+            const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(skr + AF_TX * j * QP + d);
 #pragma unroll
-            for (int i = 0; i < AF_ROWS; ++i) af_fma2(s2[i][j], a[i].x, b.x);
+            for (int i = 0; i < ROWS; ++i) af_fma2(s2[i][j], a[i].x, b.x);
 #pragma unroll
-            for (int i = 0; i < AF_ROWS; ++i) af_fma2(s2[i][j], a[i].y, b.y);
+            for (int i = 0; i < ROWS; ++i) af_fma2(s2[i][j], a[i].y, b.y);
           }
         }
 #pragma unroll
-        for (int i = 0; i < AF_ROWS; ++i)
+        for (int i = 0; i < ROWS; ++i)
 #pragma unroll
-          for (int j = 0; j < AF_KEYS; ++j) {
+          for (int j = 0; j < NS; ++j) {
             const float2 e = af_split(s2[i][j]);
             sc[i][j] = c == 0 ? e.x + e.y : sc[i][j] + (e.x + e.y);
           }
       }
+      if constexpr (ONE) sp[tx + AF_TX * ty] = sc[0][0];
       __syncthreads();                                         // K has been read
       fetch(k_pool, sk, QP, page + 1);
       const int base = page * AF_PAGE;
+      if constexpr (ONE) {
 #pragma unroll
-      for (int i = 0; i < AF_ROWS; ++i) {
+        for (int j = 0; j < AF_KEYS; ++j) sc[0][j] = sp[tx + AF_TX * j];
+      }
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i) {
         float s[AF_KEYS], mx = -INFINITY;
 #pragma unroll
         for (int j = 0; j < AF_KEYS; ++j) {
@@ -633,7 +645,8 @@ attn_f32_kernel(const float* __restrict__ q, int64_t q_row_stride, float* __rest
 #pragma unroll
         for (int j = 0; j < AF_KEYS; ++j) {
           const float p = any ? expf(s[j] - mn) : 0.0f;        // exp(-inf) = 0
-          sp[(ty + TY * i) * AF_P_PITCH + tx + AF_TX * j] = p;
+          if (!ONE) sp[(ty + TY * i) * AF_P_PITCH + tx + AF_TX * j] = p;
+          else if (j == ty) sp[AF_P_PITCH + tx + AF_TX * j] = p;
           sum += p;
         }
 #pragma unroll
@@ -650,26 +663,26 @@ attn_f32_kernel(const float* __restrict__ q, int64_t q_row_stride, float* __rest
       }
       af_wait<1>();
       __syncthreads();                                         // V of this page and P are here
-      const float* pr = sp + ty * AF_P_PITCH;
+      const float* pr = sp + (ONE ? 1 : ty) * AF_P_PITCH;
       const float* vr = sv + tx * 4;
       int all = AF_PAGE, most = 0;                             // keys that every row of this thread sees, that some does
 #pragma unroll
-      for (int i = 0; i < AF_ROWS; ++i) {
+      for (int i = 0; i < ROWS; ++i) {
         all = min(all, hi[i] - base);
         most = max(most, hi[i] - base);
       }
 #pragma unroll 1
-      for (int c0 = 0; c0 < AF_PAGE && c0 < most; c0 += AF_CHAIN / 2) {
-        unsigned long long pv[AF_ROWS][VQ][2];
+      for (int c0 = ONE ? ty * (AF_CHAIN / 2) : 0; c0 < AF_PAGE && c0 < most; c0 += ONE ? AF_PAGE : AF_CHAIN / 2) {
+        unsigned long long pv[ROWS][VQ][2];
 #pragma unroll
-        for (int i = 0; i < AF_ROWS; ++i)
+        for (int i = 0; i < ROWS; ++i)
 #pragma unroll
           for (int v = 0; v < VQ; ++v) pv[i][v][0] = pv[i][v][1] = 0;
 #pragma unroll 1
         for (int j0 = c0; j0 < c0 + AF_CHAIN / 2; j0 += 4) {
-          float4 p4[AF_ROWS];
+          float4 p4[ROWS];
 #pragma unroll
-          for (int i = 0; i < AF_ROWS; ++i) p4[i] = *reinterpret_cast<const float4*>(pr + i * TY * AF_P_PITCH + j0);
+          for (int i = 0; i < ROWS; ++i) p4[i] = *reinterpret_cast<const float4*>(pr + i * TY * AF_P_PITCH + j0);
           const bool some = j0 + 4 > all;                      // a key that a row does not see must not touch it,
 #pragma unroll                                                 // whatever its value holds
           for (int jj = 0; jj < 4; ++jj) {
@@ -677,7 +690,7 @@ attn_f32_kernel(const float* __restrict__ q, int64_t q_row_stride, float* __rest
             for (int v = 0; v < VQ; ++v) {
               const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(vr + (j0 + jj) * HD + v * 64);
 #pragma unroll
-              for (int i = 0; i < AF_ROWS; ++i) {
+              for (int i = 0; i < ROWS; ++i) {
                 const float p = jj == 0 ? p4[i].x : (jj == 1 ? p4[i].y : (jj == 2 ? p4[i].z : p4[i].w));
                 const unsigned long long pp = af_pair(p, p);
                 if (!some || base + j0 + jj < hi[i]) {
@@ -689,22 +702,36 @@ attn_f32_kernel(const float* __restrict__ q, int64_t q_row_stride, float* __rest
           }
         }
 #pragma unroll
-        for (int i = 0; i < AF_ROWS; ++i)
+        for (int i = 0; i < ROWS; ++i)
 #pragma unroll
           for (int v = 0; v < VQ; ++v)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
               const float2 a = af_split(acc[i][v][e]), x = af_split(pv[i][v][e]);
-              acc[i][v][e] = af_pair(a.x + x.x, a.y + x.y);
+              if (ONE && ty > 0) *reinterpret_cast<float2*>(sq + ty * QP + v * 64 + tx * 4 + e * 2) = x;
+              else acc[i][v][e] = af_pair(a.x + x.x, a.y + x.y);
             }
       }
       __syncthreads();                                         // V and P have been read
+      if (ONE && ty == 0) {
+#pragma unroll
+        for (int c = 1; c < TY; ++c) {                         // the other groups' chains, in order
+          if (c * (AF_CHAIN / 2) >= most) break;
+#pragma unroll
+          for (int v = 0; v < VQ; ++v) {
+            const float4 x = *reinterpret_cast<const float4*>(sq + c * QP + v * 64 + tx * 4);
+            const float2 a = af_split(acc[0][v][0]), b = af_split(acc[0][v][1]);
+            acc[0][v][0] = af_pair(a.x + x.x, a.y + x.y);
+            acc[0][v][1] = af_pair(b.x + x.z, b.y + x.w);
+          }
+        }
+      }
       fetch(v_pool, sv, HD, page + 1);
     }
     af_wait<0>();
   }
 #pragma unroll
-  for (int i = 0; i < AF_ROWS; ++i) {
+  for (int i = 0; i < ROWS; ++i) {
     const int r = ty + TY * i;
     if (r >= rows) continue;
     const int64_t at = (int64_t)(t0 + r / G) * nh + g * G + r % G;
@@ -724,24 +751,24 @@ attn_f32_kernel(const float* __restrict__ q, int64_t q_row_stride, float* __rest
   }
 }
 
-template <int HD, int TY>
+template <int HD, int TY, int ROWS, bool ONE>
 static int launch_f32(const float* q, int64_t q_row_stride, float* out, const float* k_pool, const float* v_pool,
                       const int* block_table, int bt_stride, const int* tok_pos, const int* tok_seq, const int* row_start,
                       const int* tile_seq, const int* tile_q0, int n_tiles, int T_, int nh, int nkv, float scale,
                       int split_keys, int max_splits, float* scratch, cudaStream_t stream) {
-  const size_t smem = af_smem_floats<HD, TY>() * sizeof(float);
+  const size_t smem = af_smem_floats<HD, TY, ROWS>() * sizeof(float);
   if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(attn_f32_kernel<HD, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(attn_f32_kernel<HD, TY, ROWS, ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) {
       set_error("attn_f32: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
       return (int)e;
     }
   }
-  const int tile_tokens = tile_seq ? min(128, AF_ROWS * TY / (nh / nkv)) : 1;
+  const int tile_tokens = tile_seq ? min(128, ROWS * TY / (nh / nkv)) : 1;
   const int sub = ceil_div(128, tile_tokens);
   if (max_splits > 1) scratch += ATT_COUNTER_SLOTS;            // the counters' part stays as it is
   const dim3 grid(tile_seq ? n_tiles * sub : T_, nkv, max_splits);
-  launch_pdl(attn_f32_kernel<HD, TY>, grid, dim3(AF_TX * TY), smem, stream, q, q_row_stride, out, k_pool, v_pool,
+  launch_pdl(attn_f32_kernel<HD, TY, ROWS, ONE>, grid, dim3(AF_TX * TY), smem, stream, q, q_row_stride, out, k_pool, v_pool,
              block_table, bt_stride, tok_pos, tok_seq, row_start, tile_seq, tile_q0, sub, tile_tokens, nh, nkv, scale,
              split_keys, max_splits, scratch);
   int rc = launch_status("attn_f32");
@@ -870,8 +897,9 @@ extern "C" int exl3_attn_f32(const float* q, int64_t q_row_stride, float* out, c
     return ERR_BAD_ARGUMENT;
   }
   if (nkv > 65535 || max_splits > 65535) { set_error("attn_f32: grid too large"); return ERR_UNSUPPORTED; }
-  if (!aligned16(q) || !aligned16(k_pool) || !aligned16(v_pool) || !aligned16(out) || q_row_stride % 4 != 0) {
-    set_error("attn_f32: q, k, v and out must be 16-byte aligned with a row stride in 16-byte units");
+  if (!aligned16(q) || !aligned16(k_pool) || !aligned16(v_pool) || (reinterpret_cast<uintptr_t>(out) & 7u) != 0 ||
+      q_row_stride % 4 != 0) {
+    set_error("attn_f32: q, k and v must be 16-byte aligned with a row stride in 16-byte units, out 8-byte aligned");
     return ERR_ALIGNMENT;
   }
   if (exl3_attn_tokens_scratch_bytes(T, nh, hd, max_splits) > scratch_bytes) {
@@ -879,16 +907,20 @@ extern "C" int exl3_attn_f32(const float* q, int64_t q_row_stride, float* out, c
               exl3_attn_tokens_scratch_bytes(T, nh, hd, max_splits));
     return ERR_SCRATCH;
   }
-  // single tokens with up to 16 query heads a kv head fill a quarter of the larger block's rows
-  const bool small = tile_seq == nullptr && nh / nkv <= 16;
-#define EXL3_AF(HD, TY)                                                                                            \
-  return launch_f32<HD, TY>(q, q_row_stride, out, k_pool, v_pool, block_table, bt_stride, tok_pos, tok_seq, row_start, \
-                            tile_seq, tile_q0, n_tiles, T, nh, nkv, scale, split_keys, max_splits, scratch, stream)
-  if (hd == 64) {
-    if (small) EXL3_AF(64, 4);
-    EXL3_AF(64, 16);
-  }
-  if (small) EXL3_AF(128, 4);
-  EXL3_AF(128, 16);
+  // rows of a block: the query heads of a single token, 64 of a tile's
+  const int rows = tile_seq == nullptr ? nh / nkv : 64;
+#define EXL3_AF(HD, TY, ROWS, ONE)                                                                                       \
+  return launch_f32<HD, TY, ROWS, ONE>(q, q_row_stride, out, k_pool, v_pool, block_table, bt_stride, tok_pos, tok_seq,   \
+                                       row_start, tile_seq, tile_q0, n_tiles, T, nh, nkv, scale, split_keys, max_splits, \
+                                       scratch, stream)
+#define EXL3_AF_ROWS(HD)                      \
+  if (rows == 1) EXL3_AF(HD, 4, 1, true);     \
+  if (rows <= 4) EXL3_AF(HD, 4, 1, false);    \
+  if (rows <= 8) EXL3_AF(HD, 4, 2, false);    \
+  if (rows <= 16) EXL3_AF(HD, 4, 4, false);   \
+  EXL3_AF(HD, 16, 4, false)
+  if (hd == 64) { EXL3_AF_ROWS(64); }
+  EXL3_AF_ROWS(128);
+#undef EXL3_AF_ROWS
 #undef EXL3_AF
 }

@@ -504,6 +504,25 @@ def attn_f32_supported(dtype: torch.dtype, heads: int, kv_heads: int, head_dim: 
             and heads // kv_heads <= 64)
 
 
+def attn_f32_by_tiles(T: int, n_tiles: int, heads: int, kv_heads: int, head_dim: int, split_keys: int, max_kv_len: int) -> bool:
+    """Whether a step of ``T`` new tokens in ``n_tiles`` tiles of 128 runs faster by tiles than with every token by itself
+    (same bits).  Both sides' time is the larger of a chunk's pages one after the other (3 to 6 us each for a token, 14 for
+    a block of 64 rows) and all pages over what the GPU does a us.  Measured, alone / by tiles, us: 36 heads of 64, a row
+    of 2 tokens at 1,000 12 / 56, eight rows of 16 at 300 95 / 78, 31 rows of 1 and one of 64 at 500 118 / 417, two of 300 275 /
+    93; 32 heads on 8 of 128, eight rows of 16 at 300 76 / 64, two of 300 216 / 129."""
+    group = heads // kv_heads
+    wide = head_dim > 64
+    # pages a us: single tokens by the rows of their block, tiles
+    rate = next(r for g, r in ((1, 87 if wide else 178), (4, 50 if wide else 102), (8, 50 if wide else 79), (16, 20 if wide else 40),
+                               (64, 8 if wide else 17)) if group <= g)
+    pages = (max_kv_len + 63) // 64
+    chunk = min(pages, split_keys // 64)
+    blocks = max(n_tiles, -(-T // min(128, 64 // group)))
+    alone = max((6.0 if wide else 4.0) * chunk, T * kv_heads * pages / rate)
+    tiles = max(14.0 * chunk, blocks * kv_heads * pages / (8 if wide else 17))
+    return tiles < alone
+
+
 def attn_f32(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, k_pool: torch.Tensor, v_pool: torch.Tensor,
              block_table: torch.Tensor, tok_pos: torch.Tensor, tok_seq: torch.Tensor, T: int, heads: int,
              kv_heads: int, head_dim: int, scale: float, split_keys: int, max_splits: int,

@@ -192,11 +192,19 @@ class Attention:
         scratch = None
         if n > 1:
             scratch = batch.workspace.floats(K.attn_tokens_scratch_bytes(T, s.heads, s.head_dim, n) // 4)
-        if K.attn_f32_supported(qkv.dtype, s.heads, s.kv_heads, s.head_dim, kv.page_size, s.window):
-            # float32 without a window: a page of keys at a time as two products of tiles
+        if (K.attn_f32_supported(qkv.dtype, s.heads, s.kv_heads, s.head_dim, kv.page_size, s.window)
+                and out.data_ptr() % 8 == 0):
+            # float32 without a window: a page of keys at a time as two products of tiles, by tiles of new tokens where
+            # these are full enough
+            tiles = batch.tiles.get(128) if batch.max_new > 1 else None
+            if tiles is not None:
+                key = ("attn_f32_by_tiles", s.heads, s.kv_heads, s.head_dim)
+                if key not in batch.memo:
+                    batch.memo[key] = K.attn_f32_by_tiles(T, tiles[2], s.heads, s.kv_heads, s.head_dim, split, batch.max_kv_len)
+                if not batch.memo[key]:
+                    tiles = None
             K.attn_f32(qkv, qkv.stride(0), out, kv.k, kv.v, kv.block_table, batch.tok_pos, batch.tok_seq, T, s.heads,
-                       s.kv_heads, s.head_dim, self.scale, split, n, scratch, row_start=batch.row_start,
-                       tiles=batch.tiles.get(128) if batch.max_new > 1 else None)
+                       s.kv_heads, s.head_dim, self.scale, split, n, scratch, row_start=batch.row_start, tiles=tiles)
             return
         K.attn_tokens(qkv, qkv.stride(0), out, kv.k, kv.v, kv.block_table, batch.tok_pos, batch.tok_seq, T,
                       s.heads, s.kv_heads, s.head_dim, kv.page_size, s.window, self.scale, split, n, scratch)

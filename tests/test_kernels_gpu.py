@@ -117,7 +117,9 @@ def test_gemm_simt_edges(M, N, Kd):
 # Tiles of several tokens against single tokens bit by bit, and both against 64 bits; places that no query may see hold NaN.
 @pytest.mark.parametrize("nh,nkv,hd,counts,starts", [(16, 2, 64, [90, 130, 1], [0, 0, 63]), (6, 2, 64, [70], [600]),
                                                      (5, 5, 128, [257, 3], [0, 255]), (40, 1, 64, [3, 1], [33, 500]),
-                                                     (64, 1, 128, [65], [0]), (32, 2, 64, [1, 1, 1], [0, 64, 256])])
+                                                     (64, 1, 128, [65], [0]), (32, 2, 64, [1, 1, 1], [0, 64, 256]),
+                                                     (3, 3, 64, [70, 1, 40], [0, 511, 250]), (8, 2, 128, [20, 50], [300, 0]),
+                                                     (7, 1, 128, [33], [31]), (18, 2, 64, [9, 1], [60, 129])])
 def test_attn_f32(nh, nkv, hd, counts, starts):
     g = torch.Generator(device=DEV).manual_seed(nh + hd)
     B, T, page, split = len(counts), sum(counts), 64, 256

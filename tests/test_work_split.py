@@ -99,3 +99,14 @@ def test_wide_groups_in_a_block_go_to_two_warps_per_ring():
     assert mixer(12, 1, 64)._decode_twins(1, 1) == (2, 2)
     assert mixer(36, 36, 64)._decode_twins(1, 2) == (1, 1)
     assert mixer(22, 2, 64)._decode_twins(1, 1) == (1, 1)      # 11 heads do not halve
+
+
+def test_float32_steps_of_few_tokens_run_token_by_token():
+    """Tiles of 64 rows are for prompts: a few new tokens a row, or mostly single ones, run faster one by one."""
+    from exl3_server_b200.ops.kernels import attn_f32_by_tiles as by_tiles
+    for heads, kv_heads, hd in ((36, 36, 64), (16, 16, 128), (32, 8, 64), (32, 8, 128), (16, 2, 64), (16, 1, 64), (24, 1, 64)):
+        assert not by_tiles(2, 1, heads, kv_heads, hd, 256, 1000)
+        assert not by_tiles(16, 8, heads, kv_heads, hd, 256, 300)
+        assert not by_tiles(95, 32, heads, kv_heads, hd, 256, 600)
+        assert by_tiles(4096, 32, heads, kv_heads, hd, 256, 4096)
+    assert by_tiles(128, 8, 36, 36, 64, 256, 316) and by_tiles(600, 6, 32, 8, 128, 256, 300)
