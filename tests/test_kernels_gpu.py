@@ -114,6 +114,21 @@ def test_gemm_simt_edges(M, N, Kd):
     assert torch.equal(K().gemm_simt(x, w[n:n + 1].contiguous(), b[n:n + 1].contiguous(), torch.float32)[:, 0], got[:, n])
 
 
+# Element by element: bfloat16, and float32 rows that are not on 16 bytes, around tiles, pieces and the stages asked for ahead.
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("M,N,Kd", [(1, 1, 1), (65, 63, 7), (3, 130, 9), (64, 65, 255), (129, 64, 385), (17, 70, 1030)])
+def test_gemm_simt_element_by_element(dtype, M, N, Kd):
+    g = torch.Generator(device=DEV).manual_seed(M * 31 + Kd)
+    x, w = (torch.randn(n * Kd + 1, device=DEV, generator=g).to(dtype)[1:].view(n, Kd) for n in (M, N))
+    b = torch.randn(N, device=DEV, generator=g).to(dtype)
+    got = K().gemm_simt(x, w, b, torch.float32)
+    bound = (Kd / 32 + 24) * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T + b.double().abs())
+    assert bool(((got.double() - x.double() @ w.double().T - b.double()).abs() <= bound).all())
+    assert torch.equal(K().gemm_simt(x[M // 2:M // 2 + 1].contiguous(), w, b, torch.float32)[0], got[M // 2])
+    if dtype == torch.float32:                           # 16-byte rows give the same bits
+        assert torch.equal(K().gemm_simt(x.clone(), w.clone(), b, torch.float32), got)
+
+
 # Tiles of several tokens against single tokens bit by bit, and both against 64 bits; places that no query may see hold NaN.
 @pytest.mark.parametrize("nh,nkv,hd,counts,starts", [(16, 2, 64, [90, 130, 1], [0, 0, 63]), (6, 2, 64, [70], [600]),
                                                      (5, 5, 128, [257, 3], [0, 255]), (40, 1, 64, [3, 1], [33, 500]),
