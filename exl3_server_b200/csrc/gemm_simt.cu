@@ -15,6 +15,7 @@
 // error against 64 bits is 2.1e-7, not 1.1e-6.)
 #include "api.h"
 #include "common.cuh"
+#include <algorithm>
 
 namespace exl3 {
 
@@ -45,28 +46,35 @@ __device__ inline float gs_both(unsigned long long acc) {
   return lo + hi;
 }
 
-// Many rows: a block has a tile of 64 x 64 outputs, and each of its four groups of 128 threads (8 x 4 outputs a thread) a
-// quarter of the lanes: the groups walk different pieces of K with rings and barriers of their own, and meet once at the
+// Many rows: a block has a tile of 64 x 64 outputs, and (SPLIT 4) each of its four groups of 128 threads (8 x 4 outputs a
+// thread) a quarter of the lanes: the groups walk different pieces of K with rings and barriers of their own, and meet once at the
 // end.  So a narrow output (1,024 columns at some hundred rows: fewer tiles than SMs) still has sixteen warps an SM.  The
-// sums of finished lanes wait in shared memory, which leaves the registers to the pairs of accumulators.
+// sums of finished lanes wait in shared memory, which leaves the registers to the pairs of accumulators.  With many tiles, or
+// with K too short for all lanes, a block has one group that walks all of them (SPLIT 1), four blocks an SM, whose starts and ends
+// run beside one another: 2,000 x 8,192 (rows, columns) x 64 88 us (four groups 142; one accumulator over K 103), x 1,024 928 (976).
 // Bound by the fma pipe and by what shared memory returns (12 reads of 8 bytes a lane, 128 bytes a cycle, for 32 paired fma)
 // about equally: 525 x 8,192 x 1,024 (rows, columns, K) 278 us, 32 TFLOP/s; 525 x 1,024 x 4,096 130 us (one accumulator and 4 x 4
 // outputs a thread, an element a load: 442 and 390 us; this kernel with scalar fma and the lanes' sums in registers 302 and 140).
-constexpr int GT_TILE = 64, GT_STAGES = 4, GT_GROUP = 128, GT_THREADS = GS_GROUPS * GT_GROUP;
+constexpr int GT_TILE = 64, GT_GROUP = 128;
 constexpr int GT_PITCH = GS_PIECE + 4;               // floats; rows 48 bytes apart: the reads of 8 rows do not collide
 constexpr int GT_STAGE_FLOATS = 2 * GT_TILE * GT_PITCH;
 constexpr int GT_OUT_PITCH = GT_TILE + 8;
-constexpr int GT_RING_FLOATS = GS_GROUPS * GT_STAGES * GT_STAGE_FLOATS;
-constexpr int GT_SMEM = (GT_RING_FLOATS + GT_THREADS * 32) * 4;
-static_assert(GS_GROUPS * GT_TILE * GT_OUT_PITCH <= GT_RING_FLOATS, "the groups' sums go where the rings were");
+// SPLIT: groups of threads in a block, GS_GROUPS or 1.
+template <int SPLIT> constexpr int gt_stages() { return SPLIT == 1 ? 3 : 4; }
+template <int SPLIT> constexpr int gt_ring_floats() { return SPLIT * gt_stages<SPLIT>() * GT_STAGE_FLOATS; }
+template <int SPLIT> constexpr int gt_smem() {                // the ring, sums of lanes, with one group also sums of groups
+  return (gt_ring_floats<SPLIT>() + (SPLIT == 1 ? 2 : SPLIT) * GT_GROUP * 32) * 4;
+}
+static_assert(GS_GROUPS * GT_TILE * GT_OUT_PITCH <= gt_ring_floats<GS_GROUPS>(), "the groups' sums go where the rings were");
 
 // VEC: float32, K % 4 == 0 and 16-byte aligned operands (16-byte asynchronous copies); else element by element, the loads of a
 // stage in registers while the stage before is worked on: 1,000 x 8,192 x 1,020 in bfloat16 616 us, x 1,023 in float32 616
 // (one accumulator in blocks of 64 x 64 765 and 762; every load waited for before the stage, two threads a row, 968 and 922).
-template <typename TI, typename TO, bool VEC>
-__global__ void __launch_bounds__(GT_THREADS, 1)
+template <typename TI, typename TO, bool VEC, int SPLIT>
+__global__ void __launch_bounds__(SPLIT * GT_GROUP, SPLIT == 1 ? 4 : 1)
 gemm_simt_kernel(const TI* __restrict__ x, const TI* __restrict__ w, const TI* __restrict__ bias,
                  TO* __restrict__ y, int M, int N, int K) {
+  constexpr int THREADS = SPLIT * GT_GROUP, STAGES = gt_stages<SPLIT>(), GROUP_LANES = GS_LANES / SPLIT;
   extern __shared__ __align__(16) float gt_smem[];
   pdl_wait();
   pdl_trigger();
@@ -74,10 +82,11 @@ gemm_simt_kernel(const TI* __restrict__ x, const TI* __restrict__ w, const TI* _
   // a warp has 4 x 8 threads: its reads of x are four rows, of w eight, a wavefront each
   const int tx = (t & 7) + (t >> 6) * 8, ty = ((t >> 3) & 3) + ((t >> 5) & 1) * 4;
   const int m0 = blockIdx.y * GT_TILE, n0 = blockIdx.x * GT_TILE;
-  float* ring = gt_smem + g * GT_STAGES * GT_STAGE_FLOATS;
-  float4* sums = reinterpret_cast<float4*>(gt_smem + GT_RING_FLOATS) + threadIdx.x;    // [8][threads], this thread's own
+  float* ring = gt_smem + g * STAGES * GT_STAGE_FLOATS;
+  float4* sums = reinterpret_cast<float4*>(gt_smem + gt_ring_floats<SPLIT>()) + threadIdx.x;   // [8][threads], this thread's own
+  float4* totals = sums + 8 * THREADS;                        // the same of finished groups of lanes (SPLIT 1)
   const int pieces = (K + GS_PIECE - 1) / GS_PIECE;
-  const int first_lane = g * GS_GROUP_LANES, last_lane = first_lane + GS_GROUP_LANES;
+  const int first_lane = g * GROUP_LANES, last_lane = first_lane + GROUP_LANES;
 
   // One stage: one piece of the 64 rows of x and of w.  16 bytes a thread and operand, half a row, asynchronously; or, element by
   // element, a feature of every sixteenth row (a warp's loads then share their sectors), asked for before the stage in hand is
@@ -125,12 +134,12 @@ gemm_simt_kernel(const TI* __restrict__ x, const TI* __restrict__ w, const TI* _
     return more;
   };
   {
-    Ahead v[GT_STAGES - 1];
-    bool some[GT_STAGES - 1];
+    Ahead v[STAGES - 1];
+    bool some[STAGES - 1];
 #pragma unroll
-    for (int s = 0; s < GT_STAGES - 1; ++s) some[s] = fill_next(s, v[s]);
+    for (int s = 0; s < STAGES - 1; ++s) some[s] = fill_next(s, v[s]);
 #pragma unroll
-    for (int s = 0; s < GT_STAGES - 1; ++s)
+    for (int s = 0; s < STAGES - 1; ++s)
       if (!VEC && some[s]) put(v[s], s);
   }
 
@@ -138,21 +147,21 @@ gemm_simt_kernel(const TI* __restrict__ x, const TI* __restrict__ w, const TI* _
   const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    sums[i * GT_THREADS] = zero;
+    if (SPLIT > 1) sums[i * THREADS] = zero;
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = 0;
   }
   int slot = 0;
   for (int lane = first_lane; lane < last_lane && lane < pieces; ++lane) {
     for (int q = lane; q < pieces; q += GS_LANES) {
-      if (VEC) gs_wait<GT_STAGES - 2>();
+      if (VEC) gs_wait<STAGES - 2>();
       asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");
-      const int last = slot == 0 ? GT_STAGES - 1 : slot - 1;  // the slot that was read last
+      const int last = slot == 0 ? STAGES - 1 : slot - 1;  // the slot that was read last
       Ahead v;
       const bool some = fill_next(last, v);
       const float* a = ring + slot * GT_STAGE_FLOATS + ty * GT_PITCH;
       const float* b = ring + slot * GT_STAGE_FLOATS + (GT_TILE + tx) * GT_PITCH;
-      slot = slot + 1 == GT_STAGES ? 0 : slot + 1;
+      slot = slot + 1 == STAGES ? 0 : slot + 1;
 #pragma unroll
       for (int h = 0; h < GS_PIECE / 2; ++h) {
         unsigned long long av[8];
@@ -167,26 +176,47 @@ gemm_simt_kernel(const TI* __restrict__ x, const TI* __restrict__ w, const TI* _
       }
       if (!VEC && some) put(v, last);
     }
+    // a lane is finished: to its group's sum, and with one group of threads a finished group's to the total
+    const bool first = SPLIT == 1 && lane % GS_GROUP_LANES == 0;
+    const bool ends = SPLIT == 1 && (lane % GS_GROUP_LANES == GS_GROUP_LANES - 1 || lane + 1 >= pieces);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      float4 v = sums[i * GT_THREADS];
+      float4 v = first ? zero : sums[i * THREADS];
       v.x += gs_both(acc[i][0]); v.y += gs_both(acc[i][1]); v.z += gs_both(acc[i][2]); v.w += gs_both(acc[i][3]);
-      sums[i * GT_THREADS] = v;
+      if (ends && lane >= GS_GROUP_LANES) {
+        const float4 u = totals[i * THREADS];
+        v.x = u.x + v.x; v.y = u.y + v.y; v.z = u.z + v.z; v.w = u.w + v.w;
+      }
+      (ends ? totals : sums)[i * THREADS] = v;
 #pragma unroll
       for (int j = 0; j < 4; ++j) acc[i][j] = 0;
     }
   }
   if (VEC) gs_wait<0>();
+  if constexpr (SPLIT == 1) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int m = m0 + ty + 8 * i;
+      const float4 v4 = totals[i * THREADS];
+      const float v[4] = {v4.x, v4.y, v4.z, v4.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int n = n0 + tx + 16 * j;
+        if (m < M && n < N) Elem<TO>::store(y + (int64_t)m * N + n, bias ? v[j] + Elem<TI>::load(bias + n) : v[j]);
+      }
+    }
+    return;
+  }
   __syncthreads();                                            // every ring has been read
   float* mine = gt_smem + g * GT_TILE * GT_OUT_PITCH + ty * GT_OUT_PITCH + tx;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const float4 v = sums[i * GT_THREADS];
+    const float4 v = sums[i * THREADS];
     float* o = mine + 8 * i * GT_OUT_PITCH;
     o[0] = v.x; o[16] = v.y; o[32] = v.z; o[48] = v.w;
   }
   __syncthreads();
-  for (int idx = threadIdx.x; idx < GT_TILE * GT_TILE; idx += GT_THREADS) {
+  for (int idx = threadIdx.x; idx < GT_TILE * GT_TILE; idx += THREADS) {
     const int r = idx >> 6, c = idx & 63;
     if (m0 + r >= M || n0 + c >= N) continue;
     const float* p = gt_smem + r * GT_OUT_PITCH + c;
@@ -343,16 +373,41 @@ static int gs_allow_smem(Kern kernel, size_t smem) {
   return 0;
 }
 
-template <typename TI, typename TO, bool VEC>
-static int launch(const void* x, const void* w, const void* bias, void* y, int M, int N, int K,
-                  cudaStream_t stream) {
-  dim3 grid(ceil_div(N, GT_TILE), ceil_div(M, GT_TILE));
+// The three kernels give the same bits, so a call takes the one that models of their times, fitted to 1,304 sizes (K of 4 to 4,096, 8
+// to 32,000 columns, 1 to 2,000 rows), call the fastest.  In us, streamed / tiles of four groups / of one: 300 rows x 1,024 columns,
+// K 4,096: 110 / 131 / 200; 300 x 8,192, K 64: 160 / 27 / 20; 8 x 8,192, K 64: 10 / 6.5 / 6.9; 2,000 x 8,192, K 64: - / 142 / 88,
+// K 1,024: - / 976 / 928.
+
+// Tiles: with four groups of lanes a wave is one tile an SM; with one group up to four tiles an SM share what one of them would
+// have alone (whole waves after one another, or the last one by how many an SM gets).
+static double gs_tiles_us(int M, int N, int K, bool vec, int split) {
+  const double tiles = (double)ceil_div(M, GT_TILE) * ceil_div(N, GT_TILE), sms = gs_sm_count();
+  if (split > 1)
+    return 1.0 + ceil(tiles / sms) * (vec ? std::min(2.0 + 0.047 * K, 3.5 + 0.0305 * K) : std::min(2.6 + 0.085 * K, 4.6 + 0.039 * K));
+  const double full = vec ? 2.6 + 0.127 * K : std::min(2.5 + 0.19 * K, 8.9 + 0.1465 * K);
+  const double alone = vec ? std::min(1.9 + 0.075 * K, 5.4 + 0.048 * K) : std::min(2.4 + 0.0945 * K, 6.0 + 0.067 * K);
+  const double start = vec ? std::min(4.4, 0.6 + 0.06 * K) : 2.5, waves = floor(tiles / (4 * sms));
+  const int an_sm = (int)ceil((tiles - waves * 4 * sms) / sms);
+  return waves * full + (an_sm == 0 ? 0.0 : std::max(alone, an_sm == 1 ? 0.0 : (0.1 + 0.25 * an_sm) * full + start));
+}
+
+template <typename TI, typename TO, bool VEC, int SPLIT>
+static int launch_tiles(const void* x, const void* w, const void* bias, void* y, int M, int N, int K, cudaStream_t stream) {
+  const dim3 grid(ceil_div(N, GT_TILE), ceil_div(M, GT_TILE));
   if (grid.y > 65535) { set_error("gemm_simt: M=%d is too large", M); return ERR_UNSUPPORTED; }
-  int rc = gs_allow_smem(gemm_simt_kernel<TI, TO, VEC>, GT_SMEM);
+  auto kernel = gemm_simt_kernel<TI, TO, VEC, SPLIT>;
+  int rc = gs_allow_smem(kernel, gt_smem<SPLIT>());
   if (rc) return rc;
-  launch_pdl(gemm_simt_kernel<TI, TO, VEC>, grid, dim3(GT_THREADS), GT_SMEM, stream, static_cast<const TI*>(x),
+  launch_pdl(kernel, grid, dim3(SPLIT * GT_GROUP), gt_smem<SPLIT>(), stream, static_cast<const TI*>(x),
              static_cast<const TI*>(w), static_cast<const TI*>(bias), static_cast<TO*>(y), M, N, K);
   return launch_status("gemm_simt");
+}
+
+template <typename TI, typename TO, bool VEC>
+static int launch(const void* x, const void* w, const void* bias, void* y, int M, int N, int K, cudaStream_t stream) {
+  return gs_tiles_us(M, N, K, VEC, 1) < gs_tiles_us(M, N, K, VEC, GS_GROUPS)
+             ? launch_tiles<TI, TO, VEC, 1>(x, w, bias, y, M, N, K, stream)
+             : launch_tiles<TI, TO, VEC, GS_GROUPS>(x, w, bias, y, M, N, K, stream);
 }
 
 template <int MR, int R, int U, bool V8>
@@ -367,24 +422,32 @@ static int launch_few(const float* x, const float* w, const float* bias, float* 
   return launch_status("gemm_simt_few");
 }
 
+// Rows of w a half warp: as many as leave every SM eight warps, so that the reads of x are shared.
+static int gs_few_w_rows(int M, int N, int MR) {
+  const int rows_an_sm = N / gs_sm_count() * ceil_div(M, MR);
+  return rows_an_sm >= 64 ? 4 : rows_an_sm >= 32 ? 2 : 1;
+}
+static int gs_few_x_rows(int M) { return M <= 2 ? M : M <= 4 ? 4 : 8; }
+
 template <int MR, bool V8>
 static int launch_few_rows(const float* x, const float* w, const float* bias, float* y, int M, int N, int K,
                            cudaStream_t stream) {
-  // rows of w a half warp: as many as leave every SM eight warps, so that the reads of x are shared
-  const int rows_an_sm = N / gs_sm_count() * ceil_div(M, MR);
-  if (rows_an_sm >= 64) return launch_few<MR, 4, 2, V8>(x, w, bias, y, M, N, K, stream);
-  if (rows_an_sm >= 32) return launch_few<MR, 2, 4, V8>(x, w, bias, y, M, N, K, stream);
-  return launch_few<MR, 1, 8, V8>(x, w, bias, y, M, N, K, stream);
+  switch (gs_few_w_rows(M, N, MR)) {
+    case 4: return launch_few<MR, 4, 2, V8>(x, w, bias, y, M, N, K, stream);
+    case 2: return launch_few<MR, 2, 4, V8>(x, w, bias, y, M, N, K, stream);
+    default: return launch_few<MR, 1, 8, V8>(x, w, bias, y, M, N, K, stream);
+  }
 }
 
-// Which of the two kernels: where M is large both go by the fma they do, the tiles for whole waves of 64 x 64 tiles, the
-// streaming kernel at 1 / GF_COST of their rate for the rows that there are.  1,024 x 1,024: a wave of tiles 36 us, the
-// streaming kernel 31 us for 300 rows (0.5 of a wave's products); 1,024 x 4,096: 130 us, and 102.
-constexpr double GF_COST = 1.6;
-static bool few_rows(int M, int N, int sms) {
-  const double tiles = (double)ceil_div(M, GT_TILE) * ceil_div(N, GT_TILE);
-  const double waves = (double)(int64_t)((tiles + sms - 1) / sms);
-  return GF_COST * 8.0 * ceil_div(M, 8) * N <= waves * sms * GT_TILE * GT_TILE && M <= 65535;
+// The streaming kernel: a lane's chain over K, or by pairs of a row of w and up to eight of x.
+static double gs_few_us(int M, int N, int K) {
+  const int MR = gs_few_x_rows(M);
+  if (MR < 8) return std::max(1.7 + 0.0007 * sqrt((double)MR) * K, 2.0 + (0.1 * MR + 0.0006 * K) * 1e-3 * N);
+  const double pairs = (double)ceil_div(M, 8) * N, rows_an_sm = pairs / gs_sm_count();
+  const double spread = rows_an_sm >= 128 ? 1.0 : rows_an_sm >= 64 ? 1.6 : rows_an_sm >= 32 || pairs > 8000 ? 1.8 : 2.8;
+  // a pair: whole segments of K, and every eight rows read w again, from L2 while it fits there
+  const double pair = K < GF_SEG ? 0.5 + 0.00012 * K : 0.1 + ((double)N * K > 2.5e7 ? 0.00073 : 0.00053) * GF_SEG * ceil_div(K, GF_SEG);
+  return std::max(std::max(4.6, 1.6 + 0.0035 * K), 2.0 + pair * 1e-3 * spread * pairs);
 }
 
 }  // namespace exl3
@@ -397,7 +460,8 @@ extern "C" int exl3_gemm_simt(const void* x, const void* w, const void* bias, vo
   if (M < 0 || N < 0 || K < 1) { set_error("gemm_simt: bad sizes M=%d N=%d K=%d", M, N, K); return ERR_BAD_ARGUMENT; }
   if (in_dtype == DT_F32 && out_dtype == DT_F32) {
     if (K % 4 != 0 || !aligned16(x) || !aligned16(w)) return launch<float, float, false>(x, w, bias, y, M, N, K, stream);
-    if (!few_rows(M, N, gs_sm_count())) return launch<float, float, true>(x, w, bias, y, M, N, K, stream);
+    if (M > 65535 || gs_few_us(M, N, K) > std::min(gs_tiles_us(M, N, K, true, 1), gs_tiles_us(M, N, K, true, GS_GROUPS)))
+      return launch<float, float, true>(x, w, bias, y, M, N, K, stream);
     const float *xf = static_cast<const float*>(x), *wf = static_cast<const float*>(w), *bf = static_cast<const float*>(bias);
     float* yf = static_cast<float*>(y);
     const bool v8 = K % 8 == 0 && (reinterpret_cast<uintptr_t>(w) & 31u) == 0;

@@ -129,6 +129,19 @@ def test_gemm_simt_element_by_element(dtype, M, N, Kd):
         assert torch.equal(K().gemm_simt(x.clone(), w.clone(), b, torch.float32), got)
 
 
+@pytest.mark.parametrize("M,N,Kd", [(2000, 8192, 1100), (700, 6001, 40), (3000, 64, 260)])
+def test_gemm_simt_tiles_of_one_group(M, N, Kd):
+    """So many tiles that one group of threads walks all lanes of a tile: short and long K, against rows alone."""
+    g = torch.Generator(device=DEV).manual_seed(Kd)
+    x, w = torch.randn(M, Kd, device=DEV, generator=g), torch.randn(N, Kd, device=DEV, generator=g)
+    got = K().gemm_simt(x, w, None, torch.float32)
+    for m in (0, 63, 64, M - 1):
+        assert torch.equal(K().gemm_simt(x[m:m + 1].contiguous(), w, None, torch.float32)[0], got[m])
+    rows = torch.arange(0, M, 97, device=DEV)
+    bound = (Kd / 32 + 24) * 2.0 ** -24 * (x[rows].double().abs() @ w.double().abs().T)
+    assert bool(((got[rows].double() - x[rows].double() @ w.double().T).abs() <= bound).all())
+
+
 # Tiles of several tokens against single tokens bit by bit, and both against 64 bits; places that no query may see hold NaN.
 @pytest.mark.parametrize("nh,nkv,hd,counts,starts", [(16, 2, 64, [90, 130, 1], [0, 0, 63]), (6, 2, 64, [70], [600]),
                                                      (5, 5, 128, [257, 3], [0, 255]), (40, 1, 64, [3, 1], [33, 500]),
