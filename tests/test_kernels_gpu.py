@@ -1519,6 +1519,48 @@ def test_linear_scan_a_row_alone_and_among_others(mode, dtype, off, n):
         assert torch.equal(alone, among)
 
 
+# How rows are cut, against 64 bits: by the step with bfloat16 values (chunks of 128 and 256 with a ragged end, rows beyond 128
+# tokens walked whole), by each row with float32 ones (whole, chunks of 64, of 128, of 192), and rows off 16 bytes (chunks of
+# 64); r and k of their own type, SiLU on the inputs.  Bounds as above.
+@pytest.mark.parametrize("mode,rk_type,v_type,act,H,dv,off,counts", [
+    (0, torch.bfloat16, torch.bfloat16, "none", 16, 64, 0, [2100, 40]), (1, torch.float32, torch.bfloat16, "none", 32, 128, 0, [1500, 300]),
+    (0, torch.bfloat16, torch.bfloat16, "silu", 32, 64, 0, [300] * 6), (1, torch.float32, torch.bfloat16, "silu", 16, 96, 0, [200, 131] * 4),
+    (0, torch.float32, torch.float32, "none", 8, 64, 0, [1100, 130, 100]), (1, torch.float32, torch.float32, "silu", 4, 128, 0, [3000]),
+    (0, torch.bfloat16, torch.bfloat16, "none", 16, 64, 3, [700, 65]), (1, torch.float32, torch.bfloat16, "silu", 16, 64, 3, [300, 129])])
+def test_linear_scan_cuttings(mode, rk_type, v_type, act, H, dv, off, counts):
+    dk, B, T = 64, len(counts), sum(counts)
+    g = torch.Generator(device=DEV).manual_seed(T)
+    draw = lambda d, dt, shift=0.0: (torch.randn(T, H * d + 8, device=DEV, generator=g) - shift).to(dt)[:, off:off + H * d]  # noqa: E731
+    r, k, v, w = draw(dk, rk_type), draw(dk, rk_type), draw(dv, v_type), draw(dk, v_type, 3.0)
+    w0, u = torch.randn(H * dk, device=DEV, generator=g), torch.randn(H * dk, device=DEV, generator=g)
+    decay = 1.0 - 0.1 * torch.rand(H, device=DEV, generator=g)
+    state = torch.randn(B, H, dk, dv, device=DEV, generator=g)
+    S = state.double()
+    starts = [sum(counts[:b]) for b in range(B + 1)]
+    scratch = torch.empty(K().linear_scan_scratch_bytes(B, T, H, dk, dv, max(counts)) // 4, device=DEV)
+    more = dict(wraw=w, w0=w0, u=u) if mode == 0 else dict(decay=decay)
+    got = K().linear_scan(mode, r, k, v, state, torch.arange(B, dtype=torch.int32, device=DEV),
+                          torch.tensor(starts, dtype=torch.int32, device=DEV), B, H, dk, dv, max(counts), scratch=scratch,
+                          in_act=act, **more)
+    rr, kk, vv = (torch.nn.functional.silu(x.double()) if act == "silu" else x.double() for x in (r, k, v))
+    rr, kk, vv = (x.reshape(T, H, -1) for x in (rr, kk, vv))
+    ww, uu = torch.exp(-torch.exp(w.double() + w0.double())).view(T, H, dk, 1), u.double().view(H, dk, 1)
+    want = torch.empty(T, H, dv, dtype=torch.float64, device=DEV)
+    for i in range(max(counts)):                          # the rows side by side
+        rows = [b for b in range(B) if counts[b] > i]
+        at = torch.tensor([starts[b] + i for b in rows], device=DEV)
+        kv, s, q = kk[at][..., None] * vv[at][:, :, None], S[rows], rr[at][..., None]
+        if mode == 0:
+            want[at] = ((s + uu * kv) * q).sum(2)
+            s = ww[at] * s + kv
+        else:
+            s = decay.double().view(H, 1, 1) * s + kv
+            want[at] = (s * q).sum(2)
+        S[rows] = s
+    close(got, want.view(T, H * dv), 2e-5, "outputs")
+    close(state, S, 2e-5, "states")
+
+
 @pytest.mark.parametrize("R,V", [(1, 1), (3, 2048), (8, 2049), (5, 122753)])
 def test_argmax_step(R, V):
     x = torch.randn(R, V, device=DEV)
