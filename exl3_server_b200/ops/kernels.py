@@ -168,7 +168,7 @@ def rope_kv_write(qkv: torch.Tensor, inv_freq: torch.Tensor, rot: int, pos_scale
 
 def gemm_simt(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out_dtype: torch.dtype,
               out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """``x @ w.T (+ bias)`` on the CUDA cores, float32 accumulation in K order."""
+    """``x @ w.T (+ bias)`` on the CUDA cores, float32 accumulation in one order whatever the rows (see gemm_simt.cu)."""
     M, K = x.shape
     N, K2 = w.shape
     if K != K2:
@@ -1195,7 +1195,8 @@ def sample_filtered(logits: torch.Tensor, rows: torch.Tensor, out: Optional[torc
 
 def sample_rows(logits: torch.Tensor, rows: torch.Tensor, counts: torch.Tensor, params: torch.Tensor) -> torch.Tensor:
     """``sample_filtered`` of logits with penalties (``counts`` and ``params`` as ``sample_penalties`` takes them), which
-    are applied as the logits are read: the logits stay as they are.  The chosen tokens join the counts."""
+    are applied as the logits are read: the logits stay as they are.  The chosen tokens join the counts once every row has been
+    drawn, so rows may share their counts."""
     R, V = logits.shape
     if logits.dtype != torch.float32 or rows.dtype != torch.float64 or tuple(rows.shape) != (R, 5) or \
             counts.dtype != torch.int64 or counts.numel() != R or params.dtype != torch.float32 or \
