@@ -19,7 +19,8 @@
 //             bytes, which TMA stores write out (clipped at the matrix's edges), so that no thread stores a
 //             row-strided sliver itself
 // Two accumulators (2 x 256 of the 512 columns) let the epilogue of one tile overlap the products of the next.
-// Pairs are persistent; tiles go round-robin over them, M fastest, so that pairs that run together share w in L2.
+// Pairs are persistent; tiles go round-robin over them, M fastest, so that pairs that run together share w in L2;
+// with an x that L2 does not hold, in groups of rows of tiles (gp_tile, gp_run).
 //
 // Input: x, or a norm's output in two pieces (x_raw = h * w_norm and per-row pieces of sum(h^2)): the accumulator is
 // multiplied by k = rsqrt(sum / width + eps) per row.
@@ -94,6 +95,7 @@ __device__ inline uint4* gp_box_chunk(unsigned char* box, int r, int j) {
 struct PairArgs {
   const __nv_bfloat16* bias;
   int M, N, K;
+  int group;                 // rows of tiles that are walked together (gp_tile)
   const float* ss_in;        // [rows >= M, ss_blocks] or null
   int ss_blocks;
   float eps, width;
@@ -114,6 +116,13 @@ struct PairArgs {
   __nv_bfloat16* k_pool;     // [pages, nkv, 64, 64]
   __nv_bfloat16* v_pool;
 };
+
+// The place of a tile in the order: `group` rows of tiles at a time, within them all columns of tiles, rows fastest.
+struct GpTile { int m, n; };
+__device__ inline GpTile gp_tile(int tile, int n_m, int n_n, int group) {
+  const int first = tile / (group * n_n) * group, rows = min(group, n_m - first), r = tile - first * n_n;
+  return {first + r % rows, r / rows};
+}
 
 template <int EPI>
 __global__ void __launch_bounds__(gp_threads(EPI), 1)
@@ -175,7 +184,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     // ---- producer: this block's halves of the pair's tiles ---------------------------------------------
     uint32_t it = 0;
     for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
-      const int m0 = (tile % n_m) * GP_BM + (int)rank * 128, n0 = (tile / n_m) * GP_BN + (int)rank * 128;
+      const GpTile at = gp_tile(tile, n_m, n_n, a.group);
+      const int m0 = at.m * GP_BM + (int)rank * 128, n0 = at.n * GP_BN + (int)rank * 128;
       for (int kb = 0; kb < kblocks; ++kb, ++it) {
         const int s = it % STAGES;
         if (!mbar_wait(empty + s, ((it / STAGES) & 1) ^ 1)) { ok = false; break; }
@@ -256,7 +266,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     // 2: this warp's 32 rows of a tile of h into accumulator `buf`: divided by rho * k, and the accumulator is then
     // handed to the MMA issuer; or as they are, beside the products.  False when a wait ran out.
     auto preload = [&](int tile, uint32_t buf) -> bool {
-      const int row0 = (tile % n_m) * GP_BM + (int)rank * 128 + q * 32, n0 = (tile / n_m) * GP_BN;
+      const GpTile at = gp_tile(tile, n_m, n_n, a.group);
+      const int row0 = at.m * GP_BM + (int)rank * 128 + q * 32, n0 = at.n * GP_BN;
       const float inv = beside ? 1.0f : 1.0f / (a.rho * row_factor(row0 + lane));
       if (lane == 0) tma_store_wait_read<0>();            // the last epilogue's stores have read the staging tiles
       __syncwarp();
@@ -309,7 +320,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     }
     uint32_t tcount = 0;
     for (int tile = pair; tile < n_tiles; tile += n_pairs, ++tcount) {
-      const int row0 = (tile % n_m) * GP_BM + (int)rank * 128 + q * 32, n0 = (tile / n_m) * GP_BN;
+      const GpTile at = gp_tile(tile, n_m, n_n, a.group);
+      const int row0 = at.m * GP_BM + (int)rank * 128 + q * 32, n0 = at.n * GP_BN;
       const uint32_t buf = tcount & 1;
       const int row = row0 + lane;
       // the tile's bias and norm weights, once for all rows (the previous tile's readers are past their last read:
@@ -510,7 +522,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         }
       }
       if (EPI == 2) {
-        if (row < a.M) a.ss_out[(int64_t)row * n_n + tile / n_m] = sq;
+        if (row < a.M) a.ss_out[(int64_t)row * n_n + at.n] = sq;
         // the accumulator is free: the tile after next of this pair goes into it (or nobody waits for it)
         const int next = tile + 2 * n_pairs;
         fence_before();
@@ -622,6 +634,15 @@ static int gp_run(const void* x, const void* w, const void* bias, void* y, int M
   a.M = M; a.N = N; a.K = K;
   a.ss_in = ss_in; a.ss_blocks = ss_blocks; a.eps = eps; a.width = width;
   const int tiles = ceil_div(M, GP_BM) * ceil_div(N, GP_BN);
+  // Rows of tiles that are walked together.  While x stays in L2 (126 MB, with the weights and what is written beside it)
+  // all of them: each column of w is then read once.  A larger x would be read from memory again for every few columns of
+  // tiles, so it is walked in groups of rows that stay: 64,235 rows x 1,024 columns, K 4,096 (residual) 557 -> 475 us,
+  // x 8,192, K 1,024 (gated) 919 -> 860, 16,000 x 2,304, K 5,760 401 -> 364, 6,145 x 6,144, K 4,096 258 -> 248.  Where w
+  // does not stay either, each group reads it again, so the groups are larger (4,096 x 4,096, K 16,384: 438 us whole and
+  // in twelves, 445 in eights; 6,145 x 28,672, K 4,096: 1,265 whole, 1,242 in twelves).  The sums are the same in any order.
+  const bool x_stays = (int64_t)M * K * 2 <= (40 << 20), w_stays = (int64_t)N * K * 2 <= (64 << 20);
+  a.group = ceil_div(M, GP_BM);
+  if (!x_stays && a.group > (w_stays ? 8 : 12)) a.group = w_stays ? 8 : 12;
   const int max_pairs = gp_max_pairs(epilogue);
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
   cudaLaunchConfig_t cfg;

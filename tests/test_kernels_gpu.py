@@ -550,6 +550,30 @@ def test_gemm_pair_rotates_and_writes_the_cache(lens, starts, nh, nkv, rot):
     assert K().gemm_pair_status() == 0
 
 
+@pytest.mark.parametrize("M,N,Kd", [(5300, 520, 4096),       # x is larger than what stays in L2: rows of tiles in eights, five left over
+                                    (3400, 4200, 8192)])     # and w as well: twelves, two left over
+def test_gemm_pair_walks_rows_of_tiles_in_groups(M, N, Kd):
+    """A large x is walked in groups of rows of tiles: the numbers of the same rows in calls of their own, which are not."""
+    g = torch.Generator().manual_seed(M)
+    x = (torch.randn(M, Kd, generator=g) * 0.5).to(torch.bfloat16).to(DEV)
+    w = (torch.randn(N, Kd, generator=g) / math.sqrt(Kd)).to(torch.bfloat16).to(DEV)
+    got = K().gemm_pair(x, w, None)
+    for a in range(0, M, 1700):
+        assert torch.equal(got[a:a + 1700], K().gemm_pair(x[a:a + 1700], w, None))
+    h0 = torch.randn(M, N, generator=g).to(DEV)
+    nw = torch.ones(N, device=DEV)
+    h = h0.clone()
+    _, ss = K().gemm_pair(x, w, None, resid=(h, 0.37, nw))
+    want = h0.double() + 0.37 * (x.double() @ w.double().T)
+    close(h, want, 2e-5, "residual")                          # as without groups, see above
+    for c in range(ss.shape[1]):
+        # each tile's sum in its own column, of the values that were stored: 256 float32 additions, 2^-24 each
+        part = h[:, 256 * c:256 * c + 256].double()
+        close(ss[:, c], (part * part).sum(1), 256 * 2.0 ** -24, "sums of squares of a tile")
+    torch.cuda.synchronize()
+    assert K().gemm_pair_status() == 0
+
+
 def test_gemm_pair_refuses_what_it_cannot_do():
     from exl3_server_b200.ops.lib import KernelLibraryError
     x = torch.zeros(300, 64, device=DEV).bfloat16()
