@@ -68,6 +68,11 @@ __device__ inline void fa_mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ inline void fa_mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(fa_smem_u32(bar)) : "memory");
 }
+// One arrival for the warp, when all its lanes are here.
+__device__ inline void fa_mbar_arrive_warp(uint64_t* bar) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) fa_mbar_arrive(bar);
+}
 // A bounded wait: mbarrier.try_wait (which the hardware may hold for a while before it answers; a try that
 // cannot succeed came back within a few cycles when measured) in a loop that looks at the clock after every
 // try that failed and gives up FA_WAIT_NS after the first.
@@ -231,6 +236,145 @@ __device__ inline FaTile fa_tile(int tile, const int* block_table, int bt_stride
   return t;
 }
 
+// ---- a row of 64 scores (thread = query row), for all kernels below ------------------------------------------------
+// Cap, distance biases and mask.  p0_warp: the position of the warp's first query.
+__device__ inline void fa_adjust(uint32_t (&sr)[2][32], const FaOpts& opts, int head, int key0, int p, int p_first,
+                                 int p_last, int p0_warp, int window, int chunk) {
+  const bool need_mask = (key0 + FA_BK - 1 > p_first) || (window > 0 && key0 <= p_last - window) ||
+                         (chunk > 0 && key0 < p_last / chunk * chunk);
+  if (opts.cap_in > 0.0f) {                                  // capped scores: tanh now, the cap with the scale below
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int c = 0; c < 32; ++c) sr[h][c] = __float_as_uint(fa_tanh(__uint_as_float(sr[h][c]) * opts.cap_in));
+  }
+  if (opts.dist_len > 0 && fa_near(key0, p0_warp, opts.dist_len)) {
+    // the biases of this row's distances p - key: neighbouring lanes read neighbouring entries
+    const float* tab = dist_row(opts.dist, opts.dist_len, head) + (p - key0);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int c = 0; c < 32; ++c)
+        sr[h][c] = __float_as_uint(fmaf(__ldg(tab - (h * 32 + c)), opts.dist_mul, __uint_as_float(sr[h][c])));
+  }
+  if (need_mask) {                                           // without branches: one test per page decides about the page
+    int lo_key = (window > 0) ? p - window : -1;             // keys <= lo_key are out of the window
+    if (chunk > 0) lo_key = max(lo_key, p / chunk * chunk - 1);   // or before the query's block of positions
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int c = 0; c < 32; ++c) {
+        const int key = key0 + h * 32 + c;
+        const bool dead = (key > p) | ((key <= lo_key) & (key >= opts.keep_first));   // kept first keys stay
+        sr[h][c] = dead ? 0xff800000u : sr[h][c];            // -inf
+      }
+  }
+}
+// Four independent chains for the maximum (and below for the sum): the row is long and a single chain would make every
+// step wait for the one before.
+__device__ inline float fa_row_max(const uint32_t (&sr)[2][32]) {
+  float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int c = 0; c < 32; c += 2)                          // two scores an instruction
+      mx4[(c >> 1) & 3] = fa_max3(mx4[(c >> 1) & 3], __uint_as_float(sr[h][c]), __uint_as_float(sr[h][c + 1]));
+  return fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+}
+// 2^(s * mul - mref) as bfloat16, two keys per column of P (which may lie over the row's first half); returns their sum in
+// float32.  Neighbouring keys go through the multiply-add and the additions as pairs (one issue slot for both).
+__device__ inline float fa_exponentials(const uint32_t (&sr)[2][32], float mul, float mref, uint32_t* pw) {
+  unsigned long long mul2, ref2, sum2[4] = {0, 0, 0, 0};
+  asm("mov.b64 %0, {%1, %1};" : "=l"(mul2) : "f"(mul));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(ref2) : "f"(-mref));
+#pragma unroll
+  for (int c = 0; c < 32; ++c) {
+    unsigned long long x2, e2;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(x2) : "r"(sr[(2 * c) >> 5][(2 * c) & 31]), "r"(sr[(2 * c) >> 5][(2 * c + 1) & 31]));
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(x2) : "l"(x2), "l"(mul2), "l"(ref2));
+    float e0, e1;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(e0), "=f"(e1) : "l"(x2));
+    e0 = fa_exp2(e0);
+    e1 = fa_exp2(e1);
+    asm("mov.b64 %0, {%1, %2};" : "=l"(e2) : "f"(e0), "f"(e1));
+    asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum2[c & 3]) : "l"(e2));
+    pw[c] = fa_pack(e0, e1);
+  }
+#pragma unroll
+  for (int i = 2; i > 0; i >>= 1)
+#pragma unroll
+    for (int c = 0; c < i; ++c) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum2[c]) : "l"(sum2[c + i]));
+  float lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(sum2[0]));
+  return lo + hi;
+}
+// This thread's row of O times corr.
+template <int HD> __device__ inline void fa_rescale(uint32_t taddr, float corr) {
+#pragma unroll
+  for (int h2 = 0; h2 < HD / 64; ++h2) {                     // 64 columns at a time
+    uint32_t o[2][32];
+    fa_ld32(taddr + 64 * h2, o[0]);
+    fa_ld32(taddr + 64 * h2 + 32, o[1]);
+    fa_wait_ld();
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int c = 0; c < 32; ++c) o[h][c] = __float_as_uint(__uint_as_float(o[h][c]) * corr);
+    fa_st32(taddr + 64 * h2, o[0]);
+    fa_st32(taddr + 64 * h2 + 32, o[1]);
+  }
+  fa_wait_st();
+  fa_fence_before();
+}
+// The same for 64 features, 16 columns at a time: the row of scores stays in its registers meanwhile.
+__device__ inline void fa_rescale_slowly(uint32_t taddr, float corr) {
+#pragma unroll 1
+  for (int c0 = 0; c0 < 64; c0 += 16) {
+    uint32_t o[16];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(o[0]), "=r"(o[1]), "=r"(o[2]), "=r"(o[3]), "=r"(o[4]), "=r"(o[5]), "=r"(o[6]), "=r"(o[7]),
+                   "=r"(o[8]), "=r"(o[9]), "=r"(o[10]), "=r"(o[11]), "=r"(o[12]), "=r"(o[13]), "=r"(o[14]), "=r"(o[15])
+                 : "r"(taddr + c0));
+    fa_wait_ld();
+#pragma unroll
+    for (int c = 0; c < 16; ++c) o[c] = __float_as_uint(__uint_as_float(o[c]) * corr);
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+                 ::"r"(taddr + c0), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]),
+                   "r"(o[8]), "r"(o[9]), "r"(o[10]), "r"(o[11]), "r"(o[12]), "r"(o[13]), "r"(o[14]), "r"(o[15]) : "memory");
+  }
+  fa_wait_st();
+  fa_fence_before();
+}
+// What a row of O is multiplied by at the end.  A sink is a key of score 0 without a value: one more term in the sum, in
+// the units of the reference maximum.
+__device__ inline float fa_inverse(float l_run, float m_used, int sink, const FaOpts& opts, int head, int row, int nh, bool in) {
+  float inv = 1.0f / (sink ? l_run + fa_exp2((opts.sink_vals ? __ldg(opts.sink_vals + head) * 1.4426950408889634f : 0.0f) - m_used) : l_run);
+  if (opts.gate && in) inv *= __ldcg(opts.gate + (int64_t)row * nh + head);
+  return inv;
+}
+// This thread's row of O times inv to dst (every thread reads: the load is the warp's).
+template <int HD> __device__ inline void fa_store_row(uint32_t taddr, float inv, __nv_bfloat16* dst, bool in) {
+#pragma unroll
+  for (int h2 = 0; h2 < HD / 64; ++h2) {                     // 64 columns at a time
+    uint32_t o[2][32];
+    fa_ld32(taddr + 64 * h2, o[0]);
+    fa_ld32(taddr + 64 * h2 + 32, o[1]);
+    fa_wait_ld();
+    if (in) {
+#pragma unroll
+      for (int ch = 0; ch < 8; ++ch) {
+        uint4 wd;
+        const int c = ch * 8;
+        wd.x = fa_pack(__uint_as_float(o[c >> 5][(c & 31) + 0]) * inv, __uint_as_float(o[c >> 5][(c & 31) + 1]) * inv);
+        wd.y = fa_pack(__uint_as_float(o[c >> 5][(c & 31) + 2]) * inv, __uint_as_float(o[c >> 5][(c & 31) + 3]) * inv);
+        wd.z = fa_pack(__uint_as_float(o[c >> 5][(c & 31) + 4]) * inv, __uint_as_float(o[c >> 5][(c & 31) + 5]) * inv);
+        wd.w = fa_pack(__uint_as_float(o[c >> 5][(c & 31) + 6]) * inv, __uint_as_float(o[c >> 5][(c & 31) + 7]) * inv);
+        *reinterpret_cast<uint4*>(dst + 64 * h2 + c) = wd;
+      }
+    }
+  }
+}
+
 // fold = 0: block (head, y) owns tile y.  fold = 1: it owns tiles y and n_tiles - 1 - y of the caller's list
 // (heaviest first), one after the other, so that all blocks have about the same number of pages to walk; the
 // pages of both run through the same rings and buffers as one sequence of pages, the second tile's Q in a buffer
@@ -256,8 +400,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   uint64_t* kv_full = bars + 2;                   // [stages] K and V page landed
   uint64_t* kv_free = kv_full + FA_KV_STAGES;     // [stages] the products that read the stage are done
   uint64_t* s_full = kv_free + FA_KV_STAGES;      // [2] S buffer written by the tensor core
-  uint64_t* s_free = s_full + 2;                  // [2] S buffer read by all 128 softmax threads
-  uint64_t* p_full = s_free + 2;                  // [2] P buffer written by all 128 softmax threads
+  uint64_t* s_free = s_full + 2;                  // [2] S buffer read by the four softmax warps
+  uint64_t* p_full = s_free + 2;                  // [2] P buffer written by the four softmax warps
   uint64_t* pv_done = p_full + 2;                 // [2] O += P V of that P buffer finished
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
 
@@ -281,8 +425,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     }
     for (int i = 0; i < 2; ++i) {
       fa_mbar_init(s_full + i, 1);
-      fa_mbar_init(s_free + i, 128);
-      fa_mbar_init(p_full + i, 128);
+      fa_mbar_init(s_free + i, 4);
+      fa_mbar_init(p_full + i, 4);
       fa_mbar_init(pv_done + i, 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -436,53 +580,15 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       const int st = f & 1;
       fa_wait_ld();
       fa_fence_before();
-      fa_mbar_arrive(s_free + st);
+      fa_mbar_arrive_warp(s_free + st);
       // The two barriers this page still needs (the P buffer free again, the next S written) are looked at now:
       // both have almost always flipped a page ago, and the looks' trips to shared memory pass under the
       // arithmetic below instead of standing in front of the store of P and the load of S.
       const bool p_free = f < 2 || fa_mbar_test(pv_done + st, ((f - 2) >> 1) & 1);
       const bool s_there = j + 1 < n_blocks && fa_mbar_test(s_full + (st ^ 1), ((f + 1) >> 1) & 1);
       const int key0 = (j < kept ? j : page_lo + j - kept) * FA_BK;
-      const bool need_mask = (key0 + FA_BK - 1 > p_first) || (window > 0 && key0 <= p_last - window) ||
-                             (chunk > 0 && key0 < p_last / chunk * chunk);
-      // four independent chains for the maximum (and below for the sum): the row is long and
-      // a single chain would make every step wait for the one before
-      // masking without branches (one test per page decides whether the page needs it at all)
-      if (opts.cap_in > 0.0f) {                              // capped scores: tanh now, the cap with the scale below
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int c = 0; c < 32; ++c) sr[h][c] = __float_as_uint(fa_tanh(__uint_as_float(sr[h][c]) * opts.cap_in));
-      }
-      if (opts.dist_len > 0 && fa_near(key0, p_first + warp * 32, opts.dist_len)) {
-        // the biases of this row's distances p - key: neighbouring lanes read neighbouring entries
-        const float* tab = dist_row(opts.dist, opts.dist_len, head) + (p - key0);
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int c = 0; c < 32; ++c)
-            sr[h][c] = __float_as_uint(fmaf(__ldg(tab - (h * 32 + c)), opts.dist_mul, __uint_as_float(sr[h][c])));
-      }
-      if (need_mask) {
-        int lo_key = (window > 0) ? p - window : -1;          // keys <= lo_key are out of the window
-        if (chunk > 0) lo_key = max(lo_key, p / chunk * chunk - 1);   // or before the query's block of positions
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int c = 0; c < 32; ++c) {
-            const int key = key0 + h * 32 + c;
-            const bool dead = (key > p) | ((key <= lo_key) & (key >= opts.keep_first));   // kept first keys stay
-            sr[h][c] = dead ? 0xff800000u : sr[h][c];         // -inf
-          }
-      }
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int c = 0; c < 32; c += 2)                      // two scores an instruction
-          mx4[(c >> 1) & 3] = fa_max3(mx4[(c >> 1) & 3], __uint_as_float(sr[h][c]), __uint_as_float(sr[h][c + 1]));
-      float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-      mx *= score_mul;                                       // scale > 0: max and scale commute
+      fa_adjust(sr, opts, head, key0, p, p_first, p_last, p_first + warp * 32, window, chunk);
+      const float mx = fa_row_max(sr) * score_mul;           // scale > 0: max and scale commute
       // lazy rescale: move the reference maximum only when it is far behind
       const bool grow = mx > m_used + FA_RESCALE_STEP || (m_used == -INFINITY && mx > -INFINITY);
       if (__any_sync(0xffffffffu, grow)) {
@@ -492,21 +598,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           // every earlier product must have landed in O before it is rewritten
           if (!fa_mbar_wait(pv_done + (st ^ 1), ((f - 1) >> 1) & 1)) { ok = false; break; }
           fa_fence_after();
-#pragma unroll
-          for (int h2 = 0; h2 < FA_HD / 64; ++h2) {          // 64 columns at a time
-            uint32_t o[2][32];
-            fa_ld32(tmem_o + lane_addr + 64 * h2, o[0]);
-            fa_ld32(tmem_o + lane_addr + 64 * h2 + 32, o[1]);
-            fa_wait_ld();
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-              for (int c = 0; c < 32; ++c) o[h][c] = __float_as_uint(__uint_as_float(o[h][c]) * corr);
-            fa_st32(tmem_o + lane_addr + 64 * h2, o[0]);
-            fa_st32(tmem_o + lane_addr + 64 * h2 + 32, o[1]);
-          }
-          fa_wait_st();
-          fa_fence_before();
+          fa_rescale<FA_HD>(tmem_o + lane_addr, corr);
         }
         l_run *= corr;
         m_used = m_new;
@@ -515,21 +607,12 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       // the P buffer of two pages ago must have been consumed
       if (!p_free && !fa_mbar_wait(pv_done + st, ((f - 2) >> 1) & 1)) { ok = false; break; }
       uint32_t pw[32];
-      float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-      for (int c = 0; c < 32; ++c) {                         // two keys per column
-        const float e0 = fa_exp2(fmaf(__uint_as_float(sr[(2 * c) >> 5][(2 * c) & 31]), score_mul, -mref));
-        const float e1 = fa_exp2(fmaf(__uint_as_float(sr[(2 * c + 1) >> 5][(2 * c + 1) & 31]), score_mul, -mref));
-        sum4[c & 3] += e0 + e1;
-        pw[c] = fa_pack(e0, e1);
-      }
-      const float sum = (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
-      l_run += sum;
+      l_run += fa_exponentials(sr, score_mul, mref, pw);
       fa_st32(tmem_p + lane_addr + st * 32, pw);
       if (j + 1 < n_blocks && !ask_s(f + 1, s_there)) ok = false;   // the tile's next row of S while P is being stored
       fa_wait_st();
       fa_fence_before();
-      fa_mbar_arrive(p_full + st);
+      fa_mbar_arrive_warp(p_full + st);
     }
     if (ok) {
       // last product done -> O complete
@@ -537,29 +620,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       ok = fa_mbar_wait(pv_done + (fl & 1), (fl >> 1) & 1);
       if (ok) {
         fa_fence_after();
-        // a sink is a key of score 0 without a value: one more term in the sum, in the units of the reference maximum
-        float inv = 1.0f / (sink ? l_run + fa_exp2((opts.sink_vals ? __ldg(opts.sink_vals + head) * 1.4426950408889634f : 0.0f) - m_used) : l_run);
-        if (opts.gate && r < rows) inv *= __ldcg(opts.gate + (int64_t)(tw.row0 + r) * nh + head);
-        __nv_bfloat16* dst = out + ((int64_t)(tw.row0 + r) * nh + head) * FA_HD;
-#pragma unroll
-        for (int h2 = 0; h2 < FA_HD / 64; ++h2) {            // 64 columns at a time (every thread reads: the load is the warp's)
-          uint32_t o[2][32];
-          fa_ld32(tmem_o + lane_addr + 64 * h2, o[0]);
-          fa_ld32(tmem_o + lane_addr + 64 * h2 + 32, o[1]);
-          fa_wait_ld();
-          if (r < rows) {
-#pragma unroll
-            for (int ch = 0; ch < 8; ++ch) {
-              uint4 wd;
-              const int c = ch * 8;
-              wd.x = fa_pack(__uint_as_float(o[c >> 5][(c & 31) + 0]) * inv, __uint_as_float(o[c >> 5][(c & 31) + 1]) * inv);
-              wd.y = fa_pack(__uint_as_float(o[c >> 5][(c & 31) + 2]) * inv, __uint_as_float(o[c >> 5][(c & 31) + 3]) * inv);
-              wd.z = fa_pack(__uint_as_float(o[c >> 5][(c & 31) + 4]) * inv, __uint_as_float(o[c >> 5][(c & 31) + 5]) * inv);
-              wd.w = fa_pack(__uint_as_float(o[c >> 5][(c & 31) + 6]) * inv, __uint_as_float(o[c >> 5][(c & 31) + 7]) * inv);
-              *reinterpret_cast<uint4*>(dst + 64 * h2 + c) = wd;
-            }
-          }
-        }
+        const float inv = fa_inverse(l_run, m_used, sink, opts, head, tw.row0 + r, nh, r < rows);
+        fa_store_row<FA_HD>(tmem_o + lane_addr, inv, out + ((int64_t)(tw.row0 + r) * nh + head) * FA_HD, r < rows);
         fa_fence_before();                                 // O is read: the next tile's first product may write it
       }
     }
@@ -608,7 +670,7 @@ attn_prefill_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   uint64_t* kv_full = bars + 1;                   // [2]
   uint64_t* kv_free = kv_full + F4_STAGES;        // [2]
   uint64_t* s_full = kv_free + F4_STAGES;         // S written by the tensor core
-  uint64_t* p_full = s_full + 1;                  // P written over S by all 128 softmax threads
+  uint64_t* p_full = s_full + 1;                  // P written over S by the four softmax warps
   uint64_t* pv_done = p_full + 1;                 // O += P V finished: the S columns are free again
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 1);
 
@@ -632,7 +694,7 @@ attn_prefill_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
     fa_mbar_init(q_full, 1);
     for (int i = 0; i < F4_STAGES; ++i) { fa_mbar_init(kv_full + i, 1); fa_mbar_init(kv_free + i, 1); }
     fa_mbar_init(s_full, 1);
-    fa_mbar_init(p_full, 128);
+    fa_mbar_init(p_full, 4);
     fa_mbar_init(pv_done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -713,89 +775,29 @@ attn_prefill_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
       fa_ld32(tmem_base + lane_addr + 32, sr[1]);
       fa_wait_ld();
       const int key0 = (j < kept ? j : page_lo + j - kept) * FA_BK;
-      const bool need_mask = (key0 + FA_BK - 1 > p_first) || (window > 0 && key0 <= p_last - window) ||
-                             (chunk > 0 && key0 < p_last / chunk * chunk);
-      if (opts.cap_in > 0.0f) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int c = 0; c < 32; ++c) sr[h][c] = __float_as_uint(fa_tanh(__uint_as_float(sr[h][c]) * opts.cap_in));
-      }
-      if (opts.dist_len > 0 && fa_near(key0, p_first + warp * 32, opts.dist_len)) {
-        const float* tab = dist_row(opts.dist, opts.dist_len, head) + (p - key0);
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int c = 0; c < 32; ++c)
-            sr[h][c] = __float_as_uint(fmaf(__ldg(tab - (h * 32 + c)), opts.dist_mul, __uint_as_float(sr[h][c])));
-      }
-      if (need_mask) {
-        int lo_key = (window > 0) ? p - window : -1;
-        if (chunk > 0) lo_key = max(lo_key, p / chunk * chunk - 1);
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int c = 0; c < 32; ++c) {
-            const int key = key0 + h * 32 + c;
-            const bool dead = (key > p) | ((key <= lo_key) & (key >= opts.keep_first));
-            sr[h][c] = dead ? 0xff800000u : sr[h][c];
-          }
-      }
-      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-#pragma unroll
-        for (int c = 0; c < 32; ++c) mx4[c & 3] = fmaxf(mx4[c & 3], __uint_as_float(sr[h][c]));
-      float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-      mx *= score_mul;
+      fa_adjust(sr, opts, head, key0, p, p_first, p_last, p_first + warp * 32, window, chunk);
+      const float mx = fa_row_max(sr) * score_mul;
       const bool grow = mx > m_used + FA_RESCALE_STEP || (m_used == -INFINITY && mx > -INFINITY);
       if (__any_sync(0xffffffffu, grow)) {
         const float m_new = grow ? mx : m_used;
         const float corr = (m_used == -INFINITY) ? 0.0f : fa_exp2(m_used - m_new);
-        if (j > 0) {
-          // the product of page j - 1 is in O: S_j was issued after it was done.  16 columns at a time: the
-          // row of scores stays in its registers meanwhile
-#pragma unroll 1
-          for (int c0 = 0; c0 < 64; c0 += 16) {
-            uint32_t o[16];
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                         : "=r"(o[0]), "=r"(o[1]), "=r"(o[2]), "=r"(o[3]), "=r"(o[4]), "=r"(o[5]), "=r"(o[6]), "=r"(o[7]),
-                           "=r"(o[8]), "=r"(o[9]), "=r"(o[10]), "=r"(o[11]), "=r"(o[12]), "=r"(o[13]), "=r"(o[14]), "=r"(o[15])
-                         : "r"(tmem_o + lane_addr + c0));
-            fa_wait_ld();
-#pragma unroll
-            for (int c = 0; c < 16; ++c) o[c] = __float_as_uint(__uint_as_float(o[c]) * corr);
-            asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
-                         ::"r"(tmem_o + lane_addr + c0), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]),
-                           "r"(o[8]), "r"(o[9]), "r"(o[10]), "r"(o[11]), "r"(o[12]), "r"(o[13]), "r"(o[14]), "r"(o[15]) : "memory");
-          }
-          fa_wait_st();
-        }
+        if (j > 0) fa_rescale_slowly(tmem_o + lane_addr, corr);   // the product of page j - 1 is in O: S_j was issued after it was done
         l_run *= corr;
         m_used = m_new;
       }
       const float mref = (m_used == -INFINITY) ? 0.0f : m_used;
-      float sum4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-      for (int c = 0; c < 32; ++c) {                         // two keys per column, written over the scores' registers
-        const float e0 = fa_exp2(fmaf(__uint_as_float(sr[(2 * c) >> 5][(2 * c) & 31]), score_mul, -mref));
-        const float e1 = fa_exp2(fmaf(__uint_as_float(sr[(2 * c + 1) >> 5][(2 * c + 1) & 31]), score_mul, -mref));
-        sum4[c & 3] += e0 + e1;
-        sr[0][c] = fa_pack(e0, e1);
-      }
-      l_run += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
+      l_run += fa_exponentials(sr, score_mul, mref, sr[0]);  // written over the scores' registers
       fa_st32(tmem_base + lane_addr, sr[0]);
       fa_wait_st();
       fa_fence_before();
-      fa_mbar_arrive(p_full);
+      fa_mbar_arrive_warp(p_full);
     }
     if (ok) {
       const int jl = n_blocks - 1;
       ok = fa_mbar_wait(pv_done, jl & 1);
       if (ok) {
         fa_fence_after();
-        float inv = 1.0f / (sink ? l_run + fa_exp2((opts.sink_vals ? __ldg(opts.sink_vals + head) * 1.4426950408889634f : 0.0f) - m_used) : l_run);
-        if (opts.gate && r < rows) inv *= __ldcg(opts.gate + (int64_t)(row_start[b] + q0 + r) * nh + head);
+        const float inv = fa_inverse(l_run, m_used, sink, opts, head, row_start[b] + q0 + r, nh, r < rows);
         __nv_bfloat16* dst = out + ((int64_t)(row_start[b] + q0 + r) * nh + head) * 64;
 #pragma unroll 1
         for (int c0 = 0; c0 < 64; c0 += 32) {
@@ -825,6 +827,275 @@ attn_prefill_tc4_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_
   fa_fence_after();
   if (warp == 4)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(128) : "memory");
+}
+
+// ---- heads of 128, groups of an even number of query heads: two heads side by side ---------------------------------
+// In the kernel above an SM has one block and so four softmax warps, one a scheduler, and nothing hides the latencies of a
+// page's chain.  Here a block takes the same tile of queries for two neighbouring query heads of one kv head: eight softmax
+// warps in two sets that take turns with the tensor core, and every page of keys and values is copied once for both.
+// P is written over the columns of its own S (S_(f + 2) waits for the product of P_f), which leaves room in tensor memory
+// for two buffers of S and O of both heads: 2 x (2 x 64 + 128) columns.  The second product runs as instructions of 128
+// columns over both feature boxes of V (65 cycles each; two of 64 columns take 94).  Blocks are persistent, one an SM: they
+// walk the items (tile, pair of heads), the list's heaviest tiles first and in turns from both ends (block b takes item b of
+// the first round, the mirrored one of the second), and an item's Q comes in while the last pages of the item before are
+// worked on.  Same arithmetic in the same order per row as above: the same numbers bit for bit.
+// Bound by the chain of a page's softmax, two warps a scheduler: a page takes 1.19 us for both heads (0.87 us for one head
+// above; the tensor core's share is 0.7, what it reads of shared memory).  32 heads on 8, one prompt of 6,145 tokens:
+// 465 -> 316 us, 0.98 PFLOP/s; of 2,048: 67.5 -> 47.4; 32 prompts of 19 to 147: 50.2 -> 29.4.
+//
+//   warps 0-3, 4-7   softmax and epilogue of the first and the second head (thread = query row = TMEM lane)
+//   warp 8           S = Q K^T of both heads, page by page
+//   warp 9           O += P V of both heads
+//   warp 10          copies: Q of both heads, pages of K and V
+constexpr int FP_THREADS = 352, FP_STAGES = 4;
+constexpr uint32_t FP_SMEM = 2 * fa_q_bytes(128) + 2 * FP_STAGES * fa_kv_bytes(128) + 1024 + 256;
+constexpr uint32_t FA_IDESC_PV128 = (FA_IDESC_PV & ~(63u << 17)) | ((128u >> 3) << 17);
+// V as an MN-major operand of 128 features: the second box of 64 lies FA_KVBOX_BYTES behind the first.
+__device__ inline uint64_t fa_desc_v128(uint32_t smem_addr) {
+  return (fa_desc(smem_addr) & ~(0x3fffull << 16)) | ((uint64_t)(FA_KVBOX_BYTES >> 4) << 16);
+}
+
+__global__ void __launch_bounds__(FP_THREADS, 1)
+attn_prefill_tc_pair_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+                            const __grid_constant__ CUtensorMap map_v, __nv_bfloat16* __restrict__ out,
+                            const int* __restrict__ block_table, int bt_stride, const int* __restrict__ row_start,
+                            const int* __restrict__ row_pos0, const int* __restrict__ tile_seq,
+                            const int* __restrict__ tile_q0, int n_tiles, int nh, int nkv, int window, int chunk, int sink,
+                            float scale_log2, FaOpts opts) {
+  extern __shared__ unsigned char fa_smem_raw[];
+  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(fa_smem_raw) + 1023) & ~(uintptr_t)1023);
+  constexpr uint32_t QB = fa_q_bytes(128), KVB = fa_kv_bytes(128);
+  unsigned char* sQ = base;                                  // [2 heads][2 boxes][128][64] bf16
+  unsigned char* sK = sQ + 2 * QB;                           // [stages][2 boxes][64][64]
+  unsigned char* sV = sK + FP_STAGES * KVB;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + FP_STAGES * KVB);
+  uint64_t* q_full = bars;                        // [2 heads] Q tile landed
+  uint64_t* q_free = bars + 2;                    // [2 heads] the item's last S is done
+  uint64_t* kv_full = q_free + 2;                 // [stages] K and V page landed
+  uint64_t* kv_free = kv_full + FP_STAGES;        // [stages] both heads' products that read the stage are done
+  uint64_t* s_full = kv_free + FP_STAGES;         // [2 heads][2] S buffer written by the tensor core
+  uint64_t* p_full = s_full + 4;                  // [2 heads][2] P written over it by the head's four softmax warps
+  uint64_t* pv_done = p_full + 4;                 // [2 heads][2] O += P V of that buffer finished
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 4);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n_pairs = nh >> 1, n_items = n_tiles * n_pairs;
+  auto item_of = [&](int k) {                               // the block's k-th item; n_items or more: none
+    return k * (int)gridDim.x + ((k & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
+  };
+  auto tile_of = [&](int item) {
+    return fa_tile(item / n_pairs, block_table, bt_stride, row_start, row_pos0, tile_seq, tile_q0, window, chunk, opts.keep_first);
+  };
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < 2; ++i) { fa_mbar_init(q_full + i, 1); fa_mbar_init(q_free + i, 1); }
+    for (int i = 0; i < FP_STAGES; ++i) { fa_mbar_init(kv_full + i, 1); fa_mbar_init(kv_free + i, 1); }
+    for (int i = 0; i < 4; ++i) { fa_mbar_init(s_full + i, 1); fa_mbar_init(p_full + i, 4); fa_mbar_init(pv_done + i, 1); }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 8) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(fa_smem_u32(tmem_slot)), "r"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  fa_fence_before();
+  __syncthreads();
+  fa_fence_after();
+  // so far nothing was touched that another kernel writes; the next kernel in the stream may be set up meanwhile
+  pdl_trigger();
+  pdl_wait();
+  const uint32_t tmem_base = *tmem_slot;                    // columns: S of head s at 128 s, O at 256 + 128 s
+  bool ok = true;
+
+  if (warp == 10) {
+    // ---- copies -------------------------------------------------------------------------------------------
+    // Page numbers come 32 at a time, lane i holding that of page j0 + i of the item, a batch (or the next item's
+    // first batch) ahead.
+    int c = 0, k = 0, item = item_of(0);                    // c: pages asked for
+    FaTile t = tile_of(item);
+    auto numbers = [&](const FaTile& u, int j0) {
+      const int j = j0 + lane;
+      return j < u.n_pages ? u.bt[j < u.kept ? j : u.page_lo + j - u.kept] : 0;
+    };
+    int pgs = numbers(t, 0);
+    while (ok) {
+      const int next = item_of(k + 1);
+      const FaTile tn = next < n_items ? tile_of(next) : t;
+      const int first_next = next < n_items ? numbers(tn, 0) : 0;
+      const int hp = item % n_pairs, g = 2 * hp / (nh / nkv);
+      int ahead = numbers(t, 32);
+      for (int j = 0; j < t.n_pages; ++j, ++c) {
+        if ((j & 31) == 0 && j > 0) { pgs = ahead; ahead = numbers(t, j + 32); }
+        const int st = c % FP_STAGES, pg = __shfl_sync(0xffffffffu, pgs, j & 31);
+        if (c >= FP_STAGES && !fa_mbar_wait(kv_free + st, (c / FP_STAGES - 1) & 1)) { ok = false; break; }
+        if (lane == 0) {
+          fa_mbar_expect_tx(kv_full + st, 2 * KVB);
+#pragma unroll
+          for (int x = 0; x < 2; ++x) {
+            fa_tma_2d(sK + st * KVB + x * FA_KVBOX_BYTES, &map_k, kv_full + st, 64 * x, (pg * nkv + g) * FA_BK);
+            fa_tma_2d(sV + st * KVB + x * FA_KVBOX_BYTES, &map_v, kv_full + st, 64 * x, (pg * nkv + g) * FA_BK);
+          }
+        }
+        __syncwarp();
+        if (j > 0) continue;
+        for (int s = 0; s < 2; ++s) {                        // behind the first page: Q's place may still be read
+          if (k > 0 && !fa_mbar_wait(q_free + s, (k - 1) & 1)) { ok = false; break; }
+          if (lane == 0) {
+            fa_mbar_expect_tx(q_full + s, QB);
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+              fa_tma_2d(sQ + s * QB + x * FA_QBOX_BYTES, &map_q, q_full + s, (2 * hp + s) * 128 + 64 * x, t.row0);
+          }
+          __syncwarp();
+        }
+        if (!ok) { ++c; break; }
+      }
+      if (!ok || next >= n_items) break;
+      ++k;
+      item = next;
+      t = tn;
+      pgs = first_next;
+    }
+    // what was asked for must land before the block's shared memory goes away
+    if (!ok && lane == 0) atomicExch(&g_fa_error, 1);
+    for (int u = max(0, c - FP_STAGES); u < c; ++u) fa_mbar_wait(kv_full + u % FP_STAGES, (u / FP_STAGES) & 1);
+    for (int s = 0; s < 2; ++s) fa_mbar_wait(q_full + s, k & 1);
+  } else if (warp == 8) {
+    // ---- S_f = Q K_f^T of both heads, up to two pages ahead of the softmax ------------------------------------
+    int f = 0;
+    for (int k = 0, item = item_of(0); ok && item < n_items; item = item_of(++k)) {
+      const int n_pages = tile_of(item).n_pages;
+      for (int j = 0; j < n_pages && ok; ++j, ++f) {
+        const int sb = f & 1, st = f % FP_STAGES;
+        if (!fa_mbar_wait(kv_full + st, (f / FP_STAGES) & 1)) { ok = false; break; }
+        for (int s = 0; s < 2; ++s) {
+          if (j == 0 && !fa_mbar_wait(q_full + s, k & 1)) { ok = false; break; }
+          if (f >= 2 && !fa_mbar_wait(pv_done + 2 * s + sb, ((f >> 1) - 1) & 1)) { ok = false; break; }
+          fa_fence_after();
+          if (lane == 0) {
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {                    // 64 features of the sum at a time
+              const uint64_t da = fa_desc(fa_smem_u32(sQ + s * QB + x * FA_QBOX_BYTES));
+              const uint64_t db = fa_desc(fa_smem_u32(sK + st * KVB + x * FA_KVBOX_BYTES));
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                fa_umma(tmem_base + 128 * s + 64 * sb, da + 2 * i, db + 2 * i, FA_IDESC_S, (x | i) > 0);
+            }
+            fa_commit(s_full + 2 * s + sb);
+            if (j == n_pages - 1) fa_commit(q_free + s);
+          }
+          __syncwarp();
+        }
+      }
+    }
+    if (!ok && lane == 0) atomicExch(&g_fa_error, 3);
+  } else if (warp == 9) {
+    // ---- O += P_f V_f of both heads -----------------------------------------------------------------------------
+    int f = 0;
+    for (int k = 0, item = item_of(0); ok && item < n_items; item = item_of(++k)) {
+      const int n_pages = tile_of(item).n_pages;
+      for (int j = 0; j < n_pages && ok; ++j, ++f) {
+        const int sb = f & 1, st = f % FP_STAGES;
+        for (int s = 0; s < 2; ++s) {
+          if (!fa_mbar_wait(p_full + 2 * s + sb, (f >> 1) & 1)) { ok = false; break; }
+          fa_fence_after();
+          if (lane == 0) {
+            // an item's first product starts O afresh (the softmax threads hand over P only after they have read the
+            // item before out of O)
+            const uint64_t db = fa_desc_v128(fa_smem_u32(sV + st * KVB));
+#pragma unroll
+            for (int i = 0; i < FA_BK / 16; ++i)            // 16 keys: 8 columns of P, 16 rows of V
+              fa_umma_ts(tmem_base + 256 + 128 * s, tmem_base + 128 * s + 64 * sb + 8 * i, db + 128 * i, FA_IDESC_PV128,
+                         (j > 0 || i > 0) ? 1u : 0u);
+            fa_commit(pv_done + 2 * s + sb);
+            if (s == 1) fa_commit(kv_free + st);
+          }
+          __syncwarp();
+        }
+      }
+    }
+    if (!ok && lane == 0) atomicExch(&g_fa_error, 4);
+  } else {
+    // ---- softmax and epilogue -----------------------------------------------------------------------------------
+    const int s = warp >> 2, q = warp & 3;                   // the head of the pair, and the 32 rows
+    const int r = q * 32 + lane;
+    const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
+    const uint32_t tmem_s = tmem_base + lane_addr + 128 * s, tmem_o = tmem_base + lane_addr + 256 + 128 * s;
+    const float score_mul = opts.cap_in > 0.0f ? opts.cap_log2 : scale_log2;
+    int fb = 0;                                              // the item's first page in the block's numbering
+    int k = 0, item = item_of(0);
+    FaTile t = tile_of(item);
+    while (ok) {
+      const int next = item_of(k + 1);
+      const FaTile tn = next < n_items ? tile_of(next) : t;  // asked for an item ahead
+      const int head = 2 * (item % n_pairs) + s;
+      const int p = t.p_first + r, n_pages = t.n_pages;
+      float m_used = -INFINITY, l_run = 0.0f;
+      uint32_t sr[2][32];
+      auto ask_s = [&](int f, bool there) -> bool {         // there: the barrier is known to have flipped
+        if (!there && !fa_mbar_wait(s_full + 2 * s + (f & 1), (f >> 1) & 1)) return false;
+        fa_fence_after();
+        fa_ld32(tmem_s + 64 * (f & 1), sr[0]);
+        fa_ld32(tmem_s + 64 * (f & 1) + 32, sr[1]);
+        return true;
+      };
+      ok = ask_s(fb, false);
+      for (int j = 0; j < n_pages && ok; ++j) {
+        const int f = fb + j, sb = f & 1;
+        fa_wait_ld();
+        // looked at early: see the kernel above
+        const bool s_there = j + 1 < n_pages && fa_mbar_test(s_full + 2 * s + (sb ^ 1), ((f + 1) >> 1) & 1);
+        const int key0 = (j < t.kept ? j : t.page_lo + j - t.kept) * FA_BK;
+        fa_adjust(sr, opts, head, key0, p, t.p_first, t.p_last, t.p_first + q * 32, window, chunk);
+        const float mx = fa_row_max(sr) * score_mul;         // scale > 0: max and scale commute
+        const bool grow = mx > m_used + FA_RESCALE_STEP || (m_used == -INFINITY && mx > -INFINITY);
+        if (__any_sync(0xffffffffu, grow)) {
+          const float m_new = grow ? mx : m_used;
+          const float corr = (m_used == -INFINITY) ? 0.0f : fa_exp2(m_used - m_new);   // 1 for rows that keep theirs
+          if (j > 0) {
+            // every earlier product must have landed in O before it is rewritten
+            if (!fa_mbar_wait(pv_done + 2 * s + (sb ^ 1), ((f - 1) >> 1) & 1)) { ok = false; break; }
+            fa_fence_after();
+            fa_rescale<128>(tmem_o, corr);
+          }
+          l_run *= corr;
+          m_used = m_new;
+        }
+        const float mref = (m_used == -INFINITY) ? 0.0f : m_used;
+        uint32_t pw[32];
+        l_run += fa_exponentials(sr, score_mul, mref, pw);
+        fa_st32(tmem_s + 64 * sb, pw);                       // over the row's own scores
+        if (j + 1 < n_pages && !ask_s(f + 1, s_there)) ok = false;
+        fa_wait_st();
+        fa_fence_before();
+        fa_mbar_arrive_warp(p_full + 2 * s + sb);
+      }
+      if (ok) {
+        const int fl = fb + n_pages - 1;                     // the last product done: O is complete
+        ok = fa_mbar_wait(pv_done + 2 * s + (fl & 1), (fl >> 1) & 1);
+        if (ok) {
+          fa_fence_after();
+          const bool in = r < t.rows;
+          const float inv = fa_inverse(l_run, m_used, sink, opts, head, t.row0 + r, nh, in);
+          fa_store_row<128>(tmem_o, inv, out + ((int64_t)(t.row0 + r) * nh + head) * 128, in);
+          fa_fence_before();                                 // O is read: the next item's first product may write it
+        }
+      }
+      if (!ok || next >= n_items) break;
+      fb += n_pages;
+      ++k;
+      item = next;
+      t = tn;
+    }
+    if (!ok) fa_wait_ld();                                   // a row of S may still be on its way
+    if (!ok && lane == 0) atomicExch(&g_fa_error, 2);
+  }
+
+  fa_fence_before();
+  __syncthreads();
+  fa_fence_after();
+  if (warp == 8)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
 }
 
 // ---- host side --------------------------------------------------------------------------
@@ -907,8 +1178,11 @@ extern "C" int exl3_attn_prefill_tc_opt(const void* q, int64_t q_row_stride, int
     set_error("attn_prefill_tc: needs bfloat16, head_dim 64 or 128 and pages of 64, got head_dim %d page %d", hd, page);
     return ERR_UNSUPPORTED;
   }
-  if (variant < 0 || variant > 3 || (variant == 2 && hd != 64)) {
-    set_error("attn_prefill_tc: variant is 0 (chosen), 1 (a tile a block), 2 (four blocks an SM, heads of 64) or 3 (two tiles a block), got %d", variant);
+  const bool even_groups = nkv > 0 && nh % nkv == 0 && (nh / nkv) % 2 == 0;
+  const bool pairs_fit = hd == 128 && even_groups;
+  if (variant < 0 || variant > 4 || (variant == 2 && hd != 64) || (variant == 4 && !pairs_fit)) {
+    set_error("attn_prefill_tc: variant is 0 (chosen), 1 (a tile a block), 2 (four blocks an SM, heads of 64), 3 (two tiles a block) "
+              "or 4 (pairs of heads of 128 in even groups), got %d", variant);
     return ERR_BAD_ARGUMENT;
   }
   if (n_tiles < 0 || T < 1 || nh < 1 || nkv < 1 || nh % nkv != 0 || n_tiles > 65535 || window < 0 || chunk < 0 || q_row_stride % 8 != 0) {
@@ -931,6 +1205,8 @@ extern "C" int exl3_attn_prefill_tc_opt(const void* q, int64_t q_row_stride, int
       e = cudaFuncSetAttribute(attn_prefill_tc_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fa_smem(64));
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(attn_prefill_tc_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fa_smem(128));
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(attn_prefill_tc_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FP_SMEM);
     if (e != cudaSuccess) { set_error("attn_prefill_tc: cannot get %u bytes of shared memory: %s", fa_smem(128), cudaGetErrorString(e)); return (int)e; }
     configured = true;
   }
@@ -945,12 +1221,21 @@ extern "C" int exl3_attn_prefill_tc_opt(const void* q, int64_t q_row_stride, int
   // the lightest, and so on) when a tile a block would need a second round of blocks and two tiles a block need
   // none: then every block walks about the same number of pages and the kernel ends with all of them.
   const int64_t blocks = (int64_t)n_tiles * nh, at_once = (int64_t)sms * (hd == 64 ? 2 : 1);
+  // Pairs of heads fill every SM from as many items as there are SMs (32 heads on 8 of 128: 1,500 tokens, 192 items, 33.9 us against
+  // 44.5 with a tile and head a block; 1,024 tokens, 128 items, 25.7 against 24.3).
+  const bool pairs = variant == 4 || (variant == 0 && pairs_fit && (int64_t)n_tiles * (nh / 2) >= sms);
   const bool four = hd == 64 && (variant == 2 || (variant == 0 && blocks > 4 * (int64_t)sms));
   const int fold = (variant == 3 || (variant == 0 && !four && blocks > at_once && (int64_t)((n_tiles + 1) / 2) * nh <= at_once)) ? 1 : 0;
   dim3 grid(nh, fold ? (n_tiles + 1) / 2 : n_tiles);
   __nv_bfloat16* o = static_cast<__nv_bfloat16*>(out);
   const float scale_log2 = scale * 1.4426950408889634f;
-  if (four)
+  if (pairs) {
+    const int64_t items = (int64_t)n_tiles * (nh / 2);
+    if (items > 0x3fffffff) { set_error("attn_prefill_tc: too many tiles"); return ERR_UNSUPPORTED; }
+    launch_pdl(attn_prefill_tc_pair_kernel, dim3((unsigned)(items < sms ? items : sms)), dim3(FP_THREADS), FP_SMEM, stream, map_q,
+               map_k, map_v, o, block_table, bt_stride, row_start, row_pos0, tile_seq, tile_q0, n_tiles, nh, nkv, window, chunk,
+               sink, scale_log2, opts);
+  } else if (four)
     launch_pdl(attn_prefill_tc4_kernel, grid, dim3(FA_THREADS), F4_SMEM, stream, map_q, map_k, map_v, o, block_table,
                bt_stride, row_start, row_pos0, tile_seq, tile_q0, nh, nkv, window, chunk, sink, scale_log2, opts);
   else if (hd == 64)

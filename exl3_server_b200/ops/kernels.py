@@ -1032,8 +1032,9 @@ def attn_prefill_tc(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, k_poo
     """Causal attention of whole prompts on tcgen05 tensor cores (tiles of 128 queries; see
     attention_prefill_tc.cu).  ``k_pool`` / ``v_pool``: one layer's ``[pages, kv_heads, 64, head_dim]``.
     ``variant``: 0 lets the kernel choose by the number of blocks between a tile a block, four blocks per SM (heads
-    of 64) and two tiles a block (the list's first with its last, and so on: list the tiles with the most keys
-    to visit first); 1, 2 and 3 force one of them (the same numbers every way).  ``chunk``, ``sink``, ``keep_first``,
+    of 64), two tiles a block (the list's first with its last, and so on: list the tiles with the most keys
+    to visit first) and two heads side by side (heads of 128 in even groups); 1, 2, 3 and 4 force one of them (the same
+    numbers every way).  ``chunk``, ``sink``, ``keep_first``,
     ``softcap``, ``sink_vals``, ``dist`` and ``gate`` as in ``attn_tokens_ex``."""
     dist_len = _distance_len(dist, heads, "attn_prefill_tc")
     _check_gate(gate, q.shape[0], heads, "attn_prefill_tc")

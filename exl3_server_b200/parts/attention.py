@@ -43,6 +43,31 @@ BUSY_ITEMS = 1776
 PROMPT_FUSED = os.environ.get("EXL3_PROMPT_FUSED", "1") != "0"
 
 
+def _makespan(times, slots: int, heads: int) -> float:
+    """When the last of the tiles' blocks ends: a tile's ``heads`` run side by side, a tile takes the slots that come free
+    first, in the list's order."""
+    if len(times) * heads <= slots:
+        return max(times)
+    if len(times) <= 64 and heads <= slots:
+        # every block on the slot that comes free first: a tile's heads take the slots that are free soonest
+        free = np.zeros(slots)
+        for t in times:
+            free[np.argpartition(free, heads - 1)[:heads]] += t
+        return float(free.max())
+    # many tiles: groups of slots as wide as a tile has heads, what the division leaves over given back as
+    # capacity
+    groups = slots // heads
+    if groups == 0:
+        return sum(times) * heads / slots
+    free = [0.0] * groups
+    end = 0.0
+    for t in times:
+        at = heapq.heappop(free) + t
+        heapq.heappush(free, at)
+        end = max(end, at)
+    return max(max(times), end * groups * heads / slots)
+
+
 class Attention:
     @staticmethod
     def tensor_specs(spec: MixerSpec, prefix: str) -> List[TensorSpec]:
@@ -162,7 +187,7 @@ class Attention:
             key = ("attn_prefill_variant", s.heads, s.head_dim, s.window)
             variant = batch.memo.get(key)
             if variant is None:
-                variant = batch.memo[key] = self._prefill_variant(batch.tile_keys.get(128), kv.page_size, qkv.device)
+                variant = batch.memo[key] = self._prefill_form(batch.tile_keys.get(128), kv.page_size, qkv.device)
             K.attn_prefill_tc(qkv, qkv.stride(0), out, kv.k, kv.v, kv.block_table, batch.row_start, batch.row_pos0,
                               tile_seq, tile_q0, n_tiles, s.heads, s.kv_heads, s.head_dim, kv.page_size, s.window,
                               self.scale, variant=variant)
@@ -226,31 +251,9 @@ class Attention:
             return 0
         sms = K.sm_count(device)
         n = len(tile_keys)
-        size = 128
-        pages = [((min(k, s.window + size) if s.window > 0 else k) + page - 1) // page for k in tile_keys]
+        pages = self._tile_pages(tile_keys, page)
         each = 3                                                # a tile's start and end, in pages
-
-        def makespan(times, slots):
-            if len(times) * s.heads <= slots:
-                return max(times)
-            if len(times) <= 64 and s.heads <= slots:
-                # every block on the slot that comes free first: a tile's heads take the slots that are free soonest
-                free = np.zeros(slots)
-                for t in times:
-                    free[np.argpartition(free, s.heads - 1)[:s.heads]] += t
-                return float(free.max())
-            # many tiles: groups of slots as wide as a tile has heads, what the division leaves over given back as
-            # capacity
-            groups = slots // s.heads
-            if groups == 0:
-                return sum(times) * s.heads / slots
-            free = [0.0] * groups
-            end = 0.0
-            for t in times:
-                at = heapq.heappop(free) + t
-                heapq.heappush(free, at)
-                end = max(end, at)
-            return max(max(times), end * groups * s.heads / slots)
+        makespan = lambda times, slots: _makespan(times, slots, s.heads)
 
         slots = sms * (2 if s.head_dim == 64 else 1)
         one = 0.9 * makespan([p + each for p in pages], slots)
@@ -263,6 +266,25 @@ class Attention:
             if min(one, two) >= 0.93 * four:
                 return 2
         return best
+
+    def _tile_pages(self, tile_keys, page: int):
+        """The pages that each tile of 128 queries walks."""
+        window = self.spec.window
+        return [((min(k, window + 128) if window > 0 else k) + page - 1) // page for k in tile_keys]
+
+    def _prefill_form(self, tile_keys, page: int, device: torch.device) -> int:
+        """``_prefill_variant``, or for heads of 128 in groups of an even number two heads of a tile side by side in
+        persistent blocks, one an SM (4), where that is the shorter: an item (a tile and two heads) takes its pages and 3.5
+        pages' worth at 1.19 us a page, against 0.9 us a page and head with a tile and head a block.  32 heads on 8, us for
+        forms 1 / 4: one prompt of 1,024 tokens 24.3 / 25.7, of 1,500 44.5 / 33.9, of 6,145 465 / 316; 8 of 114 to
+        500 49.0 / 32.5; 100 tokens after 3,000 44.6 / 58.5."""
+        s = self.spec
+        one = self._prefill_variant(tile_keys, page, device)
+        if s.head_dim != 128 or (s.heads // s.kv_heads) % 2 or not tile_keys:
+            return one
+        pages, sms = self._tile_pages(tile_keys, page), K.sm_count(device)
+        pairs = 1.19 * _makespan([p + 3.5 for p in pages], sms, s.heads // 2)
+        return 4 if pairs < 0.9 * _makespan([p + 3 for p in pages], sms, s.heads) else one
 
     def _decode_split(self, T: int, max_kv_len: int, page: int, device: torch.device):
         """``(keys per chunk, head_split, in_block)`` (``in_block``: 0, 1 or 2) for the tensor-core decode kernel:

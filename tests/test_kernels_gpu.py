@@ -1082,6 +1082,55 @@ def test_attn_prefill_tc(nh, nkv, hd, window):
     assert K().attn_prefill_tc_status() == 0
 
 
+@pytest.mark.parametrize("nh,nkv", [(2, 1), (12, 2), (32, 2)])     # fewer items than SMs; groups of six; several rounds of items
+@pytest.mark.parametrize("window,chunk,keep_first,softcap", [(0, 0, 0, 0.0), (100, 0, 70, 0.0), (0, 96, 0, 20.0), (24, 0, 0, 0.0)])
+def test_attn_prefill_tc_pairs_of_heads(nh, nkv, window, chunk, keep_first, softcap):
+    """Heads of 128 in even groups: two heads of a tile side by side in persistent blocks, the numbers of a tile and head a
+    block.  Keys differ in size from page to page, so that the reference maximum moves."""
+    hd = 128
+    case = PagedCase(lens=[300, 64, 1, 1500, 65, 128, 129, 900], new=[300, 64, 1, 1000, 65, 1, 129, 900], nh=nh, nkv=nkv, hd=hd,
+                     dtype=torch.bfloat16, seed=nh + window + chunk)
+    case.k_pool.mul_((1.0 + 2.0 * (torch.arange(case.k_pool.shape[0], device=DEV) % 5)).view(-1, 1, 1, 1).bfloat16())
+    T = case.q.shape[0]
+    buf = case.q.reshape(T, nh * hd).to(DEV).contiguous()
+    g = torch.Generator().manual_seed(nh)
+    sink, gate = (3.0 * torch.rand(nh, generator=g) - 1.0).to(DEV), torch.rand(T, nh, generator=g).to(DEV)
+    tile_seq, tile_q0 = case.tiles(128)
+    outs = []
+    for variant in (1, 4):
+        o = torch.full((T, nh * hd), 3.0, device=DEV, dtype=torch.bfloat16)
+        K().attn_prefill_tc(buf, buf.stride(0), o, case.k_pool, case.v_pool, case.table, case.row_start, case.row_pos0,
+                            tile_seq, tile_q0, tile_seq.numel(), nh, nkv, hd, 64, window, 0.11, variant=variant, chunk=chunk,
+                            sink=True, keep_first=keep_first, softcap=softcap, sink_vals=sink, gate=gate)
+        torch.cuda.synchronize()
+        assert K().attn_prefill_tc_status() == 0
+        outs.append(o)
+    assert torch.isfinite(outs[0].float()).all()
+    assert torch.equal(outs[0], outs[1])
+    # against the float64 reference, without the options
+    case = PagedCase(lens=[300, 64, 1, 700, 65, 128, 129], new=[300, 64, 1, 200, 65, 1, 129], nh=nh, nkv=nkv, hd=hd,
+                     dtype=torch.bfloat16, seed=nh)
+    T = case.q.shape[0]
+    buf = case.q.reshape(T, nh * hd).to(DEV).contiguous()
+    o = torch.full((T, nh * hd), 3.0, device=DEV, dtype=torch.bfloat16)
+    tile_seq, tile_q0 = case.tiles(128)
+    K().attn_prefill_tc(buf, buf.stride(0), o, case.k_pool, case.v_pool, case.table, case.row_start, case.row_pos0, tile_seq,
+                        tile_q0, tile_seq.numel(), nh, nkv, hd, 64, window, 0.11, variant=4)
+    close(o, case.reference(window, 0.11), 1e-2, "pairs of heads")
+    assert K().attn_prefill_tc_status() == 0
+
+
+@pytest.mark.parametrize("nh,hd", [(3, 128), (2, 64)])
+def test_attn_prefill_tc_pairs_of_heads_refuses_what_it_cannot_do(nh, hd):
+    from exl3_server_b200.ops.lib import KernelLibraryError
+    case = PagedCase(lens=[70], new=[70], nh=nh, nkv=1, hd=hd, dtype=torch.bfloat16, seed=1)
+    buf = case.q.reshape(70, nh * hd).to(DEV).contiguous()
+    tile_seq, tile_q0 = case.tiles(128)
+    with pytest.raises(KernelLibraryError, match="pairs of heads"):
+        K().attn_prefill_tc(buf, buf.stride(0), torch.empty_like(buf), case.k_pool, case.v_pool, case.table, case.row_start,
+                            case.row_pos0, tile_seq, tile_q0, 1, nh, 1, hd, 64, 0, 0.1, variant=4)
+
+
 @pytest.mark.parametrize("hd", [64, 128])
 def test_attn_prefill_tc_moves_its_reference_maximum(hd):
     """Keys grow page by page, so every row's running maximum rises by far more than the kernel lets its

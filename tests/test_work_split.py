@@ -110,3 +110,15 @@ def test_float32_steps_of_few_tokens_run_token_by_token():
         assert not by_tiles(95, 32, heads, kv_heads, hd, 256, 600)
         assert by_tiles(4096, 32, heads, kv_heads, hd, 256, 4096)
     assert by_tiles(128, 8, 36, 36, 64, 256, 316) and by_tiles(600, 6, 32, 8, 128, 256, 300)
+
+
+def test_prompt_kernel_form_with_pairs_of_heads():
+    eight_b = mixer(32, 8, 128)
+    assert eight_b._prefill_form(tile_keys([1024]), 64, None) in (1, 3)  # 128 items of two heads leave SMs idle
+    assert eight_b._prefill_form(tile_keys([1500]), 64, None) == 4       # 33.9 us against 44.5
+    assert eight_b._prefill_form(tile_keys([6145]), 64, None) == 4       # 316 against 465
+    assert eight_b._prefill_form(tile_keys([181]), 64, None) == 1
+    assert eight_b._prefill_form([], 64, None) == 0
+    for sizes in ((36, 36, 64), (16, 16, 128), (24, 8, 128)):            # other heads, odd groups: never
+        for lens in ([181], [6145], [300] * 30):
+            assert mixer(*sizes)._prefill_form(tile_keys(lens), 64, None) in (1, 2, 3)
