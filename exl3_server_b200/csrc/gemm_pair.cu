@@ -14,7 +14,7 @@
 //             mbarrier; no multicast, every block copies what it needs itself
 //   warp 1    even block: one thread issues the MMAs; tcgen05.commit frees ring stages in both blocks and hands
 //             accumulators to both blocks' epilogues.  Both blocks: allocates and frees the tensor memory
-//   warps 2-  epilogue (both blocks; eight warps, four with the residual epilogue): thread = row; 64 accumulator
+//   warps 2-9 epilogue (both blocks): thread = row and half of the tile's columns; 64 accumulator
 //             columns at a time from tensor memory, results into 128B-swizzled staging tiles of 32 rows x 128
 //             bytes, which TMA stores write out (clipped at the matrix's edges), so that no thread stores a
 //             row-strided sliver itself
@@ -32,11 +32,15 @@
 // added on top of it, and the epilogue only multiplies by rho * k, adds rho * bias and writes.  (The product is
 // therefore not rounded to bfloat16 before it is added, as it is where the addition is a separate step.)
 //
+// Eight warps, since an epilogue that takes longer than its tile's products bounds the kernel at short K: 64,235 rows x 1,024,
+// K 1,024 with the residual 250 -> 193 us against four warps with four staging tiles each, K 4,096 475 -> 427.
+//
 // Epilogue 3 is the q/k/v projection of heads of 64: the output, rounded to bfloat16 as the plain epilogue would
 // store it, gets the half-split rotary encoding (queries and keys; a row's sines and cosines are computed once per
-// tile, while the products run), the queries go to y, and the keys and values go straight to the token's place in
-// the paged cache: as one TMA store where a warp's 32 rows are 32 consecutive places of one page, with 16-byte
-// stores otherwise.  The key and value columns of y are not written.
+// row of tiles, while the products run), the queries go to y, and the keys and values go straight to the token's place in
+// the paged cache: as one TMA store where a warp's 32 rows are 32 consecutive places of one page, through shared memory in
+// whole rows of 128 bytes otherwise.  The key and value columns of y are not written.  64,235 rows x 1,280, K 1,024: 217 -> 177 us
+// with eight warps and the sines kept over a row of tiles (the plain projection 130).
 //
 // Every wait on an mbarrier is bounded: when one runs out the kernel records a code, leaves its loops, waits
 // (bounded) for the copies it may have in flight, meets its partner at the cluster barrier that every path reaches,
@@ -51,17 +55,15 @@ namespace exl3 {
 using namespace tc5;
 
 constexpr int GP_BM = 256, GP_BN = 256, GP_BK = 64;
-// Epilogue warps: four (one per 32 lanes of tensor memory), or eight, two per 32 lanes with half of the columns each.
-__host__ __device__ constexpr int gp_epi_warps(int epi) { return epi >= 2 ? 4 : 8; }
-__host__ __device__ constexpr int gp_threads(int epi) { return 64 + 32 * gp_epi_warps(epi); }
+// Epilogue warps: eight, two per 32 lanes of tensor memory with half of the columns each.
+constexpr int GP_EPI_WARPS = 8, GP_EPI_THREADS = 32 * GP_EPI_WARPS, GP_THREADS = 64 + GP_EPI_THREADS;
 constexpr uint32_t GP_STAGE_A = 128 * GP_BK * 2, GP_STAGE_B = 128 * GP_BK * 2;       // per block
 constexpr uint32_t GP_BOX = 32 * 128;                                                  // a staging tile: 32 rows x 128 bytes
-__host__ __device__ constexpr int gp_stages(int) { return 5; }
-__host__ __device__ constexpr int gp_boxes(int epi) { return epi == 2 ? 4 : 2; }       // staging tiles per epilogue warp
-__host__ __device__ constexpr uint32_t gp_smem(int epi) {
-  return 1024 /* alignment */ + gp_stages(epi) * (GP_STAGE_A + GP_STAGE_B) + gp_epi_warps(epi) * gp_boxes(epi) * GP_BOX +
-         GP_BN * 4 /* norm weights */ + GP_BN * 2 /* bias */ + 256 /* barriers */;
-}
+constexpr int GP_STAGES = 5;                  // four cost 5 % at K 14,336
+constexpr int GP_BOXES = 2;                   // staging tiles per epilogue warp
+constexpr uint32_t GP_SMEM = GP_STAGES * (GP_STAGE_A + GP_STAGE_B) + GP_EPI_WARPS * GP_BOXES * GP_BOX +
+                             GP_BN * 4 /* norm weights */ + GP_BN * 2 /* bias */ + 128 * 4 /* sums of squares */ + 384 /* barriers */;
+static_assert(GP_SMEM <= 227 * 1024, "shared memory of a block");
 constexpr uint32_t GP_IDESC = idesc_bf16(GP_BM, GP_BN);
 
 static __device__ int g_gp_error = 0;
@@ -125,28 +127,28 @@ __device__ inline GpTile gp_tile(int tile, int n_m, int n_n, int group) {
 }
 
 template <int EPI>
-__global__ void __launch_bounds__(gp_threads(EPI), 1)
+__global__ void __launch_bounds__(GP_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                  const __grid_constant__ CUtensorMap map_y,      // y (0, 1) or x_raw (2): bfloat16, boxes of 64 columns
                  const __grid_constant__ CUtensorMap map_h,      // 2: the float32 residual, boxes of 32 columns
                  const __grid_constant__ CUtensorMap map_k,      // 3: the key and the value pool as rows of 64 features,
                  const __grid_constant__ CUtensorMap map_v,      //    boxes of 32 rows
                  const PairArgs a) {
-  constexpr int STAGES = gp_stages(EPI), BOXES = gp_boxes(EPI), EPI_WARPS = gp_epi_warps(EPI), EPI_THREADS = 32 * EPI_WARPS;
-  extern __shared__ unsigned char gp_smem_raw[];
-  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gp_smem_raw) + 1023) & ~(uintptr_t)1023);
-  unsigned char* sA = base;
-  unsigned char* sB = base + STAGES * GP_STAGE_A;
-  unsigned char* boxes = base + STAGES * (GP_STAGE_A + GP_STAGE_B);       // [EPI_WARPS][BOXES] staging tiles
-  float* s_normw = reinterpret_cast<float*>(boxes + EPI_WARPS * BOXES * GP_BOX);
+  constexpr int STAGES = GP_STAGES, BOXES = GP_BOXES;
+  extern __shared__ __align__(1024) unsigned char gp_smem_raw[];
+  unsigned char* sA = gp_smem_raw;
+  unsigned char* sB = sA + STAGES * GP_STAGE_A;
+  unsigned char* boxes = sB + STAGES * GP_STAGE_B;                        // [epilogue warps][BOXES] staging tiles
+  float* s_normw = reinterpret_cast<float*>(boxes + GP_EPI_WARPS * BOXES * GP_BOX);
   __nv_bfloat16* s_bias = reinterpret_cast<__nv_bfloat16*>(s_normw + GP_BN);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_bias + GP_BN);
+  float* s_sq = reinterpret_cast<float*>(s_bias + GP_BN);                 // 2: [128] a row's sum of squares over columns 128 - 255
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_sq + 128);
   uint64_t* full = bars;                       // [STAGES] even block only: both blocks' copies landed
   uint64_t* empty = bars + STAGES;             // [STAGES] each block: the MMAs that read the stage are done
   uint64_t* acc_full = bars + 2 * STAGES;      // [2] each block: accumulator complete
   uint64_t* acc_empty = acc_full + 2;          // [2] even block only: both blocks' epilogues are done with it
-  uint64_t* hbar = acc_empty + 2;              // [4 warps][4] epilogue 2: a tile of h landed in a staging tile
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(hbar + 16);
+  uint64_t* hbar = acc_empty + 2;              // [epilogue warps][2] epilogue 2: a tile of h landed in a staging tile
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(hbar + 2 * GP_EPI_WARPS);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();        // 0: issues the MMAs
@@ -158,8 +160,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     if (EPI == 2) prefetch_map(&map_h);
     if (EPI == 3) { prefetch_map(&map_k); prefetch_map(&map_v); }
     for (int s = 0; s < STAGES; ++s) { mbar_init(full + s, 1); mbar_init(empty + s, 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, 2 * EPI_WARPS); }
-    for (int i = 0; i < 16; ++i) mbar_init(hbar + i, 1);
+    for (int b = 0; b < 2; ++b) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, 2 * GP_EPI_WARPS); }
+    for (int i = 0; i < 2 * GP_EPI_WARPS; ++i) mbar_init(hbar + i, 1);
     mbar_init_fence();
   }
   if (warp == 1) tmem_alloc_pair<512>(tmem_slot);
@@ -178,12 +180,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   // start from zero in the first at once, and the epilogue adds the two.  (With several tiles per pair both
   // accumulators are in use in turn, and the residual goes into the accumulator before the tile's products.)
   const bool beside = EPI == 2 && n_tiles <= n_pairs;
+  // The pair's tiles.  3: neighbours in the order (columns fastest there), so that a row's sines and cosines, 32 of each,
+  // are worked out once for all of the pair's tiles in a row; else dealt round-robin.
+  const int tile_first = EPI == 3 ? (int)((int64_t)n_tiles * pair / n_pairs) : pair;
+  const int tile_end = EPI == 3 ? (int)((int64_t)n_tiles * (pair + 1) / n_pairs) : n_tiles;
+  const int tile_step = EPI == 3 ? 1 : n_pairs;
   bool ok = true;
 
   if (warp == 0) {
     // ---- producer: this block's halves of the pair's tiles ---------------------------------------------
     uint32_t it = 0;
-    for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
+    for (int tile = tile_first; tile < tile_end && ok; tile += tile_step) {
       const GpTile at = gp_tile(tile, n_m, n_n, a.group);
       const int m0 = at.m * GP_BM + (int)rank * 128, n0 = at.n * GP_BN + (int)rank * 128;
       for (int kb = 0; kb < kblocks; ++kb, ++it) {
@@ -213,7 +220,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     // ---- MMA issuer (even block) ----------------------------------------------------------------------------
     if (rank == 0) {
       uint32_t it = 0, tcount = 0;
-      for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, ++tcount) {
+      for (int tile = tile_first; tile < tile_end && ok; tile += tile_step, ++tcount) {
         const uint32_t buf = tcount & 1;
         // 0, 1: an accumulator is free from the start and after each epilogue; 2: it is ready when the epilogue
         // warps have put the tile's residual into it
@@ -244,14 +251,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     // ---- epilogue: thread = row of this block's 128 -----------------------------------------------------------
     const int q = warp & 3;                               // the 32 TMEM lanes this warp may read
     const int t = (warp - 2) * 32 + lane;
-    // with eight warps, warps 2-5 take the tile's columns 0-127 and warps 6-9 the columns 128-255
-    const int s_lo = EPI_WARPS == 8 ? ((warp - 2) >> 2) * 2 : 0, s_hi = s_lo + (EPI_WARPS == 8 ? 2 : 4);
+    // warps 2-5 take the tile's columns 0-127 and warps 6-9 the columns 128-255, 64 at a time
+    const int s_lo = ((warp - 2) >> 2) * 2, s_hi = s_lo + 2;
     unsigned char* my_boxes = boxes + (warp - 2) * BOXES * GP_BOX;
-    uint64_t* my_hbar = hbar + q * 4;
+    uint64_t* my_hbar = hbar + (warp - 2) * 2;
     const uint32_t acc_empty_addr[2] = {cluster_addr(acc_empty, 0), cluster_addr(acc_empty + 1, 0)};
     const uint32_t lane_taddr = tmem_base + ((uint32_t)(q * 32) << 16);
     uint32_t n_store = 0;                                 // 0, 1: staging tiles stored so far (they alternate)
-    uint32_t n_hload = 0;                                 // 2: tiles of h loaded so far (four staging tiles in turn)
+    uint32_t n_hload = 0;                                 // 2: tiles of h loaded so far (the staging tiles in turn)
 
     // k of a row: what its accumulator is multiplied by
     auto row_factor = [&](int row) {
@@ -263,23 +270,26 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       }
       return k;
     };
-    // 2: this warp's 32 rows of a tile of h into accumulator `buf`: divided by rho * k, and the accumulator is then
-    // handed to the MMA issuer; or as they are, beside the products.  False when a wait ran out.
+    // 2: this warp's 32 rows and 128 columns of a tile of h into accumulator `buf`: divided by rho * k, and the accumulator is
+    // then handed to the MMA issuer; or as they are, beside the products.  False when a wait ran out.
     auto preload = [&](int tile, uint32_t buf) -> bool {
       const GpTile at = gp_tile(tile, n_m, n_n, a.group);
-      const int row0 = at.m * GP_BM + (int)rank * 128 + q * 32, n0 = at.n * GP_BN;
+      const int row0 = at.m * GP_BM + (int)rank * 128 + q * 32, n0 = at.n * GP_BN + s_lo * 64;
       const float inv = beside ? 1.0f : 1.0f / (a.rho * row_factor(row0 + lane));
       if (lane == 0) tma_store_wait_read<0>();            // the last epilogue's stores have read the staging tiles
       __syncwarp();
-      if (lane == 0)
-        for (int c = 0; c < 4; ++c) {
-          mbar_expect_tx(my_hbar + c, GP_BOX);
-          tma_load_2d(my_boxes + c * GP_BOX, &map_h, my_hbar + c, n0 + c * 32, row0);
+      auto ask = [&](int c) {                             // tile c of the four (n_hload is even here)
+        if (lane == 0) {
+          mbar_expect_tx(my_hbar + (c & 1), GP_BOX);
+          tma_load_2d(my_boxes + (c & 1) * GP_BOX, &map_h, my_hbar + (c & 1), n0 + c * 32, row0);
         }
+      };
+      ask(0);
+      ask(1);
       bool good = true;
-      for (int c = 0; c < GP_BN / 32; ++c, ++n_hload) {
-        const int k = n_hload & 3;
-        good = __all_sync(0xffffffffu, mbar_wait(my_hbar + k, (n_hload >> 2) & 1));
+      for (int c = 0; c < GP_BN / 2 / 32; ++c, ++n_hload) {
+        const uint32_t k = n_hload & 1;
+        good = __all_sync(0xffffffffu, mbar_wait(my_hbar + k, (n_hload >> 1) & 1));
         if (!good) break;
         uint32_t f[32];
         unsigned char* box = my_boxes + k * GP_BOX;
@@ -292,11 +302,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
           f[4 * j + 3] = __float_as_uint(__uint_as_float(v.w) * inv);
         }
         __syncwarp();                                     // every lane has read the staging tile
-        if (lane == 0 && c + 4 < GP_BN / 32) {
-          mbar_expect_tx(my_hbar + k, GP_BOX);
-          tma_load_2d(box, &map_h, my_hbar + k, n0 + (c + 4) * 32, row0);
-        }
-        gp_tmem_st32(lane_taddr + buf * GP_BN + c * 32, f);
+        if (c + 2 < GP_BN / 2 / 32) ask(c + 2);
+        gp_tmem_st32(lane_taddr + buf * GP_BN + s_lo * 64 + c * 32, f);
       }
       if (!good) {
         // loads that may still be in flight get the time to land before the block's shared memory goes away
@@ -318,16 +325,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         for (uint32_t b = 0; b < 2 && tile < n_tiles && ok; ++b, tile += n_pairs) ok = preload(tile, b);
       }
     }
+    float rc[EPI == 3 ? 32 : 1], rs[EPI == 3 ? 32 : 1];
+    int my_pos = 0, my_page = -1, pos0 = 0, page0 = -1, rope_m = -1;
+    bool together = false;
     uint32_t tcount = 0;
-    for (int tile = pair; tile < n_tiles; tile += n_pairs, ++tcount) {
+    for (int tile = tile_first; tile < tile_end; tile += tile_step, ++tcount) {
       const GpTile at = gp_tile(tile, n_m, n_n, a.group);
       const int row0 = at.m * GP_BM + (int)rank * 128 + q * 32, n0 = at.n * GP_BN;
       const uint32_t buf = tcount & 1;
       const int row = row0 + lane;
       // the tile's bias and norm weights, once for all rows (the previous tile's readers are past their last read:
       // they have met at the barrier after it); every thread comes here, whatever its outcome so far
-      if (!gp_epilogue_all<EPI_THREADS>(ok)) { ok = false; break; }
-      for (int c = t; c < GP_BN; c += EPI_THREADS) {
+      if (!gp_epilogue_all<GP_EPI_THREADS>(ok)) { ok = false; break; }
+      for (int c = t; c < GP_BN; c += GP_EPI_THREADS) {
         const int n = n0 + c;
         s_bias[c] = (a.bias && n < a.N) ? a.bias[n] : __float2bfloat16(0.0f);
         if (EPI == 2)
@@ -338,28 +348,37 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       const float k_bias = EPI == 2 ? a.rho : 1.0f;
       const bool plain = a.bias == nullptr && a.ss_in == nullptr && EPI != 2;      // the accumulator as it is
       // 3: the row's sines and cosines, its page, and whether the warp's rows are 32 consecutive places of one
-      // page (all of this while the tile's products run)
-      float rc[EPI == 3 ? 32 : 1], rs[EPI == 3 ? 32 : 1];
-      int my_pos = 0, my_page = -1, pos0 = 0, page0 = -1;
-      bool together = false;
-      if (EPI == 3) {
+      // page (all of this while the tile's products run, and again only in another row of tiles)
+      if (EPI == 3 && at.m != rope_m) {
+        rope_m = at.m;
         int my_seq = -1;
+        my_pos = 0;
+        my_page = -1;
         if (row < a.M) { my_pos = __ldg(a.tok_pos + row); my_seq = __ldg(a.tok_seq + row); }
         const float p = (float)my_pos * a.pos_scale;
-#pragma unroll
+        // Through the staging tiles (8 KB: 64 numbers a lane), so that the loop need not be unrolled for the registers' sake:
+        // 32 copies of sincosf are more code than the instruction cache holds (64,235 rows x 1,280, K 1,024: 190 -> 177 us).
+        if (lane == 0) tma_store_wait_read<0>();
+        __syncwarp();
+        float* mine = reinterpret_cast<float*>(my_boxes) + lane;
+#pragma unroll 2
         for (int d = 0; d < 32; ++d) {
-          if (a.inv_freq) rope_sincos(p, __ldg(a.inv_freq + d), a.inv_freq_lo ? __ldg(a.inv_freq_lo + d) : 0.0f, &rs[d], &rc[d]);
-          else { rc[d] = 1.0f; rs[d] = 0.0f; }
+          float sn = 0.0f, cs = 1.0f;
+          if (a.inv_freq) rope_sincos(p, __ldg(a.inv_freq + d), a.inv_freq_lo ? __ldg(a.inv_freq_lo + d) : 0.0f, &sn, &cs);
+          mine[32 * d] = sn;
+          mine[32 * (32 + d)] = cs;
         }
+#pragma unroll
+        for (int d = 0; d < 32; ++d) { rs[d] = mine[32 * d]; rc[d] = mine[32 * (32 + d)]; }
         if (a.write_kv && row < a.M) my_page = __ldg(a.block_table + (int64_t)my_seq * a.bt_stride + my_pos / 64);
         pos0 = __shfl_sync(0xffffffffu, my_pos, 0);
         page0 = __shfl_sync(0xffffffffu, my_page, 0);
         const int seq0 = __shfl_sync(0xffffffffu, my_seq, 0);
-        together = __all_sync(0xffffffffu, row < a.M && my_seq == seq0 && my_pos == pos0 + lane && my_page >= 0) && (pos0 & 31) == 0;
+        together = __all_sync(0xffffffffu, row < a.M && my_seq == seq0 && my_pos == pos0 + lane && my_page >= 0) && (pos0 & 63) <= 32;
       }
       // (also the barrier after which the staged bias and norm weights may be read) one outcome for all epilogue
       // threads, so that they leave the loop together
-      if (!gp_epilogue_all<EPI_THREADS>(mbar_wait(acc_full + buf, (tcount >> 1) & 1))) { ok = false; break; }
+      if (!gp_epilogue_all<GP_EPI_THREADS>(mbar_wait(acc_full + buf, (tcount >> 1) & 1))) { ok = false; break; }
       fence_after();
       const uint32_t taddr = lane_taddr + buf * GP_BN;
       float sq = 0.0f;
@@ -455,11 +474,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 }
               }
               ++n_store;
-            } else if (a.write_kv && row < a.M && my_page >= 0) {
-              uint4* dst = reinterpret_cast<uint4*>((is_k ? a.k_pool : a.v_pool) +
-                                                    (((int64_t)my_page * a.nkv + g) * 64 + (my_pos & 63)) * 64);
+            } else if (a.write_kv) {
+              // rows here and there: through the staging tile, eight lanes a row, so that a row's 128 bytes go out as one line
+              unsigned char* box = my_boxes + (n_store & 1) * GP_BOX;
 #pragma unroll
-              for (int j = 0; j < 8; ++j) dst[j] = o[j];
+              for (int j = 0; j < 8; ++j) *gp_box_chunk(box, lane, j) = o[j];
+              __syncwarp();
+              __nv_bfloat16* pool = is_k ? a.k_pool : a.v_pool;
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const int r = 4 * i + (lane >> 3), j = lane & 7;
+                const int page = __shfl_sync(0xffffffffu, my_page, r), pos = __shfl_sync(0xffffffffu, my_pos, r);
+                if (page >= 0)
+                  reinterpret_cast<uint4*>(pool + (((int64_t)page * a.nkv + g) * 64 + (pos & 63)) * 64)[j] = *gp_box_chunk(box, r, j);
+              }
             }
           }
         } else if (EPI == 1) {
@@ -486,43 +514,43 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
           }
         } else {
           // v is the new h (columns beyond N: zero in h, in the products and in the staged bias).  Per step two
-          // float32 tiles of it and one bfloat16 tile of x_raw go out, in this order; a staging tile is written
-          // again a step later (x_raw's: two steps), when all but the two newest stores have read theirs.
-          unsigned char* xbox = my_boxes + (2 + (s & 1)) * GP_BOX;
+          // float32 tiles of it and one bfloat16 tile of x_raw go out, in this order, through the two staging tiles in
+          // turn: one is written again when all but the newest store have read theirs.
 #pragma unroll
           for (int j = 0; j < 64; ++j) sq = fmaf(v[j], v[j], sq);
 #pragma unroll
-          for (int half = 0; half < 2; ++half) {
-            unsigned char* hbox = my_boxes + half * GP_BOX;
-            if (lane == 0) tma_store_wait_read<2>();
+          for (int part = 0; part < 3; ++part) {
+            unsigned char* box = my_boxes + ((s + part) & 1) * GP_BOX;     // (three a step: the steps alternate)
+            if (lane == 0) tma_store_wait_read<1>();
             __syncwarp();
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-              const float* f = v + 32 * half + 4 * j;
-              *gp_box_chunk(hbox, lane, j) = make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]), __float_as_uint(f[3]));
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float* f = v + 32 * half + 8 * j;
-              const float* wn = s_normw + s * 64 + 32 * half + 8 * j;
-              *gp_box_chunk(xbox, lane, 4 * half + j) = make_uint4(gp_pack(f[0] * wn[0], f[1] * wn[1]), gp_pack(f[2] * wn[2], f[3] * wn[3]),
-                                                                   gp_pack(f[4] * wn[4], f[5] * wn[5]), gp_pack(f[6] * wn[6], f[7] * wn[7]));
+              if (part < 2) {
+                const float* f = v + 32 * (part & 1) + 4 * j;
+                *gp_box_chunk(box, lane, j) = make_uint4(__float_as_uint(f[0]), __float_as_uint(f[1]), __float_as_uint(f[2]), __float_as_uint(f[3]));
+              } else {
+                const float* f = v + 8 * j;
+                const float* wn = s_normw + s * 64 + 8 * j;
+                *gp_box_chunk(box, lane, j) = make_uint4(gp_pack(f[0] * wn[0], f[1] * wn[1]), gp_pack(f[2] * wn[2], f[3] * wn[3]),
+                                                         gp_pack(f[4] * wn[4], f[5] * wn[5]), gp_pack(f[6] * wn[6], f[7] * wn[7]));
+              }
             }
             fence_smem_to_tma();
             __syncwarp();
             if (lane == 0 && row0 < a.M) {
-              if (n0 + s * 64 + 32 * half < a.N) tma_store_2d(&map_h, hbox, n0 + s * 64 + 32 * half, row0);
+              const int col = n0 + s * 64 + (part == 1 ? 32 : 0);
+              if (col < a.N) tma_store_2d(part < 2 ? &map_h : &map_y, box, col, row0);
               else tma_store_skip();
-              if (half == 1) {
-                if (n0 + s * 64 < a.N) tma_store_2d(&map_y, xbox, n0 + s * 64, row0);
-                else tma_store_skip();
-              }
             }
           }
         }
       }
       if (EPI == 2) {
-        if (row < a.M) a.ss_out[(int64_t)row * n_n + at.n] = sq;
+        // a row's two halves meet (the barrier is also the one after which s_sq may be written again: two more stand between)
+        const bool upper = s_lo > 0;
+        if (upper) s_sq[q * 32 + lane] = sq;
+        asm volatile("bar.sync 2, %0;" ::"n"(GP_EPI_THREADS) : "memory");
+        if (!upper && row < a.M) a.ss_out[(int64_t)row * n_n + at.n] = sq + s_sq[q * 32 + lane];
         // the accumulator is free: the tile after next of this pair goes into it (or nobody waits for it)
         const int next = tile + 2 * n_pairs;
         fence_before();
@@ -552,8 +580,8 @@ template <int EPI> static const void* gp_kernel() { return reinterpret_cast<cons
 static void gp_launch_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int blocks, int epi, cudaStream_t stream) {
   *cfg = cudaLaunchConfig_t{};
   cfg->gridDim = dim3(blocks);
-  cfg->blockDim = dim3(gp_threads(epi));
-  cfg->dynamicSmemBytes = gp_smem(epi);
+  cfg->blockDim = dim3(GP_THREADS);
+  cfg->dynamicSmemBytes = GP_SMEM;
   cfg->stream = stream;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
@@ -605,11 +633,11 @@ static int gp_run(const void* x, const void* w, const void* bias, void* y, int M
   if (ss_in && (ss_blocks < 1 || !(width > 0.0f))) { set_error("gemm_pair: the norm's pieces need blocks >= 1 and a width"); return ERR_BAD_ARGUMENT; }
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gp_smem(0));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_pair_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gp_smem(1));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_pair_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gp_smem(2));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_pair_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gp_smem(3));
-    if (e != cudaSuccess) { set_error("gemm_pair: cannot get %u bytes of shared memory: %s", gp_smem(2), cudaGetErrorString(e)); return (int)e; }
+    cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_pair_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_pair_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_pair_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
+    if (e != cudaSuccess) { set_error("gemm_pair: cannot get %u bytes of shared memory: %s", GP_SMEM, cudaGetErrorString(e)); return (int)e; }
     configured = true;
   }
   CUtensorMap map_x, map_w, map_y, map_h, map_k, map_v;
@@ -641,7 +669,8 @@ static int gp_run(const void* x, const void* w, const void* bias, void* y, int M
   // does not stay either, each group reads it again, so the groups are larger (4,096 x 4,096, K 16,384: 438 us whole and
   // in twelves, 445 in eights; 6,145 x 28,672, K 4,096: 1,265 whole, 1,242 in twelves).  The sums are the same in any order.
   const bool x_stays = (int64_t)M * K * 2 <= (40 << 20), w_stays = (int64_t)N * K * 2 <= (64 << 20);
-  a.group = ceil_div(M, GP_BM);
+  // (The rotated projection has columns fastest: see the kernel.)
+  a.group = epilogue == 3 ? 1 : ceil_div(M, GP_BM);
   if (!x_stays && a.group > (w_stays ? 8 : 12)) a.group = w_stays ? 8 : 12;
   const int max_pairs = gp_max_pairs(epilogue);
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
