@@ -195,10 +195,17 @@ class SequenceCache:
         self.lengths[slot] = 0
         for g in self.groups:
             g.pages[slot] = []
-        for t in self.state.values():
-            for part in (t if isinstance(t, tuple) else (t,)):
-                part[slot].zero_()
+        self._zero_state(slot)
         return slot
+
+    def _zero_state(self, slot: int) -> None:
+        parts = [p for t in self.state.values() for p in (t if isinstance(t, tuple) else (t,)) if p.numel()]
+        if len(parts) > 1 and all(p.is_cuda and p.device.index == torch.cuda.current_device() for p in parts):
+            from ..ops import kernels as K
+            K.zero_rows(parts, slot)                     # one launch for all of them
+        else:
+            for part in parts:
+                part[slot].zero_()
 
     def close(self, slot: int) -> None:
         self.slots.free(slot)                           # raises if the slot is not live

@@ -13,6 +13,8 @@ const char* exl3_last_error();
 int exl3_abi_version();
 long long exl3_launch_count();
 
+// Row `row` of each of the n tensors (base address, bytes of a row) becomes zero.
+int exl3_zero_rows(void* const* bases, const long long* row_bytes, int n, long long row, cudaStream_t stream);
 int exl3_embed(const int* ids, const void* table, int table_dtype, float* h, int T, int H, int V,
                float scale, cudaStream_t stream);
 int exl3_add_rmsnorm(float* h, const void* y, int y_dtype, float y_scale, const void* w, int w_dtype,

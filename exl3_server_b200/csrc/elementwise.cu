@@ -441,3 +441,42 @@ extern "C" int exl3_softcap(float* x, int64_t n, float cap, cudaStream_t stream)
   launch_pdl(exl3::softcap_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, x, n, cap, 1.0f / cap);
   return launch_status("softcap");
 }
+
+namespace exl3 {
+// Row `row` of up to ZERO_PARTS tensors becomes zero: the fixed-size state of a sequence that starts, in one launch (a fill a
+// tensor cost the host some 10 us each, 63 of them for eight sequences of a decoder of eight layers).
+constexpr int ZERO_PARTS = 96;
+struct ZeroRows { unsigned char* at[ZERO_PARTS]; long long bytes[ZERO_PARTS]; };
+__global__ void __launch_bounds__(256) zero_rows_kernel(const __grid_constant__ ZeroRows z) {
+  unsigned char* at = z.at[blockIdx.y];
+  const long long n = z.bytes[blockIdx.y], step = (long long)gridDim.x * blockDim.x, i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (((reinterpret_cast<uintptr_t>(at) | (uintptr_t)n) & 15) == 0) {
+    for (long long i = i0; i < n / 16; i += step) reinterpret_cast<uint4*>(at)[i] = make_uint4(0, 0, 0, 0);
+  } else {
+    for (long long i = i0; i < n; i += step) at[i] = 0;
+  }
+}
+}  // namespace exl3
+
+extern "C" int exl3_zero_rows(void* const* bases, const long long* row_bytes, int n, long long row, cudaStream_t stream) {
+  if (n == 0) return 0;
+  if (n < 0 || row < 0 || bases == nullptr || row_bytes == nullptr) { set_error("zero_rows: bad arguments"); return ERR_BAD_ARGUMENT; }
+  for (int i0 = 0; i0 < n; i0 += ZERO_PARTS) {
+    ZeroRows z = {};
+    const int m = n - i0 < ZERO_PARTS ? n - i0 : ZERO_PARTS;
+    long long most = 0;
+    for (int i = 0; i < m; ++i) {
+      if (bases[i0 + i] == nullptr || row_bytes[i0 + i] < 0) { set_error("zero_rows: bad part %d", i0 + i); return ERR_BAD_ARGUMENT; }
+      z.at[i] = static_cast<unsigned char*>(bases[i0 + i]) + row * row_bytes[i0 + i];
+      z.bytes[i] = row_bytes[i0 + i];
+      if (z.bytes[i] > most) most = z.bytes[i];
+    }
+    // a block takes 16 KB of a part, at most 64 blocks a part (a row of state is some hundred KB)
+    long long blocks = (most + 16383) / 16384;
+    blocks = blocks < 1 ? 1 : blocks > 64 ? 64 : blocks;
+    zero_rows_kernel<<<dim3((unsigned)blocks, (unsigned)m), 256, 0, stream>>>(z);
+    const int rc = launch_status("zero_rows");
+    if (rc) return rc;
+  }
+  return 0;
+}

@@ -1174,6 +1174,18 @@ def argmax_step(logits: torch.Tensor, out: torch.Tensor, feed: torch.Tensor, pos
                                 _ptr(scratch), _c_size_t(need), _stream()), "argmax_step")
 
 
+def zero_rows(parts, row: int) -> None:
+    """Row ``row`` of every tensor of ``parts`` (contiguous, on the current device) becomes zero, in one launch."""
+    n = len(parts)
+    for t in parts:
+        _contig(t, "zero_rows")
+        if not 0 <= row < t.shape[0]:
+            raise KernelLibraryError(f"zero_rows: row {row} of {t.shape[0]}")
+    bases = (ctypes.c_void_p * n)(*[t.data_ptr() for t in parts])
+    sizes = (ctypes.c_longlong * n)(*[t.stride(0) * t.element_size() if t.dim() > 1 else t.element_size() for t in parts])
+    _check(library().exl3_zero_rows(bases, sizes, _c_int(n), _c_int64(row), _stream()), "zero_rows")
+
+
 def sample_filtered_cap() -> int:
     """The most candidates the device sampler ranks (``top_k`` above it is the host sampler's)."""
     return int(library().exl3_sample_filtered_cap())

@@ -550,6 +550,26 @@ def test_gemm_pair_rotates_and_writes_the_cache(lens, starts, nh, nkv, rot):
     assert K().gemm_pair_status() == 0
 
 
+@pytest.mark.parametrize("shapes", [[(5, 64, 128), (5,), (5, 2048)],            # states as the recurrent layers have them
+                                    [(3, 7), (3, 1), (3, 5, 3)],                # rows that are no multiple of 16 bytes
+                                    [(4, 3)] * 97 + [(4, 300000)]])             # more parts than one launch takes
+def test_zero_rows_clears_one_row_of_every_part(shapes):
+    g = torch.Generator().manual_seed(1)
+    for dtype in (torch.float32, torch.bfloat16, torch.int32):
+        parts = [torch.randint(1, 100, s, generator=g).to(dtype).to(DEV) for s in shapes]
+        want = [p.clone() for p in parts]
+        for w in want:
+            w[2].zero_()
+        K().zero_rows(parts, 2)
+        assert all(torch.equal(p, w) for p, w in zip(parts, want))
+
+
+def test_zero_rows_refuses_a_row_that_is_not_there():
+    from exl3_server_b200.ops.lib import KernelLibraryError
+    with pytest.raises(KernelLibraryError, match="row 3 of 3"):
+        K().zero_rows([torch.zeros(3, 4, device=DEV)], 3)
+
+
 @pytest.mark.parametrize("M,N,Kd", [(5300, 520, 4096),       # x is larger than what stays in L2: rows of tiles in eights, five left over
                                     (3400, 4200, 8192)])     # and w as well: twelves, two left over
 def test_gemm_pair_walks_rows_of_tiles_in_groups(M, N, Kd):
