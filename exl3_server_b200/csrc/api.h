@@ -310,6 +310,10 @@ int exl3_sample_filtered(const float* logits, const double* rows, int* out, int 
 int exl3_sample_rows(const float* logits, const double* rows, int* const* counts, const float* params, int* out, int R,
                      int V, cudaStream_t stream);
 int exl3_sample_filtered_cap();
+// The same for up to exl3_sample_direct_rows() rows whose options are still on the host (see sampling_filtered.cu).
+int exl3_sample_direct_rows();
+int exl3_sample_batch(const float* logits, const void* packed, int R, int V, int shared_counts, int* out, int* host_out,
+                      cudaStream_t stream);
 // counts: R device pointers (null: none) to int32 [V] token counts of the rows' contexts; params: float32 [R, 3] =
 // repetition, presence and frequency penalty.  Changes logits in place.  exl3_sample_count adds the chosen tokens.
 int exl3_sample_penalties(float* logits, int R, int V, const int* const* counts, const float* params,

@@ -30,6 +30,7 @@
 #include "common.cuh"
 
 #include <math.h>
+#include <string.h>
 
 #include <algorithm>
 
@@ -49,6 +50,14 @@ __device__ inline float sf_value(uint32_t k) {
 
 struct SfRow {            // one row's options, as the host gives them (float64 [R, 5])
   double temperature, top_k, top_p, min_p, u;
+};
+
+// Up to so many rows come as a parameter of the kernel: no buffer to make and to copy (some 25 us of the host's time a call).
+constexpr int SF_DIRECT_ROWS = 64;
+struct SfBatch {
+  SfRow rows[SF_DIRECT_ROWS];
+  int* counts[SF_DIRECT_ROWS];
+  float params[SF_DIRECT_ROWS][3];
 };
 
 constexpr double SF_FIXED_US = 35.0, SF_STAGED_US = 0.00018, SF_AGAIN_US = 0.00033, SF_AGAIN_PENALTIES_US = 0.00075;
@@ -76,6 +85,8 @@ __device__ inline float sf_penalised(float x, int count, float rep, float presen
   return x;
 }
 
+// rows, counts, params: null, and `batch` holds them (with host_out, a page-locked copy of out, or null; count_now: no two
+// rows share their counts, so a row's token joins them at once).
 // counts: null, or per row a pointer to its token counts [V] (null: the row has no penalties); params [R, 3]: repetition,
 // presence, frequency.  The counts are only read: rows may share them, so the chosen tokens join them in a kernel of their
 // own, after every row has been drawn (2 us for 32 rows).  STAGED: the block's part of the row is kept in shared memory;
@@ -84,7 +95,8 @@ __device__ inline float sf_penalised(float x, int count, float rep, float presen
 template <bool STAGED, bool PENALTIES>
 __global__ void __launch_bounds__(SF_THREADS)
 sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict__ rows, const int* const* __restrict__ counts,
-                       const float* __restrict__ params, int* __restrict__ out, int V, int blocks) {
+                       const float* __restrict__ params, int* __restrict__ out, int V, int blocks,
+                       const __grid_constant__ SfBatch batch, int* host_out, bool count_now) {
   extern __shared__ __align__(16) unsigned char sf_smem[];
   unsigned* hists = reinterpret_cast<unsigned*>(sf_smem);                                      // [2][SF_BINS]
   unsigned long long* cand = reinterpret_cast<unsigned long long*>(sf_smem + 2 * SF_BINS * 4);  // the first block's: all
@@ -99,15 +111,21 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int row_id = blockIdx.x / blocks, rank = blockIdx.x % blocks;
   const float* row = logits + (int64_t)row_id * V;
-  const SfRow o = rows[row_id];
+  const SfRow o = rows ? rows[row_id] : batch.rows[row_id];
   const int M = V < SF_CAP ? V : SF_CAP;
-  const int* count = PENALTIES && counts ? counts[row_id] : nullptr;
+  const int* count = !PENALTIES ? nullptr : rows ? (counts ? counts[row_id] : nullptr) : batch.counts[row_id];
   float rep = 1.0f, presence = 0.0f, frequency = 0.0f;
   if (count) {
-    rep = params[3 * row_id];
-    presence = params[3 * row_id + 1];
-    frequency = params[3 * row_id + 2];
+    rep = rows ? params[3 * row_id] : batch.params[row_id][0];
+    presence = rows ? params[3 * row_id + 1] : batch.params[row_id][1];
+    frequency = rows ? params[3 * row_id + 2] : batch.params[row_id][2];
   }
+  // the row's token, from the thread that knows it; all of the row's blocks have read its counts by then
+  auto chosen = [&](int t) {
+    out[row_id] = t;
+    if (host_out) host_out[row_id] = t;
+    if (count && count_now && t >= 0 && t < V) atomicAdd(const_cast<int*>(count) + t, 1);
+  };
   const int per = (V + blocks - 1) / blocks;
   const int first = min(V, rank * per), n = min(V, first + per) - first;
   // f(value's key, place in the row) for every token of this block's part
@@ -297,7 +315,7 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
   }
   auto token_of = [&](int i) { return (int)(~(unsigned)(cand[i] & 0xffffffffull)); };
   if (!(o.temperature > 0.0)) {                  // greedy: the first maximum
-    if (tid == 0) out[row_id] = token_of(0);
+    if (tid == 0) chosen(token_of(0));
     return;
   }
 
@@ -337,7 +355,7 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
   __syncthreads();
   const double total = acc[M - 1];
   if (!(total > 0.0)) {
-    if (tid == 0) out[row_id] = token_of(0);
+    if (tid == 0) chosen(token_of(0));
     return;
   }
   int keep = M;
@@ -360,7 +378,7 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
   for (int i = tid; i < keep; i += SF_THREADS)
     if (acc[i] >= r) atomicMin(&first_draw, i);
   __syncthreads();
-  if (tid == 0) out[row_id] = token_of(first_draw < keep ? first_draw : keep - 1);
+  if (tid == 0) chosen(token_of(first_draw < keep ? first_draw : keep - 1));
 }
 
 // Penalties over a row's context (src/model.cpp:672-686).  counts[r] points to the row's token counts [V]
@@ -386,6 +404,14 @@ __global__ void sample_count_kernel(int* const* __restrict__ counts, const int* 
   if (t >= 0 && t < V) atomicAdd(counts[row] + t, 1);
 }
 
+struct SfCounts { int* at[SF_DIRECT_ROWS]; };
+__global__ void sample_count_batch_kernel(const __grid_constant__ SfCounts counts, const int* __restrict__ ids, int R, int V) {
+  const int row = threadIdx.x;
+  if (row >= R || counts.at[row] == nullptr) return;
+  const int t = ids[row];
+  if (t >= 0 && t < V) atomicAdd(counts.at[row] + t, 1);
+}
+
 }  // namespace exl3
 
 using namespace exl3;
@@ -393,13 +419,9 @@ using namespace exl3;
 // rows: float64 [R, 5] on the device: temperature (<= 0: greedy), top_k (0: off, at most 2048), top_p, min_p and
 // the row's uniform number in [0, 1).  out: int32 [R].  counts (may be null): as in exl3_sample_penalties, with params;
 // the penalties are applied as the logits are read, and the chosen tokens are counted when all rows have been drawn.
-extern "C" int exl3_sample_rows(const float* logits, const double* rows, int* const* counts, const float* params, int* out,
-                                int R, int V, cudaStream_t stream) {
-  if (R == 0) return 0;
-  if (R < 0 || V < 1 || (counts != nullptr && params == nullptr)) {
-    set_error("sample_filtered: bad sizes rows=%d vocab=%d, or penalties without their constants", R, V);
-    return ERR_BAD_ARGUMENT;
-  }
+// batch: the rows themselves, then rows, counts and params are null.
+static int sf_launch(const float* logits, const double* rows, int* const* counts, const float* params, int* out, int R, int V,
+                     const SfBatch& batch, bool penalties, int* host_out, bool count_now, cudaStream_t stream) {
   // Blocks a row.  An SM holds one block, and the SMs come in eight groups that a cluster must fit into; a wave of rows takes
   // some 35 us and, for a token of a block's part, 0.18 ns, or 0.33 (0.75 with penalties) where the part is too long for
   // shared memory and read in every pass.  With 8 / 4 / 2 / 1 blocks: 32 rows of 122,753 86 / 41 / 55 / 76 us, 148 rows 280 /
@@ -414,7 +436,7 @@ extern "C" int exl3_sample_rows(const float* logits, const double* rows, int* co
     const int each = ceil_div(V, b);
     const int at_once = b == 1 ? sms : 8 * std::max(1, sms / 8 / b);
     const double waves = (double)((R + at_once - 1) / at_once);
-    const double a_token = (size_t)each * 4 <= MOST ? SF_STAGED_US : counts ? SF_AGAIN_PENALTIES_US : SF_AGAIN_US;
+    const double a_token = (size_t)each * 4 <= MOST ? SF_STAGED_US : penalties ? SF_AGAIN_PENALTIES_US : SF_AGAIN_US;
     const double cost = waves * (SF_FIXED_US + a_token * each);
     if (b == 8 || cost < best) {
       best = cost;
@@ -424,7 +446,7 @@ extern "C" int exl3_sample_rows(const float* logits, const double* rows, int* co
   const size_t part = (size_t)ceil_div(V, blocks) * 4;
   const bool staged = part <= MOST;
   auto kernel = staged ? sample_filtered_kernel<true, true>
-                       : counts ? sample_filtered_kernel<false, true> : sample_filtered_kernel<false, false>;
+                       : penalties ? sample_filtered_kernel<false, true> : sample_filtered_kernel<false, false>;
   const size_t smem = SF_HEAD_BYTES + (staged ? part : 0);
   // The limit belongs to the function and not to this call: the same number from every thread, whatever its rows take, or a
   // thread with shorter rows would lower it between another one's setting it and its launch.
@@ -448,10 +470,64 @@ extern "C" int exl3_sample_rows(const float* logits, const double* rows, int* co
   cfg.attrs = attr;
   cfg.numAttrs = blocks > 1 ? 1 : 0;               // without a cluster blocks are spread over the SMs first
   cudaLaunchKernelEx(&cfg, kernel, logits, reinterpret_cast<const SfRow*>(rows), (const int* const*)counts, params, out, V,
-                     blocks);
-  int rc = launch_status("sample_filtered");
+                     blocks, batch, host_out, count_now);
+  return launch_status("sample_filtered");
+}
+
+extern "C" int exl3_sample_rows(const float* logits, const double* rows, int* const* counts, const float* params, int* out,
+                                int R, int V, cudaStream_t stream) {
+  if (R == 0) return 0;
+  if (R < 0 || V < 1 || rows == nullptr || (counts != nullptr && params == nullptr)) {
+    set_error("sample_filtered: bad sizes rows=%d vocab=%d, or penalties without their constants", R, V);
+    return ERR_BAD_ARGUMENT;
+  }
+  static const SfBatch none = {};
+  int rc = sf_launch(logits, rows, counts, params, out, R, V, none, counts != nullptr, nullptr, false, stream);
   if (rc || counts == nullptr) return rc;
   return exl3_sample_count(counts, out, R, V, stream);
+}
+
+extern "C" int exl3_sample_direct_rows() { return SF_DIRECT_ROWS; }
+
+// The reference's generator (src/model.cpp:656-665) behind its step: a state's number in [0, 1).
+static double sf_uniform(unsigned long long z) {
+  z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+  z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+  z ^= z >> 31;
+  return (double)(z >> 11) * (1.0 / 9007199254740992.0);
+}
+
+// The same for up to exl3_sample_direct_rows() rows whose options are on the host.  packed: float64 [R, 7] = temperature,
+// top_k, top_p, min_p, repetition, presence and frequency penalty; uint64 [R], the generators' states after their step (not
+// looked at for greedy rows); uint64 [R], the addresses of the rows' token counts (0: no penalties).  shared_counts: rows may
+// have the same counts.  host_out: null, or page-locked int32 [R] that gets the ids as well.
+extern "C" int exl3_sample_batch(const float* logits, const void* packed, int R, int V, int shared_counts, int* out,
+                                 int* host_out, cudaStream_t stream) {
+  if (R == 0) return 0;
+  if (R < 0 || R > SF_DIRECT_ROWS || V < 1 || packed == nullptr) {
+    set_error("sample_batch: rows=%d (at most %d) vocab=%d", R, SF_DIRECT_ROWS, V);
+    return ERR_BAD_ARGUMENT;
+  }
+  const unsigned char* at = static_cast<const unsigned char*>(packed);
+  SfBatch batch = {};
+  bool penalties = false;
+  for (int r = 0; r < R; ++r) {
+    double o[7];
+    unsigned long long state, counts;
+    memcpy(o, at + (size_t)r * 56, 56);
+    memcpy(&state, at + (size_t)R * 56 + (size_t)r * 8, 8);
+    memcpy(&counts, at + (size_t)R * 64 + (size_t)r * 8, 8);
+    batch.rows[r] = {o[0], o[1], o[2], o[3], o[0] <= 0.0 ? 0.0 : sf_uniform(state)};
+    batch.counts[r] = reinterpret_cast<int*>(counts);
+    for (int i = 0; i < 3; ++i) batch.params[r][i] = (float)o[4 + i];
+    penalties |= counts != 0;
+  }
+  int rc = sf_launch(logits, nullptr, nullptr, nullptr, out, R, V, batch, penalties, host_out, !shared_counts, stream);
+  if (rc || !penalties || !shared_counts) return rc;
+  SfCounts c = {};
+  memcpy(c.at, batch.counts, sizeof(c.at));
+  sample_count_batch_kernel<<<1, SF_DIRECT_ROWS, 0, stream>>>(c, out, R, V);
+  return launch_status("sample_count");
 }
 
 extern "C" int exl3_sample_filtered(const float* logits, const double* rows, int* out, int R, int V,

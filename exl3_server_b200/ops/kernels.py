@@ -1224,6 +1224,29 @@ def sample_rows(logits: torch.Tensor, rows: torch.Tensor, counts: torch.Tensor, 
     return out
 
 
+def sample_direct_rows() -> int:
+    """The most rows that ``sample_batch`` takes."""
+    return int(library().exl3_sample_direct_rows())
+
+
+def sample_batch(logits: torch.Tensor, packed: bytes, shared_counts: bool, host_out: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``sample_rows`` for up to ``sample_direct_rows()`` rows whose options are on the host: ``packed`` holds float64
+    ``[R, 7]`` (temperature, top_k, top_p, min_p, repetition, presence and frequency penalty), uint64 ``[R]`` (the
+    generators' states after their step) and uint64 ``[R]`` (the addresses of the rows' counts, 0: no penalties).
+    ``host_out``: page-locked int32 ``[R]`` that gets the ids as well, for a host that waits for the stream."""
+    R, V = logits.shape
+    if logits.dtype != torch.float32 or len(packed) != 72 * R:
+        raise KernelLibraryError("sample_batch: logits [R, V] must be float32 with 72 bytes of options a row")
+    _contig(logits, "logits")
+    if host_out is not None and (host_out.dtype != torch.int32 or host_out.numel() < R or not host_out.is_pinned()):
+        raise KernelLibraryError("sample_batch: host_out must be page-locked int32 [R]")
+    out = torch.empty((R,), dtype=torch.int32, device=logits.device)
+    _check(library().exl3_sample_batch(_ptr(logits), ctypes.c_char_p(packed), _c_int(R), _c_int(V), _c_int(1 if shared_counts else 0),
+                                       _ptr(out), _c_void_p(host_out.data_ptr() if host_out is not None else 0), _stream()),
+           "sample_batch")
+    return out
+
+
 def sample_penalties(logits: torch.Tensor, counts: torch.Tensor, params: torch.Tensor) -> None:
     """Repetition, presence and frequency penalties, in place.  ``counts``: int64 ``[R]`` on the device, the
     addresses of the rows' int32 ``[V]`` token counts (0: the row has none); ``params``: float32 ``[R, 3]``."""

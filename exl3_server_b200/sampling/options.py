@@ -39,12 +39,23 @@ class SplitMix64:
     def __init__(self, state: int):
         self.state = state & MASK64
 
-    def next(self) -> int:
+    def step(self) -> int:
+        """Moves on; the new state, of which ``uniform_of`` makes the number that ``uniform01`` would have returned."""
         self.state = (self.state + 0x9E3779B97F4A7C15) & MASK64
-        z = self.state
+        return self.state
+
+    def next(self) -> int:
+        return self._mix(self.step())
+
+    @staticmethod
+    def _mix(z: int) -> int:
         z = ((z ^ (z >> 30)) * 0xBF58476D1CE4E5B9) & MASK64
         z = ((z ^ (z >> 27)) * 0x94D049BB133111EB) & MASK64
         return z ^ (z >> 31)
 
+    @staticmethod
+    def uniform_of(state: int) -> float:
+        return (SplitMix64._mix(state) >> 11) * (1.0 / 9007199254740992.0)
+
     def uniform01(self) -> float:
-        return (self.next() >> 11) * (1.0 / 9007199254740992.0)
+        return self.uniform_of(self.step())

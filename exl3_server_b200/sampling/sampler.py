@@ -11,6 +11,9 @@ each other.
 """
 from __future__ import annotations
 
+import struct
+from itertools import chain
+from operator import attrgetter
 from typing import List, Optional, Sequence
 
 import numpy as np
@@ -60,6 +63,15 @@ def launch_on_device(logits: torch.Tensor, rows: Sequence[RowSampler]) -> torch.
     """Starts the sampling of one token per row on the device and returns the ids (int32 on the device)
     without waiting for them.  The generators advance now; the tokens join the rows' contexts when the caller
     has read them (``record``).  The penalties' token counts are kept up on the device."""
+    return _launch(logits, rows, None)
+
+
+# a row's options in the order in which the kernels take them
+_OPTIONS = attrgetter("temperature", "top_k", "top_p", "min_p", "repetition_penalty", "presence_penalty", "frequency_penalty")
+
+
+def _launch(logits: torch.Tensor, rows: Sequence[RowSampler], host_out: Optional[torch.Tensor]) -> torch.Tensor:
+    """``launch_on_device``; ``host_out`` as in ``kernels.sample_batch``, for at most ``sample_direct_rows()`` rows."""
     from ..engine.decode import TRANSFERRED
     from ..ops import kernels as K
     if not logits.is_contiguous():
@@ -67,35 +79,40 @@ def launch_on_device(logits: torch.Tensor, rows: Sequence[RowSampler]) -> torch.
             logits = logits.clone()                      # a slice of padded rows, or one row for all, becomes dense
         K._contig(logits, "logits")                      # before any generator has moved on
     R, V = logits.shape
-    opts, counts, params, penalised = [], [], [], []     # one pass over the rows: their options are read once each
-    for r in rows:
-        o = r.opt
-        # a greedy row draws no number from its generator, as on the host
-        opts.append((o.temperature, o.top_k, o.top_p, o.min_p, 0.0 if o.greedy else r.rng.uniform01()))
-        if o.has_penalties:
+    opts = [_OPTIONS(r.opt) for r in rows]
+    # a greedy row draws no number from its generator, as on the host
+    states = [0 if o[0] <= 0.0 else r.rng.step() for r, o in zip(rows, opts)]
+    counts, penalised = [], []
+    for r, o in zip(rows, opts):
+        if o[4] != 1.0 or o[5] != 0.0 or o[6] != 0.0:
             counts.append(r.device_counts(V, logits.device).data_ptr())
-            params.append((o.repetition_penalty, o.presence_penalty, o.frequency_penalty))
             penalised.append(r)
         else:
             counts.append(0)
-            params.append((1.0, 0.0, 0.0))
-    if not penalised:
-        host = np.array(opts, dtype=np.float64)
+    if R <= K.sample_direct_rows():
+        # the options travel with the launch.  The kernel reads the logits with their penalties (the step's own buffer stays
+        # as the model left it), and the chosen tokens join the counts without a trip to the host
+        packed = struct.pack(f"<{7 * R}d{2 * R}Q", *chain.from_iterable(opts), *states, *counts)
+        kept = [c for c in counts if c]
+        ids = K.sample_batch(logits, packed, len(set(kept)) < len(kept), host_out)
+        n_bytes = len(packed)
+    elif not penalised:
+        host = np.array([(*o[:4], SplitMix64.uniform_of(z)) for o, z in zip(opts, states)], dtype=np.float64)
         ids = K.sample_filtered(logits, torch.from_numpy(host).to(logits.device))
+        n_bytes = host.nbytes
     else:
         # options, the counts' addresses and the penalties as one buffer: one copy to the device
         host = np.empty(R * (40 + 8 + 12), dtype=np.uint8)
-        host[:R * 40].view(np.float64).reshape(R, 5)[:] = opts
+        host[:R * 40].view(np.float64).reshape(R, 5)[:] = [(*o[:4], SplitMix64.uniform_of(z)) for o, z in zip(opts, states)]
         host[R * 40:R * 48].view(np.int64)[:] = counts
-        host[R * 48:].view(np.float32).reshape(R, 3)[:] = params
+        host[R * 48:].view(np.float32).reshape(R, 3)[:] = [o[4:] if c else (1.0, 0.0, 0.0) for o, c in zip(opts, counts)]
         dev = torch.from_numpy(host).to(logits.device)
-        # the kernel reads the logits with their penalties (the step's own buffer stays as the model left it), and the
-        # chosen tokens join the counts without a trip to the host
         ids = K.sample_rows(logits, dev[:R * 40].view(torch.float64).view(R, 5), dev[R * 40:R * 48].view(torch.int64),
                             dev[R * 48:].view(torch.float32).view(R, 3))
-        for r in penalised:
-            r.counted()
-    TRANSFERRED["h2d"] += host.nbytes
+        n_bytes = host.nbytes
+    for r in penalised:
+        r.counted()
+    TRANSFERRED["h2d"] += n_bytes
     return ids
 
 
@@ -121,10 +138,16 @@ def sample_rows(logits: torch.Tensor, rows: Sequence[RowSampler],
             from ..engine.decode import TRANSFERRED
             TRANSFERRED["d2h"] += ids.numel() * 4
         elif on_device(logits, rows):
-            ids = launch_on_device(logits.to(torch.float32), rows)
-            picked = ids.cpu().tolist()
+            if len(rows) <= K.sample_direct_rows():
+                # the kernel writes the ids to page-locked memory itself
+                host = torch.empty(len(rows), dtype=torch.int32, pin_memory=True)
+                _launch(logits.to(torch.float32), rows, host)
+                torch.cuda.current_stream().synchronize()
+                picked = host.tolist()
+            else:
+                picked = launch_on_device(logits.to(torch.float32), rows).cpu().tolist()
             from ..engine.decode import TRANSFERRED
-            TRANSFERRED["d2h"] += ids.numel() * 4
+            TRANSFERRED["d2h"] += len(rows) * 4
     if picked is None:
         host = logits.detach().to(torch.float32).cpu().numpy()
         picked = [sample_token(host[i], r.opt, r.context, r.rng) for i, r in enumerate(rows)]

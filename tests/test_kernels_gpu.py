@@ -1451,6 +1451,30 @@ def test_sample_filtered_ranks_equal_logits_of_long_rows(penalties):
     assert got.tolist() == [sample_token(logits[r], opt, contexts[r], _FixedU(us[r])) for r in range(R)]
 
 
+@pytest.mark.parametrize("R", [1, 5, 64, 65])             # with the launch up to 64 rows, by a buffer beyond
+@pytest.mark.parametrize("V", [300, 40001, 330001])
+def test_sampling_of_rows_with_options_of_their_own(R, V):
+    """Greedy rows and rows that draw, with and without penalties and filters, some of them sharing their counts: the host's
+    tokens, generators and counts after several steps."""
+    from exl3_server_b200.sampling import SampleOptions
+    from exl3_server_b200.sampling.sampler import RowSampler, sample_rows
+    opts = [SampleOptions(temperature=(0.0, 0.7, 1.3)[r % 3], top_k=(0, 40, 7)[r % 3], top_p=(1.0, 0.9)[r % 2], min_p=0.02 * (r % 2),
+                          repetition_penalty=1.0 + 0.2 * (r % 4 == 1), presence_penalty=0.3 * (r % 5 == 2), seed=r * 977 + 2 ** 63)
+            for r in range(R)]
+    new = lambda: [RowSampler(o, r, [r, 5, 5, V - 1, V + 3]) for r, o in enumerate(opts)]  # noqa: E731
+    device, host = new(), new()
+    if R > 4:
+        device[3], host[3] = device[1], host[1]           # one request's sampler twice
+    for step in range(3):
+        logits = 4.0 * torch.randn(R, V, generator=torch.Generator().manual_seed(100 * R + step))
+        assert sample_rows(logits.to(DEV), device) == sample_rows(logits, host)
+    assert [d.rng.state for d in device] == [h.rng.state for h in host]
+    for d in device:
+        if d.opt.has_penalties:
+            want = torch.bincount(torch.tensor([t for t in d.context if t < V]), minlength=V)
+            assert d._counted == len(d.context) and torch.equal(d.device_counts(V, DEV).long().cpu(), want)
+
+
 @pytest.mark.parametrize("V", [300, 40001])
 def test_rows_that_share_a_sampler(V):
     """One request's sampler for all rows, more rows than run at once: every row sees the context as it was before the
