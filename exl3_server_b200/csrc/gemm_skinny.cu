@@ -86,6 +86,157 @@ __device__ inline float4 sk_ld_cluster4(uint32_t addr) {
   return v;
 }
 
+// The epilogue's second half: batch rows rank, rank + S, ... of the whole tile, S up to SMAX.  A warp takes a batch row at a
+// time, a lane four neighbouring features of it: 16-byte loads from the other blocks' shared memory (the path between SMs
+// is slow in small pieces) and 8- or 16-byte stores.  The loads of up to ROWS batch rows are in flight together (a trip to
+// another SM's shared memory takes about a microsecond, whatever it carries): with six warps all of a block's rows at up to
+// 64 rows and two cuts or more.
+template <int EPI, bool SCALE, int R, int SMAX, int ROWS>
+__device__ inline void sk_finish(const SkinnyArgs& a, const float* part, const float* s_inv, int n0, int rank, bool& arrived) {
+  constexpr int RW = R * SK_BM, WARPS = SK_THREADS / 32;
+  const int S = a.split, lane = threadIdx.x & 31;
+  {
+    const int q = threadIdx.x >> 5;
+    const int ss_out_blocks = (a.N + 15) >> 4;
+    const bool vec = (a.N & 3) == 0;                        // rows of y, h and x_raw start on 16-byte boundaries
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int f0 = r * SK_BM + 4 * lane;
+      const int n = n0 + f0;
+      uint32_t peer[SMAX];
+#pragma unroll
+      for (int j = 0; j < SMAX; ++j) peer[j] = j < S ? sk_map_rank(smem_u32(part + f0), (uint32_t)j) : 0u;
+      float bias_v[4] = {0.0f, 0.0f, 0.0f, 0.0f}, wn[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        if (n + e < a.N) {
+          if (a.bias) bias_v[e] = __bfloat162float(a.bias[n + e]);
+          if (EPI == 2)
+            wn[e] = a.norm_w_f32 ? __ldg(static_cast<const float*>(a.norm_w) + n + e)
+                                 : __bfloat162float(__ldg(static_cast<const __nv_bfloat16*>(a.norm_w) + n + e));
+        }
+      }
+      for (int i0 = q; rank + i0 * S < a.M; i0 += WARPS * ROWS) {
+        float4 vv[ROWS][SMAX];
+        float h_all[ROWS][4];
+#pragma unroll
+        for (int u = 0; u < ROWS; ++u) {
+          const int m = rank + (i0 + WARPS * u) * S;
+          const bool row = m < a.M;
+#pragma unroll
+          for (int j = 0; j < SMAX; ++j)
+            vv[u][j] = (j < S && row) ? sk_ld_cluster4(peer[j] + (uint32_t)m * RW * 4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) h_all[u][e] = 0.0f;
+          if (EPI == 2 && row) {
+            if (vec) {
+              if (n < a.N) {
+                const float4 hv = __ldcg(reinterpret_cast<const float4*>(a.h + (int64_t)m * a.N + n));
+                h_all[u][0] = hv.x; h_all[u][1] = hv.y; h_all[u][2] = hv.z; h_all[u][3] = hv.w;
+              }
+            } else {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) if (n + e < a.N) h_all[u][e] = __ldcg(a.h + (int64_t)m * a.N + n + e);
+            }
+          }
+        }
+        if (r == R - 1 && rank + (i0 + WARPS * ROWS) * S >= a.M) {     // this warp's last loads
+          float got = 0.0f;
+#pragma unroll
+          for (int u = 0; u < ROWS; ++u)
+#pragma unroll
+            for (int j = 0; j < SMAX; ++j) got += vv[u][j].x + vv[u][j].y + vv[u][j].z + vv[u][j].w;
+          sk_cluster_arrive_after(got);
+          arrived = true;
+        }
+#pragma unroll
+        for (int u = 0; u < ROWS; ++u) {
+        const int i = i0 + WARPS * u;
+        const int m = rank + i * S;
+        if (m >= a.M) break;                               // the same for every lane of the warp
+        const float4* v = vv[u];
+        const float* h_old = h_all[u];
+        float s[4] = {v[0].x, v[0].y, v[0].z, v[0].w};
+#pragma unroll
+        for (int j = 1; j < SMAX; ++j) {            // block order; the zeros of absent blocks change nothing
+          s[0] += v[j].x; s[1] += v[j].y; s[2] += v[j].z; s[3] += v[j].w;
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (SCALE) s[e] *= s_inv[i];
+          s[e] += bias_v[e];
+        }
+        if (EPI == 0) {
+          if (a.out_f32) {
+            float* dst = static_cast<float*>(a.y) + (int64_t)m * a.N + n;
+            if (vec) { if (n < a.N) *reinterpret_cast<float4*>(dst) = make_float4(s[0], s[1], s[2], s[3]); }
+            else {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) if (n + e < a.N) dst[e] = s[e];
+            }
+          } else {
+            __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(a.y) + (int64_t)m * a.N + n;
+            if (vec) {
+              if (n < a.N) {
+                const __nv_bfloat162 lo = __floats2bfloat162_rn(s[0], s[1]), hi = __floats2bfloat162_rn(s[2], s[3]);
+                *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+              }
+            } else {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) if (n + e < a.N) dst[e] = __float2bfloat16_rn(s[e]);
+            }
+          }
+        } else if (EPI == 1) {
+          // rows in eights: of every four lanes the first two hold gate rows, the other two the up rows of the same
+          // features (N is a multiple of 16 here)
+          float o[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float up = __shfl_down_sync(0xffffffffu, s[e], 2);
+            o[e] = s[e] / (1.0f + expf(-s[e])) * up;
+          }
+          if ((lane & 2) == 0 && n < a.N) {
+            const int f = ((n >> 4) << 3) + (n & 7);
+            if (a.out_f32) {
+              *reinterpret_cast<float4*>(static_cast<float*>(a.y) + (int64_t)m * (a.N >> 1) + f) = make_float4(o[0], o[1], o[2], o[3]);
+            } else {
+              const __nv_bfloat162 lo = __floats2bfloat162_rn(o[0], o[1]), hi = __floats2bfloat162_rn(o[2], o[3]);
+              *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(a.y) + (int64_t)m * (a.N >> 1) + f) =
+                  make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+            }
+          }
+        } else {
+          float hv[4], sq = 0.0f;
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            // the output is rounded to bfloat16 as it would be on its way through memory
+            hv[e] = h_old[e] + __bfloat162float(__float2bfloat16_rn(s[e])) * a.rho;
+            if (n + e < a.N) sq += hv[e] * hv[e];
+          }
+          float* hp = a.h + (int64_t)m * a.N + n;
+          __nv_bfloat16* xp = a.x_raw + (int64_t)m * a.N + n;
+          if (vec) {
+            if (n < a.N) {
+              *reinterpret_cast<float4*>(hp) = make_float4(hv[0], hv[1], hv[2], hv[3]);
+              const __nv_bfloat162 lo = __floats2bfloat162_rn(hv[0] * wn[0], hv[1] * wn[1]);
+              const __nv_bfloat162 hi = __floats2bfloat162_rn(hv[2] * wn[2], hv[3] * wn[3]);
+              *reinterpret_cast<uint2*>(xp) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (n + e < a.N) { hp[e] = hv[e]; xp[e] = __float2bfloat16_rn(hv[e] * wn[e]); }
+          }
+          sq += __shfl_xor_sync(0xffffffffu, sq, 1);
+          sq += __shfl_xor_sync(0xffffffffu, sq, 2);
+          if ((lane & 3) == 0 && n < a.N) a.ss_out[(int64_t)m * ss_out_blocks + (n >> 4)] = sq;
+        }
+        }
+      }
+    }
+  }
+}
+
 // R: 128-row tiles of w per block.
 template <int EPI, bool SCALE, int R>
 __global__ void __launch_bounds__(SK_THREADS)
@@ -104,6 +255,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   uint64_t* empty = full + a.stages;                      // [stages] the MMAs that read the stage are done
   uint64_t* acc_full = empty + a.stages;                  // the accumulator is complete
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+  int* gave_up = reinterpret_cast<int*>(tmem_slot + 1);    // a wait of this block ran out
   float* s_inv = reinterpret_cast<float*>(tmem_slot + 2); // [rows_per] SCALE: factor of the i-th batch row of this block
 
   pdl_trigger();
@@ -119,6 +271,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   if (threadIdx.x == 0) {
     for (int s = 0; s < a.stages; ++s) { mbar_init(full + s, 1); mbar_init(empty + s, 1); }
     mbar_init(acc_full, 1);
+    *gave_up = 0;
     mbar_init_fence();
     // the first weights are asked for at once: they need nothing but this thread's own barriers
     for (int i = 0; i < pre; ++i) {
@@ -224,6 +377,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     }
     fence_before();
   }
+  if (!ok) *gave_up = 1;
 
   // every block of the cluster has its partial tile in place (or has given up: then its values are not used,
   // because the error code makes the host reject the step)
@@ -232,154 +386,15 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
   // The second cluster barrier keeps a block alive while others may still read its shared memory.  A warp arrives
   // as soon as its own last loads from other blocks have come back, and waits only at the very end, so that the
   // barrier's trip overlaps the arithmetic and the stores.
+  // (All six warps take part; a block that has given up skips its rows: its error code makes the host reject the step.)
   bool arrived = false;
-  if (warp < 2 || !ok) { sk_cluster_arrive(); arrived = true; }
+  const bool all_ok = *gave_up == 0;
 
-  if (warp >= 2 && ok) {
-    // ---- epilogue, second half: batch rows rank, rank + S, ... of the whole tile ----------------------------
-    // A warp takes a batch row at a time, a lane four neighbouring features of it: 16-byte loads from the other
-    // blocks' shared memory (the path between SMs is slow in small pieces) and 8- or 16-byte stores.
-    const int q = warp & 3;
-    const int ss_out_blocks = (a.N + 15) >> 4;
-    const bool vec = (a.N & 3) == 0;                        // rows of y, h and x_raw start on 16-byte boundaries
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int f0 = r * SK_BM + 4 * lane;
-      const int n = n0 + f0;
-      uint32_t peer[SK_MAX_SPLIT];
-#pragma unroll
-      for (int j = 0; j < SK_MAX_SPLIT; ++j) peer[j] = j < S ? sk_map_rank(smem_u32(part + f0), (uint32_t)j) : 0u;
-      float bias_v[4] = {0.0f, 0.0f, 0.0f, 0.0f}, wn[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        if (n + e < a.N) {
-          if (a.bias) bias_v[e] = __bfloat162float(a.bias[n + e]);
-          if (EPI == 2)
-            wn[e] = a.norm_w_f32 ? __ldg(static_cast<const float*>(a.norm_w) + n + e)
-                                 : __bfloat162float(__ldg(static_cast<const __nv_bfloat16*>(a.norm_w) + n + e));
-        }
-      }
-      // the loads of up to ROWS batch rows are in flight together: a trip to another SM's shared memory takes about
-      // a microsecond, whatever it carries
-      constexpr int ROWS = 3;
-      for (int i0 = q; rank + i0 * S < a.M; i0 += 4 * ROWS) {
-        float4 vv[ROWS][SK_MAX_SPLIT];
-        float h_all[ROWS][4];
-#pragma unroll
-        for (int u = 0; u < ROWS; ++u) {
-          const int m = rank + (i0 + 4 * u) * S;
-          const bool row = m < a.M;
-#pragma unroll
-          for (int j = 0; j < SK_MAX_SPLIT; ++j)
-            vv[u][j] = (j < S && row) ? sk_ld_cluster4(peer[j] + (uint32_t)m * RW * 4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-#pragma unroll
-          for (int e = 0; e < 4; ++e) h_all[u][e] = 0.0f;
-          if (EPI == 2 && row) {
-            if (vec) {
-              if (n < a.N) {
-                const float4 hv = __ldcg(reinterpret_cast<const float4*>(a.h + (int64_t)m * a.N + n));
-                h_all[u][0] = hv.x; h_all[u][1] = hv.y; h_all[u][2] = hv.z; h_all[u][3] = hv.w;
-              }
-            } else {
-#pragma unroll
-              for (int e = 0; e < 4; ++e) if (n + e < a.N) h_all[u][e] = __ldcg(a.h + (int64_t)m * a.N + n + e);
-            }
-          }
-        }
-        if (r == R - 1 && rank + (i0 + 4 * ROWS) * S >= a.M) {     // this warp's last loads
-          float got = 0.0f;
-#pragma unroll
-          for (int u = 0; u < ROWS; ++u)
-#pragma unroll
-            for (int j = 0; j < SK_MAX_SPLIT; ++j) got += vv[u][j].x + vv[u][j].y + vv[u][j].z + vv[u][j].w;
-          sk_cluster_arrive_after(got);
-          arrived = true;
-        }
-#pragma unroll
-        for (int u = 0; u < ROWS; ++u) {
-        const int i = i0 + 4 * u;
-        const int m = rank + i * S;
-        if (m >= a.M) break;                               // the same for every lane of the warp
-        const float4* v = vv[u];
-        const float* h_old = h_all[u];
-        float s[4] = {v[0].x, v[0].y, v[0].z, v[0].w};
-#pragma unroll
-        for (int j = 1; j < SK_MAX_SPLIT; ++j) {            // block order; the zeros of absent blocks change nothing
-          s[0] += v[j].x; s[1] += v[j].y; s[2] += v[j].z; s[3] += v[j].w;
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          if (SCALE) s[e] *= s_inv[i];
-          s[e] += bias_v[e];
-        }
-        if (EPI == 0) {
-          if (a.out_f32) {
-            float* dst = static_cast<float*>(a.y) + (int64_t)m * a.N + n;
-            if (vec) { if (n < a.N) *reinterpret_cast<float4*>(dst) = make_float4(s[0], s[1], s[2], s[3]); }
-            else {
-#pragma unroll
-              for (int e = 0; e < 4; ++e) if (n + e < a.N) dst[e] = s[e];
-            }
-          } else {
-            __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(a.y) + (int64_t)m * a.N + n;
-            if (vec) {
-              if (n < a.N) {
-                const __nv_bfloat162 lo = __floats2bfloat162_rn(s[0], s[1]), hi = __floats2bfloat162_rn(s[2], s[3]);
-                *reinterpret_cast<uint2*>(dst) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-              }
-            } else {
-#pragma unroll
-              for (int e = 0; e < 4; ++e) if (n + e < a.N) dst[e] = __float2bfloat16_rn(s[e]);
-            }
-          }
-        } else if (EPI == 1) {
-          // rows in eights: of every four lanes the first two hold gate rows, the other two the up rows of the same
-          // features (N is a multiple of 16 here)
-          float o[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float up = __shfl_down_sync(0xffffffffu, s[e], 2);
-            o[e] = s[e] / (1.0f + expf(-s[e])) * up;
-          }
-          if ((lane & 2) == 0 && n < a.N) {
-            const int f = ((n >> 4) << 3) + (n & 7);
-            if (a.out_f32) {
-              *reinterpret_cast<float4*>(static_cast<float*>(a.y) + (int64_t)m * (a.N >> 1) + f) = make_float4(o[0], o[1], o[2], o[3]);
-            } else {
-              const __nv_bfloat162 lo = __floats2bfloat162_rn(o[0], o[1]), hi = __floats2bfloat162_rn(o[2], o[3]);
-              *reinterpret_cast<uint2*>(static_cast<__nv_bfloat16*>(a.y) + (int64_t)m * (a.N >> 1) + f) =
-                  make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-            }
-          }
-        } else {
-          float hv[4], sq = 0.0f;
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            // the output is rounded to bfloat16 as it would be on its way through memory
-            hv[e] = h_old[e] + __bfloat162float(__float2bfloat16_rn(s[e])) * a.rho;
-            if (n + e < a.N) sq += hv[e] * hv[e];
-          }
-          float* hp = a.h + (int64_t)m * a.N + n;
-          __nv_bfloat16* xp = a.x_raw + (int64_t)m * a.N + n;
-          if (vec) {
-            if (n < a.N) {
-              *reinterpret_cast<float4*>(hp) = make_float4(hv[0], hv[1], hv[2], hv[3]);
-              const __nv_bfloat162 lo = __floats2bfloat162_rn(hv[0] * wn[0], hv[1] * wn[1]);
-              const __nv_bfloat162 hi = __floats2bfloat162_rn(hv[2] * wn[2], hv[3] * wn[3]);
-              *reinterpret_cast<uint2*>(xp) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-            }
-          } else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-              if (n + e < a.N) { hp[e] = hv[e]; xp[e] = __float2bfloat16_rn(hv[e] * wn[e]); }
-          }
-          sq += __shfl_xor_sync(0xffffffffu, sq, 1);
-          sq += __shfl_xor_sync(0xffffffffu, sq, 2);
-          if ((lane & 3) == 0 && n < a.N) a.ss_out[(int64_t)m * ss_out_blocks + (n >> 4)] = sq;
-        }
-        }
-      }
-    }
+  if (all_ok) {
+    pdl_wait();                                            // (one of the warps has not waited yet)
+    if (S <= 2) sk_finish<EPI, SCALE, R, 2, 6>(a, part, s_inv, n0, rank, arrived);
+    else if (S <= 4) sk_finish<EPI, SCALE, R, 4, 4>(a, part, s_inv, n0, rank, arrived);
+    else sk_finish<EPI, SCALE, R, SK_MAX_SPLIT, 3>(a, part, s_inv, n0, rank, arrived);
   }
 
   if (!arrived) sk_cluster_arrive();
@@ -493,14 +508,14 @@ static int sk_auto_split(int N, int K) {
 }
 
 // Two tiles per block (the block's piece of x is then read once for twice the weights) where there are more
-// tiles than SMs and the blocks of two tiles still fill the GPU one and a half times, for up to 32 rows (an
+// tiles than SMs and the blocks of two tiles still fill the GPU one and a half times, for up to 64 rows (an
 // output head of 122753 x 2304: 87.8 / 90.5 / 93.3 / 97.7 us at 1 / 8 / 16 / 32 rows against 95.1 / 97.5 / 100.5 /
-// 105.1 with a tile a block, but 132.6 against 114.2 at 64 rows); for more rows only with many times more tiles
-// than SMs.  Changes no result (the cuts of K stay what N and K say).
+// 105.1 with a tile a block; two blocks an SM with two stages each at 48 and 64 rows, of 73448 x 4096, 101.4 and 104.0 against
+// 104.9 and 108.0, gated 32768 x 4096 52.2 and 54.7 against 53.0 and 55.7; with one block an SM 132.6 against 114.2).  More rows keep a tile a
+// block (128 rows: 82.7 against 67.5).  Changes no result (the cuts of K stay what N and K say).
 static int sk_auto_tiles(int N, int split, int M) {
   const int n_tiles = ceil_div(N, SK_BM), sms = sk_sm_count();
-  if (M <= 32) return n_tiles > sms && 2 * ceil_div(n_tiles, 2) * split >= 3 * sms ? 2 : 1;
-  return n_tiles * split >= 8 * sms ? 2 : 1;
+  return M <= 64 && n_tiles > sms && 2 * ceil_div(n_tiles, 2) * split >= 3 * sms ? 2 : 1;
 }
 
 template <int EPI, bool SCALE, int R>
@@ -597,13 +612,14 @@ extern "C" int exl3_gemm_skinny(const void* x, const void* w, const void* bias, 
   const int cols = R * a.MP;
   a.tmem_cols = cols <= 32 ? 32 : (cols <= 64 ? 64 : (cols <= 128 ? 128 : 256));
   // shared memory: the ring; the partial tile [MP][R * 128] floats takes its place afterwards and must fit it.
-  // As many stages as a block has steps, at most 4; fewer when two blocks can share an SM that way.
+  // As many stages as a block has steps, at most 4; three or two when two blocks can share an SM that way.
   const size_t stage = (size_t)R * SK_TILE_W + (size_t)a.MP * SK_BK * 2;
   const size_t part = (size_t)a.MP * R * SK_BM * 4;
   const size_t fixed = 1024 /* alignment */ + (size_t)(2 * 4 + 1) * 8 + 16 + (size_t)a.rows_per * 4 + 64;
   const int per_block = ceil_div(ksteps, a.split);
   int stages = per_block < 4 ? per_block : 4;
-  if (stages == 4 && fixed + 3 * stage <= 113 * 1024 && fixed + 4 * stage > 113 * 1024) stages = 3;
+  for (int n = 3; n >= 2; --n)
+    if (stages == 4 && fixed + n * stage <= 113 * 1024 && fixed + 4 * stage > 113 * 1024) stages = n;
   while ((size_t)stages * stage < part) ++stages;
   a.stages = stages;
   const size_t smem = fixed + (size_t)stages * stage;
