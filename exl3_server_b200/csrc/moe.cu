@@ -405,97 +405,140 @@ moe_gemm_kernel(const TA* A, int64_t lda, int a_div, const TW* __restrict__ Wt, 
 
 // ---- a few rows per expert (decode): the experts' matrices are read once, a warp per output feature ---------------
 //
-// out[p, n] = act(sum_k A[p / a_div, k] * W[e(p), n, k]) for tiles of at most MV_ROWS pairs.  K is walked in pieces
-// of MV_KC columns: the block puts the tile's rows of A for the piece into shared memory, and every warp takes
-// MV_FEAT output features, whose rows of W it reads in 16-byte pieces, all of a piece's loads under way before the
-// first is used.  One float32 sum per (feature, pair) and lane; the lanes' sums meet in a fixed order, so a pair's
-// result does not depend on its tile mates.
-constexpr int MV_ROWS = 4, MV_FEAT = 4, MV_WARPS = 8, MV_KC = 1024, MV_IT = MV_KC / 256;
+// out[p, n] = act(sum_k A[p / a_div, k] * W[e(p), n, k]) for tiles of at most MV_ROWS pairs.  A warp takes MV_FEAT output
+// features, whose rows of W each thread streams in its own 16-byte pieces through a ring of MV_STAGES in shared memory (only
+// the thread that copied a slot reads it: no barrier), the tile's rows of A lie in shared memory, up to MV_KC columns at a time.
+// The even and the odd columns of a lane have a float32 sum each, over K upward (neighbours in memory: a pair is one
+// fma.rn.f32x2), and are added at the end; the lanes' sums meet in a fixed order, so a pair's result does not depend on its
+// tile mates.  Bound by the instructions of a step (a tile's rows as a constant, pairs: some 90 for 2 KB of W; 290 with scalar
+// products and the rows in a loop, 0.44 a cycle and scheduler, 3 TB/s) and by the start of a block.
+// Experts of N 2,816, K 2,048 and N 2,048, K 1,408, in us for 2 / 4 / 10 of them: 8.1 / 15.0 / 30.6 and 6.2 / 8.4 / 21.5 (pieces of 1,024
+// columns in registers, a barrier between loading and multiplying: 11.1 / 19.8 / 37.2 and 8.3 / 11.8 / 29.2; four warps a block 8.0 /
+// 14.2 / 31.8 and 6.0 / 8.6 / 21.7; three or six stages are not faster).  Against 64 bits 7.0e-8 (one sum a lane: 7.4e-8).
+constexpr int MV_ROWS = 4, MV_FEAT = 4, MV_WARPS = 8, MV_STAGES = 4, MV_KC = 4096, MV_STEP = 256;
+constexpr int MV_RING_BYTES = MV_WARPS * MV_STAGES * MV_FEAT * 32 * 16;
+
+__device__ inline void mv_cp16(uint32_t smem, const void* gmem, bool ok) {
+  const int bytes = ok ? 16 : 0;                     // nothing read, zeros written
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem), "l"(gmem), "r"(bytes) : "memory");
+}
+// eight bfloat16 as four pairs of floats
+__device__ inline void mv_pairs(const uint4& v, unsigned long long (&f)[4]) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int j = 0; j < 4; ++j) asm("mov.b64 %0, {%1, %2};" : "=l"(f[j]) : "r"(w[j] << 16), "r"(w[j] & 0xffff0000u));
+}
+
+// The sums of a warp's features and the tile's NR rows: acc[f][r], of which every lane has its share.
+template <int NR>
+__device__ inline void mv_run(const __nv_bfloat16* A, int64_t lda, int a_div, const __nv_bfloat16* w0, int64_t (&row)[MV_FEAT],
+                              const int* rows, uint4* ring, uint4* xs, int steps, int K, float (&out)[MV_FEAT][MV_ROWS]) {
+  const int lane = threadIdx.x & 31, per = min(K, MV_KC) / 8;
+  unsigned long long acc[MV_FEAT][NR];
+#pragma unroll
+  for (int f = 0; f < MV_FEAT; ++f)
+#pragma unroll
+    for (int r = 0; r < NR; ++r) acc[f][r] = 0;
+  const uint32_t ring0 = (uint32_t)__cvta_generic_to_shared(ring);
+  constexpr uint32_t SLOT = MV_FEAT * 32 * 16;
+  uint32_t slot_in = ring0;
+  int asked = lane * 8;                              // the column of the next piece
+  const int last = steps * MV_STEP;                  // (0: this warp has no features)
+  auto ask = [&]() {
+    if (asked < last) {
+#pragma unroll
+      for (int f = 0; f < MV_FEAT; ++f) mv_cp16(slot_in + f * 512, w0 + row[f] + (asked < K ? asked : 0), asked < K);
+    }
+    asked += MV_STEP;
+    slot_in = slot_in == ring0 + (MV_STAGES - 1) * SLOT ? ring0 : slot_in + SLOT;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int i = 0; i < MV_STAGES - 1; ++i) ask();     // they come from DRAM: first of all
+  int slot = 0, step = 0;
+  for (int k0 = 0; k0 < K; k0 += MV_KC) {
+    __syncthreads();                                 // rows are there, the segment before has been read
+    for (int i = threadIdx.x; i < NR * per; i += MV_WARPS * 32) {
+      const int r = i / per, c = i - r * per;
+      const int p = rows[r], k = k0 + c * 8;
+      xs[i] = p >= 0 && k < K ? __ldcg(reinterpret_cast<const uint4*>(A + (int64_t)(p / a_div) * lda + k)) : make_uint4(0, 0, 0, 0);
+    }
+    __syncthreads();
+    const int end = min(steps, (k0 + MV_KC) / MV_STEP);
+    for (int c = lane; step < end; ++step, c += MV_STEP / 8) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(MV_STAGES - 2) : "memory");
+      uint4 wv[MV_FEAT];
+#pragma unroll
+      for (int f = 0; f < MV_FEAT; ++f) wv[f] = ring[(slot * MV_FEAT + f) * 32];
+      slot = slot == MV_STAGES - 1 ? 0 : slot + 1;
+      unsigned long long x[NR][4];
+#pragma unroll
+      for (int r = 0; r < NR; ++r) mv_pairs(c < per ? xs[r * per + c] : make_uint4(0, 0, 0, 0), x[r]);
+#pragma unroll
+      for (int f = 0; f < MV_FEAT; ++f) {
+        unsigned long long w[4];
+        mv_pairs(wv[f], w);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int r = 0; r < NR; ++r) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[f][r]) : "l"(x[r][j]), "l"(w[j]));
+      }
+      ask();                                         // into the slot that was read the step before
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+  for (int f = 0; f < MV_FEAT; ++f)
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      float lo, hi;
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(acc[f][r]));
+      out[f][r] = warp_sum(lo + hi);
+    }
+}
 
 template <typename TO>
 __global__ void __launch_bounds__(MV_WARPS * 32, 2)
 moe_gemv_kernel(const __nv_bfloat16* A, int64_t lda, int a_div, const __nv_bfloat16* __restrict__ Wt, const int* order,
                 const int* plan, TO* out, int N, int K, int act) {
   __shared__ int rows[MV_ROWS];
-  __shared__ uint4 xs[MV_ROWS][MV_KC / 8];
+  extern __shared__ uint4 mv_smem[];                 // [warps][stages][features][32] pieces of W, then [MV_ROWS][columns / 8] of A
   pdl_wait();
-  pdl_trigger();
   const int tile = blockIdx.x;
   if (tile >= __ldcg(plan)) return;
   const int e = __ldcg(plan + 4 + 3 * tile), start = __ldcg(plan + 5 + 3 * tile), nrows = __ldcg(plan + 6 + 3 * tile);
-  if (threadIdx.x < MV_ROWS) rows[threadIdx.x] = threadIdx.x < nrows ? __ldcg(order + start + threadIdx.x) : -1;
-  __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int n0 = (blockIdx.y * MV_WARPS + warp) * MV_FEAT;
-  const __nv_bfloat16* Wexp = Wt + (int64_t)e * N * K;
+  uint4* ring = mv_smem + warp * MV_STAGES * MV_FEAT * 32 + lane;
+  uint4* xs = mv_smem + MV_WARPS * MV_STAGES * MV_FEAT * 32;
+  if (threadIdx.x < MV_ROWS) rows[threadIdx.x] = threadIdx.x < nrows ? __ldcg(order + start + threadIdx.x) : -1;
+  int64_t row[MV_FEAT];
+#pragma unroll
+  for (int f = 0; f < MV_FEAT; ++f) row[f] = (int64_t)min(n0 + f, N - 1) * K;
+  const __nv_bfloat16* w0 = Wt + (int64_t)e * N * K;
+  const int steps = n0 < N ? (K + MV_STEP - 1) / MV_STEP : 0;
   float acc[MV_FEAT][MV_ROWS];
-#pragma unroll
-  for (int f = 0; f < MV_FEAT; ++f)
-#pragma unroll
-    for (int r = 0; r < MV_ROWS; ++r) acc[f][r] = 0.0f;
-  for (int k0 = 0; k0 < K; k0 += MV_KC) {
-    // this warp's pieces of W first: they come from DRAM
-    uint4 wv[MV_FEAT][MV_IT];
-#pragma unroll
-    for (int f = 0; f < MV_FEAT; ++f) {
-      const int n = min(n0 + f, N - 1);
-#pragma unroll
-      for (int it = 0; it < MV_IT; ++it) {
-        const int k = k0 + it * 256 + lane * 8;
-        wv[f][it] = k < K ? __ldg(reinterpret_cast<const uint4*>(Wexp + (int64_t)n * K + k)) : make_uint4(0, 0, 0, 0);
-      }
-    }
-    for (int i = threadIdx.x; i < MV_ROWS * (MV_KC / 8); i += MV_WARPS * 32) {
-      const int r = i / (MV_KC / 8), c = i - r * (MV_KC / 8);
-      const int p = rows[r], k = k0 + c * 8;
-      xs[r][c] = (p >= 0 && k < K) ? __ldcg(reinterpret_cast<const uint4*>(A + (int64_t)(p / a_div) * lda + k))
-                                   : make_uint4(0, 0, 0, 0);
-    }
-    __syncthreads();
-    if (n0 < N) {
-#pragma unroll
-      for (int it = 0; it < MV_IT; ++it) {
-#pragma unroll
-        for (int r = 0; r < MV_ROWS; ++r) {
-          if (r >= nrows) continue;
-          const uint4 xv = xs[r][it * 32 + lane];
-          const __nv_bfloat162* xp = reinterpret_cast<const __nv_bfloat162*>(&xv);
-#pragma unroll
-          for (int f = 0; f < MV_FEAT; ++f) {
-            const __nv_bfloat162* wp = reinterpret_cast<const __nv_bfloat162*>(&wv[f][it]);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float2 a = __bfloat1622float2(xp[j]), b = __bfloat1622float2(wp[j]);
-              acc[f][r] = fmaf(a.x, b.x, acc[f][r]);
-              acc[f][r] = fmaf(a.y, b.y, acc[f][r]);
-            }
-          }
-        }
-      }
-    }
-    __syncthreads();
-  }
-  if (n0 >= N) return;
+  if (nrows == 1) mv_run<1>(A, lda, a_div, w0, row, rows, ring, xs, steps, K, acc);
+  else if (nrows == 2) mv_run<2>(A, lda, a_div, w0, row, rows, ring, xs, steps, K, acc);
+  else mv_run<MV_ROWS>(A, lda, a_div, w0, row, rows, ring, xs, steps, K, acc);
+  // Not before: a kernel that was let start early would wait for this one with its shared memory taken, on SMs that the mixer's
+  // kernels on the other stream could use (two tokens of the decoder that runs both side by side: 6,274 -> 6,091 us).
+  pdl_trigger();
+  if (n0 >= N || lane != 0) return;
   if (act & MOE_GLU) {
 #pragma unroll
     for (int f = 0; f < MV_FEAT; f += 2)
 #pragma unroll
-      for (int r = 0; r < MV_ROWS; ++r) {
-        const float g = warp_sum(acc[f][r]), u = warp_sum(acc[f + 1][r]);
-        const int p = rows[r];
-        if (lane == 0 && p >= 0 && n0 + f + 1 < N)
-          moe_st(out + (int64_t)p * (N / 2) + (n0 + f) / 2, moe_act(g, act & ~MOE_GLU) * u);
-      }
+      for (int r = 0; r < MV_ROWS; ++r)
+        if (r < nrows && n0 + f + 1 < N)
+          moe_st(out + (int64_t)rows[r] * (N / 2) + (n0 + f) / 2, moe_act(acc[f][r], act & ~MOE_GLU) * acc[f + 1][r]);
     return;
   }
 #pragma unroll
   for (int f = 0; f < MV_FEAT; ++f)
 #pragma unroll
-    for (int r = 0; r < MV_ROWS; ++r) {
-      const float v = warp_sum(acc[f][r]);
-      const int p = rows[r];
-      if (lane == 0 && p >= 0 && n0 + f < N) moe_st(out + (int64_t)p * N + n0 + f, moe_act(v, act));
-    }
+    for (int r = 0; r < MV_ROWS; ++r)
+      if (r < nrows && n0 + f < N) moe_st(out + (int64_t)rows[r] * N + n0 + f, moe_act(acc[f][r], act));
 }
 
 // xs[i] = x[order[i] / top] for the planned pairs, in the plan's order (rows of K bfloat16, 16 bytes a thread).
@@ -809,11 +852,16 @@ extern "C" int exl3_moe_gemv(const void* A, int64_t lda, int a_div, const void* 
   if (grid.y > 65535) { set_error("moe_gemv: grid too large"); return ERR_UNSUPPORTED; }
   const __nv_bfloat16* a = static_cast<const __nv_bfloat16*>(A);
   const __nv_bfloat16* w = static_cast<const __nv_bfloat16*>(W);
+  const size_t smem = MV_RING_BYTES + (size_t)MV_ROWS * (K < MV_KC ? K : MV_KC) * 2;
+  constexpr int MOST = MV_RING_BYTES + MV_ROWS * MV_KC * 2;     // the same limit from every thread
+  cudaError_t err = cudaFuncSetAttribute(moe_gemv_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST);
+  if (err == cudaSuccess) err = cudaFuncSetAttribute(moe_gemv_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST);
+  if (err != cudaSuccess) { set_error("moe_gemv: %d bytes of shared memory refused: %s", MOST, cudaGetErrorString(err)); return (int)err; }
   if (out_dtype == DT_BF16)
-    launch_pdl(moe_gemv_kernel<__nv_bfloat16>, grid, dim3(MV_WARPS * 32), 0, stream, a, lda, a_div, w, order, plan,
+    launch_pdl(moe_gemv_kernel<__nv_bfloat16>, grid, dim3(MV_WARPS * 32), smem, stream, a, lda, a_div, w, order, plan,
                static_cast<__nv_bfloat16*>(out), N, K, act);
   else if (out_dtype == DT_F32)
-    launch_pdl(moe_gemv_kernel<float>, grid, dim3(MV_WARPS * 32), 0, stream, a, lda, a_div, w, order, plan,
+    launch_pdl(moe_gemv_kernel<float>, grid, dim3(MV_WARPS * 32), smem, stream, a, lda, a_div, w, order, plan,
                static_cast<float*>(out), N, K, act);
   else { set_error("moe_gemv: unsupported output type %d", out_dtype); return ERR_UNSUPPORTED; }
   return launch_status("moe_gemv");
