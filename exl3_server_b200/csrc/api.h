@@ -285,7 +285,8 @@ int exl3_gemm_pair_ss_blocks(int N);
 // 4) and merge them in shared memory; 2: a cluster of two blocks (at most 8 chunks, the first block merging, the
 // second one's records read out of its shared memory); no scratch in either.  twins 2 (with in_block 1 or 2, an even
 // head_split and groups of up to 8 heads): two groups of query heads of a kv head per block, walking the same pages
-// out of the same rings, 8 computing warps.  sink_vals and dist as in exl3_attn_tokens_opt.  See attention_decode.cu.
+// out of the same rings, 8 computing warps.  late: the next kernel of the stream starts when this one has ended.
+// sink_vals and dist as in exl3_attn_tokens_opt.  See attention_decode.cu.
 int exl3_attn_decode_supported(int dtype, int T, int nh, int nkv, int hd, int page, int split_keys, int max_splits);
 int exl3_attn_decode_status();
 int exl3_attn_decode(const void* q, int64_t q_row_stride, void* out, void* k_pool, void* v_pool,
@@ -294,7 +295,7 @@ int exl3_attn_decode(const void* q, int64_t q_row_stride, void* out, void* k_poo
                      float scale, int split_keys, int max_splits, float* scratch, size_t scratch_bytes, const float* inv_freq,
                      const float* inv_freq_lo, int rot, float pos_scale, int write_new, int head_split, int in_block,
                      int twins, const float* sink_vals, const float* dist, int dist_len, const float* gate,
-                     cudaStream_t stream);
+                     int late, cudaStream_t stream);
 
 int exl3_argmax(const float* logits, int* out, int R, int V, void* scratch, size_t scratch_bytes,
                 cudaStream_t stream);

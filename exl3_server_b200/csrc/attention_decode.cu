@@ -191,6 +191,7 @@ struct AdOpts {
   int dist_len;
   float dist_mul;                                        // 1 / scale: the biases join the scores before the scale
   const float* gate;                                     // a factor per (token, query head) on the output; null: none
+  int late;                                              // the next kernel starts when this one has ended
 };
 
 template <int HD, int NC, int TW>
@@ -242,7 +243,9 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   __syncwarp();
-  pdl_trigger();
+  // Where another stream's kernels want the SMs (late), the next kernel of this one waits for the end: let start here, it
+  // would hold their shared memory while it waits.
+  if (!opts.late) pdl_trigger();
   // Positions, sequences and page numbers are the step's inputs: no kernel of the step writes them.  When the
   // token's own key and value come from the projection (write_new), the cache pages this kernel reads hold
   // earlier steps' tokens only, so everything up to the first read of the queries, the first pages' copies
@@ -1006,7 +1009,7 @@ extern "C" int exl3_attn_decode(const void* q, int64_t q_row_stride, void* out, 
                                 float scale, int split_keys, int max_splits, float* scratch, size_t scratch_bytes,
                                 const float* inv_freq, const float* inv_freq_lo, int rot, float pos_scale,
                                 int write_new, int head_split, int in_block, int twins, const float* sink_vals,
-                                const float* dist, int dist_len, const float* gate, cudaStream_t stream) {
+                                const float* dist, int dist_len, const float* gate, int late, cudaStream_t stream) {
   if (T == 0) return 0;
   if (dist_len < 0 || (dist_len > 0 && dist == nullptr) || (sink_vals != nullptr && !sink)) {
     set_error("attn_decode: a table of %d distance biases is missing, or sink scores come without the sink", dist_len);
@@ -1073,6 +1076,7 @@ extern "C" int exl3_attn_decode(const void* q, int64_t q_row_stride, void* out, 
   opts.dist_len = dist_len;
   opts.dist_mul = 1.0f / scale;
   opts.gate = gate;
+  opts.late = late;
   // a stage is a page (heads of 64) or half a page (heads of 128): the copy's box has as many rows
   const int box_rows = hd == 64 ? 64 : 32;
   CUtensorMap map_k, map_v;

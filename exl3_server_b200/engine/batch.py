@@ -76,6 +76,8 @@ class StepBatch:
     # a second stream, in steps of one token per sequence: a block whose two sublayers do not depend on each other may run
     # one of them there (and must have joined it before it returns)
     side: Optional[Any] = None
+    # set while a block runs its mixer beside another sublayer: the mixer's kernels share the SMs with the other stream's
+    beside: bool = False
     # what a part has worked out for this step and wants to find again in the next layer (keyed as it likes)
     memo: Dict[Any, Any] = field(default_factory=dict)
 

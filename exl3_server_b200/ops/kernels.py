@@ -1089,7 +1089,7 @@ def attn_decode(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, k_pool: t
                 rot: int = 0, pos_scale: float = 1.0, write_new: bool = False, head_split: int = 1,
                 in_block: int = 0, twins: int = 1, chunk: int = 0, sink: bool = False,
                 sink_vals: Optional[torch.Tensor] = None, dist: Optional[torch.Tensor] = None,
-                gate: Optional[torch.Tensor] = None) -> torch.Tensor:
+                gate: Optional[torch.Tensor] = None, late: bool = False) -> torch.Tensor:
     """Attention of T query tokens over the paged cache on the tensor cores (see attention_decode.cu);
     arguments and scratch as ``attn_tokens``.  With ``write_new``, ``q`` is the fused q|k|v output of the
     projection, every token is its sequence's only new one and the cache holds the positions before it: the
@@ -1103,7 +1103,8 @@ def attn_decode(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, k_pool: t
     tickets; results differ from the other way's by rounding (another order of the same sums).  ``twins`` 2 (with
     ``in_block`` 1 or 2, an even ``head_split`` and groups of up to 8 heads): a block takes two groups of query heads
     of a kv head, whose warps walk the same pages out of the same rings; changes no result.  ``chunk``, ``sink``,
-    ``sink_vals``, ``dist`` and ``gate`` as in ``attn_tokens_ex``."""
+    ``sink_vals``, ``dist`` and ``gate`` as in ``attn_tokens_ex``.  ``late``: the next kernel of the stream starts when
+    this one has ended, and takes no room on the SMs before."""
     _check_gate(gate, T, heads, "attn_decode")
     if sink_vals is not None and (sink_vals.dtype != torch.float32 or sink_vals.numel() != heads or not sink):
         raise KernelLibraryError("attn_decode: sink scores must be float32 [heads], with the sink on")
@@ -1125,7 +1126,8 @@ def attn_decode(q: torch.Tensor, q_row_stride: int, out: torch.Tensor, k_pool: t
         _c_int(kv_heads), _c_int(head_dim), _c_int(page), _c_int(window), _c_int(chunk), _c_int(1 if sink else 0),
         _c_float(scale), _c_int(split_keys), _c_int(max_splits), _ptr(scratch), _c_size_t(nbytes), hi, lo, _c_int(rot),
         _c_float(pos_scale), _c_int(1 if write_new else 0), _c_int(head_split), _c_int(int(in_block)),
-        _c_int(int(twins)), _ptr(sink_vals), _ptr(dist), _c_int(dist_len), _ptr(gate), _stream()), "attn_decode")
+        _c_int(int(twins)), _ptr(sink_vals), _ptr(dist), _c_int(dist_len), _ptr(gate), _c_int(1 if late else 0),
+        _stream()), "attn_decode")
     return out
 
 

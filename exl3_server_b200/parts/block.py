@@ -244,7 +244,11 @@ class ParallelBlock:
             side.wait_stream(main)
             with torch.cuda.stream(side):
                 b, picks = self._feed(r, batch)
-            y = self.mixer.forward(r, batch, kv, state)
+            batch.beside = True
+            try:
+                y = self.mixer.forward(r, batch, kv, state)
+            finally:
+                batch.beside = False
             main.wait_stream(side)
         else:
             y = self.mixer.forward(r, batch, kv, state)

@@ -267,7 +267,8 @@ class NormedAttention:
             scratch = batch.workspace.floats(K.attn_tokens_scratch_bytes(T, H, d, n) // 4)
         K.attn_decode(q, q.stride(0), out, kv.k, kv.v, kv.block_table, batch.tok_pos, batch.tok_seq, T, H, G, d,
                       kv.page_size, self.window, self.scale, split, n, scratch, head_split=head_split, in_block=in_block,
-                      twins=twins, chunk=self.chunk, sink=self.sink, sink_vals=self.sink_vals, dist=self.dist, gate=gate)
+                      twins=twins, chunk=self.chunk, sink=self.sink, sink_vals=self.sink_vals, dist=self.dist, gate=gate,
+                      late=batch.beside)
         return True
 
     def _chunks(self, max_kv_len: int, split: int) -> int:
