@@ -87,23 +87,40 @@ __device__ inline void on_store8(float* p, const float (&v)[8]) {
 __device__ inline void on_store8(__nv_bfloat16* p, const float (&v)[8]) { store_vec(p, v); }
 
 constexpr int NA_VECS = 4;                       // pieces of 8 values per thread: rows up to 8192
+// Pieces of a thread for rows of H values: 1, 2 or 4.
+static int na_vecs(int H) { return H <= NA_THREADS * 8 ? 1 : H <= NA_THREADS * 16 ? 2 : 4; }
 
-// The same for rows of up to NA_THREADS * 8 * NA_VECS values, a multiple of 8: a thread keeps its pieces of y in
-// registers and every access is 16 or 32 bytes wide.  TX void: no copy of the residual is written.
-template <typename TY, typename TW, typename TX>
+// The same for rows of up to NA_THREADS * 8 * VECS values, a multiple of 8: a thread keeps its pieces of y in
+// registers and every access is 16 or 32 bytes wide.  TX void: no copy of the residual is written.  In this kernel and the
+// two below everything is asked for at once, the weights before the wait for the kernel before, the residual with y: behind
+// the sum of squares it would be a second trip to memory (@F1@).
+template <typename TY, typename TW, typename TX, int VECS>
 __global__ void __launch_bounds__(NA_THREADS)
 norm_add_vec_kernel(float* h, const TY* y, const TW* __restrict__ w, float eps, TX* x, int H) {
   __shared__ float red[32];
+  float wv[VECS][8];
+#pragma unroll
+  for (int p = 0; p < VECS; ++p) {
+    const int c = (p * NA_THREADS + threadIdx.x) * 8;
+    if (c < H) on_load8(w + c, wv[p], false);
+  }
   pdl_wait();
   pdl_trigger();
   const int64_t base = (int64_t)blockIdx.x * H;
-  float keep[NA_VECS][8];
+  float keep[VECS][8], hv[VECS][8];
   float ss = 0.0f;
 #pragma unroll
-  for (int p = 0; p < NA_VECS; ++p) {
+  for (int p = 0; p < VECS; ++p) {
     const int c = (p * NA_THREADS + threadIdx.x) * 8;
     if (c < H) {
       on_load8(y + base + c, keep[p], true);
+      on_load8(h + base + c, hv[p], true);
+    }
+  }
+#pragma unroll
+  for (int p = 0; p < VECS; ++p) {
+    const int c = (p * NA_THREADS + threadIdx.x) * 8;
+    if (c < H) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) ss += keep[p][e] * keep[p][e];
     }
@@ -111,16 +128,13 @@ norm_add_vec_kernel(float* h, const TY* y, const TW* __restrict__ w, float eps, 
   ss = block_sum(ss, red);
   const float inv = 1.0f / sqrtf(ss / (float)H + eps);
 #pragma unroll
-  for (int p = 0; p < NA_VECS; ++p) {
+  for (int p = 0; p < VECS; ++p) {
     const int c = (p * NA_THREADS + threadIdx.x) * 8;
     if (c < H) {
-      float hv[8], wv[8];
-      on_load8(h + base + c, hv, true);
-      on_load8(w + c, wv, false);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) hv[e] += keep[p][e] * inv * wv[e];
-      on_store8(h + base + c, hv);
-      if (x) on_store8(x + base + c, hv);
+      for (int e = 0; e < 8; ++e) hv[p][e] += keep[p][e] * inv * wv[p][e];
+      on_store8(h + base + c, hv[p]);
+      if (x) on_store8(x + base + c, hv[p]);
     }
   }
 }
@@ -169,15 +183,18 @@ __global__ void xielu_vec_kernel(const TI* z, const void* __restrict__ pq, int p
   }
 }
 
+template <typename TY, typename TW, typename TX>
+static void norm_add_vec_to(float* h, const void* y, const void* w, float eps, void* x, int T, int H, cudaStream_t stream) {
+  auto kernel = na_vecs(H) == 1 ? norm_add_vec_kernel<TY, TW, TX, 1> : na_vecs(H) == 2 ? norm_add_vec_kernel<TY, TW, TX, 2>
+                                                                                        : norm_add_vec_kernel<TY, TW, TX, 4>;
+  launch_pdl(kernel, dim3(T), dim3(NA_THREADS), 0, stream, h, static_cast<const TY*>(y), static_cast<const TW*>(w), eps,
+             static_cast<TX*>(x), H);
+}
 template <typename TY, typename TW>
 static void norm_add_vec(float* h, const void* y, const void* w, float eps, void* x, int x_dtype, int T, int H,
                          cudaStream_t stream) {
-  if (x == nullptr || x_dtype == DT_F32)
-    launch_pdl(norm_add_vec_kernel<TY, TW, float>, dim3(T), dim3(NA_THREADS), 0, stream, h, static_cast<const TY*>(y),
-               static_cast<const TW*>(w), eps, static_cast<float*>(x), H);
-  else
-    launch_pdl(norm_add_vec_kernel<TY, TW, __nv_bfloat16>, dim3(T), dim3(NA_THREADS), 0, stream, h,
-               static_cast<const TY*>(y), static_cast<const TW*>(w), eps, static_cast<__nv_bfloat16*>(x), H);
+  if (x == nullptr || x_dtype == DT_F32) norm_add_vec_to<TY, TW, float>(h, y, w, eps, x, T, H, stream);
+  else norm_add_vec_to<TY, TW, __nv_bfloat16>(h, y, w, eps, x, T, H, stream);
 }
 
 // norm_add followed by the next sublayer's input norm over the new residual, in one pass: a thread keeps its
@@ -231,23 +248,39 @@ norm_add_norm_kernel(float* h, const void* y, int y_dtype, const void* __restric
     on_store_any(x, x_dtype, base + c, h[base + c] * inv2 * on_load_any(w2, w2_dtype, c));
 }
 
-// The same for rows of up to NA_THREADS * 8 * NA_VECS values, a multiple of 8, with float32 weights: a thread keeps its
+// The same for rows of up to NA_THREADS * 8 * VECS values, a multiple of 8, with float32 weights: a thread keeps its
 // pieces of the row in registers through both norms and every access is 16 or 32 bytes wide.
-template <typename TY, typename TX>
+template <typename TY, typename TX, int VECS>
 __global__ void __launch_bounds__(NA_THREADS)
 norm_add_norm_vec_kernel(float* h, const TY* y, const float* __restrict__ w, float eps, const float* __restrict__ w2,
                          float eps2, TX* x, int H) {
   __shared__ float red[32];
+  float wv[VECS][8], wv2[VECS][8];
+#pragma unroll
+  for (int p = 0; p < VECS; ++p) {
+    const int c = (p * NA_THREADS + threadIdx.x) * 8;
+    if (c < H) {
+      on_load8(w + c, wv[p], false);
+      on_load8(w2 + c, wv2[p], false);
+    }
+  }
   pdl_wait();
   pdl_trigger();
   const int64_t base = (int64_t)blockIdx.x * H;
-  float keep[NA_VECS][8];
+  float keep[VECS][8], hv[VECS][8];
   float ss = 0.0f;
 #pragma unroll
-  for (int p = 0; p < NA_VECS; ++p) {
+  for (int p = 0; p < VECS; ++p) {
     const int c = (p * NA_THREADS + threadIdx.x) * 8;
     if (c < H) {
       on_load8(y + base + c, keep[p], true);
+      on_load8(h + base + c, hv[p], true);
+    }
+  }
+#pragma unroll
+  for (int p = 0; p < VECS; ++p) {
+    const int c = (p * NA_THREADS + threadIdx.x) * 8;
+    if (c < H) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) ss += keep[p][e] * keep[p][e];
     }
@@ -256,53 +289,69 @@ norm_add_norm_vec_kernel(float* h, const TY* y, const float* __restrict__ w, flo
   const float inv = 1.0f / sqrtf(ss / (float)H + eps);
   float ss2 = 0.0f;
 #pragma unroll
-  for (int p = 0; p < NA_VECS; ++p) {
+  for (int p = 0; p < VECS; ++p) {
     const int c = (p * NA_THREADS + threadIdx.x) * 8;
     if (c < H) {
-      float hv[8], wv[8];
-      on_load8(h + base + c, hv, true);
-      on_load8(w + c, wv, false);
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
-        hv[e] += keep[p][e] * inv * wv[e];
-        keep[p][e] = hv[e];
-        ss2 += hv[e] * hv[e];
+        hv[p][e] += keep[p][e] * inv * wv[p][e];
+        ss2 += hv[p][e] * hv[p][e];
       }
-      on_store8(h + base + c, hv);
+      on_store8(h + base + c, hv[p]);
     }
   }
   ss2 = block_sum(ss2, red);
   const float inv2 = 1.0f / sqrtf(ss2 / (float)H + eps2);
 #pragma unroll
-  for (int p = 0; p < NA_VECS; ++p) {
+  for (int p = 0; p < VECS; ++p) {
     const int c = (p * NA_THREADS + threadIdx.x) * 8;
     if (c < H) {
-      float wv[8];
-      on_load8(w2 + c, wv, false);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) keep[p][e] *= inv2 * wv[e];
-      on_store8(x + base + c, keep[p]);
+      for (int e = 0; e < 8; ++e) hv[p][e] *= inv2 * wv2[p][e];
+      on_store8(x + base + c, hv[p]);
     }
   }
 }
+template <typename TY, typename TX>
+static void norm_add_norm_vec(float* h, const void* y, const float* w, float eps, const float* w2, float eps2, void* x, int T,
+                              int H, cudaStream_t stream) {
+  auto kernel = na_vecs(H) == 1 ? norm_add_norm_vec_kernel<TY, TX, 1> : na_vecs(H) == 2 ? norm_add_norm_vec_kernel<TY, TX, 2>
+                                                                                        : norm_add_norm_vec_kernel<TY, TX, 4>;
+  launch_pdl(kernel, dim3(T), dim3(NA_THREADS), 0, stream, h, static_cast<const TY*>(y), w, eps, w2, eps2, static_cast<TX*>(x), H);
+}
 
 // The two-output norm and sum with 16-byte accesses (rows as above, float32 weights).
-template <typename TA>
+template <typename TA, int VECS>
 __global__ void __launch_bounds__(NA_THREADS)
 normed_sum2_vec_kernel(const TA* a, const TA* b, const float* __restrict__ wa, const float* __restrict__ wb, float eps,
                        float coef, float* out, int H) {
   __shared__ float red[32];
+  float wx[VECS][8], wy[VECS][8];
+#pragma unroll
+  for (int p = 0; p < VECS; ++p) {
+    const int c = (p * NA_THREADS + threadIdx.x) * 8;
+    if (c < H) {
+      on_load8(wa + c, wx[p], false);
+      on_load8(wb + c, wy[p], false);
+    }
+  }
   pdl_wait();
   pdl_trigger();
   const int64_t base = (int64_t)blockIdx.x * H;
-  float ka[NA_VECS][8], kb[NA_VECS][8];
+  float ka[VECS][8], kb[VECS][8];
   float sa = 0.0f, sb = 0.0f;
 #pragma unroll
-  for (int p = 0; p < NA_VECS; ++p) {
+  for (int p = 0; p < VECS; ++p) {
     const int c = (p * NA_THREADS + threadIdx.x) * 8;
     if (c < H) {
       on_load8(a + base + c, ka[p], true);
       on_load8(b + base + c, kb[p], true);
+    }
+  }
+#pragma unroll
+  for (int p = 0; p < VECS; ++p) {
+    const int c = (p * NA_THREADS + threadIdx.x) * 8;
+    if (c < H) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) { sa += ka[p][e] * ka[p][e]; sb += kb[p][e] * kb[p][e]; }
     }
@@ -311,17 +360,23 @@ normed_sum2_vec_kernel(const TA* a, const TA* b, const float* __restrict__ wa, c
   sb = block_sum(sb, red);
   const float ia = coef / sqrtf(sa / (float)H + eps), ib = coef / sqrtf(sb / (float)H + eps);
 #pragma unroll
-  for (int p = 0; p < NA_VECS; ++p) {
+  for (int p = 0; p < VECS; ++p) {
     const int c = (p * NA_THREADS + threadIdx.x) * 8;
     if (c < H) {
-      float wx[8], wy[8], o[8];
-      on_load8(wa + c, wx, false);
-      on_load8(wb + c, wy, false);
+      float o[8];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) o[e] = ka[p][e] * ia * wx[e] + kb[p][e] * ib * wy[e];
+      for (int e = 0; e < 8; ++e) o[e] = ka[p][e] * ia * wx[p][e] + kb[p][e] * ib * wy[p][e];
       on_store8(out + base + c, o);
     }
   }
+}
+template <typename TA>
+static void normed_sum2_vec(const void* a, const void* b, const void* wa, const void* wb, float eps, float coef, float* out, int T,
+                            int H, cudaStream_t stream) {
+  auto kernel = na_vecs(H) == 1 ? normed_sum2_vec_kernel<TA, 1> : na_vecs(H) == 2 ? normed_sum2_vec_kernel<TA, 2>
+                                                                                  : normed_sum2_vec_kernel<TA, 4>;
+  launch_pdl(kernel, dim3(T), dim3(NA_THREADS), 0, stream, static_cast<const TA*>(a), static_cast<const TA*>(b),
+             static_cast<const float*>(wa), static_cast<const float*>(wb), eps, coef, out, H);
 }
 
 // Two sublayer outputs side by side, each normed over the row with its own weight, then averaged:
@@ -397,14 +452,11 @@ extern "C" int exl3_norm_add_norm(float* h, const void* y, int y_dtype, const vo
   const float* wf = static_cast<const float*>(w);
   const float* w2f = static_cast<const float*>(w2);
   if (vec && y_dtype == DT_BF16 && x_dtype == DT_BF16)
-    launch_pdl(norm_add_norm_vec_kernel<__nv_bfloat16, __nv_bfloat16>, dim3(T), dim3(NA_THREADS), 0, stream, h,
-               static_cast<const __nv_bfloat16*>(y), wf, eps, w2f, eps2, static_cast<__nv_bfloat16*>(x), H);
+    norm_add_norm_vec<__nv_bfloat16, __nv_bfloat16>(h, y, wf, eps, w2f, eps2, x, T, H, stream);
   else if (vec && y_dtype == DT_F32 && x_dtype == DT_BF16)
-    launch_pdl(norm_add_norm_vec_kernel<float, __nv_bfloat16>, dim3(T), dim3(NA_THREADS), 0, stream, h,
-               static_cast<const float*>(y), wf, eps, w2f, eps2, static_cast<__nv_bfloat16*>(x), H);
+    norm_add_norm_vec<float, __nv_bfloat16>(h, y, wf, eps, w2f, eps2, x, T, H, stream);
   else if (vec && y_dtype == DT_F32 && x_dtype == DT_F32)
-    launch_pdl(norm_add_norm_vec_kernel<float, float>, dim3(T), dim3(NA_THREADS), 0, stream, h,
-               static_cast<const float*>(y), wf, eps, w2f, eps2, static_cast<float*>(x), H);
+    norm_add_norm_vec<float, float>(h, y, wf, eps, w2f, eps2, x, T, H, stream);
   else
     launch_pdl(norm_add_norm_kernel, dim3(T), dim3(NA_THREADS), 0, stream, h, y, y_dtype, w, w_dtype, eps, w2, w2_dtype,
                eps2, x, x_dtype, H);
@@ -420,13 +472,8 @@ extern "C" int exl3_normed_sum2(const void* a, const void* b, int ab_dtype, cons
   }
   const bool vec = H % 8 == 0 && H <= NA_THREADS * 8 * NA_VECS && w_dtype == DT_F32 && aligned16(a) && aligned16(b) &&
                    aligned16(wa) && aligned16(wb) && aligned16(out);
-  if (vec && ab_dtype == DT_BF16)
-    launch_pdl(normed_sum2_vec_kernel<__nv_bfloat16>, dim3(T), dim3(NA_THREADS), 0, stream,
-               static_cast<const __nv_bfloat16*>(a), static_cast<const __nv_bfloat16*>(b), static_cast<const float*>(wa),
-               static_cast<const float*>(wb), eps, coef, out, H);
-  else if (vec && ab_dtype == DT_F32)
-    launch_pdl(normed_sum2_vec_kernel<float>, dim3(T), dim3(NA_THREADS), 0, stream, static_cast<const float*>(a),
-               static_cast<const float*>(b), static_cast<const float*>(wa), static_cast<const float*>(wb), eps, coef, out, H);
+  if (vec && ab_dtype == DT_BF16) normed_sum2_vec<__nv_bfloat16>(a, b, wa, wb, eps, coef, out, T, H, stream);
+  else if (vec && ab_dtype == DT_F32) normed_sum2_vec<float>(a, b, wa, wb, eps, coef, out, T, H, stream);
   else
     launch_pdl(normed_sum2_kernel, dim3(T), dim3(NA_THREADS), 0, stream, a, b, ab_dtype, wa, wb, w_dtype, eps, coef, out, H);
   return launch_status("normed_sum2");

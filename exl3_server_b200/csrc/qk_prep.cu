@@ -217,7 +217,7 @@ __device__ inline void qp_load8<float>(const float* p, float (&v)[8]) {
 template <>
 __device__ inline void qp_load8<__nv_bfloat16>(const __nv_bfloat16* p, float (&v)[8]) { load_vec_cg(p, v); }
 
-template <typename TX, typename TS>
+template <typename TX, typename TS, int JOBS>
 __global__ void __launch_bounds__(QP_WARPS * 32) qk_prep_vec_kernel(QkPrepArgs a, int lph) {
   __shared__ float s_sn[QP_TABLE], s_cs[QP_TABLE];
   const int t = blockIdx.x;
@@ -240,22 +240,16 @@ __global__ void __launch_bounds__(QP_WARPS * 32) qk_prep_vec_kernel(QkPrepArgs a
   __syncthreads();
   const int per_warp = 32 / lph;
   const int jobs = a.nh + 2 * a.nkv;
-  const int job = ((int)blockIdx.y * QP_WARPS + warp) * per_warp + lane / lph;
   const int e0 = (lane % lph) * 8;
-  const bool live = job < jobs;
-  const bool is_q = job < a.nh, is_k = !is_q && job < a.nh + a.nkv;
-  const int head = is_q ? job : (is_k ? job - a.nh : job - a.nh - a.nkv);
   const TX* x = static_cast<const TX*>(a.x) + (int64_t)t * a.ld;
   __nv_bfloat16* kp = static_cast<__nv_bfloat16*>(a.k_pool);
   __nv_bfloat16* vp = static_cast<__nv_bfloat16*>(a.v_pool);
-  float v[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) v[e] = 0.0f;
   // norm 3: the factors of the token's queries and keys (see the kernel above)
   float inv_q = 1.0f, inv_k = 1.0f;
   if (a.norm == 3) {
     __shared__ float red[32];
-    const int first = (int)blockIdx.y * QP_WARPS * per_warp, end = min(jobs, first + QP_WARPS * per_warp);
+    const int first = (int)blockIdx.y * QP_WARPS * per_warp;
+    const int end = JOBS > 1 ? jobs : min(jobs, first + QP_WARPS * per_warp);
     auto row_inv = [&](int off, int n) {
       float ss = 0.0f;
       for (int e = threadIdx.x * 8; e < n; e += QP_WARPS * 32 * 8) {
@@ -269,10 +263,29 @@ __global__ void __launch_bounds__(QP_WARPS * 32) qk_prep_vec_kernel(QkPrepArgs a
     if (first < a.nh) inv_q = row_inv(a.q_off, a.nh * a.hd);
     if (end > a.nh && first < a.nh + a.nkv) inv_k = row_inv(a.k_off, a.nkv * a.hd);
   }
+  // JOBS 1: the heads are dealt to the blocks of the token; else this block takes all of them, JOBS at a time, whose pieces
+  // are asked for together
+  for (int y = (int)blockIdx.y; y * QP_WARPS * per_warp < jobs; y += JOBS) {
+  float vs[JOBS][8];
+#pragma unroll
+  for (int u = 0; u < JOBS; ++u) {
+    const int job = ((y + u) * QP_WARPS + warp) * per_warp + lane / lph;
+    const bool is_v = job >= a.nh + a.nkv;
+    const int off = job < a.nh ? a.q_off + job * a.hd : !is_v ? a.k_off + (job - a.nh) * a.hd : a.v_off + (job - a.nh - a.nkv) * a.hdv;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) vs[u][e] = 0.0f;
+    if (job < jobs && e0 < (is_v ? a.hdv : a.hd) && (!is_v || pg >= 0)) qp_load8<TX>(x + off + e0, vs[u]);
+  }
+#pragma unroll
+  for (int u = 0; u < JOBS; ++u) {
+  float (&v)[8] = vs[u];
+  const int job = ((y + u) * QP_WARPS + warp) * per_warp + lane / lph;
+  const bool live = job < jobs;
+  const bool is_q = job < a.nh, is_k = !is_q && job < a.nh + a.nkv;
+  const int head = is_q ? job : (is_k ? job - a.nh : job - a.nh - a.nkv);
   if (live && !is_q && !is_k) {
     // a value head
     if (e0 < a.hdv_pad && pg >= 0) {
-      if (e0 < a.hdv) qp_load8<TX>(x + a.v_off + (int64_t)head * a.hdv + e0, v);
       if (a.lambda != nullptr && e0 < a.hdv) {
         const float lam = qp_load(a.lambda, a.lambda_dtype, 0);
         float o[8];
@@ -285,7 +298,6 @@ __global__ void __launch_bounds__(QP_WARPS * 32) qk_prep_vec_kernel(QkPrepArgs a
   }
   const bool qk = live && (is_q || is_k);
   const bool mine = qk && e0 < a.hd;
-  if (mine) qp_load8<TX>(x + (is_q ? a.q_off : a.k_off) + (int64_t)head * a.hd + e0, v);
   float inv = is_q ? inv_q : inv_k;
   if (a.norm == 1 || a.norm == 2) {
     // every lane takes part in the shuffles; a head's lanes are neighbours
@@ -297,7 +309,7 @@ __global__ void __launch_bounds__(QP_WARPS * 32) qk_prep_vec_kernel(QkPrepArgs a
     for (int o = lph >> 1; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     inv = 1.0f / sqrtf(ss / (float)a.hd + a.eps);
   }
-  if (!qk || e0 >= a.hd_pad) return;
+  if (!qk || e0 >= a.hd_pad) continue;
   if (a.norm >= 2 && mine) {
     float w[8];
     const float* wp = static_cast<const float*>(is_q ? a.q_w : a.k_w) + (a.norm == 3 ? head * a.hd : 0) + e0;
@@ -313,9 +325,9 @@ __global__ void __launch_bounds__(QP_WARPS * 32) qk_prep_vec_kernel(QkPrepArgs a
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
       const float sn = s_sn[(e0 >> 1) + p], cs = s_cs[(e0 >> 1) + p];
-      const float u = v[2 * p], w2 = v[2 * p + 1];
-      v[2 * p] = fmaf(u, cs, -w2 * sn);
-      v[2 * p + 1] = fmaf(w2, cs, u * sn);
+      const float u2 = v[2 * p], w2 = v[2 * p + 1];
+      v[2 * p] = fmaf(u2, cs, -w2 * sn);
+      v[2 * p + 1] = fmaf(w2, cs, u2 * sn);
     }
   }
   if (is_q) {
@@ -328,6 +340,18 @@ __global__ void __launch_bounds__(QP_WARPS * 32) qk_prep_vec_kernel(QkPrepArgs a
     for (int e = 0; e < 8; ++e) v[e] *= a.k_mul;
     store_vec(kp + (((int64_t)pg * a.nkv + head) * a.page + in_page) * a.hd_pad + e0, v);
   }
+  }
+  if (JOBS == 1) break;
+  }
+}
+
+template <typename TX, typename TS>
+static void qk_prep_vec(const QkPrepArgs& a, int lph, int T, int jobs, cudaStream_t stream) {
+  const int groups = ceil_div(jobs, QP_WARPS * (32 / lph));
+  // Many tokens: a block takes all heads of its token, four pieces a thread on their way (the sines and the block's start once a
+  // token, not once for every eight warps of heads: @F2@).
+  if (groups > 1 && T >= 512) launch_pdl(qk_prep_vec_kernel<TX, TS, 4>, dim3(T), dim3(QP_WARPS * 32), 0, stream, a, lph);
+  else launch_pdl(qk_prep_vec_kernel<TX, TS, 1>, dim3(T, groups), dim3(QP_WARPS * 32), 0, stream, a, lph);
 }
 
 // What a recurrence takes: queries and keys rotated as whole heads (feature i with i + hd / 2) or not at all, as float32, without
@@ -428,14 +452,12 @@ extern "C" int exl3_qk_prep(const void* x, int x_dtype, int64_t ld, int q_off, i
       aligned16(k_pool) && aligned16(v_pool) && src_ok && (norm < 2 || (aligned16(q_w) && aligned16(k_w)))) {
     int lph = 1;
     while (lph * 8 < widest) lph <<= 1;
-    const int per_block = QP_WARPS * (32 / lph);
     const int jobs = nh + 2 * nkv;
-    const dim3 grid(T, ceil_div(jobs, per_block)), threads(QP_WARPS * 32);
     const bool xf = x_dtype == DT_F32, sf = mix_lambda != nullptr && v_src_dtype == DT_F32;
-    if (xf && sf) launch_pdl(qk_prep_vec_kernel<float, float>, grid, threads, 0, stream, a, lph);
-    else if (xf) launch_pdl(qk_prep_vec_kernel<float, __nv_bfloat16>, grid, threads, 0, stream, a, lph);
-    else if (sf) launch_pdl(qk_prep_vec_kernel<__nv_bfloat16, float>, grid, threads, 0, stream, a, lph);
-    else launch_pdl(qk_prep_vec_kernel<__nv_bfloat16, __nv_bfloat16>, grid, threads, 0, stream, a, lph);
+    if (xf && sf) qk_prep_vec<float, float>(a, lph, T, jobs, stream);
+    else if (xf) qk_prep_vec<float, __nv_bfloat16>(a, lph, T, jobs, stream);
+    else if (sf) qk_prep_vec<__nv_bfloat16, float>(a, lph, T, jobs, stream);
+    else qk_prep_vec<__nv_bfloat16, __nv_bfloat16>(a, lph, T, jobs, stream);
     return launch_status("qk_prep");
   }
   if (v_off < 0 && k_pool == nullptr && gate_out == nullptr && norm == 0 && (rot == 0 || (layout == 0 && rot == hd)) &&
