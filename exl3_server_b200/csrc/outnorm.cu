@@ -93,7 +93,8 @@ static int na_vecs(int H) { return H <= NA_THREADS * 8 ? 1 : H <= NA_THREADS * 1
 // The same for rows of up to NA_THREADS * 8 * VECS values, a multiple of 8: a thread keeps its pieces of y in
 // registers and every access is 16 or 32 bytes wide.  TX void: no copy of the residual is written.  In this kernel and the
 // two below everything is asked for at once, the weights before the wait for the kernel before, the residual with y: behind
-// the sum of squares it would be a second trip to memory (@F1@).
+// the sum of squares it would be a second trip to memory (8 rows of 2,048 with both norms 2.7 -> 2.1 us, 3,163 rows
+// 16.1 -> 14.9).
 template <typename TY, typename TW, typename TX, int VECS>
 __global__ void __launch_bounds__(NA_THREADS)
 norm_add_vec_kernel(float* h, const TY* y, const TW* __restrict__ w, float eps, TX* x, int H) {

@@ -217,13 +217,59 @@ __device__ inline void qp_load8<float>(const float* p, float (&v)[8]) {
 template <>
 __device__ inline void qp_load8<__nv_bfloat16>(const __nv_bfloat16* p, float (&v)[8]) { load_vec_cg(p, v); }
 
+// eight values as they lie in memory
+template <typename TX> struct QpRaw;
+template <> struct QpRaw<__nv_bfloat16> {
+  uint4 r;
+  __device__ void load(const __nv_bfloat16* p) { r = __ldcg(reinterpret_cast<const uint4*>(p)); }
+  __device__ void zero() { r = make_uint4(0, 0, 0, 0); }
+  __device__ void get(float (&v)[8]) const {
+    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) { v[2 * e] = __uint_as_float(w[e] << 16); v[2 * e + 1] = __uint_as_float(w[e] & 0xffff0000u); }
+  }
+};
+template <> struct QpRaw<float> {
+  float r[8];
+  __device__ void load(const float* p) { qp_load8<float>(p, r); }
+  __device__ void zero() {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) r[e] = 0.0f;
+  }
+  __device__ void get(float (&v)[8]) const {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = r[e];
+  }
+};
+
 template <typename TX, typename TS, int JOBS>
-__global__ void __launch_bounds__(QP_WARPS * 32) qk_prep_vec_kernel(QkPrepArgs a, int lph) {
+__global__ void __launch_bounds__(QP_WARPS * 32, JOBS > 1 && sizeof(TX) == 2 ? 4 : 1) qk_prep_vec_kernel(QkPrepArgs a, int lph_log2) {
   __shared__ float s_sn[QP_TABLE], s_cs[QP_TABLE];
   const int t = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // before the wait: the token's position and page, its sines and cosines (launch_pdl says why these may be read here): a step
-  // of few tokens waits 1 us less for it
+  const int lph = 1 << lph_log2, per_warp = 32 >> lph_log2;
+  const int jobs = a.nh + 2 * a.nkv;
+  const int e0 = (lane & (lph - 1)) * 8, job0 = warp * per_warp + (lane >> lph_log2);   // and u * QP_WARPS * per_warp further on
+  const TX* x = static_cast<const TX*>(a.x) + (int64_t)t * a.ld;
+  // this thread's pieces of the JOBS heads from y on
+  QpRaw<TX> raw[JOBS];
+  auto ask = [&](int y) {
+#pragma unroll
+    for (int u = 0; u < JOBS; ++u) {
+      const int job = (y + u) * QP_WARPS * per_warp + job0;
+      const bool is_v = job >= a.nh + a.nkv;
+      const int off = job < a.nh ? a.q_off + job * a.hd : !is_v ? a.k_off + (job - a.nh) * a.hd : a.v_off + (job - a.nh - a.nkv) * a.hdv;
+      if (job < jobs && e0 < (is_v ? a.hdv : a.hd)) raw[u].load(x + off + e0);
+      else raw[u].zero();
+    }
+  };
+  // With few tokens the position and page, the sines and cosines come before the wait (launch_pdl says why these may be read
+  // here): a step waits 1 us less for it.  With many the pieces are asked for first.
+  if (JOBS > 1) {
+    pdl_wait();
+    pdl_trigger();
+    ask(0);
+  }
   const int pos = __ldcg(a.tok_pos + t);
   const int pg = a.nkv > 0 ? __ldcg(a.block_table + (int64_t)__ldcg(a.tok_seq + t) * a.bt_stride + pos / a.page) : -1;
   const int in_page = a.nkv > 0 ? pos % a.page : 0;
@@ -234,16 +280,24 @@ __global__ void __launch_bounds__(QP_WARPS * 32) qk_prep_vec_kernel(QkPrepArgs a
     s_sn[i] = sn * a.mscale;
     s_cs[i] = cs * a.mscale;
   }
-  pdl_wait();
-  pdl_trigger();
+  if (JOBS == 1) {
+    pdl_wait();
+    pdl_trigger();
+    ask((int)blockIdx.y);
+  }
   qp_gates(a, t);
   __syncthreads();
-  const int per_warp = 32 / lph;
-  const int jobs = a.nh + 2 * a.nkv;
-  const int e0 = (lane % lph) * 8;
-  const TX* x = static_cast<const TX*>(a.x) + (int64_t)t * a.ld;
-  __nv_bfloat16* kp = static_cast<__nv_bfloat16*>(a.k_pool);
-  __nv_bfloat16* vp = static_cast<__nv_bfloat16*>(a.v_pool);
+  // what all of the thread's heads have in common
+  const int64_t place = (int64_t)pg * a.nkv * a.page + in_page;
+  __nv_bfloat16* kp = static_cast<__nv_bfloat16*>(a.k_pool) + place * a.hd_pad + e0;
+  __nv_bfloat16* vp = static_cast<__nv_bfloat16*>(a.v_pool) + place * a.hdv_pad + e0;
+  __nv_bfloat16* qp = static_cast<__nv_bfloat16*>(a.q_out) + (int64_t)t * a.nh * a.hd_pad + e0;
+  const float q_mul = qp_temperature(a, pos);
+  float sn[4], cs[4];
+  if (e0 < a.rot) {                                    // rot is a multiple of 8 here: all of the lane's pairs or none
+#pragma unroll
+    for (int p = 0; p < 4; ++p) { sn[p] = s_sn[(e0 >> 1) + p]; cs[p] = s_cs[(e0 >> 1) + p]; }
+  }
   // norm 3: the factors of the token's queries and keys (see the kernel above)
   float inv_q = 1.0f, inv_k = 1.0f;
   if (a.norm == 3) {
@@ -266,20 +320,12 @@ __global__ void __launch_bounds__(QP_WARPS * 32) qk_prep_vec_kernel(QkPrepArgs a
   // JOBS 1: the heads are dealt to the blocks of the token; else this block takes all of them, JOBS at a time, whose pieces
   // are asked for together
   for (int y = (int)blockIdx.y; y * QP_WARPS * per_warp < jobs; y += JOBS) {
-  float vs[JOBS][8];
+  if (y > (int)blockIdx.y) ask(y);
 #pragma unroll
   for (int u = 0; u < JOBS; ++u) {
-    const int job = ((y + u) * QP_WARPS + warp) * per_warp + lane / lph;
-    const bool is_v = job >= a.nh + a.nkv;
-    const int off = job < a.nh ? a.q_off + job * a.hd : !is_v ? a.k_off + (job - a.nh) * a.hd : a.v_off + (job - a.nh - a.nkv) * a.hdv;
-#pragma unroll
-    for (int e = 0; e < 8; ++e) vs[u][e] = 0.0f;
-    if (job < jobs && e0 < (is_v ? a.hdv : a.hd) && (!is_v || pg >= 0)) qp_load8<TX>(x + off + e0, vs[u]);
-  }
-#pragma unroll
-  for (int u = 0; u < JOBS; ++u) {
-  float (&v)[8] = vs[u];
-  const int job = ((y + u) * QP_WARPS + warp) * per_warp + lane / lph;
+  float v[8];
+  raw[u].get(v);
+  const int job = (y + u) * QP_WARPS * per_warp + job0;
   const bool live = job < jobs;
   const bool is_q = job < a.nh, is_k = !is_q && job < a.nh + a.nkv;
   const int head = is_q ? job : (is_k ? job - a.nh : job - a.nh - a.nkv);
@@ -293,7 +339,7 @@ __global__ void __launch_bounds__(QP_WARPS * 32) qk_prep_vec_kernel(QkPrepArgs a
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[e] = (1.0f - lam) * v[e] + lam * o[e];
       }
-      store_vec(vp + (((int64_t)pg * a.nkv + head) * a.page + in_page) * a.hdv_pad + e0, v);
+      store_vec(vp + head * a.page * a.hdv_pad, v);
     }
   }
   const bool qk = live && (is_q || is_k);
@@ -321,24 +367,22 @@ __global__ void __launch_bounds__(QP_WARPS * 32) qk_prep_vec_kernel(QkPrepArgs a
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] *= inv;
   }
-  if (e0 < a.rot) {                                    // rot is a multiple of 8 here: all of the lane's pairs or none
+  if (e0 < a.rot) {
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
-      const float sn = s_sn[(e0 >> 1) + p], cs = s_cs[(e0 >> 1) + p];
       const float u2 = v[2 * p], w2 = v[2 * p + 1];
-      v[2 * p] = fmaf(u2, cs, -w2 * sn);
-      v[2 * p + 1] = fmaf(w2, cs, u2 * sn);
+      v[2 * p] = fmaf(u2, cs[p], -w2 * sn[p]);
+      v[2 * p + 1] = fmaf(w2, cs[p], u2 * sn[p]);
     }
   }
   if (is_q) {
-    const float q_mul = qp_temperature(a, pos);
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] *= q_mul;
-    store_vec(static_cast<__nv_bfloat16*>(a.q_out) + ((int64_t)t * a.nh + head) * a.hd_pad + e0, v);
+    store_vec(qp + head * a.hd_pad, v);
   } else if (pg >= 0) {
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] *= a.k_mul;
-    store_vec(kp + (((int64_t)pg * a.nkv + head) * a.page + in_page) * a.hd_pad + e0, v);
+    store_vec(kp + head * a.page * a.hd_pad, v);
   }
   }
   if (JOBS == 1) break;
@@ -346,12 +390,13 @@ __global__ void __launch_bounds__(QP_WARPS * 32) qk_prep_vec_kernel(QkPrepArgs a
 }
 
 template <typename TX, typename TS>
-static void qk_prep_vec(const QkPrepArgs& a, int lph, int T, int jobs, cudaStream_t stream) {
-  const int groups = ceil_div(jobs, QP_WARPS * (32 / lph));
+static void qk_prep_vec(const QkPrepArgs& a, int lph_log2, int T, int jobs, cudaStream_t stream) {
+  const int groups = ceil_div(jobs, QP_WARPS * (32 >> lph_log2));
   // Many tokens: a block takes all heads of its token, four pieces a thread on their way (the sines and the block's start once a
-  // token, not once for every eight warps of heads: @F2@).
-  if (groups > 1 && T >= 512) launch_pdl(qk_prep_vec_kernel<TX, TS, 4>, dim3(T), dim3(QP_WARPS * 32), 0, stream, a, lph);
-  else launch_pdl(qk_prep_vec_kernel<TX, TS, 1>, dim3(T, groups), dim3(QP_WARPS * 32), 0, stream, a, lph);
+  // token, not once for every eight warps of heads: 48 heads of 128 at 512 / 2,000 / 3,163 tokens 6.1 -> 5.4, 17.3 -> 14.5,
+  // 25.8 -> 21.2 us).  With fewer the heads are spread over blocks.
+  if (groups > 1 && T >= 512) launch_pdl(qk_prep_vec_kernel<TX, TS, 4>, dim3(T), dim3(QP_WARPS * 32), 0, stream, a, lph_log2);
+  else launch_pdl(qk_prep_vec_kernel<TX, TS, 1>, dim3(T, groups), dim3(QP_WARPS * 32), 0, stream, a, lph_log2);
 }
 
 // What a recurrence takes: queries and keys rotated as whole heads (feature i with i + hd / 2) or not at all, as float32, without
@@ -450,8 +495,8 @@ extern "C" int exl3_qk_prep(const void* x, int x_dtype, int64_t ld, int q_off, i
       (rot == 0 || (layout == 1 && rot % 8 == 0 && rot / 2 <= QP_TABLE)) &&
       (norm < 2 || w_dtype == DT_F32) && (x_dtype == DT_BF16 || x_dtype == DT_F32) && aligned16(x) && aligned16(q_out) &&
       aligned16(k_pool) && aligned16(v_pool) && src_ok && (norm < 2 || (aligned16(q_w) && aligned16(k_w)))) {
-    int lph = 1;
-    while (lph * 8 < widest) lph <<= 1;
+    int lph = 0;                                       // log2 of the lanes a head takes
+    while ((8 << lph) < widest) ++lph;
     const int jobs = nh + 2 * nkv;
     const bool xf = x_dtype == DT_F32, sf = mix_lambda != nullptr && v_src_dtype == DT_F32;
     if (xf && sf) qk_prep_vec<float, float>(a, lph, T, jobs, stream);
