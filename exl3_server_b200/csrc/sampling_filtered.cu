@@ -20,12 +20,15 @@
 //
 // A row is the work of a cluster of up to eight blocks.  Each reads its part of
 // the row once, with the penalties applied on the way, and keeps the keys in
-// shared memory, where the passes of the select find them; a pass's histograms
+// shared memory, where the passes of the select find them (the first pass's
+// histogram is taken while the row is read); a pass's histograms
 // meet through distributed shared memory (every block adds all of them up and
-// finds the same digit), and the passing keys are written into the first
-// block's, which sorts and draws.  Bound by the chain of passes, barriers and the
-// sort: 32 rows of 122,753 take 41 us, 44 with penalties (one block a row that reads it five times:
-// 105 us, and the penalties were a copy of the logits and a kernel of 16 us).
+// finds the same digit), and the passing keys are dealt out to the blocks in equal
+// shares.  Each sorts its share, every block reads all the shares, and a key's place
+// among all of them goes with it into the first block, which draws.  Bound by the chain of
+// passes and barriers (of 42 us with one block sorting: the row 4.4, three passes 5 to 6 each,
+// the collection 4.4, the sort of 2,048 13.6, the draw 4): 32 rows of 122,753 take 34 us, one row 31.
+// (One block a row that reads it five times: 105 us, and the penalties were a copy of the logits and a kernel of 16 us.)
 #include "api.h"
 #include "common.cuh"
 
@@ -60,8 +63,11 @@ struct SfBatch {
   float params[SF_DIRECT_ROWS][3];
 };
 
-constexpr double SF_FIXED_US = 35.0, SF_STAGED_US = 0.00018, SF_AGAIN_US = 0.00033, SF_AGAIN_PENALTIES_US = 0.00075;
+// the model of a launch's time (sf_launch): a wave of rows with 8 / 4 / 2 / 1 blocks a row, and a token of a block's part
+constexpr double SF_FIXED_US[4] = {26.5, 23.0, 24.5, 28.0}, SF_AGAIN_FIXED_US = 6.0;
+constexpr double SF_STAGED_US = 0.00032, SF_AGAIN_US = 0.00033, SF_AGAIN_PENALTIES_US = 0.00075;
 constexpr int SF_BINS = 2048;
+constexpr int SF_BLOCKS = 8;                     // of a row, at most
 constexpr int SF_HEAD_BYTES = (2 * SF_BINS * 4) + 2 * (SF_CAP * 8);     // histograms, candidates, this block's own
 constexpr int SF_SMEM_MOST = 200 * 1024;                                // with the staged part of a row
 
@@ -99,10 +105,9 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
                        const __grid_constant__ SfBatch batch, int* host_out, bool count_now) {
   extern __shared__ __align__(16) unsigned char sf_smem[];
   unsigned* hists = reinterpret_cast<unsigned*>(sf_smem);                                      // [2][SF_BINS]
-  unsigned long long* cand = reinterpret_cast<unsigned long long*>(sf_smem + 2 * SF_BINS * 4);  // the first block's: all
-  unsigned long long* found = cand + SF_CAP;                                                   // this block's
+  unsigned long long* cand = reinterpret_cast<unsigned long long*>(sf_smem + 2 * SF_BINS * 4);  // this block's share of them
+  unsigned long long* found = cand + SF_CAP;                                                   // those of this block's tokens
   uint32_t* keys = reinterpret_cast<uint32_t*>(sf_smem + SF_HEAD_BYTES);                       // this block's part of the row
-  double* acc = reinterpret_cast<double*>(sf_smem);          // running sums of probs, once the histograms are done with
   float* probs = reinterpret_cast<float*>(found);            // and once the block's own candidates are
   __shared__ double warp_tot[SF_THREADS / 32];
   __shared__ unsigned warp_cnt[SF_THREADS / 32];
@@ -126,12 +131,23 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
     if (host_out) host_out[row_id] = t;
     if (count && count_now && t >= 0 && t < V) atomicAdd(const_cast<int*>(count) + t, 1);
   };
+  const int slots = SF_CAP / blocks;             // a block's share of the candidates (blocks is a power of two)
   const int per = (V + blocks - 1) / blocks;
   const int first = min(V, rank * per), n = min(V, first + per) - first;
   // f(value's key, place in the row) for every token of this block's part
   auto for_each = [&](auto&& f) {
     if constexpr (STAGED) {
-      for (int i = tid; i < n; i += SF_THREADS) f(keys[i], first + i);
+      const uint4* keys4 = reinterpret_cast<const uint4*>(keys);
+#pragma unroll 2
+      for (int j = tid; j < n / 4; j += SF_THREADS) {
+        const uint4 k = keys4[j];
+        const int i = first + 4 * j;
+        f(k.x, i);
+        f(k.y, i + 1);
+        f(k.z, i + 2);
+        f(k.w, i + 3);
+      }
+      for (int i = n / 4 * 4 + tid; i < n; i += SF_THREADS) f(keys[i], first + i);
     } else {
       // 16-byte loads, four of a thread on their way, with penalties two and as many of the counts (parts start at any
       // multiple of 4 bytes: the pieces before and after the aligned part go one by one)
@@ -173,7 +189,12 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
       for (int i = head + 4 * n_vec + tid; i < n; i += SF_THREADS) one(i);
     }
   };
+  for (int b = tid; b < SF_BINS; b += SF_THREADS) hists[b] = 0;
+  for (int i = tid; i < slots; i += SF_THREADS) cand[i] = 0ull;         // padding sorts last
+  if (tid == 0) n_cand = n_found = 0;
+  __syncthreads();
   if constexpr (STAGED) {
+    // the select's first histogram on the way
     constexpr int AHEAD = 8;
     for (int i0 = tid; i0 < n; i0 += SF_THREADS * AHEAD) {
       float x[AHEAD];
@@ -187,15 +208,15 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
 #pragma unroll
       for (int a = 0; a < AHEAD; ++a) {
         const int i = i0 + a * SF_THREADS;
-        if (i < n) keys[i] = sf_key(sf_penalised(x[a], c[a], rep, presence, frequency));
+        if (i < n) {
+          const uint32_t key = sf_key(sf_penalised(x[a], c[a], rep, presence, frequency));
+          keys[i] = key;
+          atomicAdd(hists + (key >> 21), 1u);
+        }
       }
     }
+    __syncthreads();
   }
-  for (int b = tid; b < SF_BINS; b += SF_THREADS) hists[b] = 0;
-  if (rank == 0)
-    for (int i = tid; i < SF_CAP; i += SF_THREADS) cand[i] = 0ull;      // padding sorts last
-  if (tid == 0) n_cand = n_found = 0;
-  __syncthreads();
 
   // ---- the M largest (value, then smaller index): radix select on the composite key -------------
   unsigned long long thresh = 0;                 // everything passes when the row is no longer than the cap
@@ -213,7 +234,9 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
       }
       const unsigned digit_mask = (1u << bits) - 1u;
       const uint32_t want = (uint32_t)(thresh >> 32);
-      if (pass < 3) {
+      if (STAGED && pass == 0) {
+        // taken above
+      } else if (pass < 3) {
         const uint32_t mask = pass == 0 ? 0u : ~0u << (shift - 32 + bits);
         for_each([&](uint32_t key, int) {
           if (((key ^ want) & mask) == 0) atomicAdd(hist + ((key >> (shift - 32)) & digit_mask), 1u);
@@ -228,11 +251,16 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
       // all blocks' histograms, from the largest digit down, two bins a thread
       const int hi = SF_BINS - 1 - 2 * tid;
       unsigned n1 = 0, n0 = 0;                    // bins hi and hi - 1
-      for (int b = 0; b < blocks; ++b) {
-        unsigned lo_bin, hi_bin;
-        asm volatile("ld.shared::cluster.v2.u32 {%0, %1}, [%2];" : "=r"(lo_bin), "=r"(hi_bin) : "r"(sf_remote(hist + hi - 1, b)));
-        n1 += hi_bin;
-        n0 += lo_bin;
+      {
+        unsigned lo_bin[SF_BLOCKS], hi_bin[SF_BLOCKS];      // all asked for before the first is added
+#pragma unroll
+        for (int b = 0; b < SF_BLOCKS; ++b) {
+          lo_bin[b] = hi_bin[b] = 0;
+          if (b < blocks)
+            asm volatile("ld.shared::cluster.v2.u32 {%0, %1}, [%2];" : "=r"(lo_bin[b]), "=r"(hi_bin[b]) : "r"(sf_remote(hist + hi - 1, b)));
+        }
+#pragma unroll
+        for (int b = 0; b < SF_BLOCKS; ++b) { n1 += hi_bin[b]; n0 += lo_bin[b]; }
       }
       unsigned run = n1 + n0;
 #pragma unroll
@@ -242,8 +270,7 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
       }
       if (lane == 31) warp_cnt[warp] = run;
       __syncthreads();
-      unsigned before = run - (n1 + n0);
-      for (int v = 0; v < warp; ++v) before += warp_cnt[v];
+      const unsigned before = run - (n1 + n0) + __reduce_add_sync(0xffffffffu, lane < warp ? warp_cnt[lane] : 0u);
       if (before < remaining && before + n1 >= remaining) {
         sel_digit = hi;
         sel_remaining = remaining - before;      // how many of this digit's tokens still pass
@@ -276,44 +303,88 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
   if (tid == 0)
     asm volatile("atom.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(at_cand) : "r"(sf_remote(&n_cand, 0)), "r"(n_found) : "memory");
   __syncthreads();
-  for (unsigned i = tid; i < n_found; i += SF_THREADS)
-    if (at_cand + i < (unsigned)SF_CAP)
-      asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(sf_remote(cand + at_cand + i, 0)), "l"(found[i]) : "memory");
-  sf_cluster_sync();                              // all candidates are there, and nobody reads another block any more
-  if (rank != 0) return;
+  for (unsigned i = tid; i < n_found; i += SF_THREADS) {
+    const unsigned at = at_cand + i;               // equal shares for the blocks
+    if (at < (unsigned)SF_CAP)
+      asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(sf_remote(cand + (at & (slots - 1)), at / slots)), "l"(found[i]) : "memory");
+  }
+  sf_cluster_sync();                              // all candidates are there
 
-  // ---- sorted descending: bitonic over the 2048 slots, two neighbours a thread: partners up to 32 places away are in
-  // the same warp, only the farther ones go through shared memory -----------------------------------
+  // ---- sorted descending: each block its share, bitonic, two neighbours a thread: partners up to 32 places away are in
+  // the same warp, only the farther ones go through shared memory.  Then a candidate's place among all of them is the
+  // sum of its places in the blocks' shares: with four blocks 7 us, one block sorting all of them 13.6 --------------
   {
-    unsigned long long a = cand[2 * tid], b = cand[2 * tid + 1];
-    for (int k = 2; k <= SF_CAP; k <<= 1) {
+    const bool mine = 2 * tid < slots;            // whole warps: a share is 256 slots or more
+    unsigned long long a = mine ? cand[2 * tid] : 0ull, b = mine ? cand[2 * tid + 1] : 0ull;
+    for (int k = 2; k <= slots; k <<= 1) {
       const bool desc = ((2 * tid) & k) == 0;     // the same for both places: k >= 2
       for (int j = k >> 1; j >= 64; j >>= 1) {
         __syncthreads();
-        cand[2 * tid] = a;
-        cand[2 * tid + 1] = b;
+        if (mine) {
+          cand[2 * tid] = a;
+          cand[2 * tid + 1] = b;
+        }
         __syncthreads();
-        const unsigned long long pa = cand[(2 * tid) ^ j], pb = cand[(2 * tid + 1) ^ j];
-        const bool larger = desc == (((2 * tid) & j) == 0);
-        a = larger ? sf_max(a, pa) : sf_min(a, pa);
-        b = larger ? sf_max(b, pb) : sf_min(b, pb);
+        if (mine) {
+          const unsigned long long pa = cand[(2 * tid) ^ j], pb = cand[(2 * tid + 1) ^ j];
+          const bool larger = desc == (((2 * tid) & j) == 0);
+          a = larger ? sf_max(a, pa) : sf_min(a, pa);
+          b = larger ? sf_max(b, pb) : sf_min(b, pb);
+        }
       }
-      for (int j = min(k >> 1, 32); j >= 2; j >>= 1) {
-        const unsigned long long pa = __shfl_xor_sync(0xffffffffu, a, j >> 1), pb = __shfl_xor_sync(0xffffffffu, b, j >> 1);
-        const bool larger = desc == (((2 * tid) & j) == 0);
-        a = larger ? sf_max(a, pa) : sf_min(a, pa);
-        b = larger ? sf_max(b, pb) : sf_min(b, pb);
+      if (mine) {
+        for (int j = min(k >> 1, 32); j >= 2; j >>= 1) {
+          const unsigned long long pa = __shfl_xor_sync(0xffffffffu, a, j >> 1), pb = __shfl_xor_sync(0xffffffffu, b, j >> 1);
+          const bool larger = desc == (((2 * tid) & j) == 0);
+          a = larger ? sf_max(a, pa) : sf_min(a, pa);
+          b = larger ? sf_max(b, pb) : sf_min(b, pb);
+        }
+        const unsigned long long top = sf_max(a, b), low = sf_min(a, b);
+        a = desc ? top : low;
+        b = desc ? low : top;
       }
-      const unsigned long long top = sf_max(a, b), low = sf_min(a, b);
-      a = desc ? top : low;
-      b = desc ? low : top;
     }
     __syncthreads();
-    cand[2 * tid] = a;
-    cand[2 * tid + 1] = b;
+    if (mine) {
+      cand[2 * tid] = a;
+      cand[2 * tid + 1] = b;
+    }
     __syncthreads();
   }
-  auto token_of = [&](int i) { return (int)(~(unsigned)(cand[i] & 0xffffffffull)); };
+  unsigned long long* sorted = cand;
+  double* acc = reinterpret_cast<double*>(sf_smem);            // running sums of probs: the histograms' place
+  if (blocks > 1) {
+    sf_cluster_sync();                            // every share is sorted
+    // all shares side by side in `found`
+    for (int i = tid; i < SF_CAP; i += SF_THREADS) {
+      unsigned long long c;
+      asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(c) : "r"(sf_remote(cand + (i & (slots - 1)), i / slots)));
+      found[i] = c;
+    }
+    unsigned* places = reinterpret_cast<unsigned*>(cand + slots);      // (a share is half of cand at most)
+    if (tid < slots) places[tid] = 0;
+    __syncthreads();
+    // SF_THREADS / slots = blocks / 2 groups of threads, a group two of the shares
+    const int e = tid & (slots - 1), group = tid / slots, groups = blocks >> 1;
+    const unsigned long long c = cand[e];
+    const unsigned long long *s0 = found + group * slots, *s1 = found + (group + groups) * slots;
+    int p0 = 0, p1 = 0;                           // how many of a share are larger
+    for (int step = slots >> 1; step > 0; step >>= 1) {
+      if (s0[p0 + step - 1] > c) p0 += step;
+      if (s1[p1 + step - 1] > c) p1 += step;
+    }
+    if (s0[p0] > c) ++p0;
+    if (s1[p1] > c) ++p1;
+    atomicAdd(places + e, (unsigned)(p0 + p1));
+    __syncthreads();
+    sorted = reinterpret_cast<unsigned long long*>(sf_smem);   // the first block's histograms' place: nobody reads those any more
+    acc = reinterpret_cast<double*>(cand);
+    if (tid < slots && c != 0ull)                 // (padding has no place: nobody looks at it)
+      asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(sf_remote(sorted + places[e], 0)), "l"(c) : "memory");
+    sf_cluster_sync();                            // and nobody reads another block any more
+    if (rank != 0) return;
+  }
+  auto token_of = [&](int i) { return (int)(~(unsigned)(sorted[i] & 0xffffffffull)); };
   if (!(o.temperature > 0.0)) {                  // greedy: the first maximum
     if (tid == 0) chosen(token_of(0));
     return;
@@ -321,9 +392,9 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
 
   // ---- probabilities as the reference rounds them, their running sums in float64 ------------------
   const float inv_t = __fdiv_rn(1.0f, (float)o.temperature);
-  const float maxl = __fmul_rn(sf_value((uint32_t)(cand[0] >> 32)), inv_t);
+  const float maxl = __fmul_rn(sf_value((uint32_t)(sorted[0] >> 32)), inv_t);
   for (int i = tid; i < SF_CAP; i += SF_THREADS)
-    probs[i] = i < M ? expf(__fsub_rn(__fmul_rn(sf_value((uint32_t)(cand[i] >> 32)), inv_t), maxl)) : 0.0f;
+    probs[i] = i < M ? expf(__fsub_rn(__fmul_rn(sf_value((uint32_t)(sorted[i] >> 32)), inv_t), maxl)) : 0.0f;
   __syncthreads();
   {
     // inclusive scan: two neighbours per thread, then warps, then the warps' totals
@@ -416,28 +487,57 @@ __global__ void sample_count_batch_kernel(const __grid_constant__ SfCounts count
 
 using namespace exl3;
 
+// Clusters of b blocks (2, 4 or 8), a block an SM, that run at once; the GPU's, so asked for once.
+static int sf_clusters_at_once(int b, int sms) {
+  struct Table { int n[SF_BLOCKS + 1]; };
+  static const Table table = [sms] {
+    Table t = {};
+    auto kernel = sample_filtered_kernel<true, true>;
+    const bool fine = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SF_SMEM_MOST) == cudaSuccess;
+    for (int c = 2; c <= SF_BLOCKS; c *= 2) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3(c * sms);
+      cfg.blockDim = dim3(SF_THREADS);
+      cfg.dynamicSmemBytes = SF_SMEM_MOST;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = c;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      if (!fine || cudaOccupancyMaxActiveClusters(&t.n[c], kernel, &cfg) != cudaSuccess || t.n[c] < 1) t.n[c] = std::max(1, sms / c);
+    }
+    cudaGetLastError();
+    return t;
+  }();
+  return table.n[b];
+}
+
 // rows: float64 [R, 5] on the device: temperature (<= 0: greedy), top_k (0: off, at most 2048), top_p, min_p and
 // the row's uniform number in [0, 1).  out: int32 [R].  counts (may be null): as in exl3_sample_penalties, with params;
 // the penalties are applied as the logits are read, and the chosen tokens are counted when all rows have been drawn.
 // batch: the rows themselves, then rows, counts and params are null.
 static int sf_launch(const float* logits, const double* rows, int* const* counts, const float* params, int* out, int R, int V,
                      const SfBatch& batch, bool penalties, int* host_out, bool count_now, cudaStream_t stream) {
-  // Blocks a row.  An SM holds one block, and the SMs come in eight groups that a cluster must fit into; a wave of rows takes
-  // some 35 us and, for a token of a block's part, 0.18 ns, or 0.33 (0.75 with penalties) where the part is too long for
-  // shared memory and read in every pass.  With 8 / 4 / 2 / 1 blocks: 32 rows of 122,753 86 / 41 / 55 / 76 us, 148 rows 280 /
-  // 168 / 108 / 77, 64 rows of 32,000 116 / 64 / 35 / 39, 100 rows of 320,001 273 / 194 / 186 / 168.
+  // Blocks a row.  An SM holds one block, and a cluster must fit into a group of SMs, so the driver says how many clusters run
+  // at once; a wave of rows takes 23 to 28 us and, for a token of a block's part, 0.32 ns, or where the part is too long for
+  // shared memory and read in every pass 6 us and 0.33 ns (0.75 with penalties).  With 8 / 4 / 2 / 1 blocks: one row of 32,000
+  // 27.8 / 25.7 / 29.6 / 38 us, 64 rows 131 / 52 / 30 / 38; 8 rows of 122,753 31.8 / 33.1 / 49 / 76, 16 rows 60 / 33 / 49 / 76,
+  // 148 rows 299 / 157 / 98 / 77; 100 rows of 320,001 289 / 200 / 168 / 163.
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   constexpr size_t MOST = SF_SMEM_MOST - SF_HEAD_BYTES;
   int blocks = 8;
   double best = 0.0;
-  for (int b = 8; b >= 1; b /= 2) {
+  for (int b = 8, i = 0; b >= 1; b /= 2, ++i) {
     const int each = ceil_div(V, b);
-    const int at_once = b == 1 ? sms : 8 * std::max(1, sms / 8 / b);
+    const int at_once = b == 1 ? sms : sf_clusters_at_once(b, sms);
     const double waves = (double)((R + at_once - 1) / at_once);
-    const double a_token = (size_t)each * 4 <= MOST ? SF_STAGED_US : penalties ? SF_AGAIN_PENALTIES_US : SF_AGAIN_US;
-    const double cost = waves * (SF_FIXED_US + a_token * each);
+    const bool kept = (size_t)each * 4 <= MOST;
+    const double a_token = kept ? SF_STAGED_US : penalties ? SF_AGAIN_PENALTIES_US : SF_AGAIN_US;
+    const double cost = waves * (SF_FIXED_US[i] + (kept ? 0.0 : SF_AGAIN_FIXED_US) + a_token * each);
     if (b == 8 || cost < best) {
       best = cost;
       blocks = b;

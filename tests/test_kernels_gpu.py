@@ -1451,6 +1451,26 @@ def test_sample_filtered_ranks_equal_logits_of_long_rows(penalties):
     assert got.tolist() == [sample_token(logits[r], opt, contexts[r], _FixedU(us[r])) for r in range(R)]
 
 
+@pytest.mark.parametrize("V,R", [(255, 3), (2047, 1), (2048, 40), (2049, 70), (4099, 1), (40001, 2), (40001, 32), (40001, 70), (40001, 149)])
+def test_sample_filtered_ranks_what_one_block_has_found(V, R):
+    """Rows that rise or fall from end to end: all candidates come from one part of the row and are dealt out to all of the
+    row's blocks (8, 4, 2 or 1 of them by the number of rows).  Logits 0, 1, 2, ... at temperature 700: neighbours in the
+    ranking differ by a seven-hundredth, so a token in a wrong place moves the draw."""
+    from exl3_server_b200.sampling import SampleOptions
+    from exl3_server_b200.sampling.host import sample_token
+    opt = SampleOptions(temperature=700.0)
+    up = np.arange(V, dtype=np.float32)
+    logits = np.stack([up if r % 2 == 0 else up[::-1] for r in range(R)])
+    us = [(r + 0.5) / R for r in range(R)]
+    rows = torch.tensor([[700.0, 0, 1.0, 0.0, u] for u in us], dtype=torch.float64)
+    got = K().sample_filtered(torch.from_numpy(logits).to(DEV), rows.to(DEV)).tolist()
+    want = [sample_token(logits[r], opt, [], _FixedU(us[r])) for r in range(R)]
+    # float32 exponentials may differ in their last bit between host and device: a sum of 2,048 of them to 2,048 * 2^-24 of
+    # itself, a draw then by one place where it falls that near to a border (one in 2,048 * 2 * 2,048 * 2^-24 = 0.5 rows)
+    off = [abs(g - w) for g, w in zip(got, want)]
+    assert max(off) <= 1 and sum(off) <= 1 + R // 2, off
+
+
 @pytest.mark.parametrize("R", [1, 5, 64, 65])             # with the launch up to 64 rows, by a buffer beyond
 @pytest.mark.parametrize("V", [300, 40001, 330001])
 def test_sampling_of_rows_with_options_of_their_own(R, V):
