@@ -13,7 +13,8 @@
 //
 // Block of 6 warps: warp 0 issues the TMA copies (weights first, before griddepcontrol.wait: they do not depend
 // on the kernel before this one; then the activations), warp 1 issues tcgen05.mma and owns the tensor memory,
-// warps 2-5 are the epilogue (thread = feature).  Epilogues as in the weight-streaming GEMV (gemv_bf16.cuh):
+// warps 2-5 bring the accumulator into shared memory (thread = feature), and all six add up the cluster's partial tiles and run
+// the epilogue.  Epilogues as in the weight-streaming GEMV (gemv_bf16.cuh):
 // 0 plain, 1 silu(gate) * up over rows interleaved in eights, 2 into the residual with the pieces of the next
 // norm (h += y * rho, x_raw = h * norm_w, sums of squares per 16 features), and optionally the consuming side of
 // such a norm (results times rsqrt(sum of the producer's sums / width + eps) per batch row).
