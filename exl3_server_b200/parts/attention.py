@@ -184,10 +184,7 @@ class Attention:
             # prompts, heads of 64 or 128: streaming softmax with both products on tcgen05 tensor cores,
             # TMA loads straight from the paged cache, a block per 128 queries
             tile_seq, tile_q0, n_tiles = batch.tiles[128]
-            key = ("attn_prefill_variant", s.heads, s.head_dim, s.window)
-            variant = batch.memo.get(key)
-            if variant is None:
-                variant = batch.memo[key] = self._prefill_form(batch.tile_keys.get(128), kv.page_size, qkv.device)
+            variant = self._step_form(batch, kv.page_size, qkv.device)
             K.attn_prefill_tc(qkv, qkv.stride(0), out, kv.k, kv.v, kv.block_table, batch.row_start, batch.row_pos0,
                               tile_seq, tile_q0, n_tiles, s.heads, s.kv_heads, s.head_dim, kv.page_size, s.window,
                               self.scale, variant=variant)
@@ -285,6 +282,16 @@ class Attention:
         pages, sms = self._tile_pages(tile_keys, page), K.sm_count(device)
         pairs = 1.19 * _makespan([p + 3.5 for p in pages], sms, s.heads // 2)
         return 4 if pairs < 0.9 * _makespan([p + 3 for p in pages], sms, s.heads) else one
+
+    def _step_form(self, batch, page: int, device: torch.device) -> int:
+        """``_prefill_form`` for a step's tiles, worked out once for all layers that it is the same for: the key holds
+        everything of the layer that the choice is made from."""
+        s = self.spec
+        key = ("attn_prefill_form", s.heads, s.kv_heads, s.head_dim, s.window, page)
+        form = batch.memo.get(key)
+        if form is None:
+            form = batch.memo[key] = self._prefill_form(batch.tile_keys.get(128), page, device)
+        return form
 
     def _decode_split(self, T: int, max_kv_len: int, page: int, device: torch.device):
         """``(keys per chunk, head_split, in_block)`` (``in_block``: 0, 1 or 2) for the tensor-core decode kernel:

@@ -246,10 +246,7 @@ class NormedAttention:
         H, G, d, T = self.H, self.G, self.d_pad, q.shape[0]
         if batch.max_new > 1 and batch.tiles and K.attn_prefill_tc_supported(torch.bfloat16, d, kv.page_size):
             tile_seq, tile_q0, n_tiles = batch.tiles[128]
-            key = ("attn_prefill_variant", H, d, self.chunk, self.window, self.keep_first)
-            variant = batch.memo.get(key)
-            if variant is None:
-                variant = batch.memo[key] = self._cuts._prefill_form(batch.tile_keys.get(128), kv.page_size, q.device)
+            variant = self._cuts._step_form(batch, kv.page_size, q.device)
             K.attn_prefill_tc(q, q.stride(0), out, kv.k, kv.v, kv.block_table, batch.row_start, batch.row_pos0, tile_seq,
                               tile_q0, n_tiles, H, G, d, kv.page_size, self.window, self.scale, variant=variant,
                               chunk=self.chunk, sink=self.sink, keep_first=self.keep_first, softcap=self.softcap,

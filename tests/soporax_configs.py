@@ -90,6 +90,9 @@ CONFIGS = {
     "only_rotated_tiles": cfg(128, 64, 1e-5, 1.5, [L(rotated(4, 2, 64, 64, 0.2, 32, 10000.0, bands(8.0, 1.0, 4.0, 64)))]),
     "only_latent": cfg(128, 64, 1e-5, 1.5, [L(latent(4, 32, 16, 24, 40, 48, 0.2, 10000.0, ramp(4.0, 64, 8.0, 1.0)))]),
     "only_moe": cfg(128, 64, 1e-5, 1.2, [L(window(1, 1, 8, 8, 0.3, 1), moe(24, 14, 3))]),
+    # layers that differ in their key/value heads alone, groups of two and of one: long prompts take other kernels for them
+    "kv_heads": cfg(96, 128, 1e-5, 1.5, [L(rotated(16, 8, 128, 128, 0.1, 64)), L(rotated(16, 16, 128, 128, 0.1, 64)),
+                                         L(rotated(16, 8, 128, 128, 0.1, 64))]),
     "only_dense": cfg(128, 64, 1e-5, 1.2, [L(window(1, 1, 8, 8, 0.3, 1), dense(48, 0.4))]),
 }
 

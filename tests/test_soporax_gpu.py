@@ -106,6 +106,23 @@ def test_configurations_drawn_from_a_seed(folders, name, dtype):
     eng.check_kernels()
 
 
+@pytest.mark.parametrize("flipped", [False, True])
+def test_long_prompt_over_layers_that_differ_in_key_value_heads(folders, flipped, monkeypatch):
+    """A prompt long enough for the kernel with two heads side by side, which only the layers with even groups can take, whichever
+    kind of layer comes first."""
+    name = "kv_heads_flipped" if flipped else "kv_heads"
+    folder = folders["kv_heads"]
+    if flipped:
+        cfg = CONFIGS["kv_heads"]
+        monkeypatch.setitem(CONFIGS, name, type(cfg)(**{**cfg.__dict__, "layers": cfg.layers[1:]}))
+        folder = make_soporax(name, folder + "_flipped")
+    requests = requests_for(name, [3000], seed=5)
+    want = {rid: plain(folder).logits(t).numpy() for rid, t in requests.items()}
+    eng = engine_for(folder, "bfloat16", max_tokens=4096)
+    check(run_trace(eng, whole_trace(requests)), want, "bfloat16", "long prompt")
+    eng.check_kernels()
+
+
 @pytest.mark.parametrize("name", ["mixed", "wide"])
 def test_float32_cuttings_agree_closely(folders, name):
     requests = requests_for(name, LENGTHS[name], seed=5)

@@ -122,3 +122,42 @@ def test_prompt_kernel_form_with_pairs_of_heads():
     for sizes in ((36, 36, 64), (16, 16, 128), (24, 8, 128)):            # other heads, odd groups: never
         for lens in ([181], [6145], [300] * 30):
             assert mixer(*sizes)._prefill_form(tile_keys(lens), 64, None) in (1, 2, 3)
+
+
+def prompt_calls(parts, step):
+    """What ``step`` hands the prompt kernel over one batch, part by part: (heads, kv_heads, variant)."""
+    keys = tile_keys([3000])
+    batch = SimpleNamespace(max_new=3000, tiles={128: (None, None, len(keys))}, tile_keys={128: keys}, memo={}, row_start=None, row_pos0=None)
+    kv = SimpleNamespace(k=None, v=None, block_table=None, page_size=64)
+    calls = []
+
+    def kernel(q, ld, out, k, v, table, row_start, row_pos0, tile_seq, tile_q0, n, heads, kv_heads, hd, page, window, scale, variant=0, **_):
+        calls.append((heads, kv_heads, variant))
+
+    with mock.patch.object(K, "attn_prefill_tc", kernel), mock.patch.object(K, "attn_prefill_tc_supported", lambda *a: True):
+        for p in parts:
+            step(p, batch, kv)
+    return calls
+
+
+@pytest.mark.parametrize("order", [(8, 16), (16, 8)])
+@pytest.mark.parametrize("normed", [False, True])
+def test_layers_with_other_kv_heads_choose_their_own_prompt_kernel(order, normed):
+    """Layers of 16 heads of 128 on 8 and on 16: pairs of heads (form 4) are for the even groups of the first alone."""
+    from exl3_server_b200.parts.normed_attention import NormedAttention
+    q = torch.zeros(1, 1)
+
+    def part(kv_heads):
+        plain = mixer(16, kv_heads, 128)
+        plain.scale = 0.1
+        if not normed:
+            return plain
+        a = NormedAttention.__new__(NormedAttention)
+        a.__dict__.update(H=16, G=kv_heads, d_pad=128, dv_pad=128, ctx=SimpleNamespace(dtype=torch.bfloat16), window=0, chunk=0, scale=0.1,
+                          sink=False, keep_first=0, softcap=0.0, sink_vals=None, dist=None, _cuts=plain)
+        return a
+
+    step = (lambda p, batch, kv: p._tensor_cores(q, q, batch, kv)) if normed else (lambda p, batch, kv: p.attend(q, q, batch, kv))
+    calls = prompt_calls([part(g) for g in order + order], step)
+    assert [c[:2] for c in calls] == [(16, g) for g in order + order]
+    assert all((v == 4) == (g == 8) and v in (1, 3, 4) for _, g, v in calls), calls
