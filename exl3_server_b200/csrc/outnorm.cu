@@ -89,53 +89,80 @@ __device__ inline void on_store8(__nv_bfloat16* p, const float (&v)[8]) { store_
 constexpr int NA_VECS = 4;                       // pieces of 8 values per thread: rows up to 8192
 // Pieces of a thread for rows of H values: 1, 2 or 4.
 static int na_vecs(int H) { return H <= NA_THREADS * 8 ? 1 : H <= NA_THREADS * 16 ? 2 : 4; }
+static int na_sms() {
+  static const int n = [] {
+    int dev = 0, v = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v > 0 ? v : 148;
+  }();
+  return n;
+}
+
+// AHEAD, in this kernel and the two below: everything is asked for at once, the weights before the wait for the kernel before,
+// the residual with y; behind the sum of squares it would be a second trip to memory.  That takes registers for all of it
+// (118 to 160 a thread with four pieces, against 56 to 86), so fewer blocks share an SM: it is right while all blocks run at once
+// anyway, and for rows of one piece, whose registers are few.  With everything at once / as it is needed, bfloat16 y: norm_add
+// 8,000 x 8,192 162 / 120 us, norm_add_norm 8 x 4,096 2.9 / 3.6, 300 x 2,304 4.6 / 4.1, 3,163 x 2,304 26.5 / 19.4, 64 x 8,192
+// 4.6 / 5.3, 300 x 8,192 12.9 / 9.9, 8,000 x 8,192 242 / 130; normed_sum2 300 x 2,304 3.6 / 3.9, 3,163 x 4,096 24 / 21, 64 x 5,120
+// 3.6 / 3.9, 300 x 5,120 8.2 / 5.7, 8,000 x 8,192 252 / 109.  Rows of one piece (2,048 with both norms): 8 of them 2.7 -> 2.1 us,
+// 3,163 19.5 -> 16.4.  The sums are the same either way.
 
 // The same for rows of up to NA_THREADS * 8 * VECS values, a multiple of 8: a thread keeps its pieces of y in
-// registers and every access is 16 or 32 bytes wide.  TX void: no copy of the residual is written.  In this kernel and the
-// two below everything is asked for at once, the weights before the wait for the kernel before, the residual with y: behind
-// the sum of squares it would be a second trip to memory (8 rows of 2,048 with both norms 2.7 -> 2.1 us, 3,163 rows
-// 16.1 -> 14.9).
-template <typename TY, typename TW, typename TX, int VECS>
+// registers and every access is 16 or 32 bytes wide.  TX void: no copy of the residual is written.
+template <typename TY, typename TW, typename TX, int VECS, bool AHEAD>
 __global__ void __launch_bounds__(NA_THREADS)
 norm_add_vec_kernel(float* h, const TY* y, const TW* __restrict__ w, float eps, TX* x, int H) {
   __shared__ float red[32];
-  float wv[VECS][8];
+  constexpr int KEPT = AHEAD ? VECS : 1;
+  float keep[VECS][8], hv[KEPT][8], wv[KEPT][8];
+  if (AHEAD) {
 #pragma unroll
-  for (int p = 0; p < VECS; ++p) {
-    const int c = (p * NA_THREADS + threadIdx.x) * 8;
-    if (c < H) on_load8(w + c, wv[p], false);
+    for (int p = 0; p < KEPT; ++p) {
+      const int c = (p * NA_THREADS + threadIdx.x) * 8;
+      if (c < H) on_load8(w + c, wv[p], false);
+    }
   }
   pdl_wait();
   pdl_trigger();
   const int64_t base = (int64_t)blockIdx.x * H;
-  float keep[VECS][8], hv[VECS][8];
   float ss = 0.0f;
 #pragma unroll
   for (int p = 0; p < VECS; ++p) {
     const int c = (p * NA_THREADS + threadIdx.x) * 8;
     if (c < H) {
       on_load8(y + base + c, keep[p], true);
-      on_load8(h + base + c, hv[p], true);
+      if (AHEAD) on_load8(h + base + c, hv[AHEAD ? p : 0], true);
+      if (!AHEAD) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) ss += keep[p][e] * keep[p][e];
+      }
     }
   }
+  if (AHEAD) {
 #pragma unroll
-  for (int p = 0; p < VECS; ++p) {
-    const int c = (p * NA_THREADS + threadIdx.x) * 8;
-    if (c < H) {
+    for (int p = 0; p < VECS; ++p) {
+      const int c = (p * NA_THREADS + threadIdx.x) * 8;
+      if (c < H) {
 #pragma unroll
-      for (int e = 0; e < 8; ++e) ss += keep[p][e] * keep[p][e];
+        for (int e = 0; e < 8; ++e) ss += keep[p][e] * keep[p][e];
+      }
     }
   }
   ss = block_sum(ss, red);
   const float inv = 1.0f / sqrtf(ss / (float)H + eps);
 #pragma unroll
   for (int p = 0; p < VECS; ++p) {
-    const int c = (p * NA_THREADS + threadIdx.x) * 8;
+    const int c = (p * NA_THREADS + threadIdx.x) * 8, k = AHEAD ? p : 0;
     if (c < H) {
+      if (!AHEAD) {
+        on_load8(h + base + c, hv[k], true);
+        on_load8(w + c, wv[k], false);
+      }
 #pragma unroll
-      for (int e = 0; e < 8; ++e) hv[p][e] += keep[p][e] * inv * wv[p][e];
-      on_store8(h + base + c, hv[p]);
-      if (x) on_store8(x + base + c, hv[p]);
+      for (int e = 0; e < 8; ++e) hv[k][e] += keep[p][e] * inv * wv[k][e];
+      on_store8(h + base + c, hv[k]);
+      if (x) on_store8(x + base + c, hv[k]);
     }
   }
 }
@@ -186,10 +213,16 @@ __global__ void xielu_vec_kernel(const TI* z, const void* __restrict__ pq, int p
 
 template <typename TY, typename TW, typename TX>
 static void norm_add_vec_to(float* h, const void* y, const void* w, float eps, void* x, int T, int H, cudaStream_t stream) {
-  auto kernel = na_vecs(H) == 1 ? norm_add_vec_kernel<TY, TW, TX, 1> : na_vecs(H) == 2 ? norm_add_vec_kernel<TY, TW, TX, 2>
-                                                                                        : norm_add_vec_kernel<TY, TW, TX, 4>;
-  launch_pdl(kernel, dim3(T), dim3(NA_THREADS), 0, stream, h, static_cast<const TY*>(y), static_cast<const TW*>(w), eps,
-             static_cast<TX*>(x), H);
+  auto launch = [&](auto kernel) {
+    launch_pdl(kernel, dim3(T), dim3(NA_THREADS), 0, stream, h, static_cast<const TY*>(y), static_cast<const TW*>(w), eps,
+               static_cast<TX*>(x), H);
+  };
+  // with two pieces ahead is never slower (8,000 x 4,096 65 against 77 us); with four a bfloat16 y gains nothing from it
+  const int vecs = na_vecs(H);
+  if (vecs == 1) launch(norm_add_vec_kernel<TY, TW, TX, 1, true>);
+  else if (vecs == 2) launch(norm_add_vec_kernel<TY, TW, TX, 2, true>);
+  else if (sizeof(TY) == 4 && T <= 3 * na_sms()) launch(norm_add_vec_kernel<TY, TW, TX, 4, true>);
+  else launch(norm_add_vec_kernel<TY, TW, TX, 4, false>);
 }
 template <typename TY, typename TW>
 static void norm_add_vec(float* h, const void* y, const void* w, float eps, void* x, int x_dtype, int T, int H,
@@ -251,31 +284,33 @@ norm_add_norm_kernel(float* h, const void* y, int y_dtype, const void* __restric
 
 // The same for rows of up to NA_THREADS * 8 * VECS values, a multiple of 8, with float32 weights: a thread keeps its
 // pieces of the row in registers through both norms and every access is 16 or 32 bytes wide.
-template <typename TY, typename TX, int VECS>
+template <typename TY, typename TX, int VECS, bool AHEAD>
 __global__ void __launch_bounds__(NA_THREADS)
 norm_add_norm_vec_kernel(float* h, const TY* y, const float* __restrict__ w, float eps, const float* __restrict__ w2,
                          float eps2, TX* x, int H) {
   __shared__ float red[32];
-  float wv[VECS][8], wv2[VECS][8];
+  constexpr int KEPT = AHEAD ? VECS : 1;
+  float keep[VECS][8], hv[KEPT][8], wv[KEPT][8], wv2[KEPT][8];
+  if (AHEAD) {
 #pragma unroll
-  for (int p = 0; p < VECS; ++p) {
-    const int c = (p * NA_THREADS + threadIdx.x) * 8;
-    if (c < H) {
-      on_load8(w + c, wv[p], false);
-      on_load8(w2 + c, wv2[p], false);
+    for (int p = 0; p < KEPT; ++p) {
+      const int c = (p * NA_THREADS + threadIdx.x) * 8;
+      if (c < H) {
+        on_load8(w + c, wv[p], false);
+        on_load8(w2 + c, wv2[p], false);
+      }
     }
   }
   pdl_wait();
   pdl_trigger();
   const int64_t base = (int64_t)blockIdx.x * H;
-  float keep[VECS][8], hv[VECS][8];
   float ss = 0.0f;
 #pragma unroll
   for (int p = 0; p < VECS; ++p) {
     const int c = (p * NA_THREADS + threadIdx.x) * 8;
     if (c < H) {
       on_load8(y + base + c, keep[p], true);
-      on_load8(h + base + c, hv[p], true);
+      if (AHEAD) on_load8(h + base + c, hv[AHEAD ? p : 0], true);
     }
   }
 #pragma unroll
@@ -291,55 +326,69 @@ norm_add_norm_vec_kernel(float* h, const TY* y, const float* __restrict__ w, flo
   float ss2 = 0.0f;
 #pragma unroll
   for (int p = 0; p < VECS; ++p) {
-    const int c = (p * NA_THREADS + threadIdx.x) * 8;
+    const int c = (p * NA_THREADS + threadIdx.x) * 8, k = AHEAD ? p : 0;
     if (c < H) {
+      if (!AHEAD) {
+        on_load8(h + base + c, hv[k], true);
+        on_load8(w + c, wv[k], false);
+      }
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
-        hv[p][e] += keep[p][e] * inv * wv[p][e];
-        ss2 += hv[p][e] * hv[p][e];
+        keep[p][e] = hv[k][e] + keep[p][e] * inv * wv[k][e];
+        ss2 += keep[p][e] * keep[p][e];
       }
-      on_store8(h + base + c, hv[p]);
+      on_store8(h + base + c, keep[p]);
     }
   }
   ss2 = block_sum(ss2, red);
   const float inv2 = 1.0f / sqrtf(ss2 / (float)H + eps2);
 #pragma unroll
   for (int p = 0; p < VECS; ++p) {
-    const int c = (p * NA_THREADS + threadIdx.x) * 8;
+    const int c = (p * NA_THREADS + threadIdx.x) * 8, k = AHEAD ? p : 0;
     if (c < H) {
+      if (!AHEAD) on_load8(w2 + c, wv2[k], false);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) hv[p][e] *= inv2 * wv2[p][e];
-      on_store8(x + base + c, hv[p]);
+      for (int e = 0; e < 8; ++e) keep[p][e] *= inv2 * wv2[k][e];
+      on_store8(x + base + c, keep[p]);
     }
   }
 }
 template <typename TY, typename TX>
 static void norm_add_norm_vec(float* h, const void* y, const float* w, float eps, const float* w2, float eps2, void* x, int T,
                               int H, cudaStream_t stream) {
-  auto kernel = na_vecs(H) == 1 ? norm_add_norm_vec_kernel<TY, TX, 1> : na_vecs(H) == 2 ? norm_add_norm_vec_kernel<TY, TX, 2>
-                                                                                        : norm_add_norm_vec_kernel<TY, TX, 4>;
-  launch_pdl(kernel, dim3(T), dim3(NA_THREADS), 0, stream, h, static_cast<const TY*>(y), w, eps, w2, eps2, static_cast<TX*>(x), H);
+  auto launch = [&](auto kernel) {
+    launch_pdl(kernel, dim3(T), dim3(NA_THREADS), 0, stream, h, static_cast<const TY*>(y), w, eps, w2, eps2, static_cast<TX*>(x), H);
+  };
+  const int vecs = na_vecs(H);
+  const bool ahead = T <= na_sms();
+  if (vecs == 1) launch(norm_add_norm_vec_kernel<TY, TX, 1, true>);
+  else if (vecs == 2 && ahead) launch(norm_add_norm_vec_kernel<TY, TX, 2, true>);
+  else if (vecs == 2) launch(norm_add_norm_vec_kernel<TY, TX, 2, false>);
+  else if (ahead) launch(norm_add_norm_vec_kernel<TY, TX, 4, true>);
+  else launch(norm_add_norm_vec_kernel<TY, TX, 4, false>);
 }
 
 // The two-output norm and sum with 16-byte accesses (rows as above, float32 weights).
-template <typename TA, int VECS>
+template <typename TA, int VECS, bool AHEAD>
 __global__ void __launch_bounds__(NA_THREADS)
 normed_sum2_vec_kernel(const TA* a, const TA* b, const float* __restrict__ wa, const float* __restrict__ wb, float eps,
                        float coef, float* out, int H) {
   __shared__ float red[32];
-  float wx[VECS][8], wy[VECS][8];
+  constexpr int KEPT = AHEAD ? VECS : 1;
+  float ka[VECS][8], kb[VECS][8], wx[KEPT][8], wy[KEPT][8];
+  if (AHEAD) {
 #pragma unroll
-  for (int p = 0; p < VECS; ++p) {
-    const int c = (p * NA_THREADS + threadIdx.x) * 8;
-    if (c < H) {
-      on_load8(wa + c, wx[p], false);
-      on_load8(wb + c, wy[p], false);
+    for (int p = 0; p < KEPT; ++p) {
+      const int c = (p * NA_THREADS + threadIdx.x) * 8;
+      if (c < H) {
+        on_load8(wa + c, wx[p], false);
+        on_load8(wb + c, wy[p], false);
+      }
     }
   }
   pdl_wait();
   pdl_trigger();
   const int64_t base = (int64_t)blockIdx.x * H;
-  float ka[VECS][8], kb[VECS][8];
   float sa = 0.0f, sb = 0.0f;
 #pragma unroll
   for (int p = 0; p < VECS; ++p) {
@@ -362,11 +411,15 @@ normed_sum2_vec_kernel(const TA* a, const TA* b, const float* __restrict__ wa, c
   const float ia = coef / sqrtf(sa / (float)H + eps), ib = coef / sqrtf(sb / (float)H + eps);
 #pragma unroll
   for (int p = 0; p < VECS; ++p) {
-    const int c = (p * NA_THREADS + threadIdx.x) * 8;
+    const int c = (p * NA_THREADS + threadIdx.x) * 8, k = AHEAD ? p : 0;
     if (c < H) {
+      if (!AHEAD) {
+        on_load8(wa + c, wx[k], false);
+        on_load8(wb + c, wy[k], false);
+      }
       float o[8];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) o[e] = ka[p][e] * ia * wx[p][e] + kb[p][e] * ib * wy[p][e];
+      for (int e = 0; e < 8; ++e) o[e] = ka[p][e] * ia * wx[k][e] + kb[p][e] * ib * wy[k][e];
       on_store8(out + base + c, o);
     }
   }
@@ -374,10 +427,16 @@ normed_sum2_vec_kernel(const TA* a, const TA* b, const float* __restrict__ wa, c
 template <typename TA>
 static void normed_sum2_vec(const void* a, const void* b, const void* wa, const void* wb, float eps, float coef, float* out, int T,
                             int H, cudaStream_t stream) {
-  auto kernel = na_vecs(H) == 1 ? normed_sum2_vec_kernel<TA, 1> : na_vecs(H) == 2 ? normed_sum2_vec_kernel<TA, 2>
-                                                                                  : normed_sum2_vec_kernel<TA, 4>;
-  launch_pdl(kernel, dim3(T), dim3(NA_THREADS), 0, stream, static_cast<const TA*>(a), static_cast<const TA*>(b),
-             static_cast<const float*>(wa), static_cast<const float*>(wb), eps, coef, out, H);
+  auto launch = [&](auto kernel) {
+    launch_pdl(kernel, dim3(T), dim3(NA_THREADS), 0, stream, static_cast<const TA*>(a), static_cast<const TA*>(b),
+               static_cast<const float*>(wa), static_cast<const float*>(wb), eps, coef, out, H);
+  };
+  const int vecs = na_vecs(H);
+  if (vecs == 1) launch(normed_sum2_vec_kernel<TA, 1, true>);
+  else if (vecs == 2 && T <= 4 * na_sms()) launch(normed_sum2_vec_kernel<TA, 2, true>);
+  else if (vecs == 2) launch(normed_sum2_vec_kernel<TA, 2, false>);
+  else if (T <= na_sms()) launch(normed_sum2_vec_kernel<TA, 4, true>);
+  else launch(normed_sum2_vec_kernel<TA, 4, false>);
 }
 
 // Two sublayer outputs side by side, each normed over the row with its own weight, then averaged:

@@ -332,6 +332,36 @@ def test_norm_add_norm(y_dt, H):
         close(x, want_h / torch.sqrt((want_h * want_h).mean(-1, keepdim=True) + 2e-6) * w2.double(), x_dt, "next norm")
 
 
+@pytest.mark.parametrize("y_dt", TYPES)
+@pytest.mark.parametrize("H", [8, 2048, 2056, 4096, 4104, 8192])         # one, two and four pieces a thread, the last one short or full
+def test_norms_of_rows_in_pieces(y_dt, H):
+    """Few rows ask for everything at once, many as it is needed: float64's numbers, and a row's bits whatever rows stand beside it."""
+    g = torch.Generator().manual_seed(H)
+    T, few = 700, 3
+    h = torch.randn(T, H, generator=g).to(DEV)
+    y, z = ((torch.randn(T, H, generator=g) * s).to(y_dt).to(DEV) for s in (4, 1))
+    w, w2 = ((1 + 0.2 * torch.randn(H, generator=g)).to(DEV) for _ in range(2))
+    n = lambda v, weight, eps: v / torch.sqrt((v * v).mean(-1, keepdim=True) + eps) * weight.double()
+    want = h.double() + n(y.double(), w, 1e-5)
+
+    def each(rows):
+        a, b, c = (h[:rows].clone() for _ in range(3))
+        xa = K().norm_add(a, y[:rows], w, 1e-5, torch.bfloat16)
+        assert K().norm_add(b, y[:rows], w, 1e-5, None) is None and torch.equal(a, b)
+        xc = [K().norm_add_norm(c if dt == y_dt else h[:rows].clone(), y[:rows], w, 1e-5, w2, 2e-6, dt) for dt in TYPES]
+        return [a, xa, c, *xc, K().normed_sum2(y[:rows], z[:rows], w, w2, 1e-6, 0.5)]
+
+    outs = each(T)
+    close(outs[0], want, torch.float32, "residual")
+    assert torch.equal(outs[1], outs[0].bfloat16())
+    close(outs[2], want, torch.float32, "residual under both norms")
+    for dt, x in zip(TYPES, outs[3:5]):
+        close(x, n(want, w2, 2e-6), dt, "next norm")
+    close(outs[5], 0.5 * (n(y.double(), w, 1e-6) + n(z.double(), w2, 1e-6)), torch.float32, "two norms")
+    for rows in (few, 148, 149, 444, 445, 592, 593):
+        assert all(torch.equal(a, b[:rows]) for a, b in zip(each(rows), outs)), rows
+
+
 def test_gelu_in_the_projection():
     g = torch.Generator().manual_seed(9)
     M, N, Kd = 5, 72, 128
