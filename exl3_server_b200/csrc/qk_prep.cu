@@ -242,8 +242,18 @@ template <> struct QpRaw<float> {
   }
 };
 
-template <typename TX, typename TS, int JOBS>
-__global__ void __launch_bounds__(QP_WARPS * 32, JOBS > 1 && sizeof(TX) == 2 ? 4 : 1) qk_prep_vec_kernel(QkPrepArgs a, int lph_log2) {
+// The forms (qk_prep_vec chooses):
+//   QP_FEW    a token's heads are dealt to blocks, a thread asks for its piece before anything else: all blocks run at once
+//   QP_HEADS  the same with nothing kept that can be had again, in 32 registers: as many blocks on an SM as it can hold
+//   QP_TOKEN  a block takes all heads of its token, four at a time a thread, whose pieces are asked for together; what the heads
+//             have in common is worked out once
+constexpr int QP_FEW = 0, QP_HEADS = 1, QP_TOKEN = 2;
+constexpr int QP_HEADS_BLOCKS = 8, QP_TOKEN_BLOCKS = 4;      // on an SM
+
+template <typename TX, typename TS, int FORM>
+__global__ void __launch_bounds__(QP_WARPS * 32, FORM == QP_HEADS ? QP_HEADS_BLOCKS : FORM == QP_TOKEN ? QP_TOKEN_BLOCKS : 1)
+qk_prep_vec_kernel(QkPrepArgs a, int lph_log2) {
+  constexpr int JOBS = FORM == QP_TOKEN ? 4 : 1;
   __shared__ float s_sn[QP_TABLE], s_cs[QP_TABLE];
   const int t = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -283,7 +293,7 @@ __global__ void __launch_bounds__(QP_WARPS * 32, JOBS > 1 && sizeof(TX) == 2 ? 4
   if (JOBS == 1) {
     pdl_wait();
     pdl_trigger();
-    ask((int)blockIdx.y);
+    if (FORM == QP_FEW) ask((int)blockIdx.y);
   }
   qp_gates(a, t);
   __syncthreads();
@@ -294,10 +304,11 @@ __global__ void __launch_bounds__(QP_WARPS * 32, JOBS > 1 && sizeof(TX) == 2 ? 4
   __nv_bfloat16* qp = static_cast<__nv_bfloat16*>(a.q_out) + (int64_t)t * a.nh * a.hd_pad + e0;
   const float q_mul = qp_temperature(a, pos);
   float sn[4], cs[4];
-  if (e0 < a.rot) {                                    // rot is a multiple of 8 here: all of the lane's pairs or none
+  auto angles = [&]() {
 #pragma unroll
     for (int p = 0; p < 4; ++p) { sn[p] = s_sn[(e0 >> 1) + p]; cs[p] = s_cs[(e0 >> 1) + p]; }
-  }
+  };
+  if (FORM != QP_HEADS && e0 < a.rot) angles();                // rot is a multiple of 8 here: all of the lane's pairs or none
   // norm 3: the factors of the token's queries and keys (see the kernel above)
   float inv_q = 1.0f, inv_k = 1.0f;
   if (a.norm == 3) {
@@ -324,7 +335,12 @@ __global__ void __launch_bounds__(QP_WARPS * 32, JOBS > 1 && sizeof(TX) == 2 ? 4
 #pragma unroll
   for (int u = 0; u < JOBS; ++u) {
   float v[8];
-  raw[u].get(v);
+  if (FORM != QP_HEADS) {
+    raw[u].get(v);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = 0.0f;
+  }
   const int job = (y + u) * QP_WARPS * per_warp + job0;
   const bool live = job < jobs;
   const bool is_q = job < a.nh, is_k = !is_q && job < a.nh + a.nkv;
@@ -332,6 +348,7 @@ __global__ void __launch_bounds__(QP_WARPS * 32, JOBS > 1 && sizeof(TX) == 2 ? 4
   if (live && !is_q && !is_k) {
     // a value head
     if (e0 < a.hdv_pad && pg >= 0) {
+      if (FORM == QP_HEADS && e0 < a.hdv) qp_load8<TX>(x + a.v_off + head * a.hdv + e0, v);
       if (a.lambda != nullptr && e0 < a.hdv) {
         const float lam = qp_load(a.lambda, a.lambda_dtype, 0);
         float o[8];
@@ -344,6 +361,7 @@ __global__ void __launch_bounds__(QP_WARPS * 32, JOBS > 1 && sizeof(TX) == 2 ? 4
   }
   const bool qk = live && (is_q || is_k);
   const bool mine = qk && e0 < a.hd;
+  if (FORM == QP_HEADS && mine) qp_load8<TX>(x + (is_q ? a.q_off : a.k_off) + head * a.hd + e0, v);
   float inv = is_q ? inv_q : inv_k;
   if (a.norm == 1 || a.norm == 2) {
     // every lane takes part in the shuffles; a head's lanes are neighbours
@@ -368,6 +386,7 @@ __global__ void __launch_bounds__(QP_WARPS * 32, JOBS > 1 && sizeof(TX) == 2 ? 4
     for (int e = 0; e < 8; ++e) v[e] *= inv;
   }
   if (e0 < a.rot) {
+    if (FORM == QP_HEADS) angles();
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
       const float u2 = v[2 * p], w2 = v[2 * p + 1];
@@ -389,14 +408,33 @@ __global__ void __launch_bounds__(QP_WARPS * 32, JOBS > 1 && sizeof(TX) == 2 ? 4
   }
 }
 
+// Which form.  Few tokens whose blocks all run at once (bfloat16 four, float32 one on an SM): QP_FEW (a token of 16 heads of 64
+// on 2: 2.0 us against 2.3; but 511 tokens of 64 on 64 of 128 23 against 18, float32 42 against 19).  QP_TOKEN by the
+// rounds of its blocks, a round for every four groups of heads (the eight warps' heads are a group), against the rounds of the
+// groups alone; its round takes 1.15 times as long with bfloat16, 1.45 with float32, whose pieces fill the registers.  QP_TOKEN /
+// QP_HEADS in us, bfloat16 without a norm: 16 on 16 of 128 (three groups) 512 / 700 / 1,000 / 2,000 / 8,000 tokens 5.4 / 8.0 / 8.7 /
+// 15.4 / 54 and 6.0 / 7.9 / 10.5 / 18.0 / 66; 36 on 36 of 64 (four) 5.7 / 7.7 / 9.2 / 16 / 58 and 7.2 / 9.1 / 12.2 / 22 / 81; 12 on 4 of 80 (two) 2,000
+// tokens 13.2 and 11.3; 64 on 64 of 128 (twelve) 300 tokens 11.4 and 11.9, 2,000 41 and 65.  float32: 16 on 16 of 128, 2,000 tokens 20.3
+// and 18.5; 36 on 36 of 64 21.6 and 21.9; 64 on 64 of 128 54 and 64.
 template <typename TX, typename TS>
 static void qk_prep_vec(const QkPrepArgs& a, int lph_log2, int T, int jobs, cudaStream_t stream) {
+  static const int sms = [] {
+    int dev = 0, v = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v > 0 ? v : 148;
+  }();
+  const bool wide = sizeof(TX) == 4;
   const int groups = ceil_div(jobs, QP_WARPS * (32 >> lph_log2));
-  // Many tokens: a block takes all heads of its token, four pieces a thread on their way (the sines and the block's start once a
-  // token, not once for every eight warps of heads: 48 heads of 128 at 512 / 2,000 / 3,163 tokens 6.1 -> 5.4, 17.3 -> 14.5,
-  // 25.8 -> 21.2 us).  With fewer the heads are spread over blocks.
-  if (groups > 1 && T >= 512) launch_pdl(qk_prep_vec_kernel<TX, TS, 4>, dim3(T), dim3(QP_WARPS * 32), 0, stream, a, lph_log2);
-  else launch_pdl(qk_prep_vec_kernel<TX, TS, 1>, dim3(T, groups), dim3(QP_WARPS * 32), 0, stream, a, lph_log2);
+  const int64_t blocks = (int64_t)T * groups;
+  const double token_rounds = (double)ceil_div(T, QP_TOKEN_BLOCKS * sms) * ceil_div(groups, 4);
+  const double head_rounds = (double)blocks / (QP_HEADS_BLOCKS * sms);
+  if (token_rounds * (wide ? 1.45 : 1.15) < head_rounds)
+    launch_pdl(qk_prep_vec_kernel<TX, TS, QP_TOKEN>, dim3(T), dim3(QP_WARPS * 32), 0, stream, a, lph_log2);
+  else if (blocks <= (wide ? 1 : 4) * sms)
+    launch_pdl(qk_prep_vec_kernel<TX, TS, QP_FEW>, dim3(T, groups), dim3(QP_WARPS * 32), 0, stream, a, lph_log2);
+  else
+    launch_pdl(qk_prep_vec_kernel<TX, TS, QP_HEADS>, dim3(T, groups), dim3(QP_WARPS * 32), 0, stream, a, lph_log2);
 }
 
 // What a recurrence takes: queries and keys rotated as whole heads (feature i with i + hd / 2) or not at all, as float32, without

@@ -140,6 +140,69 @@ def test_qk_prep_into_the_cache(dt, aligned, H, G, d, dv, norm, rot, layout, mix
     close(vp, want_v, dt, "values, and no other place of the pool")
 
 
+@pytest.mark.parametrize("dt", TYPES)
+@pytest.mark.parametrize("H, G, d, dv, dp, dvp, norm, rot, mix, gated, temp", [
+    (16, 16, 128, 128, 128, 128, 1, 128, False, False, None),       # three groups of heads: a block a token in one round
+    (36, 36, 64, 64, 64, 64, 3, 64, True, True, (0.4, 50.0)),       # four
+    (80, 72, 56, 40, 64, 64, 2, 48, True, True, None),              # seven: a second round, cut short; padded rows
+    (64, 64, 128, 128, 128, 128, 3, 0, False, False, (0.1, 7.0)),   # twelve
+    (12, 4, 80, 96, 128, 128, 0, 80, True, True, (0.2, 3.0))])      # two: the heads dealt to blocks
+def test_qk_prep_of_few_and_of_many_tokens(dt, H, G, d, dv, dp, dvp, norm, rot, mix, gated, temp):
+    """Which form of the 16-byte kernel runs goes by tokens and heads: float64's numbers from the form for many tokens, and the same
+    bits for the same tokens in calls of fewer."""
+    g = torch.Generator().manual_seed(H + norm)
+    k_ = K()
+    T, off, other = 560, 8, TYPES[1 - TYPES.index(dt)]
+    g_off = off + (H + G) * d + G * dv
+    x = torch.randn(T, (g_off + H + 7) // 8 * 8, generator=g).to(dt).to(DEV)
+    n_w = (H * d, G * d) if norm == 3 else (d, d)
+    qw, kw = ((1 + 0.3 * torch.randn(n, generator=g)).to(DEV) if norm >= 2 else None for n in n_w)
+    f = torch.tensor([300.0 ** (-2.0 * i / max(rot, 1)) for i in range(rot // 2)], dtype=torch.float64)
+    lam, src = torch.tensor([0.35], device=DEV), torch.randn(T, G * dv + 8, generator=g).to(other).to(DEV)
+    pos = torch.cat([torch.arange(300), torch.arange(40, 300)]).int().to(DEV)
+    seq = (torch.arange(T) >= 300).int().to(DEV)
+    bt = torch.tensor([[9, 1, 4, 0, 7], [3, 8, -1, 5, 2]], dtype=torch.int32, device=DEV)      # a page that is not kept
+
+    def call(a, b):
+        kp, vp = (torch.full((10, G, 64, n), 7.0, dtype=torch.bfloat16, device=DEV) for n in (dp, dvp))
+        out = k_.qk_prep(x[a:b], off, off + H * d, off + (H + G) * d, H, G, d, dv, dp, dvp, norm, qw, kw, 1e-5, rot, 1,
+                         k_.rotary_table(f).to(DEV) if rot else None, 1.1, 0.9, (lam, src[a:b, 8:]) if mix else None, pos[a:b], seq[a:b], bt, 64,
+                         torch.bfloat16, kp, vp, temperature=temp, gate_off=g_off if gated else None)
+        return [out[0], kp, vp] + ([out[2]] if gated else [])
+
+    q, kp, vp, *gate = call(0, T)
+    xd = x.double()
+    qr, kr, vr = (xd[:, a:a + n * w].reshape(T, n, w) for a, n, w in ((off, H, d), (off + H * d, G, d), (off + (H + G) * d, G, dv)))
+    n = lambda a, dims, w: a / torch.sqrt((a * a).mean(dims, keepdim=True) + 1e-5) * (w.double().reshape(-1, d) if w is not None else 1.0)
+    if norm:
+        qr, kr = (n(a, (1, 2) if norm == 3 else 2, w) for a, w in ((qr, qw), (kr, kw)))
+    if rot:
+        qr, kr = (rotate_ref(a, pos, f.to(DEV), 1.1, rot, True) for a in (qr, kr))
+    if temp:
+        qr = qr * (1 + temp[0] * torch.log(torch.floor((pos.double() + 1) / temp[1]) + 1))[:, None, None]
+    if mix:
+        vr = (1 - lam.double()) * vr + lam.double() * src[:, 8:].double().reshape(T, G, dv)
+    pad = lambda a, w: torch.nn.functional.pad(a, (0, w - a.shape[-1]))
+    close(q.reshape(T, H, dp), pad(qr, dp), torch.bfloat16, "q")
+    pg = bt[seq.long(), (pos // 64).long()].long()
+    kept = pg >= 0
+    for got, want, w, what in ((kp, 0.9 * kr, dp, "keys"), (vp, vr, dvp, "values")):
+        pool = torch.full(got.shape, 7.0, dtype=torch.float64, device=DEV)
+        pool[pg[kept], :, (pos % 64).long()[kept]] = pad(want, w)[kept]
+        close(got, pool, torch.bfloat16, what + ", and no other place of the pool")
+    if gated:
+        close(gate[0], torch.sigmoid(xd[:, g_off:g_off + H]), torch.float32, "gates")
+    for step in (7, 130):
+        parts = [call(a, min(T, a + step)) for a in range(0, T, step)]
+        assert torch.equal(torch.cat([p[0] for p in parts]), q)
+        for i, whole in ((1, kp), (2, vp)):
+            written = torch.stack([p[i] != 7.0 for p in parts]).any(0)
+            merged = sum((p[i].double() - 7.0) for p in parts) + 7.0          # each place is written by one call at most
+            assert torch.equal(merged.bfloat16(), whole) and torch.equal(written, whole != 7.0)
+        if gated:
+            assert torch.equal(torch.cat([p[3] for p in parts]), gate[0])
+
+
 def test_qk_prep_without_a_cache_keeps_float32():
     g = torch.Generator().manual_seed(3)
     k_ = K()
