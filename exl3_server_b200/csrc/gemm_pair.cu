@@ -35,12 +35,13 @@
 // Eight warps, since an epilogue that takes longer than its tile's products bounds the kernel at short K: 64,235 rows x 1,024,
 // K 1,024 with the residual 250 -> 193 us against four warps with four staging tiles each, K 4,096 475 -> 427.
 //
-// Epilogue 3 is the q/k/v projection of heads of 64: the output, rounded to bfloat16 as the plain epilogue would
-// store it, gets the half-split rotary encoding (queries and keys; a row's sines and cosines are computed once per
-// row of tiles, while the products run), the queries go to y, and the keys and values go straight to the token's place in
-// the paged cache: as one TMA store where a warp's 32 rows are 32 consecutive places of one page, through shared memory in
-// whole rows of 128 bytes otherwise.  The key and value columns of y are not written.  64,235 rows x 1,280, K 1,024: 217 -> 177 us
-// with eight warps and the sines kept over a row of tiles (the plain projection 130).
+// Epilogues 3 and 4 are the q/k/v projection of heads of 64: the output, rounded to bfloat16 as the plain epilogue would
+// store it, gets the half-split rotary encoding (queries and keys; a row's sines and cosines are computed while the products
+// run), the queries go to y, and the keys and values go straight to the token's place in
+// the paged cache: as one TMA store where a warp's 32 rows are 32 consecutive places of one page, row by row otherwise.  The key and
+// value columns of y are not written.  3, for short K and many tiles: eight warps, the sines kept over a row of tiles, rows here and there
+// through shared memory in whole lines of 128 bytes (64,235 rows x 1,280, K 1,024: 217 -> 177 us; the plain projection 130).  4: four
+// warps, which have the registers for a whole row, and the sines for every tile.
 //
 // Every wait on an mbarrier is bounded: when one runs out the kernel records a code, leaves its loops, waits
 // (bounded) for the copies it may have in flight, meets its partner at the cluster barrier that every path reaches,
@@ -55,8 +56,10 @@ namespace exl3 {
 using namespace tc5;
 
 constexpr int GP_BM = 256, GP_BN = 256, GP_BK = 64;
-// Epilogue warps: eight, two per 32 lanes of tensor memory with half of the columns each.
-constexpr int GP_EPI_WARPS = 8, GP_EPI_THREADS = 32 * GP_EPI_WARPS, GP_THREADS = 64 + GP_EPI_THREADS;
+// Epilogue warps: eight, two per 32 lanes of tensor memory with half of the columns each (epilogue 4: four).
+constexpr int GP_EPI_WARPS = 8;
+__host__ __device__ constexpr int gp_epi_threads(int epi) { return 32 * (epi == 4 ? 4 : GP_EPI_WARPS); }
+__host__ __device__ constexpr int gp_threads(int epi) { return 64 + gp_epi_threads(epi); }
 constexpr uint32_t GP_STAGE_A = 128 * GP_BK * 2, GP_STAGE_B = 128 * GP_BK * 2;       // per block
 constexpr uint32_t GP_BOX = 32 * 128;                                                  // a staging tile: 32 rows x 128 bytes
 constexpr int GP_STAGES = 5;                  // four cost 5 % at K 14,336
@@ -127,14 +130,15 @@ __device__ inline GpTile gp_tile(int tile, int n_m, int n_n, int group) {
 }
 
 template <int EPI>
-__global__ void __launch_bounds__(GP_THREADS, 1)
+__global__ void __launch_bounds__(gp_threads(EPI), 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w,
                  const __grid_constant__ CUtensorMap map_y,      // y (0, 1) or x_raw (2): bfloat16, boxes of 64 columns
                  const __grid_constant__ CUtensorMap map_h,      // 2: the float32 residual, boxes of 32 columns
                  const __grid_constant__ CUtensorMap map_k,      // 3: the key and the value pool as rows of 64 features,
                  const __grid_constant__ CUtensorMap map_v,      //    boxes of 32 rows
                  const PairArgs a) {
-  constexpr int STAGES = GP_STAGES, BOXES = GP_BOXES;
+  constexpr int STAGES = GP_STAGES, BOXES = GP_BOXES, EPI_THREADS = gp_epi_threads(EPI), EPI_WARPS = EPI_THREADS / 32;
+  constexpr bool ROPE = EPI >= 3, ALONG = EPI == 3;
   extern __shared__ __align__(1024) unsigned char gp_smem_raw[];
   unsigned char* sA = gp_smem_raw;
   unsigned char* sB = sA + STAGES * GP_STAGE_A;
@@ -158,9 +162,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     prefetch_map(&map_w);
     prefetch_map(&map_y);
     if (EPI == 2) prefetch_map(&map_h);
-    if (EPI == 3) { prefetch_map(&map_k); prefetch_map(&map_v); }
+    if (ROPE) { prefetch_map(&map_k); prefetch_map(&map_v); }
     for (int s = 0; s < STAGES; ++s) { mbar_init(full + s, 1); mbar_init(empty + s, 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, 2 * GP_EPI_WARPS); }
+    for (int b = 0; b < 2; ++b) { mbar_init(acc_full + b, 1); mbar_init(acc_empty + b, 2 * EPI_WARPS); }
     for (int i = 0; i < 2 * GP_EPI_WARPS; ++i) mbar_init(hbar + i, 1);
     mbar_init_fence();
   }
@@ -182,9 +186,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
   const bool beside = EPI == 2 && n_tiles <= n_pairs;
   // The pair's tiles.  3: neighbours in the order (columns fastest there), so that a row's sines and cosines, 32 of each,
   // are worked out once for all of the pair's tiles in a row; else dealt round-robin.
-  const int tile_first = EPI == 3 ? (int)((int64_t)n_tiles * pair / n_pairs) : pair;
-  const int tile_end = EPI == 3 ? (int)((int64_t)n_tiles * (pair + 1) / n_pairs) : n_tiles;
-  const int tile_step = EPI == 3 ? 1 : n_pairs;
+  const int tile_first = ALONG ? (int)((int64_t)n_tiles * pair / n_pairs) : pair;
+  const int tile_end = ALONG ? (int)((int64_t)n_tiles * (pair + 1) / n_pairs) : n_tiles;
+  const int tile_step = ALONG ? 1 : n_pairs;
   bool ok = true;
 
   if (warp == 0) {
@@ -251,8 +255,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     // ---- epilogue: thread = row of this block's 128 -----------------------------------------------------------
     const int q = warp & 3;                               // the 32 TMEM lanes this warp may read
     const int t = (warp - 2) * 32 + lane;
-    // warps 2-5 take the tile's columns 0-127 and warps 6-9 the columns 128-255, 64 at a time
-    const int s_lo = ((warp - 2) >> 2) * 2, s_hi = s_lo + 2;
+    // warps 2-5 take the tile's columns 0-127 (with four warps all of them) and warps 6-9 the columns 128-255, 64 at a time
+    const int s_lo = ((warp - 2) >> 2) * 2, s_hi = s_lo + (EPI_WARPS == 4 ? 4 : 2);
     unsigned char* my_boxes = boxes + (warp - 2) * BOXES * GP_BOX;
     uint64_t* my_hbar = hbar + (warp - 2) * 2;
     const uint32_t acc_empty_addr[2] = {cluster_addr(acc_empty, 0), cluster_addr(acc_empty + 1, 0)};
@@ -325,7 +329,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         for (uint32_t b = 0; b < 2 && tile < n_tiles && ok; ++b, tile += n_pairs) ok = preload(tile, b);
       }
     }
-    float rc[EPI == 3 ? 32 : 1], rs[EPI == 3 ? 32 : 1];
+    float rc[ROPE ? 32 : 1], rs[ROPE ? 32 : 1];
     int my_pos = 0, my_page = -1, pos0 = 0, page0 = -1, rope_m = -1;
     bool together = false;
     uint32_t tcount = 0;
@@ -336,8 +340,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       const int row = row0 + lane;
       // the tile's bias and norm weights, once for all rows (the previous tile's readers are past their last read:
       // they have met at the barrier after it); every thread comes here, whatever its outcome so far
-      if (!gp_epilogue_all<GP_EPI_THREADS>(ok)) { ok = false; break; }
-      for (int c = t; c < GP_BN; c += GP_EPI_THREADS) {
+      if (!gp_epilogue_all<EPI_THREADS>(ok)) { ok = false; break; }
+      for (int c = t; c < GP_BN; c += EPI_THREADS) {
         const int n = n0 + c;
         s_bias[c] = (a.bias && n < a.N) ? a.bias[n] : __float2bfloat16(0.0f);
         if (EPI == 2)
@@ -347,29 +351,37 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       const float k_row = (EPI == 2 ? a.rho : 1.0f) * row_factor(row);
       const float k_bias = EPI == 2 ? a.rho : 1.0f;
       const bool plain = a.bias == nullptr && a.ss_in == nullptr && EPI != 2;      // the accumulator as it is
-      // 3: the row's sines and cosines, its page, and whether the warp's rows are 32 consecutive places of one
-      // page (all of this while the tile's products run, and again only in another row of tiles)
-      if (EPI == 3 && at.m != rope_m) {
+      // 3, 4: the row's sines and cosines, its page, and whether the warp's rows are 32 consecutive places of one
+      // page (all of this while the tile's products run; 3: again only in another row of tiles)
+      if (ROPE && (!ALONG || at.m != rope_m)) {
         rope_m = at.m;
         int my_seq = -1;
         my_pos = 0;
         my_page = -1;
         if (row < a.M) { my_pos = __ldg(a.tok_pos + row); my_seq = __ldg(a.tok_seq + row); }
         const float p = (float)my_pos * a.pos_scale;
-        // Through the staging tiles (8 KB: 64 numbers a lane), so that the loop need not be unrolled for the registers' sake:
-        // 32 copies of sincosf are more code than the instruction cache holds (64,235 rows x 1,280, K 1,024: 190 -> 177 us).
-        if (lane == 0) tma_store_wait_read<0>();
-        __syncwarp();
-        float* mine = reinterpret_cast<float*>(my_boxes) + lane;
+        if (ALONG) {
+          // Through the staging tiles (8 KB: 64 numbers a lane), so that the loop need not be unrolled for the registers' sake:
+          // 32 copies of sincosf are more code than the instruction cache holds (64,235 rows x 1,280, K 1,024: 190 -> 177 us).
+          if (lane == 0) tma_store_wait_read<0>();
+          __syncwarp();
+          float* mine = reinterpret_cast<float*>(my_boxes) + lane;
 #pragma unroll 2
-        for (int d = 0; d < 32; ++d) {
-          float sn = 0.0f, cs = 1.0f;
-          if (a.inv_freq) rope_sincos(p, __ldg(a.inv_freq + d), a.inv_freq_lo ? __ldg(a.inv_freq_lo + d) : 0.0f, &sn, &cs);
-          mine[32 * d] = sn;
-          mine[32 * (32 + d)] = cs;
-        }
+          for (int d = 0; d < 32; ++d) {
+            float sn = 0.0f, cs = 1.0f;
+            if (a.inv_freq) rope_sincos(p, __ldg(a.inv_freq + d), a.inv_freq_lo ? __ldg(a.inv_freq_lo + d) : 0.0f, &sn, &cs);
+            mine[32 * d] = sn;
+            mine[32 * (32 + d)] = cs;
+          }
 #pragma unroll
-        for (int d = 0; d < 32; ++d) { rs[d] = mine[32 * d]; rc[d] = mine[32 * (32 + d)]; }
+          for (int d = 0; d < 32; ++d) { rs[d] = mine[32 * d]; rc[d] = mine[32 * (32 + d)]; }
+        } else {
+#pragma unroll
+          for (int d = 0; d < 32; ++d) {
+            if (a.inv_freq) rope_sincos(p, __ldg(a.inv_freq + d), a.inv_freq_lo ? __ldg(a.inv_freq_lo + d) : 0.0f, &rs[d], &rc[d]);
+            else { rc[d] = 1.0f; rs[d] = 0.0f; }
+          }
+        }
         if (a.write_kv && row < a.M) my_page = __ldg(a.block_table + (int64_t)my_seq * a.bt_stride + my_pos / 64);
         pos0 = __shfl_sync(0xffffffffu, my_pos, 0);
         page0 = __shfl_sync(0xffffffffu, my_page, 0);
@@ -378,7 +390,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
       }
       // (also the barrier after which the staged bias and norm weights may be read) one outcome for all epilogue
       // threads, so that they leave the loop together
-      if (!gp_epilogue_all<GP_EPI_THREADS>(mbar_wait(acc_full + buf, (tcount >> 1) & 1))) { ok = false; break; }
+      if (!gp_epilogue_all<EPI_THREADS>(mbar_wait(acc_full + buf, (tcount >> 1) & 1))) { ok = false; break; }
       fence_after();
       const uint32_t taddr = lane_taddr + buf * GP_BN;
       float sq = 0.0f;
@@ -388,7 +400,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         __syncwarp();
         tmem_ld32_issue(taddr + s * 64, r0);
         tmem_ld32_issue(taddr + s * 64 + 32, r1);
-        if (EPI == 0 || EPI == 3 || (EPI == 1 && (s & 1) == 0)) {
+        if (EPI == 0 || ROPE || (EPI == 1 && (s & 1) == 0)) {
           // the store before the last one used this staging tile
           if (lane == 0) tma_store_wait_read<1>();
           __syncwarp();
@@ -438,7 +450,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             else tma_store_skip();
           }
           ++n_store;
-        } else if (EPI == 3) {
+        } else if (ROPE) {
           const int col = n0 + s * 64, head = col >> 6;
           if (col < a.N) {                                  // (the same for the whole warp)
             // as the plain epilogue would store it, then rotated: pairs d, d + 32
@@ -474,8 +486,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 }
               }
               ++n_store;
+            } else if (!ALONG) {
+              // rows here and there: from each thread
+              if (a.write_kv && row < a.M && my_page >= 0) {
+                uint4* dst = reinterpret_cast<uint4*>((is_k ? a.k_pool : a.v_pool) + (((int64_t)my_page * a.nkv + g) * 64 + (my_pos & 63)) * 64);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) dst[j] = o[j];
+              }
             } else if (a.write_kv) {
-              // rows here and there: through the staging tile, eight lanes a row, so that a row's 128 bytes go out as one line
+              // through the staging tile, eight lanes a row, so that a row's 128 bytes go out as one line
               unsigned char* box = my_boxes + (n_store & 1) * GP_BOX;
 #pragma unroll
               for (int j = 0; j < 8; ++j) *gp_box_chunk(box, lane, j) = o[j];
@@ -549,7 +568,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         // a row's two halves meet (the barrier is also the one after which s_sq may be written again: two more stand between)
         const bool upper = s_lo > 0;
         if (upper) s_sq[q * 32 + lane] = sq;
-        asm volatile("bar.sync 2, %0;" ::"n"(GP_EPI_THREADS) : "memory");
+        asm volatile("bar.sync 2, %0;" ::"n"(EPI_THREADS) : "memory");
         if (!upper && row < a.M) a.ss_out[(int64_t)row * n_n + at.n] = sq + s_sq[q * 32 + lane];
         // the accumulator is free: the tile after next of this pair goes into it (or nobody waits for it)
         const int next = tile + 2 * n_pairs;
@@ -580,7 +599,7 @@ template <int EPI> static const void* gp_kernel() { return reinterpret_cast<cons
 static void gp_launch_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int blocks, int epi, cudaStream_t stream) {
   *cfg = cudaLaunchConfig_t{};
   cfg->gridDim = dim3(blocks);
-  cfg->blockDim = dim3(GP_THREADS);
+  cfg->blockDim = dim3(gp_threads(epi));
   cfg->dynamicSmemBytes = GP_SMEM;
   cfg->stream = stream;
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -595,7 +614,7 @@ static void gp_launch_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr,
 
 // Pairs that the GPU runs at once (a pair needs two SMs of one cluster-capable group).
 static int gp_max_pairs(int epi) {
-  static int pairs[4] = {0, 0, 0, 0};
+  static int pairs[5] = {};
   if (pairs[epi]) return pairs[epi];
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
@@ -606,7 +625,7 @@ static int gp_max_pairs(int epi) {
   gp_launch_config(&cfg, attr, sms & ~1, epi, nullptr);
   cfg.numAttrs = 1;
   int clusters = 0;
-  const void* fn = epi == 0 ? gp_kernel<0>() : epi == 1 ? gp_kernel<1>() : epi == 2 ? gp_kernel<2>() : gp_kernel<3>();
+  const void* fn = epi == 0 ? gp_kernel<0>() : epi == 1 ? gp_kernel<1>() : epi == 2 ? gp_kernel<2>() : epi == 3 ? gp_kernel<3>() : gp_kernel<4>();
   if (cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) == cudaSuccess && clusters > 0 && clusters < n) n = clusters;
   cudaGetLastError();
   pairs[epi] = n > 0 ? n : 1;
@@ -637,9 +656,17 @@ static int gp_run(const void* x, const void* w, const void* bias, void* y, int M
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_pair_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_pair_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_pair_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_pair_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GP_SMEM);
     if (e != cudaSuccess) { set_error("gemm_pair: cannot get %u bytes of shared memory: %s", GP_SMEM, cudaGetErrorString(e)); return (int)e; }
     configured = true;
   }
+  // The rotated projection: where a pair has one tile there are no sines to keep, and from K 2,048 on a tile's products take longer
+  // than working them out again, while the eight warps' registers do not hold a row beside them and the columns' order reads w again
+  // for every row of tiles.  Form 3 / 4, us: K 1,024, 64,000 x 1,280 162 / 215 and 2,048 x 1,280 (40 tiles) 15.1 / 14.1; K 1,536,
+  // 8,192 x 2,560 58 / 66; K 1,792, 30,000 x 5,376 523 / 586; K 2,048, 8,192 x 3,072 80 / 82 and 20,000 x 6,144 492 / 446; K 2,304, 8,192 x
+  // 6,912 203 / 187; K 8,192, 700 x 24,576 253 / 209.
+  const int tiles = ceil_div(M, GP_BM) * ceil_div(N, GP_BN);
+  if (epilogue == 3 && (K >= 2048 || tiles <= gp_max_pairs(3))) epilogue = 4;
   CUtensorMap map_x, map_w, map_y, map_h, map_k, map_v;
   int rc = make_map_k64(&map_x, x, M, K, 128, "gemm_pair");
   if (rc) return rc;
@@ -652,7 +679,7 @@ static int gp_run(const void* x, const void* w, const void* bias, void* y, int M
     rc = make_map_128b(&map_h, h, M, N, 4, 32, "gemm_pair");
     if (rc) return rc;
   }
-  if (epilogue == 3 && a.write_kv) {
+  if (epilogue >= 3 && a.write_kv) {
     rc = make_map_128b(&map_k, a.k_pool, pool_rows, 64, 2, 32, "gemm_pair");
     if (rc) return rc;
     rc = make_map_128b(&map_v, a.v_pool, pool_rows, 64, 2, 32, "gemm_pair");
@@ -661,7 +688,6 @@ static int gp_run(const void* x, const void* w, const void* bias, void* y, int M
   a.bias = static_cast<const __nv_bfloat16*>(bias);
   a.M = M; a.N = N; a.K = K;
   a.ss_in = ss_in; a.ss_blocks = ss_blocks; a.eps = eps; a.width = width;
-  const int tiles = ceil_div(M, GP_BM) * ceil_div(N, GP_BN);
   // Rows of tiles that are walked together.  While x stays in L2 (126 MB, with the weights and what is written beside it)
   // all of them: each column of w is then read once.  A larger x would be read from memory again for every few columns of
   // tiles, so it is walked in groups of rows that stay: 64,235 rows x 1,024 columns, K 4,096 (residual) 557 -> 475 us,
@@ -669,9 +695,9 @@ static int gp_run(const void* x, const void* w, const void* bias, void* y, int M
   // does not stay either, each group reads it again, so the groups are larger (4,096 x 4,096, K 16,384: 438 us whole and
   // in twelves, 445 in eights; 6,145 x 28,672, K 4,096: 1,265 whole, 1,242 in twelves).  The sums are the same in any order.
   const bool x_stays = (int64_t)M * K * 2 <= (40 << 20), w_stays = (int64_t)N * K * 2 <= (64 << 20);
-  // (The rotated projection has columns fastest: see the kernel.)
-  a.group = epilogue == 3 ? 1 : ceil_div(M, GP_BM);
+  a.group = ceil_div(M, GP_BM);
   if (!x_stays && a.group > (w_stays ? 8 : 12)) a.group = w_stays ? 8 : 12;
+  if (epilogue == 3) a.group = 1;                        // columns fastest: see the kernel
   const int max_pairs = gp_max_pairs(epilogue);
   const int pairs = tiles < max_pairs ? tiles : max_pairs;
   cudaLaunchConfig_t cfg;
@@ -681,7 +707,8 @@ static int gp_run(const void* x, const void* w, const void* bias, void* y, int M
   if (epilogue == 0) e = cudaLaunchKernelEx(&cfg, gemm_pair_kernel<0>, map_x, map_w, map_y, map_h, map_k, map_v, a);
   else if (epilogue == 1) e = cudaLaunchKernelEx(&cfg, gemm_pair_kernel<1>, map_x, map_w, map_y, map_h, map_k, map_v, a);
   else if (epilogue == 2) e = cudaLaunchKernelEx(&cfg, gemm_pair_kernel<2>, map_x, map_w, map_y, map_h, map_k, map_v, a);
-  else e = cudaLaunchKernelEx(&cfg, gemm_pair_kernel<3>, map_x, map_w, map_y, map_h, map_k, map_v, a);
+  else if (epilogue == 3) e = cudaLaunchKernelEx(&cfg, gemm_pair_kernel<3>, map_x, map_w, map_y, map_h, map_k, map_v, a);
+  else e = cudaLaunchKernelEx(&cfg, gemm_pair_kernel<4>, map_x, map_w, map_y, map_h, map_k, map_v, a);
   if (e != cudaSuccess) { set_error("gemm_pair: launch failed: %s", cudaGetErrorString(e)); return (int)e; }
   return launch_status("gemm_pair");
 }

@@ -550,6 +550,45 @@ def test_gemm_pair_rotates_and_writes_the_cache(lens, starts, nh, nkv, rot):
     assert K().gemm_pair_status() == 0
 
 
+@pytest.mark.parametrize("lens,starts,nh,nkv,Kd", [
+    ([100, 31, 64] * 27 + [35], [7, 0, 32] * 27 + [61], 16, 2, 72),    # five tiles in a row, some 1.4 a pair: sines kept, rows of tiles changed, places here and there
+    ([9000, 9990], [0, 64], 6, 1, 136),                                # two tiles in a row, two a pair, whole pages
+    ([100, 31, 64] * 27 + [35], [7, 0, 32] * 27 + [61], 16, 2, 2048),  # K from which the sines are worked out for every tile
+    ([5200], [31], 16, 2, 2056)])
+@pytest.mark.parametrize("rot", [64, 0])
+def test_gemm_pair_rotates_with_several_tiles_a_pair(lens, starts, nh, nkv, Kd, rot):
+    """More tiles than pairs, in both forms of the rotated epilogue: the projection followed by the kernel of the position step."""
+    g = torch.Generator(device=DEV).manual_seed(Kd + len(lens))
+    hd, page, T, N = 64, 64, sum(lens), (nh + 2 * nkv) * 64
+    assert ((T + 255) // 256) * ((N + 255) // 256) > 74
+    x = (torch.randn(T, Kd, device=DEV, generator=g) * 0.5).bfloat16()
+    w = (torch.randn(N, Kd, device=DEV, generator=g) / math.sqrt(Kd)).bfloat16()
+    need = [(s0 + n + page - 1) // page for s0, n in zip(starts, lens)]
+    n_pages, at = sum(need) + 3, 0
+    perm = torch.randperm(n_pages, generator=torch.Generator().manual_seed(1)).int()
+    table = torch.full((len(lens), max(need)), -1, dtype=torch.int32)
+    for i, n in enumerate(need):
+        table[i, :n] = perm[at:at + n]
+        at += n
+    table = table.to(DEV)
+    tok_pos = torch.cat([torch.arange(s0, s0 + n) for s0, n in zip(starts, lens)]).int().to(DEV)
+    tok_seq = torch.repeat_interleave(torch.arange(len(lens)), torch.tensor(lens)).int().to(DEV)
+    inv_freq = K().rotary_table(10000.0 ** (-torch.arange(32, dtype=torch.float64) / 32)).to(DEV)
+    junk = torch.randn(2, n_pages, nkv, page, hd, device=DEV, generator=g).bfloat16()
+    (k1, v1), (k2, v2) = junk.clone(), junk.clone()
+    want = K().gemm_pair(x, w, None)
+    K().rope_kv_write(want, inv_freq, rot, 1.0, tok_pos, tok_seq, table, k1, v1, nh, nkv, hd, page, True)
+    got = K().gemm_pair_rope(x, w, None, None, tok_pos, tok_seq, table, inv_freq, rot, 1.0, nh, nkv, hd, page, k2, v2, True)
+    close(got[:, :nh * hd], want[:, :nh * hd], 1e-2, "rotated queries")
+    close(k2, k1, 1e-2, "key cache")
+    assert torch.equal(v2, v1)                           # values are copied, not computed with: and nothing is written anywhere else
+    written = torch.zeros(n_pages, page, dtype=torch.bool, device=DEV)
+    written[table[tok_seq.long(), (tok_pos // page).long()].long(), (tok_pos % page).long()] = True
+    assert torch.equal(k2.transpose(1, 2)[~written], junk[0].transpose(1, 2)[~written])
+    torch.cuda.synchronize()
+    assert K().gemm_pair_status() == 0
+
+
 @pytest.mark.parametrize("shapes", [[(5, 64, 128), (5,), (5, 2048)],            # states as the recurrent layers have them
                                     [(3, 7), (3, 1), (3, 5, 3)],                # rows that are no multiple of 16 bytes
                                     [(4, 3)] * 97 + [(4, 300000)]])             # more parts than one launch takes
