@@ -55,17 +55,31 @@ struct SfRow {            // one row's options, as the host gives them (float64 
   double temperature, top_k, top_p, min_p, u;
 };
 
-// Up to so many rows come as a parameter of the kernel: no buffer to make and to copy (some 25 us of the host's time a call).
+// The options of a call's rows.  Up to so many rows come as a parameter of the kernel: no buffer to make and to copy (some
+// 25 us of the host's time a call).
 constexpr int SF_DIRECT_ROWS = 64;
 struct SfBatch {
   SfRow rows[SF_DIRECT_ROWS];
-  int* counts[SF_DIRECT_ROWS];
-  float params[SF_DIRECT_ROWS][3];
+  int* counts_of[SF_DIRECT_ROWS];
+  float params_of[SF_DIRECT_ROWS][3];
+  __device__ SfRow row(int r) const { return rows[r]; }
+  __device__ const int* counts(int r) const { return counts_of[r]; }
+  __device__ const float* params(int r) const { return params_of[r]; }
+};
+// Or they lie in buffers on the device.  (A type of its own: 4 KB of parameters that nobody reads cost a launch 1 us.)
+struct SfTables {
+  const SfRow* rows;
+  int* const* counts_of;                         // null: no row has penalties
+  const float* params_of;
+  __device__ SfRow row(int r) const { return rows[r]; }
+  __device__ const int* counts(int r) const { return counts_of ? counts_of[r] : nullptr; }
+  __device__ const float* params(int r) const { return params_of + 3 * r; }
 };
 
 // the model of a launch's time (sf_launch): a wave of rows with 8 / 4 / 2 / 1 blocks a row, and a token of a block's part
 constexpr double SF_FIXED_US[4] = {26.5, 23.0, 24.5, 28.0}, SF_AGAIN_FIXED_US = 6.0;
-constexpr double SF_STAGED_US = 0.00032, SF_AGAIN_US = 0.00033, SF_AGAIN_PENALTIES_US = 0.00075;
+constexpr double SF_STAGED_US = 0.00032, SF_AGAIN_US = 0.00033, SF_AGAIN_PENALTIES_US = 0.00066, SF_AGAIN_FAR_US = 0.00075, SF_PENALTIES_US = 2.1;
+constexpr double SF_NEAR_BYTES = 100e6;          // logits and counts of the rows under way that L2 holds
 constexpr int SF_BINS = 2048;
 constexpr int SF_BLOCKS = 8;                     // of a row, at most
 constexpr int SF_HEAD_BYTES = (2 * SF_BINS * 4) + 2 * (SF_CAP * 8);     // histograms, candidates, this block's own
@@ -91,18 +105,16 @@ __device__ inline float sf_penalised(float x, int count, float rep, float presen
   return x;
 }
 
-// rows, counts, params: null, and `batch` holds them (with host_out, a page-locked copy of out, or null; count_now: no two
-// rows share their counts, so a row's token joins them at once).
-// counts: null, or per row a pointer to its token counts [V] (null: the row has no penalties); params [R, 3]: repetition,
-// presence, frequency.  The counts are only read: rows may share them, so the chosen tokens join them in a kernel of their
-// own, after every row has been drawn (2 us for 32 rows).  STAGED: the block's part of the row is kept in shared memory;
+// of_rows: the rows' options, per row a pointer to its token counts [V] (null: the row has no penalties) and three numbers:
+// repetition, presence, frequency.  host_out: null, or a page-locked copy of out.  count_now: no two rows share their counts,
+// so a row's token joins them at once; else they are only read, and the chosen tokens join them in a kernel of their own, after
+// every row has been drawn (2 us for 32 rows).  STAGED: the block's part of the row is kept in shared memory;
 // else (parts too long for that) every pass reads it again, 16 bytes a load: one block a row takes 76 us for 122,753
 // tokens (4 bytes a load, and 64-bit keys compared in every pass: 107), 142 for 320,001.  PENALTIES: there may be counts.
-template <bool STAGED, bool PENALTIES>
+template <bool STAGED, bool PENALTIES, typename ROWS>
 __global__ void __launch_bounds__(SF_THREADS)
-sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict__ rows, const int* const* __restrict__ counts,
-                       const float* __restrict__ params, int* __restrict__ out, int V, int blocks,
-                       const __grid_constant__ SfBatch batch, int* host_out, bool count_now) {
+sample_filtered_kernel(const float* __restrict__ logits, const __grid_constant__ ROWS of_rows, int* __restrict__ out, int V,
+                       int blocks, int* host_out, bool count_now) {
   extern __shared__ __align__(16) unsigned char sf_smem[];
   unsigned* hists = reinterpret_cast<unsigned*>(sf_smem);                                      // [2][SF_BINS]
   unsigned long long* cand = reinterpret_cast<unsigned long long*>(sf_smem + 2 * SF_BINS * 4);  // this block's share of them
@@ -116,14 +128,15 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int row_id = blockIdx.x / blocks, rank = blockIdx.x % blocks;
   const float* row = logits + (int64_t)row_id * V;
-  const SfRow o = rows ? rows[row_id] : batch.rows[row_id];
+  const SfRow o = of_rows.row(row_id);
   const int M = V < SF_CAP ? V : SF_CAP;
-  const int* count = !PENALTIES ? nullptr : rows ? (counts ? counts[row_id] : nullptr) : batch.counts[row_id];
+  const int* count = PENALTIES ? of_rows.counts(row_id) : nullptr;
   float rep = 1.0f, presence = 0.0f, frequency = 0.0f;
   if (count) {
-    rep = rows ? params[3 * row_id] : batch.params[row_id][0];
-    presence = rows ? params[3 * row_id + 1] : batch.params[row_id][1];
-    frequency = rows ? params[3 * row_id + 2] : batch.params[row_id][2];
+    const float* params = of_rows.params(row_id);
+    rep = params[0];
+    presence = params[1];
+    frequency = params[2];
   }
   // the row's token, from the thread that knows it; all of the row's blocks have read its counts by then
   auto chosen = [&](int t) {
@@ -194,7 +207,7 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
   if (tid == 0) n_cand = n_found = 0;
   __syncthreads();
   if constexpr (STAGED) {
-    // the select's first histogram on the way
+    // the select's first histogram on the way, where there is a select
     constexpr int AHEAD = 8;
     for (int i0 = tid; i0 < n; i0 += SF_THREADS * AHEAD) {
       float x[AHEAD];
@@ -211,7 +224,7 @@ sample_filtered_kernel(const float* __restrict__ logits, const SfRow* __restrict
         if (i < n) {
           const uint32_t key = sf_key(sf_penalised(x[a], c[a], rep, presence, frequency));
           keys[i] = key;
-          atomicAdd(hists + (key >> 21), 1u);
+          if (V > SF_CAP) atomicAdd(hists + (key >> 21), 1u);
         }
       }
     }
@@ -492,7 +505,7 @@ static int sf_clusters_at_once(int b, int sms) {
   struct Table { int n[SF_BLOCKS + 1]; };
   static const Table table = [sms] {
     Table t = {};
-    auto kernel = sample_filtered_kernel<true, true>;
+    auto kernel = sample_filtered_kernel<true, true, SfTables>;
     const bool fine = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SF_SMEM_MOST) == cudaSuccess;
     for (int c = 2; c <= SF_BLOCKS; c *= 2) {
       cudaLaunchConfig_t cfg = {};
@@ -517,12 +530,13 @@ static int sf_clusters_at_once(int b, int sms) {
 // rows: float64 [R, 5] on the device: temperature (<= 0: greedy), top_k (0: off, at most 2048), top_p, min_p and
 // the row's uniform number in [0, 1).  out: int32 [R].  counts (may be null): as in exl3_sample_penalties, with params;
 // the penalties are applied as the logits are read, and the chosen tokens are counted when all rows have been drawn.
-// batch: the rows themselves, then rows, counts and params are null.
-static int sf_launch(const float* logits, const double* rows, int* const* counts, const float* params, int* out, int R, int V,
-                     const SfBatch& batch, bool penalties, int* host_out, bool count_now, cudaStream_t stream) {
+template <typename ROWS>
+static int sf_launch(const float* logits, const ROWS& of_rows, int* out, int R, int V, bool penalties, int* host_out, bool count_now,
+                     cudaStream_t stream) {
   // Blocks a row.  An SM holds one block, and a cluster must fit into a group of SMs, so the driver says how many clusters run
-  // at once; a wave of rows takes 23 to 28 us and, for a token of a block's part, 0.32 ns, or where the part is too long for
-  // shared memory and read in every pass 6 us and 0.33 ns (0.75 with penalties).  With 8 / 4 / 2 / 1 blocks: one row of 32,000
+  // at once; a wave of rows takes 23 to 28 us (2 more with penalties) and, for a token of a block's part, 0.32 ns, or where the part is
+  // too long for shared memory and read in every pass 6 us and 0.33 ns (with penalties 0.66 where L2 holds the rows under way, else 0.75:
+  // 256 rows of 50,257 take one block a row, 133 us, and not two, 144; 75 of 320,001 two, 237, and not one, 266).  With 8 / 4 / 2 / 1 blocks: one row of 32,000
   // 27.8 / 25.7 / 29.6 / 38 us, 64 rows 131 / 52 / 30 / 38; 8 rows of 122,753 31.8 / 33.1 / 49 / 76, 16 rows 60 / 33 / 49 / 76,
   // 148 rows 299 / 157 / 98 / 77; 100 rows of 320,001 289 / 200 / 168 / 163.
   int dev = 0, sms = 148;
@@ -536,8 +550,9 @@ static int sf_launch(const float* logits, const double* rows, int* const* counts
     const int at_once = b == 1 ? sms : sf_clusters_at_once(b, sms);
     const double waves = (double)((R + at_once - 1) / at_once);
     const bool kept = (size_t)each * 4 <= MOST;
-    const double a_token = kept ? SF_STAGED_US : penalties ? SF_AGAIN_PENALTIES_US : SF_AGAIN_US;
-    const double cost = waves * (SF_FIXED_US[i] + (kept ? 0.0 : SF_AGAIN_FIXED_US) + a_token * each);
+    const bool near = 8.0 * V * std::min(R, at_once) < SF_NEAR_BYTES;
+    const double a_token = kept ? SF_STAGED_US : !penalties ? SF_AGAIN_US : near ? SF_AGAIN_PENALTIES_US : SF_AGAIN_FAR_US;
+    const double cost = waves * (SF_FIXED_US[i] + (kept ? penalties ? SF_PENALTIES_US : 0.0 : SF_AGAIN_FIXED_US) + a_token * each);
     if (b == 8 || cost < best) {
       best = cost;
       blocks = b;
@@ -545,8 +560,8 @@ static int sf_launch(const float* logits, const double* rows, int* const* counts
   }
   const size_t part = (size_t)ceil_div(V, blocks) * 4;
   const bool staged = part <= MOST;
-  auto kernel = staged ? sample_filtered_kernel<true, true>
-                       : penalties ? sample_filtered_kernel<false, true> : sample_filtered_kernel<false, false>;
+  auto kernel = staged ? sample_filtered_kernel<true, true, ROWS>
+                       : penalties ? sample_filtered_kernel<false, true, ROWS> : sample_filtered_kernel<false, false, ROWS>;
   const size_t smem = SF_HEAD_BYTES + (staged ? part : 0);
   // The limit belongs to the function and not to this call: the same number from every thread, whatever its rows take, or a
   // thread with shorter rows would lower it between another one's setting it and its launch.
@@ -569,8 +584,7 @@ static int sf_launch(const float* logits, const double* rows, int* const* counts
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = blocks > 1 ? 1 : 0;               // without a cluster blocks are spread over the SMs first
-  cudaLaunchKernelEx(&cfg, kernel, logits, reinterpret_cast<const SfRow*>(rows), (const int* const*)counts, params, out, V,
-                     blocks, batch, host_out, count_now);
+  cudaLaunchKernelEx(&cfg, kernel, logits, of_rows, out, V, blocks, host_out, count_now);
   return launch_status("sample_filtered");
 }
 
@@ -581,8 +595,8 @@ extern "C" int exl3_sample_rows(const float* logits, const double* rows, int* co
     set_error("sample_filtered: bad sizes rows=%d vocab=%d, or penalties without their constants", R, V);
     return ERR_BAD_ARGUMENT;
   }
-  static const SfBatch none = {};
-  int rc = sf_launch(logits, rows, counts, params, out, R, V, none, counts != nullptr, nullptr, false, stream);
+  const SfTables tables = {reinterpret_cast<const SfRow*>(rows), counts, params};
+  int rc = sf_launch(logits, tables, out, R, V, counts != nullptr, nullptr, false, stream);
   if (rc || counts == nullptr) return rc;
   return exl3_sample_count(counts, out, R, V, stream);
 }
@@ -618,14 +632,14 @@ extern "C" int exl3_sample_batch(const float* logits, const void* packed, int R,
     memcpy(&state, at + (size_t)R * 56 + (size_t)r * 8, 8);
     memcpy(&counts, at + (size_t)R * 64 + (size_t)r * 8, 8);
     batch.rows[r] = {o[0], o[1], o[2], o[3], o[0] <= 0.0 ? 0.0 : sf_uniform(state)};
-    batch.counts[r] = reinterpret_cast<int*>(counts);
-    for (int i = 0; i < 3; ++i) batch.params[r][i] = (float)o[4 + i];
+    batch.counts_of[r] = reinterpret_cast<int*>(counts);
+    for (int i = 0; i < 3; ++i) batch.params_of[r][i] = (float)o[4 + i];
     penalties |= counts != 0;
   }
-  int rc = sf_launch(logits, nullptr, nullptr, nullptr, out, R, V, batch, penalties, host_out, !shared_counts, stream);
+  int rc = sf_launch(logits, batch, out, R, V, penalties, host_out, !shared_counts, stream);
   if (rc || !penalties || !shared_counts) return rc;
   SfCounts c = {};
-  memcpy(c.at, batch.counts, sizeof(c.at));
+  memcpy(c.at, batch.counts_of, sizeof(c.at));
   sample_count_batch_kernel<<<1, SF_DIRECT_ROWS, 0, stream>>>(c, out, R, V);
   return launch_status("sample_count");
 }
