@@ -1490,24 +1490,24 @@ def test_sample_filtered_ranks_equal_logits_of_long_rows(penalties):
     assert got.tolist() == [sample_token(logits[r], opt, contexts[r], _FixedU(us[r])) for r in range(R)]
 
 
-@pytest.mark.parametrize("V,R", [(255, 3), (2047, 1), (2048, 40), (2049, 70), (4099, 1), (40001, 2), (40001, 32), (40001, 70), (40001, 149)])
-def test_sample_filtered_ranks_what_one_block_has_found(V, R):
-    """Rows that rise or fall from end to end: all candidates come from one part of the row and are dealt out to all of the
-    row's blocks (8, 4, 2 or 1 of them by the number of rows).  Logits 0, 1, 2, ... at temperature 700: neighbours in the
-    ranking differ by a seven-hundredth, so a token in a wrong place moves the draw."""
-    from exl3_server_b200.sampling import SampleOptions
-    from exl3_server_b200.sampling.host import sample_token
-    opt = SampleOptions(temperature=700.0)
-    up = np.arange(V, dtype=np.float32)
-    logits = np.stack([up if r % 2 == 0 else up[::-1] for r in range(R)])
-    us = [(r + 0.5) / R for r in range(R)]
-    rows = torch.tensor([[700.0, 0, 1.0, 0.0, u] for u in us], dtype=torch.float64)
-    got = K().sample_filtered(torch.from_numpy(logits).to(DEV), rows.to(DEV)).tolist()
-    want = [sample_token(logits[r], opt, [], _FixedU(us[r])) for r in range(R)]
-    # float32 exponentials may differ in their last bit between host and device: a sum of 2,048 of them to 2,048 * 2^-24 of
-    # itself, a draw then by one place where it falls that near to a border (one in 2,048 * 2 * 2,048 * 2^-24 = 0.5 rows)
-    off = [abs(g - w) for g, w in zip(got, want)]
-    assert max(off) <= 1 and sum(off) <= 1 + R // 2, off
+@pytest.mark.parametrize("V,R", [(255, 3), (2047, 1), (2048, 40), (2049, 70), (4099, 1), (40001, 2), (40001, 32), (40001, 70), (40001, 149),
+                                 (320001, 1), (320001, 70)])     # kept in shared memory, and parts too long for it
+def test_sample_filtered_puts_every_candidate_in_its_place(V, R):
+    """Candidates that lie anywhere, and all of them in one part of the row, dealt out to the row's blocks (8, 4, 2 or 1 of them
+    by the number of rows).  At a temperature at which all terms are one (1 - 4e-5 at the least) top_k = k and a number of 1 - 1 / (4 k) draw
+    the k-th candidate: the running sums around it are k - 1 and k, to 2,048 * 4e-5 = 0.08, and the draw looks for k - 0.25."""
+    g = torch.Generator(device=DEV).manual_seed(V + R)
+    ramp = torch.arange(V, dtype=torch.float32, device=DEV)
+    orders = [ramp, ramp.flip(0), ramp[torch.randperm(V, generator=g, device=DEV)]]
+    logits = torch.stack([orders[r % 3] for r in range(R)])
+    ranking = [torch.argsort(o, descending=True).tolist() for o in orders]
+    ks = [k for k in (1, 2, 127, 128, 255, 256, 257, 511, 512, 513, 768, 769, 1023, 1024, 1025, 1536, 1793, 2047, 2048) if k <= V]
+    heat = 2.5e4 * V
+    for shift in range(0, len(ks), max(1, min(R, 4))):
+        rows = [[heat, ks[(r // 3 + shift) % len(ks)], 1.0, 0.0] for r in range(R)]
+        rows = torch.tensor([r + [1.0 - 0.25 / r[1]] for r in rows], dtype=torch.float64)
+        got = K().sample_filtered(logits, rows.to(DEV)).tolist()
+        assert got == [ranking[r % 3][int(rows[r, 1]) - 1] for r in range(R)]
 
 
 @pytest.mark.parametrize("R", [1, 5, 64, 65])             # with the launch up to 64 rows, by a buffer beyond
