@@ -238,8 +238,10 @@ __device__ inline void sk_finish(const SkinnyArgs& a, const float* part, const f
   }
 }
 
-// R: 128-row tiles of w per block.
-template <int EPI, bool SCALE, int R>
+// R: 128-row tiles of w per block.  WIDE: clusters of more than four blocks, whose sums take a form of their own; in a kernel with
+// the other two it cost 0.1 to 0.2 us of 5 to 10 (2304 x 2304 in 8 cuts at 17 / 24 / 32 / 33 rows 5.6 / 5.8 / 6.1 / 6.3 -> 5.6 / 5.7 / 5.9 /
+// 6.1 us).
+template <int EPI, bool SCALE, int R, bool WIDE>
 __global__ void __launch_bounds__(SK_THREADS)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
                    const SkinnyArgs a) {
@@ -393,9 +395,9 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
 
   if (all_ok) {
     pdl_wait();                                            // (one of the warps has not waited yet)
-    if (S <= 2) sk_finish<EPI, SCALE, R, 2, 6>(a, part, s_inv, n0, rank, arrived);
-    else if (S <= 4) sk_finish<EPI, SCALE, R, 4, 4>(a, part, s_inv, n0, rank, arrived);
-    else sk_finish<EPI, SCALE, R, SK_MAX_SPLIT, 3>(a, part, s_inv, n0, rank, arrived);
+    if constexpr (WIDE) sk_finish<EPI, SCALE, R, SK_MAX_SPLIT, 3>(a, part, s_inv, n0, rank, arrived);
+    else if (S <= 2) sk_finish<EPI, SCALE, R, 2, 6>(a, part, s_inv, n0, rank, arrived);
+    else sk_finish<EPI, SCALE, R, 4, 4>(a, part, s_inv, n0, rank, arrived);
   }
 
   if (!arrived) sk_cluster_arrive();
@@ -497,7 +499,7 @@ static int sk_auto_split(int N, int K) {
   if (s < 1) s = 1;
   // More tiles than SMs, and no cut: the cuts that pairs of tiles would get when a block takes two (as it does
   // for few rows, below): 32768 x 4096 at 1 to 32 rows 42.9-46.2 us with two tiles a block and two cuts against
-  // 45.3-48.2 us with one and none; at 48 and 64 rows, a tile a block, the two cuts cost 1 us of 50.
+  // 45.3-48.2 us with one and none; at 48 and 64 rows 46.5 and 47.6 against 49.2 and 51.3 with a tile a block and two cuts.
   if (s == 1 && n_tiles > sk_sm_count()) {
     const int pairs = ceil_div(n_tiles, 2);
     int s2 = 2 * sk_sm_count() / pairs;
@@ -519,12 +521,12 @@ static int sk_auto_tiles(int N, int split, int M) {
   return M <= 64 && n_tiles > sms && 2 * ceil_div(n_tiles, 2) * split >= 3 * sms ? 2 : 1;
 }
 
-template <int EPI, bool SCALE, int R>
-static int sk_launch(const CUtensorMap& mw, const CUtensorMap& mx, const SkinnyArgs& a, int n_blocks, size_t smem,
+template <int EPI, bool SCALE, int R, bool WIDE>
+static int sk_launch_form(const CUtensorMap& mw, const CUtensorMap& mx, const SkinnyArgs& a, int n_blocks, size_t smem,
                      cudaStream_t stream) {
   static size_t configured = 0;
   if (smem > configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<EPI, SCALE, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<EPI, SCALE, R, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) { set_error("gemm_skinny: cannot get %zu bytes of shared memory: %s", smem, cudaGetErrorString(e)); return (int)e; }
     configured = smem;
   }
@@ -542,8 +544,14 @@ static int sk_launch(const CUtensorMap& mw, const CUtensorMap& mx, const SkinnyA
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 2 : 1;
-  cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<EPI, SCALE, R>, mw, mx, a);
+  cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<EPI, SCALE, R, WIDE>, mw, mx, a);
   return launch_status("gemm_skinny");
+}
+template <int EPI, bool SCALE, int R>
+static int sk_launch(const CUtensorMap& mw, const CUtensorMap& mx, const SkinnyArgs& a, int n_blocks, size_t smem,
+                     cudaStream_t stream) {
+  return a.split > 4 ? sk_launch_form<EPI, SCALE, R, true>(mw, mx, a, n_blocks, smem, stream)
+                     : sk_launch_form<EPI, SCALE, R, false>(mw, mx, a, n_blocks, smem, stream);
 }
 
 }  // namespace exl3
@@ -623,7 +631,10 @@ extern "C" int exl3_gemm_skinny(const void* x, const void* w, const void* bias, 
     if (stages == 4 && fixed + n * stage <= 113 * 1024 && fixed + 4 * stage > 113 * 1024) stages = n;
   while ((size_t)stages * stage < part) ++stages;
   a.stages = stages;
-  const size_t smem = fixed + (size_t)stages * stage;
+  // two blocks an SM at most, which is what the cuts are counted for: a third one leaves SMs to which it would have gone idle
+  // (16,384 x 2048 at 8 rows 14.3 -> 15.1 us with up to three)
+  size_t smem = fixed + (size_t)stages * stage;
+  if (smem < 76 * 1024) smem = 76 * 1024;
   if (smem > 227 * 1024) { set_error("gemm_skinny: %zu bytes of shared memory needed", smem); return ERR_UNSUPPORTED; }
   CUtensorMap mw, mx;
   int rc = sk_map(&mw, w, N, K, R * SK_BM);
