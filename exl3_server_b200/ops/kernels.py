@@ -1184,7 +1184,8 @@ def zero_rows(parts, row: int) -> None:
         if not 0 <= row < t.shape[0]:
             raise KernelLibraryError(f"zero_rows: row {row} of {t.shape[0]}")
     bases = (ctypes.c_void_p * n)(*[t.data_ptr() for t in parts])
-    sizes = (ctypes.c_longlong * n)(*[t.stride(0) * t.element_size() if t.dim() > 1 else t.element_size() for t in parts])
+    # (not by the stride: that of a dimension of one row may be anything)
+    sizes = (ctypes.c_longlong * n)(*[t.numel() // t.shape[0] * t.element_size() for t in parts])
     _check(library().exl3_zero_rows(bases, sizes, _c_int(n), _c_int64(row), _stream()), "zero_rows")
 
 

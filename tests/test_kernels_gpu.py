@@ -603,6 +603,15 @@ def test_zero_rows_clears_one_row_of_every_part(shapes):
         assert all(torch.equal(p, w) for p, w in zip(parts, want))
 
 
+def test_zero_rows_of_tensors_of_one_row():
+    """The only row of a view may have any stride, and nothing beside it is touched."""
+    base = torch.ones(8, 4, device=DEV)
+    K().zero_rows([base[2::4][:1], base[5:6]], 0)
+    want = torch.ones(8, 4, device=DEV)
+    want[2] = want[5] = 0
+    assert torch.equal(base, want)
+
+
 def test_zero_rows_refuses_a_row_that_is_not_there():
     from exl3_server_b200.ops.lib import KernelLibraryError
     with pytest.raises(KernelLibraryError, match="row 3 of 3"):
