@@ -3,9 +3,12 @@
 //
 // Same mathematics as attention_simt.cu (the
 // reference's masked scaled-dot-product attention, src/model.cpp:539-548,
-// 576-578).  A block owns 128 consecutive queries of one sequence and one head
-// (or two such tiles, one after the other: see the kernel) and walks the key pages
-// its queries may see:
+// 576-578).  Three kernels.  The first: a block owns 128 consecutive queries of one
+// sequence and one head (or two such tiles, one after the other) and walks the key pages
+// its queries may see, as below.  The second, for heads of 64 and many rounds of blocks: four
+// smaller blocks an SM.  The third, for heads of 128 in groups of an even number: two
+// heads of a tile side by side in persistent blocks.
+//
 //
 //   warp 5     S = Q K^T as tcgen05.mma into one of two S buffers of 64 columns in tensor
 //              memory, as soon as a page has landed and the buffer has been read: up to two
@@ -68,7 +71,10 @@ __device__ inline void fa_mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
 __device__ inline void fa_mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(fa_smem_u32(bar)) : "memory");
 }
-// One arrival for the warp, when all its lanes are here.
+// One arrival for the warp, when all its lanes are here.  Right where softmax warps share a scheduler (the kernels with eight of them
+// or four blocks an SM: 32 prompts of 19 to 147 tokens, 36 heads of 64, 26.3 us against 27.2 with an arrival a thread); where a warp has
+// its scheduler to itself or nearly, waiting for its lanes stands in its chain (100 tokens after 3,000, 16 heads of 64 on 2: 41.6 us with an
+// arrival a thread, 43.0 with one a warp; 16 prompts of 200 with 36 heads 34.3 and 35.6).
 __device__ inline void fa_mbar_arrive_warp(uint64_t* bar) {
   __syncwarp();
   if ((threadIdx.x & 31) == 0) fa_mbar_arrive(bar);
@@ -400,8 +406,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
   uint64_t* kv_full = bars + 2;                   // [stages] K and V page landed
   uint64_t* kv_free = kv_full + FA_KV_STAGES;     // [stages] the products that read the stage are done
   uint64_t* s_full = kv_free + FA_KV_STAGES;      // [2] S buffer written by the tensor core
-  uint64_t* s_free = s_full + 2;                  // [2] S buffer read by the four softmax warps
-  uint64_t* p_full = s_free + 2;                  // [2] P buffer written by the four softmax warps
+  uint64_t* s_free = s_full + 2;                  // [2] S buffer read by all 128 softmax threads
+  uint64_t* p_full = s_free + 2;                  // [2] P buffer written by all 128 softmax threads
   uint64_t* pv_done = p_full + 2;                 // [2] O += P V of that P buffer finished
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2);
 
@@ -425,8 +431,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     }
     for (int i = 0; i < 2; ++i) {
       fa_mbar_init(s_full + i, 1);
-      fa_mbar_init(s_free + i, 4);
-      fa_mbar_init(p_full + i, 4);
+      fa_mbar_init(s_free + i, 128);
+      fa_mbar_init(p_full + i, 128);
       fa_mbar_init(pv_done + i, 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -580,7 +586,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       const int st = f & 1;
       fa_wait_ld();
       fa_fence_before();
-      fa_mbar_arrive_warp(s_free + st);
+      fa_mbar_arrive(s_free + st);
       // The two barriers this page still needs (the P buffer free again, the next S written) are looked at now:
       // both have almost always flipped a page ago, and the looks' trips to shared memory pass under the
       // arithmetic below instead of standing in front of the store of P and the load of S.
@@ -612,7 +618,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       if (j + 1 < n_blocks && !ask_s(f + 1, s_there)) ok = false;   // the tile's next row of S while P is being stored
       fa_wait_st();
       fa_fence_before();
-      fa_mbar_arrive_warp(p_full + st);
+      fa_mbar_arrive(p_full + st);
     }
     if (ok) {
       // last product done -> O complete

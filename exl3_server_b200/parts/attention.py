@@ -238,10 +238,11 @@ class Attention:
         pages to walk plus three pages' worth for every tile (its start and its end), a page taking 0.9 us on one
         of the two slots an SM has for the first two forms (one slot for heads of 128) and 1.5 us on one of the four
         of the third; the tiles' heads run side by side on as many slots, and a tile goes to the slots that come
-        free first, in the list's order.  Constants fitted to thirteen measured workloads (to 9 % in the mean; us
-        for forms 1 / 2 / 3, 36 heads of 64 unless said): one prompt of 2,048 tokens 41.9 / 59.1 / 40.2, of 1,536
-        28.5 / 39.3 / 34.0, of 8,192 442 / 429 / 455, 24 prompts of 16 to 2,048 tokens 447 / 392 / 470, one of 5,000
-        with 16 heads 88.8 / 130 / 130.  The four-block kernel is taken when the better of the others is not
+        free first, in the list's order.  Constants fitted to thirteen workloads, to 9 % in the mean; the kernel
+        has become 2 to 5 % faster since, in all three forms (us for forms 1 / 2 / 3 now, 36 heads of 64 unless said: one prompt of
+        2,048 tokens 45.2 / 62.2 / 43.7, of 1,500 31.2 / 43.5 / 36.9, of 8,192 490 / 476 / 504, 24 prompts of 16 to 2,048 tokens
+        425 / 394 / 407, one of 4,096 with 16 heads on 2 66.9 / 104 / 71.4, and the worst choice found, 2 for one of 6,145 of them, 140 /
+        163 / 176).  The four-block kernel is taken when the better of the others is not
         below 0.93 of it (the model flatters them where tiles are short)."""
         s = self.spec
         if not tile_keys:
@@ -273,8 +274,8 @@ class Attention:
         """``_prefill_variant``, or for heads of 128 in groups of an even number two heads of a tile side by side in
         persistent blocks, one an SM (4), where that is the shorter: an item (a tile and two heads) takes its pages and 3.5
         pages' worth at 1.19 us a page, against 0.9 us a page and head with a tile and head a block.  32 heads on 8, us for
-        forms 1 / 4: one prompt of 1,024 tokens 24.3 / 25.7, of 1,500 44.5 / 33.9, of 6,145 465 / 316; 8 of 114 to
-        500 49.0 / 32.5; 100 tokens after 3,000 44.6 / 58.5."""
+        forms 1 / 4: one prompt of 1,024 tokens 23.7 / 25.3, of 1,500 43.9 / 33.4, of 6,145 464 / 314; 8 of 114 to
+        500 41.7 / 31.3; 100 tokens after 3,000 44.4 / 57.5."""
         s = self.spec
         one = self._prefill_variant(tile_keys, page, device)
         if s.head_dim != 128 or (s.heads // s.kv_heads) % 2 or not tile_keys:
