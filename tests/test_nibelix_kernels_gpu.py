@@ -176,6 +176,24 @@ def test_experts_of_a_few_rows(T, top, E, n_out, W, inner):
     close(y[rows], want_y[rows], dt, "down")
 
 
+@pytest.mark.parametrize("Kd", [4088, 4096, 4104, 8192, 9000])           # the rows of A go in by pieces of 4,096 columns
+@pytest.mark.parametrize("rows", [1, 2, 3, 4, 9])                         # tiles of one row, of two, of up to four, several of an expert
+@pytest.mark.parametrize("glu", [False, True])
+def test_experts_of_a_few_long_rows(Kd, rows, glu):
+    """Inputs longer than the columns that a block holds, with a remainder that is no step; a feature count that ends inside a warp."""
+    g = torch.Generator().manual_seed(Kd + rows)
+    E, N = 3, 42
+    x = torch.randn(rows, Kd, generator=g).bfloat16()
+    w = (torch.randn(E, N, Kd, generator=g) / math.sqrt(Kd)).bfloat16()
+    idx = torch.tensor([[2, 0]], dtype=torch.int32).repeat(rows, 1)       # every token picks these two, nobody the third
+    order, plan = K().moe_plan(idx.to(DEV), E, K().moe_tile_rows("few"))
+    got = K().moe_gemv(x.to(DEV), 2, w.to(DEV), order, plan, torch.float32, act="silu" if glu else "none", glu=glu)
+    z = torch.stack([x.double() @ w[e].double().T for e in (2, 0)], dim=1).reshape(2 * rows, N)
+    if glu:
+        z = torch.nn.functional.silu(z[:, 0::2]) * z[:, 1::2]
+    close(got, z, torch.float32)
+
+
 @pytest.mark.parametrize("T, top, E, n_out, W, inner", [(300, 2, 3, 4, 64, 72), (1100, 3, 9, 10, 200, 328), (513, 1, 2, 2, 520, 264)])
 def test_experts_on_tensor_cores(T, top, E, n_out, W, inner):
     """The prompt-sized product: rows gathered into the plan's order, tiles of 128 rows that run into the next

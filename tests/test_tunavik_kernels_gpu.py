@@ -230,7 +230,7 @@ def test_distance_biases_for_prompts(nh, nkv, hd, near, cap, window):
     want = torch.cat(outs).reshape(-1, nh * hd)
     tile_seq, tile_q0 = case.tiles(128)
     got = []
-    for variant in ((0, 1, 2, 3) if hd == 64 else (0, 1, 3)):
+    for variant in ((0, 1, 2, 3) if hd == 64 else (0, 1, 3) if G % 2 else (0, 1, 3, 4)):
         o = torch.full((T, nh * hd), 3.0, device=DEV, dtype=torch.bfloat16)
         k_.attn_prefill_tc(buf, buf.stride(0), o, case.k_pool, case.v_pool, case.table, case.row_start, case.row_pos0,
                            tile_seq, tile_q0, tile_seq.numel(), nh, nkv, hd, 64, window, scale, variant=variant, sink=True,
