@@ -305,9 +305,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
           f[4 * j + 2] = __float_as_uint(__uint_as_float(v.z) * inv);
           f[4 * j + 3] = __float_as_uint(__uint_as_float(v.w) * inv);
         }
-        __syncwarp();                                     // every lane has read the staging tile
-        if (c + 2 < GP_BN / 2 / 32) ask(c + 2);
         gp_tmem_st32(lane_taddr + buf * GP_BN + s_lo * 64 + c * 32, f);
+        // Every lane has its values, and only then may the next tile of h land on them: a lane's reads are ordered before the copies
+        // that another lane asks for by the fence alone (the meeting of the warp orders them before its loads and stores, not before
+        // TMA's; with the load asked for before the values were used, a row now and then got the last 16 bytes of the tile after).
+        fence_smem_to_tma();
+        __syncwarp();
+        if (c + 2 < GP_BN / 2 / 32) ask(c + 2);
       }
       if (!good) {
         // loads that may still be in flight get the time to land before the block's shared memory goes away

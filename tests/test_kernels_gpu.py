@@ -618,6 +618,28 @@ def test_zero_rows_refuses_a_row_that_is_not_there():
         K().zero_rows([torch.zeros(3, 4, device=DEV)], 3)
 
 
+@pytest.mark.parametrize("M", [2048, 4000])                  # the residual beside the products, and in the accumulators of several tiles
+def test_gemm_pair_residual_repeats_itself(M):
+    """The residual comes in through staging tiles that the next copy lands on: a hundred calls in a row, with weights that come from
+    memory, give the same bits, and float64's numbers."""
+    g = torch.Generator(device=DEV).manual_seed(M)
+    N, Kd, calls = 2304, 5760, 100 if M < 4000 else 50
+    x = (torch.randn(M, Kd, device=DEV, generator=g) * 0.5).bfloat16()
+    w = (torch.randn(N, Kd, device=DEV, generator=g) / math.sqrt(Kd)).bfloat16()
+    ws = [w.clone() for _ in range(8)]
+    nw = torch.ones(N, device=DEV)
+    h0 = 30.0 * torch.randn(M, N, device=DEV, generator=g)
+    hs = h0.expand(calls, M, N).contiguous()
+    outs = [K().gemm_pair(x, ws[i % 8], None, resid=(hs[i], 0.25, nw)) for i in range(calls)]
+    want = h0.double() + 0.25 * (x.double() @ w.double().T)
+    close(hs[0], want, 2e-5, "residual")
+    for i in range(1, calls):
+        wrong = hs[i] != hs[0]
+        assert not wrong.any(), (i, int(wrong.sum()), wrong.nonzero()[:4].tolist())
+        assert torch.equal(outs[i][0], outs[0][0]) and torch.equal(outs[i][1], outs[0][1])
+    assert K().gemm_pair_status() == 0
+
+
 @pytest.mark.parametrize("M,N,Kd", [(5300, 520, 4096),       # x is larger than what stays in L2: rows of tiles in eights, five left over
                                     (3400, 4200, 8192)])     # and w as well: twelves, two left over
 def test_gemm_pair_walks_rows_of_tiles_in_groups(M, N, Kd):
