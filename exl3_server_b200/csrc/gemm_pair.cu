@@ -39,7 +39,7 @@
 // store it, gets the half-split rotary encoding (queries and keys; a row's sines and cosines are computed while the products
 // run), the queries go to y, and the keys and values go straight to the token's place in
 // the paged cache: as one TMA store where a warp's 32 rows are 32 consecutive places of one page, row by row otherwise.  The key and
-// value columns of y are not written.  3, for short K and many tiles: eight warps, the sines kept over a row of tiles, rows here and there
+// value columns of y are not written.  3, for short K and many tiles (gp_run): eight warps, the sines kept over a row of tiles, rows here and there
 // through shared memory in whole lines of 128 bytes (64,235 rows x 1,280, K 1,024: 217 -> 177 us; the plain projection 130).  4: four
 // warps, which have the registers for a whole row, and the sines for every tile.
 //
@@ -664,13 +664,17 @@ static int gp_run(const void* x, const void* w, const void* bias, void* y, int M
     if (e != cudaSuccess) { set_error("gemm_pair: cannot get %u bytes of shared memory: %s", GP_SMEM, cudaGetErrorString(e)); return (int)e; }
     configured = true;
   }
-  // The rotated projection: where a pair has one tile there are no sines to keep, and from K 2,048 on a tile's products take longer
-  // than working them out again, while the eight warps' registers do not hold a row beside them and the columns' order reads w again
-  // for every row of tiles.  Form 3 / 4, us: K 1,024, 64,000 x 1,280 162 / 215 and 2,048 x 1,280 (40 tiles) 15.1 / 14.1; K 1,536,
-  // 8,192 x 2,560 58 / 66; K 1,792, 30,000 x 5,376 523 / 586; K 2,048, 8,192 x 3,072 80 / 82 and 20,000 x 6,144 492 / 446; K 2,304, 8,192 x
-  // 6,912 203 / 187; K 8,192, 700 x 24,576 253 / 209.
+  // The rotated projection: where a pair has one tile there are no sines to keep.  The longer K, the more of a tile's products cover
+  // working them out again, while form 3 has too few registers for a row and its order reads w again for every row of tiles, which
+  // costs where L2 does not hold x beside it.  The kernel alone, form 3 / 4, us: K 1,024, 64,000 x 1,280 162 / 215 and 2,048 x 1,280 (40 tiles)
+  // 15.1 / 14.1; K 1,536, 8,192 x 2,560 58 / 66; K 2,304, 20,000 x 6,912 630 / 480; K 8,192, 700 x 24,576 253 / 209.  Between K 2,048 and 3,072 the
+  // kernel behind itself in a chain says little (weights that no other kernel has pushed out of L2), so these are prompts of eight
+  // layers: 36 heads, K 2,304, 2,048 tokens 2,180 / 2,267, 8,192 11,149 / 11,410, 20,000 42,237 / 40,649; 32 on 32, K 2,048, 2,048 tokens 1,926 /
+  // 2,054, 20,000 36,330 / 35,660; K 2,560, 4,000 tokens 5,413 / 5,472, 20,000 44,300 / 43,636; K 3,072, 2,048 tokens 3,444 / 3,419, 20,000 57,233 /
+  // 55,976.
   const int tiles = ceil_div(M, GP_BM) * ceil_div(N, GP_BN);
-  if (epilogue == 3 && (K >= 2048 || tiles <= gp_max_pairs(3))) epilogue = 4;
+  const bool keeps_sines = K < 2048 || (K < 3072 && (int64_t)M * K * 2 <= (48 << 20));
+  if (epilogue == 3 && (!keeps_sines || tiles <= gp_max_pairs(3))) epilogue = 4;
   CUtensorMap map_x, map_w, map_y, map_h, map_k, map_v;
   int rc = make_map_k64(&map_x, x, M, K, 128, "gemm_pair");
   if (rc) return rc;

@@ -553,8 +553,9 @@ def test_gemm_pair_rotates_and_writes_the_cache(lens, starts, nh, nkv, rot):
 @pytest.mark.parametrize("lens,starts,nh,nkv,Kd", [
     ([100, 31, 64] * 27 + [35], [7, 0, 32] * 27 + [61], 16, 2, 72),    # five tiles in a row, some 1.4 a pair: sines kept, rows of tiles changed, places here and there
     ([9000, 9990], [0, 64], 6, 1, 136),                                # two tiles in a row, two a pair, whole pages
-    ([100, 31, 64] * 27 + [35], [7, 0, 32] * 27 + [61], 16, 2, 2048),  # K from which the sines are worked out for every tile
-    ([5200], [31], 16, 2, 2056)])
+    ([100, 31, 64] * 27 + [35], [7, 0, 32] * 27 + [61], 16, 2, 3072),  # K from which the sines are worked out for every tile
+    ([5200], [31], 16, 2, 3080),
+    ([12300], [3], 4, 2, 2048)])                                       # an x of more than 48 MB: the same
 @pytest.mark.parametrize("rot", [64, 0])
 def test_gemm_pair_rotates_with_several_tiles_a_pair(lens, starts, nh, nkv, Kd, rot):
     """More tiles than pairs, in both forms of the rotated epilogue: the projection followed by the kernel of the position step."""
