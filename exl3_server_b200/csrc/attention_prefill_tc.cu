@@ -651,9 +651,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
 // over S, a ring of two pages) for blocks: 128 columns of tensor memory, 49 KB of shared memory and at most 102
 // registers a thread let four blocks share an SM, sixteen softmax warps instead of eight.  A block alone is
 // slower (1.64 against 1.53 us a page), so the variant is used when the blocks do not all fit the GPU at once
-// (more than four per SM): 452 against 530 us at 8,192 tokens with 36 heads, 84 against 96 us at 3,072, 117 against
-// 142 us for 24 prompts of 16 to 2,048 tokens with 16 heads; at 2,048 tokens, where one wave of blocks runs and the
-// heaviest tile's 32 pages are the kernel's length, the kernel above stays (48.7 against 52.6 us).  Same
+// (more than four per SM): 476 against 490 us at 8,192 tokens with 36 heads, 394 against 425 us for 24 prompts of 16 to
+// 2,048 tokens; at 2,048 tokens, where one wave of blocks runs and the
+// heaviest tile's 32 pages are the kernel's length, the kernel above stays (45.2 against 62.2 us).  Same
 // arithmetic in the same order per row: the two give the same numbers bit for bit.
 constexpr int F4_STAGES = 2;
 constexpr uint32_t F4_SMEM = fa_q_bytes(64) + 2 * F4_STAGES * fa_kv_bytes(64) + 1024 + 128;
