@@ -97,7 +97,8 @@ __device__ inline void sk_finish(const SkinnyArgs& a, const float* part, const f
   constexpr int RW = R * SK_BM, WARPS = SK_THREADS / 32;
   const int S = a.split, lane = threadIdx.x & 31;
   {
-    const int q = threadIdx.x >> 5;
+    // the accumulator's warps take the first rows: with few of them the copying and the issuing warp have none to wait for
+    const int q = ((threadIdx.x >> 5) + WARPS - 2) % WARPS;
     const int ss_out_blocks = (a.N + 15) >> 4;
     const bool vec = (a.N & 3) == 0;                        // rows of y, h and x_raw start on 16-byte boundaries
 #pragma unroll
