@@ -108,7 +108,7 @@ struct PairArgs {
   const void* norm_w;        // [N], float32 or bfloat16
   int norm_w_f32;
   float* ss_out;             // [M, tiles of 256 columns]
-  // epilogue 3
+  // epilogues 3 and 4
   const int* tok_pos;        // [M] position of each row's token
   const int* tok_seq;        // [M] its row of the block table
   const int* block_table;
